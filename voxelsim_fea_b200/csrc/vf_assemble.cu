@@ -19,6 +19,7 @@
 
 #include "../../include/voxfea.h"
 #include "vf_common.cuh"
+#include "vf_workspace.cuh"
 
 namespace vf {
 extern thread_local std::string g_last_error;
@@ -83,24 +84,6 @@ __global__ void k_popcount_bits(long long n, const uint8_t* __restrict__ bits, u
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
 
-// Device buffers of one call, released on every exit path.
-struct Scratch {
-  std::vector<void*> p;
-  cudaStream_t st = nullptr;
-  ~Scratch() {
-    if (st) cudaStreamSynchronize(st);
-    for (void* q : p) cudaFree(q);
-    if (st) cudaStreamDestroy(st);
-  }
-  template <typename T> bool alloc(T** out, size_t count) {
-    void* q = nullptr;
-    if (cudaMalloc(&q, count * sizeof(T) + 16) != cudaSuccess) return false;
-    p.push_back(q);
-    *out = (T*)q;
-    return true;
-  }
-};
-
 int fail(const std::string& msg, int code) {
   vf::g_last_error = msg;
   return code;
@@ -123,8 +106,8 @@ int vf_assemble_grid(int32_t nx, int32_t ny, int32_t nz, int32_t n_roles, const 
   const bool dev = (flags & VF_SOLVE_DEVICE_PTRS) != 0;
   const long long ne = (long long)nx * ny * nz;
   const long long nn = (long long)(nx + 1) * (ny + 1) * (nz + 1);
-  Scratch sc;
-  if (cudaStreamCreateWithFlags(&sc.st, cudaStreamNonBlocking) != cudaSuccess)
+  vf::Workspace sc;
+  if (!sc.open())
     return fail("vf_assemble_grid: no CUDA stream", VF_ERR_CUDA);
   cudaStream_t st = sc.st;
   uint8_t *d_act = nullptr, *d_bits = nullptr, *d_mask = nullptr;
@@ -200,8 +183,8 @@ int vf_drop_unsupported_islands_mask(int32_t nx, int32_t ny, int32_t nz, const u
   const bool dev = (flags & VF_SOLVE_DEVICE_PTRS) != 0;
   const long long ne = (long long)nx * ny * nz;
   const long long nn = (long long)(nx + 1) * (ny + 1) * (nz + 1);
-  Scratch sc;
-  if (cudaStreamCreateWithFlags(&sc.st, cudaStreamNonBlocking) != cudaSuccess)
+  vf::Workspace sc;
+  if (!sc.open())
     return fail("vf_drop_unsupported_islands_mask: no CUDA stream", VF_ERR_CUDA);
   cudaStream_t st = sc.st;
   uint8_t *d_act = nullptr, *d_fix = nullptr, *d_kept = nullptr, *d_in = nullptr, *d_bits = nullptr;

@@ -5,6 +5,7 @@
 // (core/fea.py:165-227) as an in-place 6-connected flood fill.
 #include "../../include/voxfea.h"
 #include "vf_common.cuh"
+#include "vf_workspace.cuh"
 
 namespace vf {
 
@@ -197,22 +198,15 @@ __global__ void k_elem_disp(int nx, int ny, int nz, const double* __restrict__ u
 extern "C" int vf_element_displacement(int32_t nx, int32_t ny, int32_t nz, const double* u, float* disp_out) {
   if (nx < 1 || ny < 1 || nz < 1 || !u || !disp_out) return VF_ERR_ARG;
   const size_t ndof = 3 * (size_t)(nx + 1) * (ny + 1) * (nz + 1), ne = (size_t)nx * ny * nz;
-  cudaStream_t st = nullptr;
-  if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return VF_ERR_CUDA;
+  vf::Workspace ws;
+  if (!ws.open()) return VF_ERR_CUDA;
+  cudaStream_t st = ws.st;
   double* d_u = nullptr;
   float* d_o = nullptr;
-  int rc = VF_OK;
-  if (cudaMalloc(&d_u, sizeof(double) * ndof) != cudaSuccess || cudaMalloc(&d_o, sizeof(float) * ne) != cudaSuccess) {
-    rc = VF_ERR_NOMEM;
-  } else {
-    cudaMemcpyAsync(d_u, u, sizeof(double) * ndof, cudaMemcpyHostToDevice, st);
-    const long long b = ((long long)ne + 255) / 256;
-    vf::launch_k(vf::k_elem_disp, (int)(b < 148 * 16 ? b : 148 * 16), 256, 0, st, nx, ny, nz, (const double*)d_u, d_o);
-    cudaMemcpyAsync(disp_out, d_o, sizeof(float) * ne, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = VF_ERR_CUDA;
-  }
-  cudaFree(d_u);
-  cudaFree(d_o);
-  cudaStreamDestroy(st);
-  return rc;
+  if (!ws.alloc(&d_u, ndof) || !ws.alloc(&d_o, ne)) return VF_ERR_NOMEM;
+  cudaMemcpyAsync(d_u, u, sizeof(double) * ndof, cudaMemcpyHostToDevice, st);
+  const long long b = ((long long)ne + 255) / 256;
+  vf::launch_k(vf::k_elem_disp, (int)(b < 148 * 16 ? b : 148 * 16), 256, 0, st, nx, ny, nz, (const double*)d_u, d_o);
+  cudaMemcpyAsync(disp_out, d_o, sizeof(float) * ne, cudaMemcpyDeviceToHost, st);
+  return cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess ? VF_ERR_CUDA : VF_OK;
 }

@@ -28,6 +28,7 @@
 #include "vf_hex8.h"
 #include "vf_reduce.cuh"
 #include "vf_nn.cuh"
+#include "vf_workspace.cuh"
 #include <cuda_fp16.h>
 
 namespace vf {
@@ -212,6 +213,11 @@ template <typename T>
 int dalloc(vf_solver* s, T** p, size_t count) {
   void* q = nullptr;
   cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
+  if (e == cudaErrorMemoryAllocation) {   // what the stateless calls keep may be in the way
+    cudaGetLastError();
+    workspace_trim();
+    e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
+  }
   if (e != cudaSuccess) {
     s->err = std::string("cudaMalloc(") + std::to_string(count * sizeof(T)) + " B): " + cudaGetErrorString(e);
     return VF_ERR_NOMEM;
@@ -1960,22 +1966,14 @@ int vf_drop_unsupported_islands(int32_t nx, int32_t ny, int32_t nz, const uint8_
   }
   uint8_t *d_act = nullptr, *d_fix = nullptr, *d_kept = nullptr;
   int* d_changed = nullptr;
-  cudaStream_t st = nullptr;
   int rc = VF_OK;
-  auto cleanup = [&]() {
-    if (d_act) cudaFree(d_act);
-    if (d_fix) cudaFree(d_fix);
-    if (d_kept) cudaFree(d_kept);
-    if (d_changed) cudaFree(d_changed);
-    if (st) cudaStreamDestroy(st);
-  };
-  if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess || cudaMalloc(&d_act, ne) != cudaSuccess ||
-      cudaMalloc(&d_fix, nn) != cudaSuccess || cudaMalloc(&d_kept, ne) != cudaSuccess ||
-      cudaMalloc(&d_changed, sizeof(int)) != cudaSuccess) {
+  Workspace ws;
+  if (!ws.open() || !ws.alloc(&d_act, ne) || !ws.alloc(&d_fix, nn) || !ws.alloc(&d_kept, ne) ||
+      !ws.alloc(&d_changed, 1)) {
     g_last_error = "device allocation failed";
-    cleanup();
     return VF_ERR_NOMEM;
   }
+  cudaStream_t st = ws.st;
   std::vector<uint8_t> act01(ne);
   long long n_active = 0;
   for (size_t e = 0; e < ne; ++e) { act01[e] = active[e] ? 1 : 0; n_active += act01[e]; }
@@ -1985,7 +1983,6 @@ int vf_drop_unsupported_islands(int32_t nx, int32_t ny, int32_t nz, const uint8_
   std::vector<uint8_t> kept(ne);
   if (!rc && cudaMemcpyAsync(kept.data(), d_kept, ne, cudaMemcpyDeviceToHost, st) != cudaSuccess) rc = VF_ERR_CUDA;
   if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = VF_ERR_CUDA;
-  cleanup();
   if (rc) { g_last_error = "CUDA error in flood fill"; return rc; }
   long long n_kept = 0;
   for (size_t e = 0; e < ne; ++e) n_kept += kept[e];

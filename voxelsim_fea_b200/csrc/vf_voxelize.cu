@@ -19,6 +19,7 @@
 
 #include "../../include/voxfea.h"
 #include "vf_common.cuh"
+#include "vf_workspace.cuh"
 
 namespace vf {
 
@@ -116,40 +117,31 @@ int inside_run(int mode, const double* verts, int64_t nv, const int64_t* faces, 
   if (npts <= 0) return VF_OK;
   for (int64_t k = 0; k < 3 * nf; ++k)   // the kernels index verts by these: check them here
     if (faces[k] < 0 || faces[k] >= nv) return VF_ERR_ARG;
-  cudaStream_t st = nullptr;
-  if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return VF_ERR_CUDA;
+  Workspace ws;
+  if (!ws.open()) return VF_ERR_CUDA;
+  cudaStream_t st = ws.st;
   double *d_v = nullptr, *d_tri = nullptr, *d_p = nullptr;
   int64_t* d_f = nullptr;
   uint8_t* d_o = nullptr;
-  int rc = VF_OK;
   const size_t nfs = (size_t)(nf > 0 ? nf : 1);
-  if (cudaMalloc(&d_v, sizeof(double) * 3 * (size_t)(nv > 0 ? nv : 1)) != cudaSuccess ||
-      cudaMalloc(&d_f, sizeof(int64_t) * 3 * nfs) != cudaSuccess ||
-      cudaMalloc(&d_tri, sizeof(double) * kTriVals * nfs) != cudaSuccess ||
-      cudaMalloc(&d_o, (size_t)npts) != cudaSuccess ||
-      (mode == 0 && cudaMalloc(&d_p, sizeof(double) * 3 * (size_t)npts) != cudaSuccess)) {
-    rc = VF_ERR_NOMEM;
-  }
+  if (!ws.alloc(&d_v, 3 * (size_t)(nv > 0 ? nv : 1)) || !ws.alloc(&d_f, 3 * nfs) || !ws.alloc(&d_tri, kTriVals * nfs) ||
+      !ws.alloc(&d_o, (size_t)npts) || (mode == 0 && !ws.alloc(&d_p, 3 * (size_t)npts)))
+    return VF_ERR_NOMEM;
   Dir d;
   for (int c = 0; c < 3; ++c) d.d[c] = dir3[c];
-  if (rc == VF_OK) {
-    if (nf > 0) {
-      cudaMemcpyAsync(d_v, verts, sizeof(double) * 3 * (size_t)nv, cudaMemcpyHostToDevice, st);
-      cudaMemcpyAsync(d_f, faces, sizeof(int64_t) * 3 * (size_t)nf, cudaMemcpyHostToDevice, st);
-      launch_k(k_prepare_tris, (int)((nf + 255) / 256 < 4096 ? (nf + 255) / 256 : 4096), 256, 0, st,
-               (const double*)d_v, (const int64_t*)d_f, nf, d, d_tri);
-    }
-    if (mode == 0) cudaMemcpyAsync(d_p, pts, sizeof(double) * 3 * (size_t)npts, cudaMemcpyHostToDevice, st);
-    const int nx = dims ? dims[0] : 0, ny = dims ? dims[1] : 0, nz = dims ? dims[2] : 0;
-    const double ox = origin ? origin[0] : 0.0, oy = origin ? origin[1] : 0.0, oz = origin ? origin[2] : 0.0;
-    launch_k(k_inside, (unsigned)((npts + 255) / 256), 256, 0, st, mode, (const double*)d_p, npts, nx, ny, nz, ox, oy,
-             oz, vsize, (const double*)d_tri, nf, d, d_o);
-    cudaMemcpyAsync(out, d_o, (size_t)npts, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = VF_ERR_CUDA;
+  if (nf > 0) {
+    cudaMemcpyAsync(d_v, verts, sizeof(double) * 3 * (size_t)nv, cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(d_f, faces, sizeof(int64_t) * 3 * (size_t)nf, cudaMemcpyHostToDevice, st);
+    launch_k(k_prepare_tris, (int)((nf + 255) / 256 < 4096 ? (nf + 255) / 256 : 4096), 256, 0, st,
+             (const double*)d_v, (const int64_t*)d_f, nf, d, d_tri);
   }
-  cudaFree(d_v); cudaFree(d_f); cudaFree(d_tri); cudaFree(d_o); cudaFree(d_p);
-  cudaStreamDestroy(st);
-  return rc;
+  if (mode == 0) cudaMemcpyAsync(d_p, pts, sizeof(double) * 3 * (size_t)npts, cudaMemcpyHostToDevice, st);
+  const int nx = dims ? dims[0] : 0, ny = dims ? dims[1] : 0, nz = dims ? dims[2] : 0;
+  const double ox = origin ? origin[0] : 0.0, oy = origin ? origin[1] : 0.0, oz = origin ? origin[2] : 0.0;
+  launch_k(k_inside, (unsigned)((npts + 255) / 256), 256, 0, st, mode, (const double*)d_p, npts, nx, ny, nz, ox, oy,
+           oz, vsize, (const double*)d_tri, nf, d, d_o);
+  cudaMemcpyAsync(out, d_o, (size_t)npts, cudaMemcpyDeviceToHost, st);
+  return cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess ? VF_ERR_CUDA : VF_OK;
 }
 
 }  // namespace

@@ -242,7 +242,10 @@ def assemble(descr, masks, dims):
     _lib.check(_lib.load().vf_assemble_grid(nx, ny, nz, n, _lib.ptr(roles), ptrs, _lib.ptr(meta), 0,
                                             _lib.ptr(active), _lib.ptr(bits), _lib.ptr(force),
                                             ctypes.byref(n_act), ctypes.byref(n_fix)), None, "assemble")
-    fixed_dofs = np.flatnonzero(((bits[:, None] >> np.arange(3, dtype=np.uint8)) & 1).ravel()).astype(np.int64)
+    # (the supports touch few nodes: expand those alone, in the same ascending order)
+    nodes = np.flatnonzero(bits)
+    fixed = ((bits[nodes, None] >> np.arange(3, dtype=np.uint8)) & 1).astype(bool)
+    fixed_dofs = (3 * nodes[:, None] + np.arange(3))[fixed].astype(np.int64)
     return active.astype(bool), fixed_dofs, force, bits
 
 
