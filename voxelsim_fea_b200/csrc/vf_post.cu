@@ -100,29 +100,56 @@ __global__ void k_island_seed(int nx, int ny, int nz, const uint8_t* __restrict_
   }
 }
 
-// One in-place dilation pass (monotone: kept only grows, so any visiting
-// order reaches the same fixed point as fea.py:193-204's synchronous passes).
-__global__ void k_island_grow(int nx, int ny, int nz, const uint8_t* __restrict__ active, uint8_t* kept,
-                              int* changed) {
-  const long long ne = (long long)nx * ny * nz;
-  int any = 0;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ne; e += (long long)gridDim.x * blockDim.x) {
-    if (!active[e] || kept[e]) continue;
-    const int iz = (int)(e % nz);
-    const long long t = e / nz;
-    const int iy = (int)(t % ny), ix = (int)(t / ny);
-    const long long sx = (long long)ny * nz, sy = nz;
-    uint8_t g = 0;
-    if (ix > 0) g |= ((volatile uint8_t*)kept)[e - sx];
-    if (ix + 1 < nx) g |= ((volatile uint8_t*)kept)[e + sx];
-    if (iy > 0) g |= ((volatile uint8_t*)kept)[e - sy];
-    if (iy + 1 < ny) g |= ((volatile uint8_t*)kept)[e + sy];
-    if (iz > 0) g |= ((volatile uint8_t*)kept)[e - 1];
-    if (iz + 1 < nz) g |= ((volatile uint8_t*)kept)[e + 1];
-    if (g) { kept[e] = 1; any = 1; }
+// One pass of the fill (monotone: kept only grows, so any visiting order
+// reaches the same fixed point as fea.py:193-204's synchronous passes).  A
+// block owns a tile of voxels and dilates it in shared memory until the tile
+// no longer changes, so a pass carries the fill across whole tiles: one voxel
+// a pass took 104 launches and 13 host checks on a 128x96x64 part (0.9 ms).
+constexpr int kFillX = 4, kFillY = 8, kFillZ = 32, kFillThreads = 256;
+__global__ void __launch_bounds__(kFillThreads) k_island_grow(int nx, int ny, int nz, const uint8_t* __restrict__ active,
+                                                              uint8_t* kept, int* changed) {
+  constexpr int HX = kFillX + 2, HY = kFillY + 2, HZ = kFillZ + 2, PER = kFillX * kFillY * kFillZ / kFillThreads;
+  __shared__ uint8_t s_kept[HX][HY][HZ];
+  const int tz = (nz + kFillZ - 1) / kFillZ, ty = (ny + kFillY - 1) / kFillY;
+  const int z0 = (int)(blockIdx.x % tz) * kFillZ, y0 = (int)(blockIdx.x / tz % ty) * kFillY;
+  const int x0 = (int)(blockIdx.x / tz / ty) * kFillX;
+  for (int i = threadIdx.x; i < HX * HY * HZ; i += kFillThreads) {
+    const int iz = i % HZ, iy = i / HZ % HY, ix = i / (HZ * HY);
+    const int x = x0 + ix - 1, y = y0 + iy - 1, z = z0 + iz - 1;
+    const bool in = x >= 0 && x < nx && y >= 0 && y < ny && z >= 0 && z < nz;
+    s_kept[ix][iy][iz] = in ? ((volatile uint8_t*)kept)[((long long)x * ny + y) * nz + z] : (uint8_t)0;
   }
-  if (any) *changed = 1;
+  const int lz = threadIdx.x % kFillZ, ly = threadIdx.x / kFillZ;   // this thread: PER voxels along x
+  const int y = y0 + ly, z = z0 + lz;
+  unsigned open = 0, grown = 0;   // bit k: voxel k is active and not kept yet / became kept here
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int x = x0 + k;
+    if (x < nx && y < ny && z < nz && active[((long long)x * ny + y) * nz + z] && !s_kept[k + 1][ly + 1][lz + 1])
+      open |= 1u << k;
+  }
+  for (;;) {
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      if (!((open >> k) & 1)) continue;
+      volatile uint8_t* c = &s_kept[k + 1][ly + 1][lz + 1];
+      if (c[-HY * HZ] | c[HY * HZ] | c[-HZ] | c[HZ] | c[-1] | c[1]) {
+        *c = 1;
+        open &= ~(1u << k);
+        grown |= 1u << k;
+        any = true;
+      }
+    }
+    if (!__syncthreads_or(any)) break;
+  }
+#pragma unroll
+  for (int k = 0; k < PER; ++k)
+    if ((grown >> k) & 1) ((volatile uint8_t*)kept)[((long long)(x0 + k) * ny + y) * nz + z] = 1;
+  if (grown) *changed = 1;
 }
+static_assert(kFillY * kFillZ == kFillThreads, "one thread per column of the tile along x");
 
 }  // namespace
 
@@ -153,13 +180,15 @@ int flood_fill_islands(int nx, int ny, int nz, const uint8_t* d_active, const ui
   int blocks = (int)((ne + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
   launch_k(k_island_seed, blocks, 256, 0, st, nx, ny, nz, d_active, d_fixed_node, d_kept);
+  const long long tiles = ((long long)(nx + kFillX - 1) / kFillX) * ((ny + kFillY - 1) / kFillY) * ((nz + kFillZ - 1) / kFillZ);
   int passes = 0;
   const long long max_passes = 4 * ((long long)nx + ny + nz) + ne;   // monotone: ends long before
   for (;;) {
     int h_changed = 0;
     cudaMemsetAsync(d_changed, 0, sizeof(int), st);
-    for (int k = 0; k < 8; ++k) launch_k(k_island_grow, blocks, 256, 0, st, nx, ny, nz, d_active, d_kept, d_changed);
-    passes += 8;
+    for (int k = 0; k < 4; ++k)
+      launch_k(k_island_grow, (unsigned)tiles, kFillThreads, 0, st, nx, ny, nz, d_active, d_kept, d_changed);
+    passes += 4;
     cudaMemcpyAsync(&h_changed, d_changed, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
     if (!h_changed || passes > max_passes) break;

@@ -4,18 +4,27 @@
 // One fixed ray direction d per query; a point is inside a closed triangle
 // mesh when the ray from it crosses an odd number of triangles
 // (Moeller-Trumbore: u >= -1e-7, v >= -1e-7, u + v <= 1 + 1e-7, t > 1e-7,
-// triangles with |det| < 1e-9 skipped).  One thread per point; triangles are
-// streamed through shared memory in tiles, pre-transformed once (v0, e1, e2,
-// p = d x e2, 1/det).  Every product and sum is an explicitly rounded FP64
+// triangles with |det| < 1e-9 skipped).  Triangles are pre-transformed once
+// (v0, e1, e2, p = d x e2, 1/det).  Every product and sum is an explicitly rounded FP64
 // operation in the reference's evaluation order (no contraction into FMAs),
 // so the inside/outside decisions are the reference's bit for bit.
-// The points are either given, or generated on the fly for a voxel grid
-// (voxel centers in element order iz-fastest, or nodes in node order
-// x-fastest: inside_worker.py:voxel_centers / node_coords).
+//
+// Given points: one thread per point, every triangle streamed through shared
+// memory (k_inside).  Points of a voxel grid (voxel centers in element order
+// iz-fastest, or nodes in node order x-fastest: inside_worker.py:voxel_centers /
+// node_coords): each triangle visits only the grid points whose ray can meet
+// it (k_inside_grid), found from the bounds of its projection along the ray,
+// widened by the test's own tolerance and a bound of its rounding, and flips
+// their parity; the test of a visited point is the same arithmetic, and a
+// point that is not visited could not have passed it.  All points against all
+// triangles cost points x triangles tests at the FP64 rate (786,432 centers x
+// 10,000 triangles: 18.8 ms); now their number is the grid lines that each
+// triangle covers times the points before it.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <vector>
+#include <algorithm>
+#include <cmath>
 
 #include "../../include/voxfea.h"
 #include "vf_common.cuh"
@@ -43,6 +52,23 @@ __device__ __forceinline__ void cross3(const double* a, const double* b, double*
 }
 
 struct Dir { double d[3]; };
+
+// Whether the ray from p meets prepared triangle T (T[12] != 0).
+__device__ __forceinline__ bool hits_triangle(const double* p, const double* T, const Dir& dir) {
+  const double inv = T[12];
+  const double tv[3] = {sub(p[0], T[0]), sub(p[1], T[1]), sub(p[2], T[2])};
+  const double u = mul(dot3(tv, T + 9), inv);
+  double q[3];
+  cross3(tv, T + 3, q);
+  const double v = mul(dot3(dir.d, q), inv);
+  const double t = mul(dot3(T + 6, q), inv);
+  return u >= -1e-7 && v >= -1e-7 && add(u, v) <= 1.0 + 1e-7 && t > 1e-7;
+}
+
+// Coordinate c of grid point k along its axis (mode 1: centers, 2: nodes).
+__device__ __forceinline__ double grid_coord(int mode, int k, double vs, double o) {
+  return add(mul(mode == 1 ? k + 0.5 : (double)k, vs), o);
+}
 
 __global__ void k_prepare_tris(const double* __restrict__ verts, const int64_t* __restrict__ faces, int64_t nf,
                                Dir dir, double* __restrict__ tri) {
@@ -75,17 +101,14 @@ __global__ void k_inside(int mode, const double* __restrict__ pts, int64_t npts,
   if (live) {
     if (mode == 0) {
       p[0] = pts[3 * i]; p[1] = pts[3 * i + 1]; p[2] = pts[3 * i + 2];
-    } else if (mode == 1) {   // element order: (ix * ny + iy) * nz + iz
-      const int iz = (int)(i % nz), iy = (int)((i / nz) % ny), ix = (int)(i / ((int64_t)nz * ny));
-      p[0] = add(mul(ix + 0.5, vs), ox);
-      p[1] = add(mul(iy + 0.5, vs), oy);
-      p[2] = add(mul(iz + 0.5, vs), oz);
-    } else {                  // node order: ix + (nx+1) (iy + (ny+1) iz)
+    } else {   // element order (ix * ny + iy) * nz + iz, node order ix + (nx+1) (iy + (ny+1) iz)
       const int nxp = nx + 1, nyp = ny + 1;
-      const int ix = (int)(i % nxp), iy = (int)((i / nxp) % nyp), iz = (int)(i / ((int64_t)nxp * nyp));
-      p[0] = add(mul((double)ix, vs), ox);
-      p[1] = add(mul((double)iy, vs), oy);
-      p[2] = add(mul((double)iz, vs), oz);
+      const int ix = mode == 1 ? (int)(i / ((int64_t)nz * ny)) : (int)(i % nxp);
+      const int iy = mode == 1 ? (int)((i / nz) % ny) : (int)((i / nxp) % nyp);
+      const int iz = mode == 1 ? (int)(i % nz) : (int)(i / ((int64_t)nxp * nyp));
+      p[0] = grid_coord(mode, ix, vs, ox);
+      p[1] = grid_coord(mode, iy, vs, oy);
+      p[2] = grid_coord(mode, iz, vs, oz);
     }
   }
   int hits = 0;
@@ -97,18 +120,106 @@ __global__ void k_inside(int mode, const double* __restrict__ pts, int64_t npts,
     if (!live) continue;
     for (int k = 0; k < nt; ++k) {
       const double* T = s_tri + kTriVals * k;
-      const double inv = T[12];
-      if (inv == 0.0) continue;   // |det| < 1e-9
-      const double tv[3] = {sub(p[0], T[0]), sub(p[1], T[1]), sub(p[2], T[2])};
-      const double u = mul(dot3(tv, T + 9), inv);
-      double q[3];
-      cross3(tv, T + 3, q);
-      const double v = mul(dot3(dir.d, q), inv);
-      const double t = mul(dot3(T + 6, q), inv);
-      hits += (u >= -1e-7 && v >= -1e-7 && add(u, v) <= 1.0 + 1e-7 && t > 1e-7) ? 1 : 0;
+      if (T[12] == 0.0) continue;   // |det| < 1e-9
+      hits += hits_triangle(p, T, dir) ? 1 : 0;
     }
   }
   if (live) out[i] = (uint8_t)(hits & 1);
+}
+
+// The grid of k_inside_grid: n points along each axis, the ray's dominant axis
+// a and the other two b, c; sb, sc: the ray's slopes along them.
+struct RayGrid {
+  int mode, n[3], a, b, c;
+  double o[3], vs, sb, sc;
+};
+
+// The points that one triangle's test can pass, as ranges of the projected
+// coordinates B = p_b - sb p_a and C = p_c - sc p_a (constant along the ray)
+// and of p_a.  A point passes only if, in exact arithmetic,
+//   p + t d = v0 + u e1 + v e2,  u, v >= -tau, u + v <= 1 + tau, t >= -tau_t
+// with tau the test's 1e-7 plus what rounding can add: u and v are sums of a
+// few products of |tv| <= R, |e1|, |e2|, |d| times 1/det, each within 16 eps
+// of them and 1/det itself within 16 eps |e1| |e2| |d| / |det| of its own
+// (64 eps here).  So B lies within 3 tau (|B(e1)| + |B(e2)|) of the vertices'
+// range.  Bounds that are not finite come out as the whole axis.
+struct TriBounds { double b0, b1, c0, c1, amin, amax; };
+__device__ __forceinline__ TriBounds tri_bounds(const double* T, const Dir& dir, const RayGrid& G) {
+  auto norm1 = [](const double* v) { return fabs(v[0]) + fabs(v[1]) + fabs(v[2]); };
+  double R = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    const double lo = G.o[k], hi = G.o[k] + G.n[k] * G.vs;
+    R += fmax(fabs(lo - T[k]), fabs(hi - T[k])) + fabs(lo) * 1e-15 + fabs(T[k]) * 1e-15;
+  }
+  const double l1 = norm1(T + 3), l2 = norm1(T + 6), ld = norm1(dir.d);
+  const double eps = 64.0 * 2.3e-16 * fabs(T[12]) * ld;
+  const double S = R + l1 + l2;
+  const double tau = 4e-7 + eps * S * (l1 + l2), tau_t = eps / ld * S * l1 * l2 + 1e-7;
+  auto B = [&](const double* v) { return v[G.b] - G.sb * v[G.a]; };
+  auto C = [&](const double* v) { return v[G.c] - G.sc * v[G.a]; };
+  const double vb = B(T), vc = C(T), b1 = B(T + 3), b2 = B(T + 6), c1 = C(T + 3), c2 = C(T + 6);
+  // (the projections' own rounding, and 1e-6 of a voxel for the index arithmetic)
+  const double slack = 1e-6 * G.vs + 1e-14 * (norm1(T) + R);
+  const double mb = 3.0 * tau * (fabs(b1) + fabs(b2)) + slack, mc = 3.0 * tau * (fabs(c1) + fabs(c2)) + slack;
+  const double a1 = T[3 + G.a], a2 = T[6 + G.a];
+  const double ma = 3.0 * tau * (fabs(a1) + fabs(a2)) + tau_t * fabs(dir.d[G.a]) + slack;
+  TriBounds r;
+  r.b0 = vb + fmin(0.0, fmin(b1, b2)) - mb;
+  r.b1 = vb + fmax(0.0, fmax(b1, b2)) + mb;
+  r.c0 = vc + fmin(0.0, fmin(c1, c2)) - mc;
+  r.c1 = vc + fmax(0.0, fmax(c1, c2)) + mc;
+  r.amin = T[G.a] + fmin(0.0, fmin(a1, a2)) - ma;
+  r.amax = T[G.a] + fmax(0.0, fmax(a1, a2)) + ma;
+  return r;
+}
+// first / last grid index whose coordinate is >= lo / <= hi (NaN: the whole axis)
+__device__ __forceinline__ int first_index(double lo, double o, double vs, double half, int n) {
+  return (int)fmin(fmax(ceil((lo - o) / vs - half), 0.0), (double)n);
+}
+__device__ __forceinline__ int last_index(double hi, double o, double vs, double half, int n) {
+  return (int)fmax(fmin(floor((hi - o) / vs - half), (double)(n - 1)), -1.0);
+}
+
+// blockIdx.x: triangle; the blocks of a triangle (gridDim.y) share its
+// candidate points: the grid positions along the ray's axis times the widest
+// rectangle of grid lines its projection covers at any of them.
+__global__ void __launch_bounds__(128) k_inside_grid(RayGrid G, const double* __restrict__ tri, Dir dir,
+                                                     unsigned* __restrict__ out) {
+  const double* Tg = tri + (int64_t)kTriVals * blockIdx.x;
+  double T[kTriVals];
+#pragma unroll
+  for (int k = 0; k < kTriVals; ++k) T[k] = __ldg(Tg + k);
+  if (T[12] == 0.0) return;
+  const TriBounds r = tri_bounds(T, dir, G);
+  const double half = G.mode == 1 ? 0.5 : 0.0;
+  const int na = G.n[G.a], nb = G.n[G.b], nc = G.n[G.c];
+  // the ray runs along +a or -a: points before the triangle's far end
+  int ia0 = 0, ia1 = na - 1;
+  if (dir.d[G.a] > 0.0) ia1 = last_index(r.amax, G.o[G.a], G.vs, half, na);
+  else ia0 = first_index(r.amin, G.o[G.a], G.vs, half, na);
+  const int la = ia1 - ia0 + 1;
+  if (la <= 0) return;
+  const int wb = (int)fmin(floor((r.b1 - r.b0) / G.vs) + 2.0, (double)nb);
+  const int wc = (int)fmin(floor((r.c1 - r.c0) / G.vs) + 2.0, (double)nc);
+  const int64_t total = (int64_t)la * wb * wc;
+  for (int64_t i = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.y * blockDim.x) {
+    int64_t q = i / wc;
+    const int jc = (int)(i - q * wc), ja = (int)(q / wb), jb = (int)(q - (int64_t)ja * wb);
+    int k[3];
+    double p[3];
+    k[G.a] = ia0 + ja;
+    p[G.a] = grid_coord(G.mode, k[G.a], G.vs, G.o[G.a]);
+    const double sb = G.sb * p[G.a], sc = G.sc * p[G.a];
+    k[G.b] = first_index(r.b0 + sb, G.o[G.b], G.vs, half, nb) + jb;
+    k[G.c] = first_index(r.c0 + sc, G.o[G.c], G.vs, half, nc) + jc;
+    if (k[G.b] >= nb || k[G.c] >= nc) continue;
+    p[G.b] = grid_coord(G.mode, k[G.b], G.vs, G.o[G.b]);
+    p[G.c] = grid_coord(G.mode, k[G.c], G.vs, G.o[G.c]);
+    if (!hits_triangle(p, T, dir)) continue;
+    const int64_t e = G.mode == 1 ? ((int64_t)k[0] * G.n[1] + k[1]) * G.n[2] + k[2]
+                                  : k[0] + (int64_t)G.n[0] * (k[1] + (int64_t)G.n[1] * k[2]);
+    atomicXor(out + (e >> 2), 1u << (8 * (e & 3)));   // one byte per point
+  }
 }
 
 int inside_run(int mode, const double* verts, int64_t nv, const int64_t* faces, int64_t nf, const double* pts,
@@ -138,8 +249,32 @@ int inside_run(int mode, const double* verts, int64_t nv, const int64_t* faces, 
   if (mode == 0) cudaMemcpyAsync(d_p, pts, sizeof(double) * 3 * (size_t)npts, cudaMemcpyHostToDevice, st);
   const int nx = dims ? dims[0] : 0, ny = dims ? dims[1] : 0, nz = dims ? dims[2] : 0;
   const double ox = origin ? origin[0] : 0.0, oy = origin ? origin[1] : 0.0, oz = origin ? origin[2] : 0.0;
-  launch_k(k_inside, (unsigned)((npts + 255) / 256), 256, 0, st, mode, (const double*)d_p, npts, nx, ny, nz, ox, oy,
-           oz, vsize, (const double*)d_tri, nf, d, d_o);
+  int axis = 0;
+  for (int c = 1; c < 3; ++c)
+    if (std::fabs(dir3[c]) > std::fabs(dir3[axis])) axis = c;
+  const int64_t kMaxTri = 1 << 30;   // a block each
+  if (mode == 0 || nf > kMaxTri || !(vsize > 0.0) || !(std::fabs(dir3[axis]) > 0.0) || !std::isfinite(dir3[0] + dir3[1] + dir3[2])) {
+    // given points, or a grid or ray that has no lines to speak of
+    launch_k(k_inside, (unsigned)((npts + 255) / 256), 256, 0, st, mode, (const double*)d_p, npts, nx, ny, nz, ox, oy,
+             oz, vsize, (const double*)d_tri, nf, d, d_o);
+  } else {
+    cudaMemsetAsync(d_o, 0, (size_t)npts, st);
+    RayGrid G;
+    G.mode = mode;
+    for (int c = 0; c < 3; ++c) {
+      G.n[c] = dims[c] + (mode == 2 ? 1 : 0);
+      G.o[c] = origin[c];
+    }
+    G.a = axis; G.b = (axis + 1) % 3; G.c = (axis + 2) % 3;
+    G.vs = vsize;
+    G.sb = dir3[G.b] / dir3[axis];
+    G.sc = dir3[G.c] / dir3[axis];
+    // a mesh of few triangles (a support box: 12) covers many points with each:
+    // enough blocks to fill the device share a triangle's candidates
+    const unsigned per = (unsigned)std::max<int64_t>(1, std::min<int64_t>((16 * 148 + nf - 1) / std::max<int64_t>(nf, 1), 256));
+    if (nf > 0)
+      launch_k(k_inside_grid, dim3((unsigned)nf, per), 128, 0, st, G, (const double*)d_tri, d, (unsigned*)d_o);
+  }
   cudaMemcpyAsync(out, d_o, (size_t)npts, cudaMemcpyDeviceToHost, st);
   return cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess ? VF_ERR_CUDA : VF_OK;
 }
