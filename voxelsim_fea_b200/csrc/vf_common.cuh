@@ -265,7 +265,7 @@ template <typename T> void launch_dense_solve(const double* Ainv, int n, const i
 void launch_dense_solve_f32(const float* Ainv32, int n, const int* perm, const float* b, float* x, const KrylovState* ks, cudaStream_t st);
 
 // vf_krylov.cu -- fused PCG vector kernels with deterministic FP64 reductions
-constexpr int kVecBlocks = 148 * 8;     // grid of the vector kernels (fixed => deterministic)
+constexpr int kVecBlocks = 148 * 8;     // largest grid of the vector kernels (by size alone => deterministic)
 constexpr int kVecThreads = 256;
 template <typename T> void launch_dot(const Grid& g, const T* a, const T* b, double* partials, KrylovState* ks, int slot, cudaStream_t st);
 template <typename T> void launch_cg_update(const Grid& g, T* x, const T* p, T* r, const T* Ap, double* partials, KrylovState* ks, double* hist, cudaStream_t st);
@@ -273,6 +273,9 @@ template <typename T> void launch_p_update(const Grid& g, T* p, const T* z, Kryl
 template <typename T> void launch_dot_fcg(const Grid& g, const T* r, const T* z, const T* Ap, double* partials,
                                           KrylovState* ks, cudaStream_t st);
 template <typename T> void launch_jacobi_precond(const Grid& g, const T* r, const T* minv3, const uint8_t* mask, T* z, const KrylovState* ks, cudaStream_t st);
+// Jacobi-PCG: the vector update with r.r and r.z (z = Minv r), and p = z + beta p
+template <typename T> void launch_jacobi_update(const Grid& g, T* x, const T* p, T* r, const T* Ap, const T* minv3, double* partials, KrylovState* ks, double* hist, cudaStream_t st);
+template <typename T> void launch_jacobi_direction(const Grid& g, T* p, const T* r, const T* minv3, const KrylovState* ks, cudaStream_t st);
 template <typename T> void launch_copy_vec(const Grid& g, const T* src, T* dst, const KrylovState* ks, cudaStream_t st);
 void launch_norm2_f64(const Grid& g, const double* v, double* partials, KrylovState* ks, int slot, cudaStream_t st);
 void launch_ir_prepare(const Grid& g, const double* r64, float* r32, KrylovState* ks, cudaStream_t st);

@@ -22,12 +22,14 @@ template <> struct V16<float> {
   __device__ __forceinline__ static V axpy(float s, V x, V y) {   // y + s x
     return make_float4(fmaf(s, x.x, y.x), fmaf(s, x.y, y.y), fmaf(s, x.z, y.z), fmaf(s, x.w, y.w));
   }
+  __device__ __forceinline__ static V mul(V a, V b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 };
 template <> struct V16<double> {
   using V = double2;
   static constexpr int W = 2;
   __device__ __forceinline__ static double dot(V a, V b) { return a.x * b.x + a.y * b.y; }
   __device__ __forceinline__ static V axpy(double s, V x, V y) { return make_double2(fma(s, x.x, y.x), fma(s, x.y, y.y)); }
+  __device__ __forceinline__ static V mul(V a, V b) { return make_double2(a.x * b.x, a.y * b.y); }
 };
 
 template <typename T>
@@ -219,6 +221,60 @@ __global__ void k_jacobi_precond(int n, const T* __restrict__ r, const T* __rest
   }
 }
 
+// Jacobi-PCG's vector update: x += alpha p, r -= alpha A p and, with
+// z = Minv r (fea.py:566-571) only ever formed here and in the direction
+// update, both sums r.r and r.z: one pass in place of the update, the
+// preconditioner and the dot product, 7 reads and writes a value instead of
+// 12.  With k_jacobi_direction, two launches fewer an iteration, which short
+// vectors are bound by: a job on a 61x43x37 grid 92.9 -> 55.9 ms (with the
+// smaller grids of vec_blocks and several chunks per look at the state).
+template <typename T>
+__global__ void __launch_bounds__(kVecThreads) k_jacobi_update(long long n3, T* __restrict__ x, const T* __restrict__ p,
+                                                               T* __restrict__ r, const T* __restrict__ Ap,
+                                                               const T* __restrict__ minv, double* partials,
+                                                               KrylovState* ks, double* hist) {
+  if (ks->done) return;
+  using H = V16<T>;
+  using V = typename H::V;
+  const T alpha = (T)ks->alpha;
+  const long long nv = n3 / H::W;
+  V* xv = reinterpret_cast<V*>(x);
+  V* rv = reinterpret_cast<V*>(r);
+  const V* pv = reinterpret_cast<const V*>(p);
+  const V* av = reinterpret_cast<const V*>(Ap);
+  const V* mv = reinterpret_cast<const V*>(minv);
+  double s = 0.0, sz = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
+    const V pi = __ldg(pv + i), ai = __ldg(av + i), mi = __ldg(mv + i);
+    xv[i] = H::axpy(alpha, pi, xv[i]);
+    const V ri = H::axpy(-alpha, ai, rv[i]);
+    rv[i] = ri;
+    s += H::dot(ri, ri);
+    sz += H::dot(ri, H::mul(mi, ri));
+  }
+  reduce_rr_rz(s, sz, partials, ks, hist);
+}
+
+// p = Minv r + beta p (r is zero on the DOFs that are not free)
+template <typename T>
+__global__ void __launch_bounds__(kVecThreads) k_jacobi_direction(long long n3, T* __restrict__ p,
+                                                                  const T* __restrict__ r, const T* __restrict__ minv,
+                                                                  const KrylovState* ks) {
+  if (ks->done) return;
+  using H = V16<T>;
+  using V = typename H::V;
+  const bool restart = ks->restart != 0;
+  const T beta = restart ? (T)0 : (T)ks->beta;
+  const long long nv = n3 / H::W;
+  V* pv = reinterpret_cast<V*>(p);
+  const V* rv = reinterpret_cast<const V*>(r);
+  const V* mv = reinterpret_cast<const V*>(minv);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
+    const V z = H::mul(__ldg(mv + i), __ldg(rv + i));
+    pv[i] = restart ? z : H::axpy(beta, pv[i], z);
+  }
+}
+
 template <typename T>
 __global__ void k_copy(long long n3, const T* __restrict__ s, T* __restrict__ d, const KrylovState* ks) {
   if (ks && ks->done) return;
@@ -345,6 +401,15 @@ __global__ void k_cheb_coefs(const double* lambda, int nl, int ratio, double* co
   c[3] = 2.0 * rho1 / delta;
 }
 
+// Blocks of a vector pass over nv 16-byte values: two values a thread on short
+// vectors, the fixed full grid on long ones.  The grid depends on the size
+// alone (determinism); on short vectors idle blocks only lengthen the sum of
+// the partials (1,184 blocks on 176,000 values: k_dot 9.4 us, now 345).
+inline int vec_blocks(long long nv) {
+  const long long b = (nv + 2 * kVecThreads - 1) / (2 * kVecThreads);
+  return (int)(b < 1 ? 1 : (b > kVecBlocks ? kVecBlocks : b));
+}
+
 }  // namespace
 
 void launch_cheb_coefs(const double* lambda, int nl, int ratio, double* coef, cudaStream_t st) {
@@ -353,15 +418,15 @@ void launch_cheb_coefs(const double* lambda, int nl, int ratio, double* coef, cu
 
 template <typename T>
 void launch_power_init(const Grid& g, T* x, const uint8_t* mask, cudaStream_t st) {
-  launch_k(k_power_init<T>, kVecBlocks, kVecThreads, 0, st, (long long)g.n, x, mask);
+  launch_k(k_power_init<T>, vec_blocks((long long)g.n), kVecThreads, 0, st, (long long)g.n, x, mask);
 }
 template <typename T>
 void launch_power_scale(const Grid& g, T* y, const T* minv3, double* partials, KrylovState* ks, cudaStream_t st) {
-  launch_k(k_power_scale<T>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, y, minv3, partials, ks);
+  launch_k(k_power_scale<T>, vec_blocks(3LL * g.n), kVecThreads, 0, st, 3LL * g.n, y, minv3, partials, ks);
 }
 template <typename T>
 void launch_power_normalize(const Grid& g, const T* y, T* x, const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_power_normalize<T>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, y, x, ks);
+  launch_k(k_power_normalize<T>, vec_blocks(3LL * g.n), kVecThreads, 0, st, 3LL * g.n, y, x, ks);
 }
 #define VF_INST_POWER(T)                                                                                   \
   template void launch_power_init<T>(const Grid&, T*, const uint8_t*, cudaStream_t);                       \
@@ -377,28 +442,38 @@ void launch_power_omega(const KrylovState* ks, double omega_rel, double safety, 
 
 template <typename T>
 void launch_dot(const Grid& g, const T* a, const T* b, double* partials, KrylovState* ks, int slot, cudaStream_t st) {
-  launch_k(k_dot<T>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, a, b, partials, ks, slot);
+  launch_k(k_dot<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, a, b, partials, ks, slot);
 }
 template <typename T>
 void launch_cg_update(const Grid& g, T* x, const T* p, T* r, const T* Ap, double* partials, KrylovState* ks,
                       double* hist, cudaStream_t st) {
-  launch_k(k_cg_update<T>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, x, p, r, Ap, partials, ks, hist);
+  launch_k(k_cg_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, p, r, Ap, partials, ks, hist);
 }
 template <typename T>
 void launch_p_update(const Grid& g, T* p, const T* z, KrylovState* ks, cudaStream_t st) {
-  launch_k(k_p_update<T>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, p, z, ks);
+  launch_k(k_p_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, p, z, ks);
 }
 template <typename T>
 void launch_jacobi_precond(const Grid& g, const T* r, const T* minv3, const uint8_t* mask, T* z,
                            const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_jacobi_precond<T>, kVecBlocks, kVecThreads, 0, st, g.n, r, minv3, mask, z, ks);
+  launch_k(k_jacobi_precond<T>, vec_blocks(g.n), kVecThreads, 0, st, g.n, r, minv3, mask, z, ks);
+}
+template <typename T>
+void launch_jacobi_update(const Grid& g, T* x, const T* p, T* r, const T* Ap, const T* minv3, double* partials,
+                          KrylovState* ks, double* hist, cudaStream_t st) {
+  launch_k(k_jacobi_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, p, r, Ap, minv3,
+           partials, ks, hist);
+}
+template <typename T>
+void launch_jacobi_direction(const Grid& g, T* p, const T* r, const T* minv3, const KrylovState* ks, cudaStream_t st) {
+  launch_k(k_jacobi_direction<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, p, r, minv3, ks);
 }
 template <typename T>
 void launch_copy_vec(const Grid& g, const T* src, T* dst, const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_copy<T>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, src, dst, ks);
+  launch_k(k_copy<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, src, dst, ks);
 }
 void launch_norm2_f64(const Grid& g, const double* v, double* partials, KrylovState* ks, int slot, cudaStream_t st) {
-  launch_k(k_dot<double>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, v, v, partials, ks, slot);
+  launch_k(k_dot<double>, vec_blocks(3LL * g.n / 2), kVecThreads, 0, st, 3LL * g.n, v, v, partials, ks, slot);
 }
 void launch_ir_prepare(const Grid& g, const double* r64, float* r32, KrylovState* ks, cudaStream_t st) {
   launch_k(k_ir_prepare, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, r64, r32, ks);
@@ -428,14 +503,14 @@ void launch_sub_from(const Grid& g, const double* f, double* r, cudaStream_t st)
 
 void launch_cg_update_split(const Grid& g, double* r, const double* Ap, float* r32, double* partials,
                             KrylovState* ks, double* hist, cudaStream_t st) {
-  launch_k(k_cg_update_split, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, r, Ap, r32, partials, ks, hist);
+  launch_k(k_cg_update_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, r, Ap, r32, partials, ks, hist);
 }
 void launch_p_update_split(const Grid& g, double* x, double* p, const float* z, KrylovState* ks, cudaStream_t st) {
-  launch_k(k_p_update_split, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, x, p, z, ks);
+  launch_k(k_p_update_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, x, p, z, ks);
 }
 void launch_dot_fcg_split(const Grid& g, const float* r, const float* z, const double* Ap, double* partials,
                           KrylovState* ks, cudaStream_t st) {
-  launch_k(k_dot_fcg_split, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
+  launch_k(k_dot_fcg_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
 }
 void launch_scale64(const Grid& g, const double* x, double* y, double sc, cudaStream_t st) {
   launch_k(k_scale64, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, x, y, sc);
@@ -444,7 +519,7 @@ void launch_scale64(const Grid& g, const double* x, double* y, double sc, cudaSt
 template <typename T>
 void launch_dot_fcg(const Grid& g, const T* r, const T* z, const T* Ap, double* partials, KrylovState* ks,
                     cudaStream_t st) {
-  launch_k(k_dot_fcg<T>, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
+  launch_k(k_dot_fcg<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
 }
 
 #define VF_INST(T)                                                                                            \
@@ -453,6 +528,8 @@ void launch_dot_fcg(const Grid& g, const T* r, const T* z, const T* Ap, double* 
   template void launch_p_update<T>(const Grid&, T*, const T*, KrylovState*, cudaStream_t);                   \
   template void launch_dot_fcg<T>(const Grid&, const T*, const T*, const T*, double*, KrylovState*, cudaStream_t); \
   template void launch_jacobi_precond<T>(const Grid&, const T*, const T*, const uint8_t*, T*, const KrylovState*, cudaStream_t); \
+  template void launch_jacobi_update<T>(const Grid&, T*, const T*, T*, const T*, const T*, double*, KrylovState*, double*, cudaStream_t); \
+  template void launch_jacobi_direction<T>(const Grid&, T*, const T*, const T*, const KrylovState*, cudaStream_t); \
   template void launch_copy_vec<T>(const Grid&, const T*, T*, const KrylovState*, cudaStream_t);
 VF_INST(double)
 VF_INST(float)

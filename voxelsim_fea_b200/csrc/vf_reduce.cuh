@@ -104,6 +104,47 @@ __device__ inline void finalize_slot(KrylovState* ks, int slot, double total, do
   }
 }
 
+// The pairs of partials summed by the last CTA (valid in thread 0)
+__device__ __forceinline__ void sum_partials2(const double* partials, int nb, double& a, double& b) {
+  double ta = 0.0, tb = 0.0;
+  const double2* p2 = reinterpret_cast<const double2*>(partials);
+#pragma unroll 4
+  for (int i = lin_tid(); i < nb; i += lin_nthreads()) {
+    const double2 v = __ldcg(p2 + i);
+    ta += v.x;
+    tb += v.y;
+  }
+  a = block_sum(ta);
+  b = block_sum(tb);
+}
+
+// Jacobi-PCG: r.r and r.z in one pass; the last CTA finalizes r.r (ratio,
+// history, stopping tests) and, if the iteration goes on, r.z (beta)
+__device__ inline void reduce_rr_rz(double rr, double rz, double* partials, KrylovState* ks, double* hist) {
+  __shared__ bool s_last3;
+  const double sa = block_sum(rr);
+  const double sb = block_sum(rz);
+  const int tid = lin_tid();
+  const unsigned nb = lin_nblocks();
+  if (tid == 0) {
+    partials[2 * lin_bid()] = sa;
+    partials[2 * lin_bid() + 1] = sb;
+    __threadfence();
+    s_last3 = (atomicAdd(&ks->counter[SLOT_RR], 1u) == nb - 1);
+  }
+  __syncthreads();
+  if (!s_last3) return;
+  __threadfence();
+  double ta, tb;
+  sum_partials2(partials, (int)nb, ta, tb);
+  if (tid == 0) {
+    finalize_slot(ks, SLOT_RR, ta, hist);
+    if (!ks->done) finalize_slot(ks, SLOT_RZ, tb, nullptr);
+    ks->counter[SLOT_RR] = 0u;
+    __threadfence();
+  }
+}
+
 // Two sums in one pass (partials hold 2 doubles per CTA); the last CTA finalizes
 // both together.  Used by the flexible-CG beta.
 __device__ inline void reduce2_and_finalize(double a, double b, double* partials, KrylovState* ks, int slot) {
@@ -122,13 +163,8 @@ __device__ inline void reduce2_and_finalize(double a, double b, double* partials
   __syncthreads();
   if (!s_last2) return;
   __threadfence();
-  double ta = 0.0, tb = 0.0;
-  for (int i = tid; i < (int)nb; i += lin_nthreads()) {
-    ta += ((volatile double*)partials)[2 * i];
-    tb += ((volatile double*)partials)[2 * i + 1];
-  }
-  ta = block_sum(ta);
-  tb = block_sum(tb);
+  double ta, tb;
+  sum_partials2(partials, (int)nb, ta, tb);
   if (tid == 0) {
     // FCG(1): p_new = z - (z.Ap / p.Ap) p; alpha next = (r.z) / (p_new.Ap_new)
     ks->rz_new = ta;
@@ -159,7 +195,9 @@ __device__ inline void reduce_and_finalize(double v, double* partials, KrylovSta
   if (!s_last) return;
   __threadfence();
   double t = 0.0;
-  for (int i = tid; i < (int)nb; i += lin_nthreads()) t += ((volatile double*)partials)[i];
+  // (through L2, several in flight: the partials come from other SMs)
+#pragma unroll 4
+  for (int i = tid; i < (int)nb; i += lin_nthreads()) t += __ldcg(partials + i);
   t = block_sum(t);
   if (tid == 0) {
     finalize_slot(ks, slot, t, hist);

@@ -576,6 +576,11 @@ void pcg_iteration(vf_solver* s) {
   const Grid& g = s->L[0].g;
   // the fine operator (level 0), masked, fused with p.Ap -> alpha
   level_op<T>(s, 0, EPI_APPLY, p, Ap, nullptr, s->ks, s->d_partials, SLOT_PAP);
+  if (!use_mg(s) && !flexible(s)) {   // Jacobi-PCG: z = Minv r is formed where it is used
+    launch_jacobi_update<T>(g, x, p, r, Ap, Sel<T>::minv(s->L[0]), s->d_partials, s->ks, s->d_hist, s->st);
+    launch_jacobi_direction<T>(g, p, r, Sel<T>::minv(s->L[0]), s->ks, s->st);
+    return;
+  }
   launch_cg_update<T>(g, x, p, r, Ap, s->d_partials, s->ks, s->d_hist, s->st);
   precondition<T>(s, r, z, s->ks, fused_rz(s) ? SLOT_RZ : -1);
   update_direction<T>(s, r, z, p, Ap);
@@ -635,14 +640,22 @@ int run_chunks(vf_solver* s, void (*iteration)(vf_solver*), int gslot,
   // ever fails to advance, report an error instead of polling forever.
   const long long max_chunks = (long long)(s->h_ks->max_it + K - 1) / K + 4;
   long long chunks = 0;
+  int burst = 1;
   for (;;) {
     if (++chunks > max_chunks) {
       s->err = "PCG state did not reach max_it/convergence within the expected number of chunks";
       return VF_ERR_CUDA;
     }
     if (s->o.use_graphs) {
-      VF_TRY(cudaGraphLaunch(s->chunk[gslot], s->st));
-      g_launches += s->chunk_kernels[gslot];
+      // nobody watches a Jacobi solve without callbacks: several chunks per
+      // look at the state (the wait, the copies and the relaunch cost ~30 us
+      // of every 8 short iterations), a few more each time; the launches past
+      // the end are no-ops
+      if (!progress && !use_mg(s) && chunks > 1) burst = std::min(2 * burst, 16);
+      for (int k = 0; k < burst; ++k) {
+        VF_TRY(cudaGraphLaunch(s->chunk[gslot], s->st));
+        g_launches += s->chunk_kernels[gslot];
+      }
     } else {
       for (int k = 0; k < K; ++k) iteration(s);
       VF_CHECK_LAUNCH();

@@ -362,7 +362,7 @@ class MGSolver:
             except BaseException as exc:  # noqa: BLE001  re-raised after the call
                 cb_error.append(exc)
 
-        cfun = _lib.PROGRESS_FN(_tramp)
+        cfun = _lib.PROGRESS_FN(_tramp) if progress_cb is not None else _lib.PROGRESS_FN()   # null: nobody watches
         L = _lib.load()
         rc = L.vf_solve_cb(self._handle(), _lib.ptr(f), _lib.ptr(x0a), float(tol),
                            int(max_cg or 0), 0, _lib.ptr(u), ctypes.byref(info), cfun, None)
