@@ -15,7 +15,9 @@
 //   * at most kMaxBlocks blocks of 256 threads, i.e. (nx+1)(ny+1)(nz+1) <=
 //     kMaxNodes grid nodes; larger grids are rejected with VF_ERR_ARG;
 //   * every call on a device shares the one array and it keeps the last call's
-//     contents; the completion counter is cleared at the start of each call.
+//     contents; successive calls take successive completion counters of a
+//     ring, and a call's last block clears its own and the one half a ring
+//     ahead, so a counter that an overlap spoilt does not stay spoilt.
 //     Calls whose kernels overlap on the GPU (different streams, no ordering)
 //     race on the array and give wrong results: order them on one stream;
 //   * the first call on each device looks up the array's device address
@@ -27,12 +29,15 @@
 //     while others write y, so an in-place call is rejected.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <string>
 
 #include "../../include/voxfea.h"
 #include "vf_common.cuh"
 #include "vf_hex8.h"
+#include "vf_modal.cuh"
 
 namespace vf {
 extern thread_local std::string g_last_error;
@@ -44,8 +49,9 @@ constexpr int kThreads = 256;
 constexpr int kMaxBlocks = 32768;
 constexpr long long kMaxNodes = (long long)kMaxBlocks * kThreads;   // 8,388,608 nodes
 constexpr int kMaxDevices = 64;
-// [0, kMaxBlocks) doubles: per-block partials; then one unsigned counter.
-constexpr size_t kScratchBytes = sizeof(double) * kMaxBlocks + 256;
+constexpr int kRing = 64;
+// [0, kMaxBlocks) doubles: per-block partials; then kRing unsigned counters.
+constexpr size_t kScratchBytes = sizeof(double) * kMaxBlocks + kRing * sizeof(unsigned);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -53,6 +59,7 @@ struct KeParam { double k[576]; };
 
 unsigned char* g_scratch_addr[kMaxDevices] = {};
 std::mutex g_scratch_mu;
+std::atomic<unsigned> g_call{0};
 
 // Device address of g_noalloc_scratch on the current device (set up once per device).
 int scratch_for_device(unsigned char** out) {
@@ -72,12 +79,199 @@ int scratch_for_device(unsigned char** out) {
   return VF_OK;
 }
 
+// Block sum in a fixed order; the last block sums the partials in order.
+__device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_out, double* __restrict__ partials,
+                                           unsigned int* __restrict__ counters, unsigned slot) {
+  __shared__ double s_w[kThreads / 32];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  __syncthreads();
+  if ((tid & 31) == 0) s_w[tid >> 5] = dot;
+  __syncthreads();
+  if (tid == 0) {
+    double b = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) b += s_w[w];
+    partials[blockIdx.x] = b;
+    __threadfence();
+    s_last = (atomicAdd(counters + slot, 1u) == gridDim.x - 1);
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double s = 0.0;
+#pragma unroll 4
+  for (int i = tid; i < (int)gridDim.x; i += kThreads) s += __ldcg(partials + i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((tid & 31) == 0) s_w[tid >> 5] = s;
+  __syncthreads();
+  if (tid == 0) {
+    double tot = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) tot += s_w[w];
+    *dot_out = tot;
+    counters[slot] = 0u;
+    counters[(slot + kRing / 2) % kRing] = 0u;
+  }
+}
+
+// The operator in modal form (vf_modal.cuh), marching along z: 32 x 8 threads
+// own a 31 x 7 tile of nodes and a chunk of planes; each thread transforms the
+// face of its element column once per plane, couples it with the plane below
+// and keeps the upper face's forces for the next step, so a node's value is
+// loaded once per tile and a voxel costs ~170 operations instead of the 576
+// products per node of the gather form below.  The caller's arrays are in
+// reference order with rows of any alignment, so planes are staged with plain
+// coalesced loads, one plane ahead in registers, three planes in shared
+// memory; the corner forces are exchanged through a double buffer (one barrier
+// a plane).  251x127x129 voxels: 387 us (gather) -> 161 us; 48x24x24: 29 -> 12 us
+// (there also without a clearing launch and the host's 24x24 tables).
+constexpr int kMX = 32, kMY = 8;
+constexpr int kRow = 3 * (kMX + 1) + 1, kPlane = (kMY + 1) * kRow;   // 33 x 9 halo nodes
+constexpr size_t kMarchSmem = sizeof(double) * (3 * kPlane + 2 * 3 * 3 * kMY * kMX);
+struct March { int ntx, nty, zchunk, units; };
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_apply_march(int nx, int ny, int nz, const double* __restrict__ E, const uint8_t* __restrict__ mask,
+                  const double* __restrict__ u, double* __restrict__ y, double* __restrict__ dot_out,
+                  double* __restrict__ partials, unsigned int* __restrict__ counters, unsigned slot,
+                  const vf::ModalConst mc, March mp) {
+  using O = vf::modal::Pack<double>;
+  extern __shared__ double smem[];
+  double (*s_u)[kPlane] = reinterpret_cast<double (*)[kPlane]>(smem);
+  double (*s_c)[3][3][kMY][kMX] = reinterpret_cast<double (*)[3][3][kMY][kMX]>(smem + 3 * kPlane);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + kMX * ty;
+  const int nx1 = nx + 1, ny1 = ny + 1;
+  constexpr int NL = (3 * (kMX + 1) * (kMY + 1) + kThreads - 1) / kThreads;   // halo values per thread
+  double dot = 0.0;
+#pragma unroll 1
+  for (int unit = blockIdx.x; unit < mp.units; unit += gridDim.x) {
+    const int X0 = unit % mp.ntx * (kMX - 1), Y0 = unit / mp.ntx % mp.nty * (kMY - 1);
+    const int zb = unit / (mp.ntx * mp.nty) * mp.zchunk, ze = min(zb + mp.zchunk, nz + 1);
+    const int Xc = X0 - 1 + tx, Yc = Y0 - 1 + ty;
+    const bool out_col = tx >= 1 && ty >= 1 && Xc <= nx && Yc <= ny;
+    const bool elem_col = Xc >= 0 && Xc < nx && Yc >= 0 && Yc < ny;
+    const double* Ecol = E + (elem_col ? ((long long)Xc * ny + Yc) * nz : 0);
+    const int node_col = out_col ? Xc + nx1 * Yc : 0;
+    int goff[NL], soff[NL];   // this thread's halo values: offset within a plane of u (-1: outside), in s_u
+#pragma unroll
+    for (int q = 0; q < NL; ++q) {
+      const int e = tid + q * kThreads, j = e / (3 * (kMX + 1)), i = e % (3 * (kMX + 1));
+      const int gx = X0 - 1 + i / 3, gy = Y0 - 1 + j;
+      soff[q] = j < kMY + 1 ? j * kRow + i : -1;
+      goff[q] = (j < kMY + 1 && gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) ? 3 * (gx + nx1 * gy) + i % 3 : -1;
+    }
+    double pre[NL];
+    auto fetch = [&](int z) {
+#pragma unroll
+      for (int q = 0; q < NL; ++q)
+        pre[q] = (goff[q] >= 0 && z >= 0 && z <= nz) ? __ldg(u + 3LL * nx1 * ny1 * z + goff[q]) : 0.0;
+    };
+    auto store = [&](int b) {
+#pragma unroll
+      for (int q = 0; q < NL; ++q)
+        if (soff[q] >= 0) s_u[b][soff[q]] = pre[q];
+    };
+    double hiPrev[3][4], Fp[3][4], own[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      own[c] = 0.0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) { hiPrev[c][m] = 0.0; Fp[c][m] = 0.0; }
+    }
+    // plane s of this unit is z = zb - 1 + s; layer s lies between planes s - 1 and s
+    const int nsteps = ze - zb + 2;
+    __syncthreads();   // the previous unit's readers are done
+    fetch(zb - 1);
+    store(0);
+    fetch(zb);
+    double En = 0.0;
+    uint8_t mk = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s < nsteps; ++s) {
+      const int z = zb - 1 + s;
+      if (s + 1 < nsteps) store((s + 1) % 3);
+      if (s + 2 < nsteps) fetch(z + 2);
+      const double Ee = En;   // of layer s
+      En = (elem_col && z >= 0 && z < nz && s + 1 < nsteps) ? __ldg(Ecol + z) : 0.0;
+      const uint8_t m8 = mk;
+      mk = (out_col && s >= 1 && z >= 0 && z <= nz) ? __ldg(mask + node_col + (long long)nx1 * ny1 * z) : (uint8_t)0;
+      const double* us = s_u[s % 3] + ty * kRow + 3 * tx;
+      double Fc[3][4], u0[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double u00 = us[c], u10 = us[3 + c], u01 = us[kRow + c], u11 = us[kRow + 3 + c];
+        const double e0 = u10 + u00, e1 = u10 - u00, e2 = u11 + u01, e3 = u11 - u01;
+        u0[c] = u00;
+        Fc[c][0] = e0 + e2;
+        Fc[c][1] = e1 + e3;
+        Fc[c][2] = e2 - e0;
+        Fc[c][3] = e3 - e1;
+      }
+      if (s >= 1) {
+        double A[3][8], B[3][8];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            A[c][m] = Fp[c][m] + Fc[c][m];
+            A[c][m + 4] = Fc[c][m] - Fp[c][m];
+          }
+        vf::modal::modal_physics<O, double, double>(A, B, Ee, Ee, mc);
+        double c00[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          double acc[4];
+          acc[0] = hiPrev[c][0] - B[c][4];
+          hiPrev[c][0] = B[c][4];
+#pragma unroll
+          for (int m = 1; m < 4; ++m) {
+            acc[m] = hiPrev[c][m] + (B[c][m] - B[c][m + 4]);
+            hiPrev[c][m] = B[c][m] + B[c][m + 4];
+          }
+          const double t0 = acc[0] - acc[2], t1 = acc[1] - acc[3], t2 = acc[0] + acc[2], t3 = acc[1] + acc[3];
+          c00[c] = t0 - t1;
+          s_c[s & 1][0][c][ty][tx] = t0 + t1;
+          s_c[s & 1][1][c][ty][tx] = t2 - t3;
+          s_c[s & 1][2][c][ty][tx] = t2 + t3;
+        }
+        __syncthreads();
+        if (s >= 2 && out_col) {
+          const long long p3 = 3 * (node_col + (long long)nx1 * ny1 * (z - 1));
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const double v = (c00[c] + s_c[s & 1][0][c][ty][tx - 1]) +
+                             (s_c[s & 1][1][c][ty - 1][tx] + s_c[s & 1][2][c][ty - 1][tx - 1]);
+            const double k = ((m8 >> c) & 1) ? v : 0.0;
+            y[p3 + c] = k;
+            dot += own[c] * k;
+          }
+        }
+      } else {
+        __syncthreads();
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        own[c] = u0[c];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) Fp[c][m] = Fc[c][m];
+      }
+    }
+  }
+  finish_dot(dot, dot_out, partials, counters, slot);
+}
+
+// The operator as a node-centric gather over KE, one thread per node: better
+// only on grids too thin to fill the marching form's tiles.
 __global__ void __launch_bounds__(kThreads) k_apply_noalloc(int nx, int ny, int nz, const double* __restrict__ E,
                                                             const uint8_t* __restrict__ mask,
                                                             const double* __restrict__ u, double* __restrict__ y,
                                                             double* __restrict__ dot_out,
                                                             double* __restrict__ partials,
-                                                            unsigned int* __restrict__ counter, const KeParam K) {
+                                                            unsigned int* __restrict__ counters, unsigned slot,
+                                                            const KeParam K) {
   const int nx1 = nx + 1, ny1 = ny + 1;
   const long long nn = (long long)nx1 * ny1 * (nz + 1);
   const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -119,36 +313,30 @@ __global__ void __launch_bounds__(kThreads) k_apply_noalloc(int nx, int ny, int 
     y[3 * r] = a0; y[3 * r + 1] = a1; y[3 * r + 2] = a2;
     dot = u[3 * r] * a0 + u[3 * r + 1] * a1 + u[3 * r + 2] * a2;
   }
-  // block sum in a fixed order, then the last block sums the partials in order
-  __shared__ double s_w[kThreads / 32];
-  __shared__ bool s_last;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = dot;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) b += s_w[w];
-    partials[blockIdx.x] = b;
-    __threadfence();
-    s_last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+  finish_dot(dot, dot_out, partials, counters, slot);
+}
+
+// Planes per chunk of the marching form: the split whose waves of two blocks
+// per SM take the fewest steps (a chunk of n planes marches n + 2).
+March march_plan(int nx, int ny, int nz) {
+  March m;
+  m.ntx = (nx + kMX - 1) / (kMX - 1);
+  m.nty = (ny + kMY - 1) / (kMY - 1);
+  const long long tiles = (long long)m.ntx * m.nty, planes = nz + 1, room = 2 * 148;
+  long long best = -1;
+  m.zchunk = (int)planes;
+  for (long long n = 1; n <= planes && n <= 4096; ++n) {
+    const long long zc = (planes + n - 1) / n;
+    const long long waves = (tiles * ((planes + zc - 1) / zc) + room - 1) / room;
+    const long long cost = waves * (zc + 2);
+    if (best < 0 || cost < best) {
+      best = cost;
+      m.zchunk = (int)zc;
+    }
+    if (tiles * n > 8 * room) break;   // (more chunks only add their two extra steps)
   }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  double s = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) s += ((volatile double*)partials)[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) tot += s_w[w];
-    *dot_out = tot;
-    *counter = 0u;
-  }
+  m.units = (int)(tiles * ((planes + m.zchunk - 1) / m.zchunk));
+  return m;
 }
 
 }  // namespace
@@ -185,21 +373,29 @@ extern "C" int vf_apply_noalloc(int32_t nx, int32_t ny, int32_t nz, double nu, c
   int rc = scratch_for_device(&base);
   if (rc) return rc;
   double* partials = (double*)base;
-  unsigned int* counter = (unsigned int*)(base + sizeof(double) * kMaxBlocks);
+  unsigned int* counters = (unsigned int*)(base + sizeof(double) * kMaxBlocks);
+  const unsigned slot = g_call.fetch_add(1) % kRing;
   cudaStream_t st = (cudaStream_t)stream;
-  KeParam K;
-  double tab[1728], b0[144];
-  vf::hex8_tables(nu, tab, b0);
-  for (int i = 0; i < 576; ++i) K.k[i] = tab[i];
-  cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), st);
-  if (e != cudaSuccess) {
-    vf::g_last_error = std::string("vf_apply_noalloc: ") + cudaGetErrorString(e);
-    return VF_ERR_CUDA;
+  // The marching form computes whole 31 x 7 tiles: where less than a fifth of
+  // their columns are nodes of the grid the gather form is no slower (gather /
+  // marching form, us: 3x40x3000 51 / 92, 2x100x400 24 / 38, 1x1x100000 43 /
+  // 406; above the line 10x3x200 24 / 10, 30x6x1000 29 / 14, 61x43x37 23 / 12).
+  const March m = march_plan(nx, ny, nz);
+  if (5LL * (nx + 1) * (ny + 1) >= (long long)m.ntx * (kMX - 1) * m.nty * (kMY - 1)) {
+    static std::atomic<int> per_dev[vf::kMaxDevices];
+    vf::kernel_prepare(per_dev, k_apply_march, kMarchSmem, kThreads);
+    vf::launch_k(k_apply_march, dim3((unsigned)std::min(m.units, kMaxBlocks)), dim3(kMX, kMY), kMarchSmem, st, nx, ny,
+                 nz, E, free_mask, u, y, u_dot_y, partials, counters, slot, vf::modal_constants(nu, false), m);
+  } else {
+    KeParam K;
+    double tab[1728], b0[144];
+    vf::hex8_tables(nu, tab, b0);
+    for (int i = 0; i < 576; ++i) K.k[i] = tab[i];
+    const int blocks = (int)((nn + kThreads - 1) / kThreads);
+    vf::launch_k(k_apply_noalloc, blocks, kThreads, 0, st, nx, ny, nz, E, free_mask, u, y, u_dot_y, partials, counters,
+                 slot, K);
   }
-  const int blocks = (int)((nn + kThreads - 1) / kThreads);
-  vf::launch_k(k_apply_noalloc, blocks, kThreads, 0, st, nx, ny, nz, E, free_mask, u, y, u_dot_y, partials,
-               counter, K);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     vf::g_last_error = std::string("vf_apply_noalloc launch: ") + cudaGetErrorString(e);
     return VF_ERR_CUDA;
