@@ -255,14 +255,25 @@ template <typename T> void launch_restrict_first(const Grid& f, const T* rf, con
 template <typename T> void launch_jacobi_from_zero(const Grid& g, const T* b, const T* minv3, const uint8_t* mask, double omega, const double* omega_dev, T* u, const KrylovState* ks, cudaStream_t st);
 
 // vf_dense.cu -- coarsest-level dense FP64 direct solve
+// parts == 1: one explicit inverse of n DOFs; parts > 1: the grid dissected
+// along `axis` into interiors of at most ni DOFs and separators of rm = reach
+// planes of m DOFs each (ns in all)
+struct DensePlan { int n, axis, reach, parts, planes, nx1, ny1, m, rm, ni, ns; };
+DensePlan dense_plan(const Grid& c, int reach);
+size_t dense_store_count(const DensePlan& P);     // doubles of the inverse / the blocks
+size_t dense_store32_count(const DensePlan& P);   // floats of their FP32 copy
+size_t dense_work_count(const DensePlan& P);      // doubles of the set-up's scratch
+size_t dense_perm_count(const DensePlan& P);
+size_t dense_vec_count(const DensePlan& P);       // doubles of a solve's intermediate vectors (one per stream)
 int dense_assemble(const Grid& c, const double* stencil, const uint8_t* cmask, double* A, int n, cudaStream_t st);
-int dense_cholesky_inverse(double* A, double* work, int n, int bw, int* d_info, cudaStream_t st);
-size_t dense_work_count(int n);
 int dense_ld32(int n);   // row stride (floats) of the padded FP32 inverse
-void launch_dense_perm(const Grid& c, int* perm, int n, cudaStream_t st);
-void launch_dense_convert_pad(const double* A, float* B, int n, cudaStream_t st);
-template <typename T> void launch_dense_solve(const double* Ainv, int n, const int* perm, const T* b, T* x, const KrylovState* ks, cudaStream_t st);
-void launch_dense_solve_f32(const float* Ainv32, int n, const int* perm, const float* b, float* x, const KrylovState* ks, cudaStream_t st);
+void dense_prepare_smem();
+void launch_dense_perm(const Grid& c, const DensePlan& P, int* perm, cudaStream_t st);
+void dense_build(const Grid& c, const DensePlan& P, const double* stencil, int reach, const uint8_t* cmask,
+                 double* store, double* work, int* d_info, cudaStream_t st);
+void dense_build32(const DensePlan& P, const double* store, float* store32, cudaStream_t st);
+// x = A^-1 b: FP64 blocks for double, their FP32 copy for float (FP64 sums in both)
+template <typename T> void launch_dense_solve(const DensePlan& P, const double* store, const float* store32, const int* perm, double* vec, const T* b, T* x, const KrylovState* ks, cudaStream_t st);
 
 // vf_krylov.cu -- fused PCG vector kernels with deterministic FP64 reductions
 constexpr int kVecBlocks = 148 * 8;     // largest grid of the vector kernels (by size alone => deterministic)

@@ -2,8 +2,9 @@
 // identity rows on non-free DOFs) is factored A = L L^T by a blocked
 // right-looking Cholesky, inverted as A^{-1} = Y^T Y with Y = L^{-1}, and each
 // V-cycle applies the explicit inverse with one GEMV.  All kernels are plain
-// CUDA-core FP64 (the coarsest level holds a few thousand DOFs at most);
-// the factorization runs once per set_material, outside the iteration.
+// CUDA-core FP64; the factorization runs once per set_material, outside the
+// iteration.  A coarsest level of many DOFs (a grid that halves only once or
+// twice) is dissected instead: see DensePlan below.
 // Replaces the reference's 30-sweep Jacobi "coarse solve" (core/multigrid.py:428-429)
 // when VF_COARSEST_CHOLESKY is selected.
 #include <algorithm>
@@ -46,12 +47,16 @@ __global__ void k_dense_assemble(Grid c, const double* __restrict__ st, const ui
 // 1024 threads, one per (row t, column c) of the block; the panel solve and
 // the block-row solve of the inverse phase then multiply by linv instead of
 // substituting row by row.
-__global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int k, int nb, int* info, double* linv) {
+// (blockIdx.x: matrix of a batch, sA / sL values apart.)
+__global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int k, int nb, int* info, double* linv,
+                                                           size_t sA, size_t sL) {
+  A += sA * blockIdx.x;
+  linv += sL * blockIdx.x;
   // L: the block being reduced (column j is read, columns > j updated in step
   // j); F: the factor, each entry written once -- so one barrier per column:
   // every thread takes the pivot's square root itself, and nothing reads
   // what step j writes until step j + 1
-  __shared__ double L[NB][NB + 1], F[NB][NB + 1], X[NB][NB + 1];
+  __shared__ double L[NB][NB + 1], F[NB][NB + 1], X[NB][NB + 1], rec[NB];
   const int c = threadIdx.x % NB, t = threadIdx.x / NB;
   L[t][c] = (t < nb && c <= t) ? A[(long long)(k + t) * n + k + c] : 0.0;
   F[t][c] = 0.0;
@@ -63,6 +68,7 @@ __global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int
     const double rinv = 1.0 / piv;
     if (t == j && c == j) {
       F[j][j] = piv;
+      rec[j] = rinv;
       if (bad && *info == 0) *info = k + j + 1;
     }
     if (t > j && t < nb) {
@@ -78,7 +84,7 @@ __global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int
   double xv = (t == c) ? 1.0 : 0.0;
   for (int r = 0; r < nb; ++r) {
     if (t == r) {
-      xv = xv / F[r][r];
+      xv *= rec[r];   // (a division here was a third of the kernel's chain)
       X[r][c] = xv;
     }
     __syncthreads();
@@ -90,7 +96,10 @@ __global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int
 
 // Rows i >= k+nb: A[i, k:k+nb] <- A[i, k:k+nb] L_kk^-T, i.e.
 // X[i][j] = sum_{l <= j} A[i][k+l] linv[j][l].  64 rows per CTA.
-__global__ void __launch_bounds__(256) k_trsm_panel(double* A, int n, int k, int nb, const double* linv) {
+__global__ void __launch_bounds__(256) k_trsm_panel(double* A, int n, int k, int nb, const double* linv, size_t sA,
+                                                    size_t sL) {
+  A += sA * blockIdx.y;
+  linv += sL * blockIdx.y;
   __shared__ double P[64][NB + 1], Li[NB][NB + 1];
   const int tid = threadIdx.x;
   const int i0 = k + nb + blockIdx.x * 64;
@@ -117,7 +126,8 @@ constexpr int TB = 64;
 
 // Trailing update (lower triangle): A[i][j] -= sum_l A[i][k+l] A[j][k+l].
 // Grid: one CTA per 64 x 64 tile pair bi >= bj of the trailing matrix.
-__global__ void __launch_bounds__(256) k_syrk_update(double* A, int n, int k, int nb) {
+__global__ void __launch_bounds__(256) k_syrk_update(double* A, int n, int k, int nb, size_t sA) {
+  A += sA * blockIdx.z;
   const int t0 = k + nb;
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (bj > bi) return;
@@ -167,7 +177,7 @@ constexpr int kMaxJobs = 128;
 struct GemmBatch {
   GemmJob job[kMaxJobs];
   int count;
-  double alpha;
+  double alpha, beta;     // C = alpha A B + beta C (C is not read when beta is 0)
   int a_lower, b_lower;   // A / B lower triangular (square): skip the zero part of the K range
   // a_bw > 0: A is a block L21 of a band matrix, its row 0 K rows below its
   // column 0, so A[i][k] = 0 for k < i + K - a_bw
@@ -218,12 +228,17 @@ __global__ void __launch_bounds__(256) k_gemm_batched(const __grid_constant__ Ge
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const int i = i0 + ty + 16 * q, j = j0 + tx + 16 * w;
-      if (i < jb.M && j < jb.N) jb.C[(long long)i * jb.ldc + j] = bt.alpha * acc[q][w];
+      if (i < jb.M && j < jb.N) {
+        double* C = jb.C + (long long)i * jb.ldc + j;
+        *C = bt.beta != 0.0 ? bt.alpha * acc[q][w] + bt.beta * *C : bt.alpha * acc[q][w];
+      }
     }
 }
 
 // Y = 0 with the inverted diagonal blocks L_kk^-1 on the diagonal.
-__global__ void k_y_init(double* Y, int n, const double* linv_all) {
+__global__ void k_y_init(double* Y, int n, const double* linv_all, size_t sY, size_t sL) {
+  Y += sY * blockIdx.y;
+  linv_all += sL * blockIdx.y;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)n * n;
        e += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(e / n), j = (int)(e % n);
@@ -239,7 +254,9 @@ __global__ void k_y_init(double* Y, int n, const double* linv_all) {
 // Ainv = Y^T Y (Y lower triangular): Ainv[i][j] = sum_{l >= max(i,j)} Y[l][i] Y[l][j].
 // A^-1 = Y^T Y is symmetric: one CTA per 64x64 tile of the lower triangle
 // (blockIdx.x enumerates the pairs bi >= bj), written to both triangles.
-__global__ void __launch_bounds__(256) k_yty(const double* Y, double* Ainv, int n) {
+__global__ void __launch_bounds__(256) k_yty(const double* Y, double* Ainv, int n, size_t sY, size_t sA) {
+  Y += sY * blockIdx.y;
+  Ainv += sA * blockIdx.y;
   int bi = (int)((sqrt(8.0 * blockIdx.x + 1.0) - 1.0) * 0.5);
   while ((bi + 1) * (bi + 2) / 2 <= (int)blockIdx.x) ++bi;
   while (bi * (bi + 1) / 2 > (int)blockIdx.x) --bi;
@@ -388,40 +405,42 @@ int dense_assemble(const Grid& c, const double* stencil, const uint8_t* cmask, d
   return 0;
 }
 
-// Doubles of the work buffer: Y = L^-1 (n x n) and the inverted diagonal
-// blocks (NB x NB each).
-size_t dense_work_count(int n) {
-  return (size_t)n * n + (size_t)((n + NB - 1) / NB) * NB * NB + (size_t)n * n / 2 + (size_t)NB * n;
+// Doubles of the work buffer for a batch of n x n matrices: each Y = L^-1, its
+// inverted diagonal blocks (NB x NB each) and the products' temporaries.
+static size_t cholesky_work(int n, int batch) {
+  return (size_t)batch * ((size_t)n * n + (size_t)((n + NB - 1) / NB) * NB * NB + (size_t)n * n / 2 + (size_t)NB * n);
 }
 
-// A (n x n, lower part) is overwritten by L; work (dense_work_count(n))
-// receives Y = L^-1 and the inverted diagonal blocks; A <- Y^T Y = A^-1.
-// d_info > 0 flags a non-positive pivot.  bw: A[i][j] == 0 for |i - j| > bw
-// (a stencil operator in lexicographic node order is banded).  A Cholesky
-// factor keeps the band, so the panel solve and the trailing update of block
-// column k only touch the rows below it that lie within the band: the rows
-// they skip would receive exact zeros (the factor is the same bit for bit).
-int dense_cholesky_inverse(double* A, double* work, int n, int bw, int* d_info, cudaStream_t st) {
-  cudaMemsetAsync(d_info, 0, sizeof(int), st);
-  double* linv_all = work + (size_t)n * n;
+// A (batch matrices n x n, sA values apart, lower parts) is overwritten by L;
+// work (cholesky_work) receives Y = L^-1 and the inverted diagonal blocks;
+// A <- Y^T Y = A^-1.  d_info > 0 flags a non-positive pivot.  bw: A[i][j] == 0
+// for |i - j| > bw (a stencil operator in lexicographic node order is banded).
+// A Cholesky factor keeps the band, so the panel solve and the trailing update
+// of block column k only touch the rows below it that lie within the band: the
+// rows they skip would receive exact zeros (the factor is the same bit for
+// bit).
+static void cholesky_inverse(double* A, double* work, int n, int bw, int* d_info, cudaStream_t st, int batch,
+                             size_t sA) {
+  const int nbk = (n + NB - 1) / NB;
+  const size_t sY = (size_t)n * n, sL = (size_t)nbk * NB * NB;
+  double* linv_all = work + sY * batch;
   if (bw < 0 || bw > n) bw = n;
   for (int k = 0; k < n; k += NB) {
     const int nb = (n - k < NB) ? (n - k) : NB;
     double* linv = linv_all + (size_t)(k / NB) * NB * NB;
-    launch_k(k_potrf_diag, 1, NB * NB, 0, st, A, n, k, nb, d_info, linv);
+    launch_k(k_potrf_diag, batch, NB * NB, 0, st, A, n, k, nb, d_info, linv, sA, sL);
     // rows > k + nb - 1 + bw of columns k .. k + nb - 1 are zero
     const int rest = std::min(n, k + nb + bw) - (k + nb);
     if (rest > 0) {
-      launch_k(k_trsm_panel, (rest + 63) / 64, 256, 0, st, A, n, k, nb, (const double*)linv);
+      launch_k(k_trsm_panel, dim3((rest + 63) / 64, batch), 256, 0, st, A, n, k, nb, (const double*)linv, sA, sL);
       const int tiles = (rest + TB - 1) / TB;
-      launch_k(k_syrk_update, dim3(tiles, tiles), 256, 0, st, A, n, k, nb);
+      launch_k(k_syrk_update, dim3(tiles, tiles, batch), 256, 0, st, A, n, k, nb, sA);
     }
   }
   // Y = L^{-1} into work: diagonal blocks from the factorization, then the
   // off-diagonal blocks level by level (T in the scratch after linv_all)
-  launch_k(k_y_init, 148 * 4, 256, 0, st, work, n, (const double*)linv_all);
-  double* tbuf = linv_all + (size_t)((n + NB - 1) / NB) * NB * NB;
-  const int nbk = (n + NB - 1) / NB;
+  launch_k(k_y_init, dim3(std::max(1, 148 * 4 / batch), batch), 256, 0, st, work, n, (const double*)linv_all, sY, sL);
+  double* tbuf = linv_all + sL * batch;
   for (int g = 1; g < nbk; g *= 2) {
     GemmBatch b1{}, b2{};
     b1.alpha = 1.0; b1.b_lower = 1;     // T = L21 Y11
@@ -436,67 +455,424 @@ int dense_cholesky_inverse(double* A, double* work, int n, int bw, int* d_info, 
       b1.count = b2.count = 0;
       max_tiles = 0;
     };
-    for (int p0 = 0; p0 < nbk; p0 += 2 * g) {
-      const int r0 = p0 * NB, r1 = std::min((p0 + g) * NB, n), r2 = std::min((p0 + 2 * g) * NB, n);
-      if (r1 >= r2) continue;
-      const int m = r2 - r1, h = r1 - r0;
-      double* T = tbuf + toff;   // distinct per pair within a level (sum of m h <= n^2 / 4)
-      toff += (size_t)m * h;
-      // L21 = L[r1:r2, r0:r1] is zero below its row bw (the band), and so
-      // is T: only its first mb rows are formed, and only they enter Y21
-      const int mb = std::min(m, bw);
-      b1.job[b1.count++] = GemmJob{A + (size_t)r1 * n + r0, work + (size_t)r0 * n + r0, T, n, n, h, mb, h, h};
-      b2.job[b2.count++] = GemmJob{work + (size_t)r1 * n + r1, T, work + (size_t)r1 * n + r0, n, h, n, m, h, mb};
-      max_tiles = std::max(max_tiles, ((m + TB - 1) / TB) * ((h + TB - 1) / TB));
-      if (b1.count == kMaxJobs) flush();
+    for (int q = 0; q < batch; ++q) {
+      double *Aq = A + sA * q, *Yq = work + sY * q;
+      for (int p0 = 0; p0 < nbk; p0 += 2 * g) {
+        const int r0 = p0 * NB, r1 = std::min((p0 + g) * NB, n), r2 = std::min((p0 + 2 * g) * NB, n);
+        if (r1 >= r2) continue;
+        const int m = r2 - r1, h = r1 - r0;
+        double* T = tbuf + toff;   // distinct per pair within a level (sum of m h <= n^2 / 4 per matrix)
+        toff += (size_t)m * h;
+        // L21 = L[r1:r2, r0:r1] is zero below its row bw (the band), and so
+        // is T: only its first mb rows are formed, and only they enter Y21
+        const int mb = std::min(m, bw);
+        b1.job[b1.count++] = GemmJob{Aq + (size_t)r1 * n + r0, Yq + (size_t)r0 * n + r0, T, n, n, h, mb, h, h};
+        b2.job[b2.count++] = GemmJob{Yq + (size_t)r1 * n + r1, T, Yq + (size_t)r1 * n + r0, n, h, n, m, h, mb};
+        max_tiles = std::max(max_tiles, ((m + TB - 1) / TB) * ((h + TB - 1) / TB));
+        if (b1.count == kMaxJobs) flush();
+      }
     }
     flush();
   }
   // A <- Y^T Y (lower-triangle tiles, mirrored)
   const int tiles = (n + TB - 1) / TB;
-  launch_k(k_yty, dim3(tiles * (tiles + 1) / 2), 256, 0, st, work, A, n);
-  return 0;
+  launch_k(k_yty, dim3(tiles * (tiles + 1) / 2, batch), 256, 0, st, (const double*)work, A, n, sY, sA);
+}
+
+// ---------------------------------------------------------------------------
+// The dissected coarsest solve.
+//
+// The explicit inverse of n DOFs costs n / 32 dependent block steps and n^3
+// products to build and reads n^2 values at each use: on a coarsest level of
+// 10,920 DOFs (25x13x9 voxels) 52 ms of a job's set-up and 368 us (FP64) a
+// V-cycle.  Planes of nodes along the grid's longest axis split it instead into
+// `parts` interiors and, between them, separators as thick as the stencil's
+// reach, which nothing couples across.  With Z_i = A_ii^-1, C_i the coupling of
+// interior i to its two separators, W_i = Z_i C_i and the Schur complement
+// S = A_ss - sum C_i^T W_i,
+//     x_s = S^-1 (b_s - sum W_i^T b_i),   x_i = Z_i b_i - W_i x_s,
+// three products with explicit blocks: [Z_i; W_i^T] b_i, S^-1 and W_i x_s.  The
+// interiors are factored as one batch, so the chain of block steps is
+// (ni + ns) / 32.  Same solution, same FP64 (the FP32 V-cycle reads FP32 copies
+// of the blocks and accumulates in FP64, as it does with the explicit inverse).
+//   storage of part i: (ni + 2 Rm) x ni values, Z_i above W_i^T (left separator's
+//   rows, then the right one's), ni padded with identity rows to the longest
+//   part and a multiple of 4; then S^-1, ns x ns.
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr int kMaxParts = 12;
+
+__host__ __device__ __forceinline__ int part_planes(const DensePlan& P, int i) {
+  const int T = P.planes - (P.parts - 1) * P.reach;
+  return (int)((long long)(i + 1) * T / P.parts) - (int)((long long)i * T / P.parts);
+}
+__host__ __device__ __forceinline__ int part_first(const DensePlan& P, int i) {
+  const int T = P.planes - (P.parts - 1) * P.reach;
+  return (int)((long long)i * T / P.parts) + i * P.reach;
+}
+struct DisLoc { int part, sep, row; };   // part or sep -1; row: DOF of the node's component 0 in it
+__device__ __forceinline__ DisLoc dis_locate(const DensePlan& P, int x, int y, int z) {
+  const int k = P.axis == 0 ? x : (P.axis == 1 ? y : z);
+  const int e = P.axis == 0 ? y + P.ny1 * z : (P.axis == 1 ? x + P.nx1 * z : x + P.nx1 * y);
+  DisLoc l{-1, -1, 0};
+  for (int i = 0; i < P.parts; ++i) {
+    const int f = part_first(P, i), c = part_planes(P, i);
+    if (k < f + c) {
+      l.part = i;
+      l.row = (k - f) * P.m + 3 * e;
+      return l;
+    }
+    if (k < f + c + P.reach) {
+      l.sep = i;
+      l.row = i * P.rm + (k - f - c) * P.m + 3 * e;
+      return l;
+    }
+  }
+  return l;
+}
+
+// Offsets in the FP64 store and the set-up's work buffer.
+__host__ __device__ __forceinline__ size_t dis_part(const DensePlan& P) { return (size_t)(P.ni + 2 * P.rm) * P.ni; }
+
+// A_ii, C (interior x separator) and C^T, A_ss from the level's full stencil
+// (27 or 125 blocks), identity on DOFs that are not free.
+__global__ void k_dis_assemble(Grid c, DensePlan P, const double* __restrict__ st, const uint8_t* __restrict__ cm,
+                               double* __restrict__ store, double* __restrict__ coup) {
+  const int R = P.reach, W = 2 * R + 1, NBK = W * W * W, SC = NBK / 2;
+  const long long nint = (long long)P.nx1 * P.ny1 * (c.lz + 1), ns = c.n;
+  const size_t blk = (size_t)P.rm * P.rm;
+  double* S = store + P.parts * dis_part(P);
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nint * NBK;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int r = (int)(t / NBK), s = (int)(t % NBK);
+    const int x = r % P.nx1, y = r / P.nx1 % P.ny1, z = r / (P.nx1 * P.ny1);
+    const int X = x + s % W - R, Y = y + (s / W) % W - R, Z = z + s / (W * W) - R;
+    if (X < 0 || X > c.lx || Y < 0 || Y > c.ly || Z < 0 || Z > c.lz) continue;
+    const DisLoc a = dis_locate(P, x, y, z), b = dis_locate(P, X, Y, Z);
+    const int p = c.idx(x, y, z);
+    const uint8_t m = cm[p];
+    for (int i = 0; i < 3; ++i)
+      for (int j = 0; j < 3; ++j) {
+        double v = st[((long long)s * 9 + 3 * i + j) * ns + p];
+        if (s == SC && i == j && !((m >> i) & 1)) v = 1.0;
+        const int ra = a.row + i, rb = b.row + j;
+        if (a.part >= 0 && b.part >= 0) {
+          store[a.part * dis_part(P) + (size_t)ra * P.ni + rb] = v;
+        } else if (a.sep >= 0 && b.sep >= 0) {
+          S[(size_t)ra * P.ns + rb] = v;
+        } else {
+          // coup: per part C_left, C_left^T, C_right, C_right^T (Rm x Rm each)
+          const bool in_a = a.part >= 0;
+          const int part = in_a ? a.part : b.part, sep = in_a ? b.sep : a.sep;
+          const int right = sep == part ? 1 : 0;   // separator i lies right of part i
+          const int shift = right ? part_planes(P, part) * P.m - P.rm : 0;
+          const int ii = (in_a ? ra : rb) - shift, ss = (in_a ? rb : ra) - sep * P.rm;
+          double* C = coup + ((size_t)part * 4 + 2 * right) * blk;
+          if (in_a) C[(size_t)ii * P.rm + ss] = v;
+          else C[blk + (size_t)ss * P.rm + ii] = v;
+        }
+      }
+  }
+}
+__global__ void k_dis_pad(DensePlan P, double* __restrict__ store) {
+  const int i = blockIdx.y;
+  for (int r = part_planes(P, i) * P.m + blockIdx.x * blockDim.x + threadIdx.x; r < P.ni; r += gridDim.x * blockDim.x)
+    store[i * dis_part(P) + (size_t)r * P.ni + r] = 1.0;
+}
+// perm[i * ni + r]: padded-vector index of row r of part i (-1: padding); then the separators' rows
+__global__ void k_dis_perm(Grid c, DensePlan P, int* __restrict__ perm) {
+  const int nint = P.nx1 * P.ny1 * (c.lz + 1);
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nint; r += gridDim.x * blockDim.x) {
+    const int x = r % P.nx1, y = r / P.nx1 % P.ny1, z = r / (P.nx1 * P.ny1);
+    const DisLoc a = dis_locate(P, x, y, z);
+    const int base = a.part >= 0 ? a.part * P.ni : P.parts * P.ni;
+    for (int k = 0; k < 3; ++k) perm[base + a.row + k] = 3 * c.idx(x, y, z) + k;
+  }
+}
+
+// 16 bytes of a row against the staged vector, FP64 sums
+__device__ __forceinline__ double dot16(const double* row, const double* b) {
+  const double2 v = __ldg(reinterpret_cast<const double2*>(row));
+  return v.x * b[0] + v.y * b[1];
+}
+__device__ __forceinline__ double dot16(const float* row, const double* b) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(row));
+  return ((double)v.x * b[0] + (double)v.y * b[1]) + ((double)v.z * b[2] + (double)v.w * b[3]);
+}
+// A warp's product of a 16-byte aligned row of `n` values (a multiple of VW)
+// with b in shared memory; eight loads in flight per lane.
+template <typename S>
+__device__ __forceinline__ double warp_row(const S* row, int n, const double* b, int lane) {
+  constexpr int VW = 16 / (int)sizeof(S);
+  double part[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  int j = lane * VW;
+  for (; j + 7 * 32 * VW < n; j += 8 * 32 * VW) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) part[k] += dot16(row + j + 32 * VW * k, b + j + 32 * VW * k);
+  }
+  for (; j < n; j += 32 * VW) part[7] += dot16(row + j, b + j);
+  double s = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+constexpr int kDisRows = 32;   // rows per block: the staged vector serves four rows a warp
+
+// y_i = [Z_i; W_i^T] b_i
+template <typename T, typename S>
+__global__ void __launch_bounds__(256) k_dis_parts(DensePlan P, const S* __restrict__ store,
+                                                   const int* __restrict__ perm, const T* __restrict__ b,
+                                                   double* __restrict__ y, const KrylovState* ks) {
+  if (ks && ks->done) return;
+  extern __shared__ double sb[];
+  const int i = blockIdx.y, rows = P.ni + 2 * P.rm;
+  for (int k = threadIdx.x; k < P.ni; k += blockDim.x) {
+    const int q = __ldg(perm + i * P.ni + k);
+    sb[k] = q >= 0 ? (double)b[q] : 0.0;
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const S* M = store + i * dis_part(P);
+  for (int r = blockIdx.x * kDisRows + warp; r < min(rows, (int)(blockIdx.x + 1) * kDisRows); r += 8) {
+    const double v = warp_row<S>(M + (size_t)r * P.ni, P.ni, sb, lane);
+    if (lane == 0) y[(size_t)i * rows + r] = v;
+  }
+}
+// x_s = S^-1 (b_s - the parts' W^T b); S in rows of ld values
+template <typename T, typename S>
+__global__ void __launch_bounds__(256) k_dis_schur(DensePlan P, const S* __restrict__ Sinv, int ld,
+                                                   const int* __restrict__ perm, const T* __restrict__ b,
+                                                   const double* __restrict__ y, double* __restrict__ xs,
+                                                   T* __restrict__ x, const KrylovState* ks) {
+  if (ks && ks->done) return;
+  extern __shared__ double sb[];
+  const int rows = P.ni + 2 * P.rm;
+  for (int k = threadIdx.x; k < ld; k += blockDim.x) {
+    double v = 0.0;
+    if (k < P.ns) {
+      const int sep = k / P.rm, l = k - sep * P.rm;
+      v = (double)b[__ldg(perm + P.parts * P.ni + k)] - y[(size_t)sep * rows + P.ni + P.rm + l] -
+          y[(size_t)(sep + 1) * rows + P.ni + l];
+    }
+    sb[k] = v;
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = blockIdx.x * 8 + warp; r < P.ns; r += gridDim.x * 8) {
+    const double v = warp_row<S>(Sinv + (size_t)r * ld, ld, sb, lane);
+    if (lane == 0) {
+      xs[r] = v;
+      x[__ldg(perm + P.parts * P.ni + r)] = (T)v;
+    }
+  }
+}
+// x_i = (Z_i b_i) - W_i x_s: lanes take 32 rows, warps share the separators' DOFs
+template <typename T, typename S>
+__global__ void __launch_bounds__(256) k_dis_back(DensePlan P, const S* __restrict__ store,
+                                                  const int* __restrict__ perm, const double* __restrict__ y,
+                                                  const double* __restrict__ xs, T* __restrict__ x,
+                                                  const KrylovState* ks) {
+  if (ks && ks->done) return;
+  __shared__ double part[8][33];
+  const int i = blockIdx.y, rows = P.ni + 2 * P.rm;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * 32 + lane;
+  const S* W = store + i * dis_part(P) + (size_t)P.ni * P.ni;
+  const int c0 = i > 0 ? 0 : P.rm, c1 = i + 1 < P.parts ? 2 * P.rm : P.rm;
+  const double* xl = xs + (long long)(i - 1) * P.rm;   // column c belongs to row c of the pair (separators i - 1, i)
+  double s = 0.0;
+  if (r < P.ni) {
+#pragma unroll 8
+    for (int c = c0 + warp; c < c1; c += 8) s += (double)__ldg(W + (size_t)c * P.ni + r) * xl[c];
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && r < P.ni) {
+    const int q = __ldg(perm + i * P.ni + r);
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += part[w][lane];
+    if (q >= 0) x[q] = (T)(y[(size_t)i * rows + r] - t);
+  }
+}
+
+}  // namespace
+
+// The cheapest split by a model of the set-up and 80 uses, in microseconds:
+// 60 per block step of 32 columns, 2.5e-8 per n^3 (both measured on 10,920
+// DOFs: 342 steps, 32 ms of products), 8 bytes per value read at 4.5 TB/s, and
+// for a split 150 of set-up launches and 8 per use for the two more kernels.
+// It keeps the explicit inverse up to about 700 DOFs, and splits 10,920 of them
+// into 7 parts of 1,260 (a 100x52x36 job, FP64: 99 -> 34 ms).
+DensePlan dense_plan(const Grid& c, int reach) {
+  DensePlan best{};
+  const int dims[3] = {c.lx + 1, c.ly + 1, c.lz + 1};
+  best.n = 3 * dims[0] * dims[1] * dims[2];
+  best.parts = 1;
+  best.ni = best.n;
+  const double n = best.n;
+  double least = n / 32 * 60 + n * n * n * 2.5e-8 + 80 * (n * n * 8 / 4.5e6);
+  int axis = 0;
+  for (int a = 1; a < 3; ++a)
+    if (dims[a] > dims[axis]) axis = a;
+  for (int parts = 2; parts <= kMaxParts; ++parts) {
+    DensePlan P{};
+    P.n = best.n;
+    P.axis = axis;
+    P.reach = reach < 1 ? 1 : reach;
+    P.parts = parts;
+    P.planes = dims[axis];
+    P.nx1 = dims[0];
+    P.ny1 = dims[1];
+    P.m = P.n / dims[axis];
+    P.rm = P.reach * P.m;
+    const int inner = P.planes - (parts - 1) * P.reach;
+    if (inner < parts * P.reach) break;   // a part at least as thick as the reach keeps its separators apart
+    P.ni = ((inner + parts - 1) / parts * P.m + 3) / 4 * 4;
+    P.ns = (parts - 1) * P.rm;
+    if (P.ns % 2) continue;   // rows of S^-1 start on 16 bytes
+    const double ni = P.ni, ns = P.ns, rm = P.rm;
+    const double cost = 150 + (ni + ns) / 32 * 60 + (parts * ni * ni * ni + ns * ns * ns) * 2.5e-8 +
+                        80 * (8 + (parts * (ni * ni + 4 * rm * ni) + ns * ns) * 8 / 4.5e6);
+    if (cost < least) {
+      least = cost;
+      best = P;
+    }
+  }
+  return best;
+}
+
+size_t dense_store_count(const DensePlan& P) {
+  return P.parts == 1 ? (size_t)P.n * P.n : P.parts * dis_part(P) + (size_t)P.ns * P.ns;
+}
+size_t dense_store32_count(const DensePlan& P) {
+  return P.parts == 1 ? (size_t)P.n * dense_ld32(P.n) : P.parts * dis_part(P) + (size_t)P.ns * dense_ld32(P.ns);
+}
+size_t dense_perm_count(const DensePlan& P) { return P.parts == 1 ? (size_t)P.n : (size_t)P.parts * P.ni + P.ns; }
+size_t dense_vec_count(const DensePlan& P) {
+  return P.parts == 1 ? 1 : (size_t)P.parts * (P.ni + 2 * P.rm) + P.ns;
+}
+size_t dense_work_count(const DensePlan& P) {
+  if (P.parts == 1) return cholesky_work(P.n, 1);
+  return std::max(cholesky_work(P.ni, P.parts), cholesky_work(P.ns, 1)) + (size_t)P.parts * 4 * P.rm * P.rm;
+}
+void launch_dense_perm(const Grid& c, const DensePlan& P, int* perm, cudaStream_t st) {
+  if (P.parts == 1) {
+    launch_k(k_dense_perm, (P.n + 255) / 256, 256, 0, st, c, perm, P.n);
+    return;
+  }
+  cudaMemsetAsync(perm, 0xff, sizeof(int) * dense_perm_count(P), st);
+  launch_k(k_dis_perm, (P.n / 3 + 255) / 256, 256, 0, st, c, P, perm);
+}
+
+// The coarsest operator's explicit inverse, or the dissected one's blocks, in
+// `store`, from the level's full stencil.  d_info > 0: a non-positive pivot.
+void dense_build(const Grid& c, const DensePlan& P, const double* stencil, int reach, const uint8_t* cmask,
+                 double* store, double* work, int* d_info, cudaStream_t st) {
+  cudaMemsetAsync(d_info, 0, sizeof(int), st);
+  if (P.parts == 1) {
+    if (reach > 1) wide_dense_assemble(c, reach, stencil, cmask, store, P.n, st);
+    else dense_assemble(c, stencil, cmask, store, P.n, st);
+    // DOF bandwidth of the reach-R stencil in reference node order
+    const long long nx1 = c.lx + 1, ny1 = c.ly + 1;
+    const long long bw = 3LL * std::max(reach, 1) * (1 + nx1 + nx1 * ny1) + 2;
+    cholesky_inverse(store, work, P.n, (int)std::min<long long>(bw, P.n), d_info, st, 1, 0);
+    return;
+  }
+  const size_t sp = dis_part(P), blk = (size_t)P.rm * P.rm;
+  double* coup = work + std::max(cholesky_work(P.ni, P.parts), cholesky_work(P.ns, 1));
+  double* S = store + P.parts * sp;
+  cudaMemsetAsync(store, 0, sizeof(double) * dense_store_count(P), st);
+  cudaMemsetAsync(coup, 0, sizeof(double) * P.parts * 4 * blk, st);
+  const int W = 2 * P.reach + 1;
+  const long long pairs = (long long)(P.n / 3) * W * W * W;
+  launch_k(k_dis_assemble, (int)std::min<long long>((pairs + 255) / 256, 148LL * 64), 256, 0, st, c, P, stencil, cmask,
+           store, coup);
+  launch_k(k_dis_pad, dim3(4, P.parts), 256, 0, st, P, store);
+  // within a part the DOFs run plane by plane: the band is reach + 1 planes
+  cholesky_inverse(store, work, P.ni, P.rm + P.m, d_info, st, P.parts, sp);
+  GemmBatch w{}, r{}, l{};
+  w.alpha = 1.0;
+  r.alpha = l.alpha = -1.0;
+  r.beta = l.beta = 1.0;
+  const int rm = P.rm, ni = P.ni;
+  for (int i = 0; i < P.parts; ++i) {
+    double *Z = store + i * sp, *WL = Z + (size_t)ni * ni, *WR = WL + (size_t)rm * ni, *C = coup + (size_t)i * 4 * blk;
+    const int last = part_planes(P, i) * P.m - rm;   // first row of the planes next to the right separator
+    // W^T = C^T Z (Z is symmetric); S -= W^T C, the lower blocks
+    if (i > 0) w.job[w.count++] = GemmJob{C + blk, Z, WL, rm, ni, ni, rm, ni, rm};
+    if (i + 1 < P.parts) w.job[w.count++] = GemmJob{C + 3 * blk, Z + (size_t)last * ni, WR, rm, ni, ni, rm, ni, rm};
+    double* Sii = S + (size_t)i * rm * P.ns + (size_t)i * rm;   // separator i against itself
+    if (i + 1 < P.parts) r.job[r.count++] = GemmJob{WR + last, C + 2 * blk, Sii, ni, rm, P.ns, rm, rm, rm};
+    if (i > 0) {
+      l.job[l.count++] = GemmJob{WL, C, Sii - (size_t)rm * P.ns - rm, ni, rm, P.ns, rm, rm, rm};
+      if (i + 1 < P.parts) l.job[l.count++] = GemmJob{WR, C, Sii - rm, ni, rm, P.ns, rm, rm, rm};
+    }
+  }
+  const int t = (rm + TB - 1) / TB;
+  launch_k(k_gemm_batched, dim3(t * ((ni + TB - 1) / TB), w.count), 256, 0, st, w);
+  launch_k(k_gemm_batched, dim3(t * t, r.count), 256, 0, st, r);
+  launch_k(k_gemm_batched, dim3(t * t, l.count), 256, 0, st, l);
+  cholesky_inverse(S, work, P.ns, 2 * rm, d_info, st, 1, 0);
+}
+void dense_build32(const DensePlan& P, const double* store, float* store32, cudaStream_t st) {
+  const size_t head = P.parts == 1 ? 0 : P.parts * dis_part(P);
+  const int n = P.parts == 1 ? P.n : P.ns;
+  if (head) launch_convert<double, float>(store, store32, (long long)head, st);
+  const long long total = (long long)n * dense_ld32(n);
+  launch_k(k_convert_pad, (int)std::min<long long>((total + 255) / 256, 148LL * 32), 256, 0, st, store + head,
+           store32 + head, n, dense_ld32(n));
+}
+
+template <typename T, typename S>
+static void dissected_solve(const DensePlan& P, const S* store, int ld, const int* perm, double* vec, const T* b, T* x,
+                            const KrylovState* ks, cudaStream_t st) {
+  double* xs = vec + (size_t)P.parts * (P.ni + 2 * P.rm);
+  launch_k(k_dis_parts<T, S>, dim3((P.ni + 2 * P.rm + kDisRows - 1) / kDisRows, P.parts), 256, sizeof(double) * P.ni, st,
+           P, store, perm, b, vec, ks);
+  launch_k(k_dis_schur<T, S>, (P.ns + 7) / 8, 256, sizeof(double) * ld, st, P, store + P.parts * dis_part(P), ld, perm, b,
+           (const double*)vec, xs, x, ks);
+  launch_k(k_dis_back<T, S>, dim3((P.ni + 31) / 32, P.parts), 256, 0, st, P, store, perm, (const double*)vec,
+           (const double*)xs, x, ks);
 }
 
 // b is staged in dynamic shared memory (n doubles, n <= 16384).  The limit is
 // a per-function attribute shared by every solver of the process (solvers of
 // different sizes run concurrently in batch solves): always the maximum.
-void dense_prepare_smem(int n) {
-  (void)n;
+void dense_prepare_smem() {
   const int bytes = (int)sizeof(double) * 16384;
-  cudaFuncSetAttribute(k_dense_solve<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_dense_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_dense_solve_f32<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  auto allow = [&](const void* f) { cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+  allow((const void*)k_dense_solve<double>);
+  allow((const void*)k_dense_solve<float>);
+  allow((const void*)k_dense_solve_f32<float>);
+  allow((const void*)k_dis_parts<double, double>);
+  allow((const void*)k_dis_parts<float, float>);
+  allow((const void*)k_dis_schur<double, double>);
+  allow((const void*)k_dis_schur<float, float>);
 }
 
 int dense_ld32(int n) { return (n + 3) / 4 * 4; }
 
-void launch_dense_perm(const Grid& c, int* perm, int n, cudaStream_t st) {
-  launch_k(k_dense_perm, (n + 255) / 256, 256, 0, st, c, perm, n);
+template <>
+void launch_dense_solve<double>(const DensePlan& P, const double* store, const float*, const int* perm, double* vec,
+                                const double* b, double* x, const KrylovState* ks, cudaStream_t st) {
+  if (P.parts > 1) {
+    // (ns is even or its rows would not start on 16 bytes: see dense_plan)
+    dissected_solve<double, double>(P, store, P.ns, perm, vec, b, x, ks, st);
+    return;
+  }
+  launch_k(k_dense_solve<double>, (P.n + 7) / 8, 256, sizeof(double) * P.n, st, store, P.n, perm, b, x, ks);
 }
-
-void launch_dense_convert_pad(const double* A, float* B, int n, cudaStream_t st) {
-  const int ld = dense_ld32(n);
-  const long long total = (long long)n * ld;
-  launch_k(k_convert_pad, (int)std::min<long long>((total + 255) / 256, 148LL * 32), 256, 0, st, A, B, n, ld);
-}
-
-template <typename T>
-void launch_dense_solve(const double* Ainv, int n, const int* perm, const T* b, T* x, const KrylovState* ks,
-                        cudaStream_t st) {
-  const int blocks = (n + 7) / 8;   // one row per warp: every row's stream in flight at once
-  launch_k(k_dense_solve<T>, blocks, 256, sizeof(double) * n, st, Ainv, n, perm, b, x, ks);
-}
-template void launch_dense_solve<double>(const double*, int, const int*, const double*, double*,
-                                         const KrylovState*, cudaStream_t);
-template void launch_dense_solve<float>(const double*, int, const int*, const float*, float*,
-                                        const KrylovState*, cudaStream_t);
-
-void launch_dense_solve_f32(const float* Ainv32, int n, const int* perm, const float* b, float* x,
-                            const KrylovState* ks, cudaStream_t st) {
-  const int ld = dense_ld32(n);
-  const int blocks = (n + 7) / 8;
-  launch_k(k_dense_solve_f32<float>, blocks, 256, sizeof(double) * ld, st, Ainv32, n, ld, perm, b, x, ks);
+template <>
+void launch_dense_solve<float>(const DensePlan& P, const double*, const float* store32, const int* perm, double* vec,
+                               const float* b, float* x, const KrylovState* ks, cudaStream_t st) {
+  if (P.parts > 1) {
+    dissected_solve<float, float>(P, store32, dense_ld32(P.ns), perm, vec, b, x, ks, st);
+    return;
+  }
+  const int ld = dense_ld32(P.n);
+  launch_k(k_dense_solve_f32<float>, (P.n + 7) / 8, 256, sizeof(double) * ld, st, store32, P.n, ld, perm, b, x, ks);
 }
 
 }  // namespace vf

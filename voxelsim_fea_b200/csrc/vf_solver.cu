@@ -42,7 +42,6 @@ void launch_stencil_from_elements(const Grid& g, const double* E, const double* 
                                   double* stencil, const double* Ktab, int lame, cudaStream_t st);
 void launch_galerkin_mask(const Grid& c, double* stencil, uint8_t* cmask, double* minv3, cudaStream_t st);
 void launch_stencil_diag(const Grid& c, double* stencil, const uint8_t* cmask, double* minv3, cudaStream_t st);
-void dense_prepare_smem(int n);
 void launch_strain_energy_tab(const Grid& g, const double* u_pad, const uint8_t* active_ref, const double* KE,
                               double* se_ref, cudaStream_t st);
 }  // namespace vf
@@ -137,11 +136,12 @@ struct vf_solver {
   bool have_active = false;
   uint8_t* d_allfree = nullptr;
   // coarsest dense factor
-  double* d_Ainv = nullptr;
-  float* d_Ainv32 = nullptr;    // FP32 copy of the coarsest inverse for the FP32 V-cycle (rows of dense_ld32(n))
+  double* d_Ainv = nullptr;     // the inverse, or the dissected one's blocks (DensePlan)
+  float* d_Ainv32 = nullptr;    // their FP32 copy for the FP32 V-cycle
   int* d_dense_perm = nullptr;  // padded-vector index of each coarsest DOF
   double* d_dense_work = nullptr;
-  int dense_n = 0;
+  double* d_dense_vec = nullptr;   // this solver's own (a child shares the blocks, not these)
+  DensePlan dense{};
   int* d_info = nullptr;
   // Krylov vectors on level 0: x, r, z, p, Ap
   double* k64[5] = {};
@@ -444,12 +444,7 @@ template <typename T>
 void coarse_solve(vf_solver* s, int li, const T* b, T* x, KrylovState* ks) {
   Level& l = s->L[li];
   if (s->o.coarsest == VF_COARSEST_CHOLESKY && s->d_Ainv) {
-    if constexpr (sizeof(T) == 4) {
-      if (s->d_Ainv32) launch_dense_solve_f32(s->d_Ainv32, s->dense_n, s->d_dense_perm, b, x, ks, s->st);
-      else launch_dense_solve<T>(s->d_Ainv, s->dense_n, s->d_dense_perm, b, x, ks, s->st);
-    } else {
-      launch_dense_solve<T>(s->d_Ainv, s->dense_n, s->d_dense_perm, b, x, ks, s->st);
-    }
+    launch_dense_solve<T>(s->dense, s->d_Ainv, s->d_Ainv32, s->d_dense_perm, s->d_dense_vec, b, x, ks, s->st);
   } else {
     smooth<T>(s, li, x, Sel<T>::w(l, 1), b, s->o.coarse_sweeps, true, ks);
   }
@@ -859,13 +854,14 @@ int build_levels(vf_solver* s) {
     Level& lc = s->L.back();
     const int n = 3 * lc.g.nodes_ref();
     if (n <= 16384) {
-      VF_ALLOC(s->d_Ainv, (size_t)n * n);
-      VF_ALLOC(s->d_Ainv32, (size_t)n * dense_ld32(n));
-      VF_ALLOC(s->d_dense_perm, (size_t)n);
-      VF_ALLOC(s->d_dense_work, dense_work_count(n));
-      s->dense_n = n;
-      dense_prepare_smem(n);
-      launch_dense_perm(lc.g, s->d_dense_perm, n, s->st);
+      s->dense = dense_plan(lc.g, lc.reach);
+      VF_ALLOC(s->d_Ainv, dense_store_count(s->dense));
+      VF_ALLOC(s->d_Ainv32, dense_store32_count(s->dense));
+      VF_ALLOC(s->d_dense_perm, dense_perm_count(s->dense));
+      VF_ALLOC(s->d_dense_work, dense_work_count(s->dense));
+      VF_ALLOC(s->d_dense_vec, dense_vec_count(s->dense));
+      dense_prepare_smem();
+      launch_dense_perm(lc.g, s->dense, s->d_dense_perm, s->st);
       if (!lc.galerkin && !lc.st64) VF_ALLOC(lc.st64, 243 * (size_t)lc.g.n);
     }
   }
@@ -1091,15 +1087,6 @@ int build_dense_coarsest(vf_solver* s) {
              "(use more levels or VF_COARSEST_JACOBI)";
     return VF_ERR_UNSUPPORTED;
   }
-  if (s->dense_n != n) {
-    VF_ALLOC(s->d_Ainv, (size_t)n * n);
-    VF_ALLOC(s->d_Ainv32, (size_t)n * dense_ld32(n));
-    VF_ALLOC(s->d_dense_perm, (size_t)n);
-    VF_ALLOC(s->d_dense_work, dense_work_count(n));
-    s->dense_n = n;
-    dense_prepare_smem(n);
-    launch_dense_perm(lc.g, s->d_dense_perm, n, s->st);   // after its zeroing on st; read on st
-  }
   double* st = lc.st64;
   if (!lc.galerkin) {
     // stencil of the rediscretized element operator on the coarsest level
@@ -1108,13 +1095,8 @@ int build_dense_coarsest(vf_solver* s) {
     launch_stencil_from_elements(lc.g, lc.E64, s->lame ? lc.mu64 : nullptr, lc.mask, st,
                                  s->lame ? s->d_Ktab_lame : s->d_Ktab, s->lame ? 1 : 0, sd);
   }
-  if (lc.reach > 1) wide_dense_assemble(lc.g, lc.reach, st, lc.mask, s->d_Ainv, n, sd);
-  else dense_assemble(lc.g, st, lc.mask, s->d_Ainv, n, sd);
-  // DOF bandwidth of the reach-R stencil in reference node order
-  const long long nx1 = lc.g.lx + 1, ny1 = lc.g.ly + 1;
-  const long long bw = 3LL * std::max(lc.reach, 1) * (1 + nx1 + nx1 * ny1) + 2;
-  dense_cholesky_inverse(s->d_Ainv, s->d_dense_work, n, (int)std::min<long long>(bw, n), s->d_info, sd);
-  launch_dense_convert_pad(s->d_Ainv, s->d_Ainv32, n, sd);
+  dense_build(lc.g, s->dense, st, lc.reach, lc.mask, s->d_Ainv, s->d_dense_work, s->d_info, sd);
+  dense_build32(s->dense, s->d_Ainv, s->d_Ainv32, sd);
   VF_CHECK_LAUNCH();
   int info = 0;
   VF_TRY(cudaMemcpyAsync(&info, s->d_info, sizeof(int), cudaMemcpyDeviceToHost, sd));
@@ -2265,7 +2247,7 @@ void share_operator(vf_solver* c, const vf_solver* m) {
   c->d_Ainv = m->d_Ainv;
   c->d_Ainv32 = m->d_Ainv32;
   c->d_dense_perm = m->d_dense_perm;
-  c->dense_n = m->dense_n;
+  c->dense = m->dense;
   c->d_omega = m->d_omega;
   c->d_lambda = m->d_lambda;
   c->d_cheb = m->d_cheb;
@@ -2321,6 +2303,7 @@ int make_child(vf_solver* m, vf_solver** out) {
     VF_ALLOC(s->d_partials, partials_needed(s));
     VF_ALLOC(s->d_info, 1);
     VF_ALLOC(s->d_err, 1);
+    if (m->d_Ainv) VF_ALLOC(s->d_dense_vec, dense_vec_count(m->dense));
     VF_TRY(cudaMallocHost(&s->h_ks, sizeof(KrylovState)));
     memset(s->h_ks, 0, sizeof(KrylovState));
     int rc = ensure_hist(s, 4096);
