@@ -163,6 +163,8 @@ struct OpArgs {
   const void* dprev;
   void* dout;
   const double* c1_dev;
+  // APPLY: out = Minv A u (a step of the power iteration) instead of A u
+  const void* apply_minv;
 };
 template <typename T> void launch_fine_op(const Grid& g, int epi, const OpArgs& a, cudaStream_t st);
 
@@ -304,8 +306,7 @@ template <typename T> void launch_axpy_gamma(const Grid& g, T* z, const T* c, co
                                              cudaStream_t st);
 // power iteration on D^-1 A (per-level damping)
 template <typename T> void launch_power_init(const Grid& g, T* x, const uint8_t* mask, cudaStream_t st);
-template <typename T>
-void launch_power_scale(const Grid& g, T* y, const T* minv3, double* partials, KrylovState* ks, cudaStream_t st);
+template <typename T> void launch_power_norm(const Grid& g, const T* x, double* partials, KrylovState* ks, cudaStream_t st);
 template <typename T>
 void launch_power_normalize(const Grid& g, const T* y, T* x, const KrylovState* ks, cudaStream_t st);
 void launch_cheb_coefs(const double* lambda, int nl, int ratio, double* coef, cudaStream_t st);

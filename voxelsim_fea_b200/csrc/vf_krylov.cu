@@ -350,20 +350,22 @@ __global__ void k_power_init(long long n, T* __restrict__ x, const uint8_t* __re
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_power_scale(long long n, T* __restrict__ y,
-                                                             const T* __restrict__ minv, double* partials,
-                                                             KrylovState* ks) {
+__global__ void __launch_bounds__(kVecThreads) k_power_norm(long long n3, const T* __restrict__ x, double* partials,
+                                                            KrylovState* ks) {
+  using H = V16<T>;
+  using V = typename H::V;
+  const long long nv = n3 / H::W;
+  const V* xv = reinterpret_cast<const V*>(x);
   double s = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const T v = y[i] * minv[i];
-    y[i] = v;
-    s += (double)v * (double)v;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
+    const V v = __ldg(xv + i);
+    s += H::dot(v, v);
   }
   reduce_and_finalize(s, partials, ks, SLOT_PLAIN, nullptr);
 }
 
 template <typename T>
-__global__ void k_power_normalize(long long n, const T* __restrict__ y, T* __restrict__ x, const KrylovState* ks) {
+__global__ void k_power_normalize(long long n, const T* y, T* x, const KrylovState* ks) {   // (in place)
   const T inv = ks->rr > 0.0 ? (T)(1.0 / sqrt(ks->rr)) : (T)0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     x[i] = y[i] * inv;
@@ -421,8 +423,8 @@ void launch_power_init(const Grid& g, T* x, const uint8_t* mask, cudaStream_t st
   launch_k(k_power_init<T>, vec_blocks((long long)g.n), kVecThreads, 0, st, (long long)g.n, x, mask);
 }
 template <typename T>
-void launch_power_scale(const Grid& g, T* y, const T* minv3, double* partials, KrylovState* ks, cudaStream_t st) {
-  launch_k(k_power_scale<T>, vec_blocks(3LL * g.n), kVecThreads, 0, st, 3LL * g.n, y, minv3, partials, ks);
+void launch_power_norm(const Grid& g, const T* x, double* partials, KrylovState* ks, cudaStream_t st) {
+  launch_k(k_power_norm<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, partials, ks);
 }
 template <typename T>
 void launch_power_normalize(const Grid& g, const T* y, T* x, const KrylovState* ks, cudaStream_t st) {
@@ -430,7 +432,7 @@ void launch_power_normalize(const Grid& g, const T* y, T* x, const KrylovState* 
 }
 #define VF_INST_POWER(T)                                                                                   \
   template void launch_power_init<T>(const Grid&, T*, const uint8_t*, cudaStream_t);                       \
-  template void launch_power_scale<T>(const Grid&, T*, const T*, double*, KrylovState*, cudaStream_t);     \
+  template void launch_power_norm<T>(const Grid&, const T*, double*, KrylovState*, cudaStream_t);           \
   template void launch_power_normalize<T>(const Grid&, const T*, T*, const KrylovState*, cudaStream_t);
 VF_INST_POWER(double)
 VF_INST_POWER(float)

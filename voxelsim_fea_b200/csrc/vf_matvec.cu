@@ -102,6 +102,10 @@ __global__ void __launch_bounds__(kOpThreads) k_fine_op(Grid g, OpArgs a, const 
     k2 = (m & 4) ? k2 : (T)0;
     const long long p3 = 3 * (long long)p;
     if (EPI == EPI_APPLY) {
+      if (a.apply_minv) {
+        const T* am = (const T*)a.apply_minv;
+        k0 *= __ldg(am + p3); k1 *= __ldg(am + p3 + 1); k2 *= __ldg(am + p3 + 2);
+      }
       out[p3] = k0; out[p3 + 1] = k1; out[p3 + 2] = k2;
       if (a.dot_partials)
         dot += (double)u[p3] * (double)k0 + (double)u[p3 + 1] * (double)k1 + (double)u[p3 + 2] * (double)k2;

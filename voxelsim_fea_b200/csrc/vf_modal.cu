@@ -250,10 +250,14 @@ __global__ void __launch_bounds__(TX * TY, 2) k_modal_op(Grid g, OpArgs a, Modal
           if (zs < oend[l]) {
             const int p3 = 3 * ((zs + 1) * sz + colbase);
             const uint8_t m8 = mk[l];
-            const T k0 = (m8 & 1) ? O::lane(y[0], l) : (T)0;
-            const T k1 = (m8 & 2) ? O::lane(y[1], l) : (T)0;
-            const T k2 = (m8 & 4) ? O::lane(y[2], l) : (T)0;
+            T k0 = (m8 & 1) ? O::lane(y[0], l) : (T)0;
+            T k1 = (m8 & 2) ? O::lane(y[1], l) : (T)0;
+            T k2 = (m8 & 4) ? O::lane(y[2], l) : (T)0;
             if (EPI == EPI_APPLY) {
+              if (a.apply_minv) {
+                const T* am = (const T*)a.apply_minv + p3;
+                k0 *= __ldg(am); k1 *= __ldg(am + 1); k2 *= __ldg(am + 2);
+              }
               out[p3] = k0; out[p3 + 1] = k1; out[p3 + 2] = k2;
               if (a.dot_partials) {
                 const T u0 = O::lane(Sp.u[0][ty][tx], l), u1 = O::lane(Sp.u[1][ty][tx], l);

@@ -289,7 +289,7 @@ struct SweepStep {
 
 template <typename T>
 void level_op(vf_solver* s, int li, int epi, const T* u, T* out, const T* b, KrylovState* ks, double* partials,
-              int slot, const SweepStep* step = nullptr) {
+              int slot, const SweepStep* step = nullptr, const T* apply_minv = nullptr) {
   Level& l = s->L[li];
   OpArgs a{};
   a.u = u; a.out = out; a.b = b;
@@ -309,6 +309,7 @@ void level_op(vf_solver* s, int li, int epi, const T* u, T* out, const T* b, Kry
   a.dot_slot = slot;
   a.ke_tab = s->tab;
   a.err = s->d_err;
+  a.apply_minv = apply_minv;
   if (l.galerkin) {
     if (s->o.coarse_storage == VF_STENCIL_FULL) launch_stencil_op<T>(l.g, epi, a, Sel<T>::st(l), s->st);
     else level_sym_op<T>(s, l, epi, a);
@@ -1039,11 +1040,20 @@ int power_level(vf_solver* s, int li) {
   init_ks(*s->h_ks, 1.0, 1, 0, 0, 1.0);
   VF_TRY(cudaMemcpyAsync(s->ks, s->h_ks, sizeof(KrylovState), cudaMemcpyHostToDevice, s->st));
   Level& l = s->L[li];
-  launch_power_init<float>(l.g, l.w32[0], l.mask, s->st);
-  for (int k = 0; k < std::max(2, s->o.power_iters); ++k) {
-    level_op<float>(s, li, EPI_APPLY, l.w32[0], l.w32[1], nullptr, nullptr, nullptr, 0);
-    launch_power_scale<float>(l.g, l.w32[1], l.minv32, s->d_partials, s->ks, s->st);
-    launch_power_normalize<float>(l.g, l.w32[1], l.w32[0], s->ks, s->st);
+  // lambda = ||D^-1 A x|| for the last, unit x.  In between the iterate only
+  // needs to stay in range: an eigenvalue of D^-1 A is at most a few dozen, so
+  // it is scaled to unit length every 8 steps, and a step is one launch (it
+  // was three: product, scaling with its reduction, normalisation)
+  float *x = l.w32[0], *y = l.w32[1];
+  launch_power_init<float>(l.g, x, l.mask, s->st);
+  const int steps = std::max(2, s->o.power_iters);
+  for (int k = 0; k < steps; ++k) {
+    level_op<float>(s, li, EPI_APPLY, x, y, nullptr, nullptr, nullptr, 0, nullptr, l.minv32);
+    if (k == steps - 1 || k == steps - 2 || k % 8 == 7) {
+      launch_power_norm<float>(l.g, y, s->d_partials, s->ks, s->st);
+      if (k < steps - 1) launch_power_normalize<float>(l.g, y, y, s->ks, s->st);
+    }
+    std::swap(x, y);
   }
   launch_power_omega(s->ks, s->o.omega_rel, 1.1, s->d_omega + li, s->d_lambda + li, s->st);
   VF_CHECK_LAUNCH();

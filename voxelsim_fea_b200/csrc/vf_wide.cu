@@ -508,19 +508,21 @@ __global__ void k_wide_apply_mask(Grid c, int R, double* __restrict__ st, const 
                                   double* __restrict__ minv3) {
   const int W = wide_w(R), NB = wide_nb(R), SC = NB / 2;
   const long long n = c.n;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < c.n; p += gridDim.x * blockDim.x) {
+  // one thread per node and block: a thread per node walked 125 blocks alone
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * NB; i += (long long)gridDim.x * blockDim.x) {
+    const int s = (int)(i / n), p = (int)(i - s * n);
     int x, y, z;
     decode(c, p, x, y, z);
     const bool in = inside(c, x, y, z);
     const uint8_t mp = cmask[p];
-    for (int s = 0; s < NB; ++s) {
+    {
       const int qx = x + s % W - R, qy = y + (s / W) % W - R, qz = z + s / (W * W) - R;
       const uint8_t mq = (in && inside(c, qx, qy, qz)) ? cmask[c.idx(qx, qy, qz)] : (uint8_t)0;
       for (int r = 0; r < 3; ++r)
         for (int cc = 0; cc < 3; ++cc)
           if (!(in && ((mp >> r) & 1) && ((mq >> cc) & 1))) st[((long long)s * 9 + 3 * r + cc) * n + p] = 0.0;
     }
-    for (int r = 0; r < 3; ++r) {
+    if (s == SC) for (int r = 0; r < 3; ++r) {
       const double d = st[((long long)SC * 9 + 4 * r) * n + p];
       minv3[3LL * p + r] = ((mp >> r) & 1) && d != 0.0 ? 1.0 / d : 0.0;
     }
@@ -540,7 +542,11 @@ __global__ void k_wide_compress(Grid g, const double* __restrict__ st, const uin
   using Q = typename L::Q;
   constexpr int W = 2 * R + 1, NB = W * W * W, SC = NB / 2, G = L::G;
   const long long n = g.n;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < g.n; p += gridDim.x * blockDim.x) {
+  // one thread per node and block slot, a node's lanes consecutive (a thread
+  // per node walked 64 slots alone: 0.27 ms on 2,400 nodes and on 20,000)
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * G * L::NJ;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int jj = (int)(i / (n * G)), p = (int)((i - jj * n * G) / G), u = jj * G + (int)(i % G);
     int x, y, z;
     decode(g, p, x, y, z);
     const bool in = inside(g, x, y, z);
@@ -548,10 +554,12 @@ __global__ void k_wide_compress(Grid g, const double* __restrict__ st, const uin
     for (int r = 0; r < 3; ++r) {
       const double d = in ? st[((long long)SC * 9 + 4 * r) * n + p] : 0.0;
       sp[r] = (in && ((mask[p] >> r) & 1) && d > 0.0) ? 1.0 / sqrt(d) : 0.0;
-      sqrtd[3LL * p + r] = (Q)(sp[r] > 0.0 ? 1.0 / sp[r] : 0.0);
+      if (u == 0) sqrtd[3LL * p + r] = (Q)(sp[r] > 0.0 ? 1.0 / sp[r] : 0.0);
     }
-    for (int u = 0; u < L::G * L::NJ; ++u) {
-      const long long v = (long long)p * G + u % G;
+    const long long v = (long long)p * G + u % G;
+    if (jj == 0)
+      for (int k = 9 * L::NJ; k < L::NVL; ++k) stc[L::off(v, k)] = to_s<S>(0.0);
+    {
       const int k0 = 9 * (u / G);
       if (u >= L::NBLK) {
         for (int k = 0; k < 9; ++k) stc[L::off(v, k0 + k)] = to_s<S>(0.0);
@@ -574,8 +582,6 @@ __global__ void k_wide_compress(Grid g, const double* __restrict__ st, const uin
           stc[L::off(v, k0 + 3 * r + cc)] = to_s<S>(val);
         }
     }
-    for (int gl = 0; gl < G; ++gl)
-      for (int k = 9 * L::NJ; k < L::NVL; ++k) stc[L::off((long long)p * G + gl, k)] = to_s<S>(0.0);
   }
 }
 
@@ -710,7 +716,7 @@ __global__ void __launch_bounds__(128) k_wide_op(Grid g, OpArgs a, const S* __re
     const T kc = ((m >> c) & 1) ? (T)(ac * (A)sqd[pc]) : (T)0;
     const T bc = b ? b[pc] : (T)0;
     if (EPI == EPI_APPLY) {
-      out[pc] = kc;
+      out[pc] = a.apply_minv ? kc * __ldg((const T*)a.apply_minv + pc) : kc;
       if (a.dot_partials) dot += (double)u[pc] * (double)kc;
     } else if (EPI == EPI_SMOOTH) {
       const T u0 = u[pc];
@@ -809,13 +815,13 @@ void launch_wide_galerkin(const Grid& f, const double* stf, int Rf, const uint8_
 
 void launch_wide_mask(const Grid& c, int R, double* stc, uint8_t* cmask, double* minv3, cudaStream_t st) {
   launch_k(k_wide_mask_from_diag, blocks_for(c.n, 256), 256, 0, st, c, R, stc, cmask);
-  launch_k(k_wide_apply_mask, blocks_for(c.n, 128), 128, 0, st, c, R, stc, cmask, minv3);
+  launch_k(k_wide_apply_mask, blocks_for((long long)c.n * wide_nb(R), 128), 128, 0, st, c, R, stc, cmask, minv3);
 }
 
 template <typename S, int R>
 void launch_wide_compress(const Grid& g, const double* st, const uint8_t* mask, S* stc,
                           typename WideLayout<S, R>::Q* sqrtd, cudaStream_t st_) {
-  launch_k(k_wide_compress<S, R>, blocks_for(g.n, 128), 128, 0, st_, g, st, mask, stc, sqrtd);
+  launch_k(k_wide_compress<S, R>, blocks_for((long long)g.n * WideLayout<S, R>::G * WideLayout<S, R>::NJ, 128), 128, 0, st_, g, st, mask, stc, sqrtd);
 }
 template void launch_wide_compress<__half, 2>(const Grid&, const double*, const uint8_t*, __half*, float*, cudaStream_t);
 template void launch_wide_compress<float, 2>(const Grid&, const double*, const uint8_t*, float*, float*, cudaStream_t);
