@@ -50,6 +50,7 @@ __global__ void k_dense_assemble(Grid c, const double* __restrict__ st, const ui
 // (blockIdx.x: matrix of a batch, sA / sL values apart.)
 __global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int k, int nb, int* info, double* linv,
                                                            size_t sA, size_t sL) {
+  pdl_enter();
   A += sA * blockIdx.x;
   linv += sL * blockIdx.x;
   // L: the block being reduced (column j is read, columns > j updated in step
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int
 // X[i][j] = sum_{l <= j} A[i][k+l] linv[j][l].  64 rows per CTA.
 __global__ void __launch_bounds__(256) k_trsm_panel(double* A, int n, int k, int nb, const double* linv, size_t sA,
                                                     size_t sL) {
+  pdl_enter();
   A += sA * blockIdx.y;
   linv += sL * blockIdx.y;
   __shared__ double P[64][NB + 1], Li[NB][NB + 1];
@@ -127,6 +129,7 @@ constexpr int TB = 64;
 // Trailing update (lower triangle): A[i][j] -= sum_l A[i][k+l] A[j][k+l].
 // Grid: one CTA per 64 x 64 tile pair bi >= bj of the trailing matrix.
 __global__ void __launch_bounds__(256) k_syrk_update(double* A, int n, int k, int nb, size_t sA) {
+  pdl_enter();
   A += sA * blockIdx.z;
   const int t0 = k + nb;
   const int bi = blockIdx.y, bj = blockIdx.x;
@@ -187,6 +190,7 @@ struct GemmBatch {
 // One 64 x 64 output tile per CTA (blockIdx.x: tile of job blockIdx.y),
 // 4 x 4 register blocks, K in chunks of 32 through shared memory.
 __global__ void __launch_bounds__(256) k_gemm_batched(const __grid_constant__ GemmBatch bt) {
+  pdl_enter();
   const GemmJob& jb = bt.job[blockIdx.y];
   const int tn = (jb.N + TB - 1) / TB, tm = (jb.M + TB - 1) / TB;
   if ((int)blockIdx.x >= tn * tm) return;
@@ -255,6 +259,7 @@ __global__ void k_y_init(double* Y, int n, const double* linv_all, size_t sY, si
 // A^-1 = Y^T Y is symmetric: one CTA per 64x64 tile of the lower triangle
 // (blockIdx.x enumerates the pairs bi >= bj), written to both triangles.
 __global__ void __launch_bounds__(256) k_yty(const double* Y, double* Ainv, int n, size_t sY, size_t sA) {
+  pdl_enter();
   Y += sY * blockIdx.y;
   Ainv += sA * blockIdx.y;
   int bi = (int)((sqrt(8.0 * blockIdx.x + 1.0) - 1.0) * 0.5);
@@ -330,6 +335,7 @@ __global__ void k_convert_pad(const double* __restrict__ A, float* __restrict__ 
 template <typename T>
 __global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int* __restrict__ perm,
                               const T* __restrict__ b, T* __restrict__ x, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];
   for (int i = threadIdx.x; i < n; i += blockDim.x) sb[i] = (double)b[__ldg(perm + i)];
@@ -361,6 +367,7 @@ __global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int*
 template <typename T>
 __global__ void k_dense_solve_f32(const float* __restrict__ Ainv, int n, int ld, const int* __restrict__ perm,
                                   const T* __restrict__ b, T* __restrict__ x, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];   // ld values, zero past n
   for (int i = threadIdx.x; i < ld; i += blockDim.x) sb[i] = i < n ? (double)b[__ldg(perm + i)] : 0.0;
@@ -428,13 +435,13 @@ static void cholesky_inverse(double* A, double* work, int n, int bw, int* d_info
   for (int k = 0; k < n; k += NB) {
     const int nb = (n - k < NB) ? (n - k) : NB;
     double* linv = linv_all + (size_t)(k / NB) * NB * NB;
-    launch_k(k_potrf_diag, batch, NB * NB, 0, st, A, n, k, nb, d_info, linv, sA, sL);
+    launch_pdl(k_potrf_diag, batch, NB * NB, 0, st, A, n, k, nb, d_info, linv, sA, sL);
     // rows > k + nb - 1 + bw of columns k .. k + nb - 1 are zero
     const int rest = std::min(n, k + nb + bw) - (k + nb);
     if (rest > 0) {
-      launch_k(k_trsm_panel, dim3((rest + 63) / 64, batch), 256, 0, st, A, n, k, nb, (const double*)linv, sA, sL);
+      launch_pdl(k_trsm_panel, dim3((rest + 63) / 64, batch), 256, 0, st, A, n, k, nb, (const double*)linv, sA, sL);
       const int tiles = (rest + TB - 1) / TB;
-      launch_k(k_syrk_update, dim3(tiles, tiles, batch), 256, 0, st, A, n, k, nb, sA);
+      launch_pdl(k_syrk_update, dim3(tiles, tiles, batch), 256, 0, st, A, n, k, nb, sA);
     }
   }
   // Y = L^{-1} into work: diagonal blocks from the factorization, then the
@@ -450,8 +457,8 @@ static void cholesky_inverse(double* A, double* work, int n, int bw, int* d_info
     size_t toff = 0;
     auto flush = [&]() {
       if (b1.count == 0) return;
-      launch_k(k_gemm_batched, dim3(max_tiles, b1.count), 256, 0, st, b1);
-      launch_k(k_gemm_batched, dim3(max_tiles, b2.count), 256, 0, st, b2);
+      launch_pdl(k_gemm_batched, dim3(max_tiles, b1.count), 256, 0, st, b1);
+      launch_pdl(k_gemm_batched, dim3(max_tiles, b2.count), 256, 0, st, b2);
       b1.count = b2.count = 0;
       max_tiles = 0;
     };
@@ -476,7 +483,7 @@ static void cholesky_inverse(double* A, double* work, int n, int bw, int* d_info
   }
   // A <- Y^T Y (lower-triangle tiles, mirrored)
   const int tiles = (n + TB - 1) / TB;
-  launch_k(k_yty, dim3(tiles * (tiles + 1) / 2, batch), 256, 0, st, (const double*)work, A, n, sY, sA);
+  launch_pdl(k_yty, dim3(tiles * (tiles + 1) / 2, batch), 256, 0, st, (const double*)work, A, n, sY, sA);
 }
 
 // ---------------------------------------------------------------------------
@@ -625,6 +632,7 @@ template <typename T, typename S>
 __global__ void __launch_bounds__(256) k_dis_parts(DensePlan P, const S* __restrict__ store,
                                                    const int* __restrict__ perm, const T* __restrict__ b,
                                                    double* __restrict__ y, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];
   const int i = blockIdx.y, rows = P.ni + 2 * P.rm;
@@ -646,6 +654,7 @@ __global__ void __launch_bounds__(256) k_dis_schur(DensePlan P, const S* __restr
                                                    const int* __restrict__ perm, const T* __restrict__ b,
                                                    const double* __restrict__ y, double* __restrict__ xs,
                                                    T* __restrict__ x, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];
   const int rows = P.ni + 2 * P.rm;
@@ -674,6 +683,7 @@ __global__ void __launch_bounds__(256) k_dis_back(DensePlan P, const S* __restri
                                                   const int* __restrict__ perm, const double* __restrict__ y,
                                                   const double* __restrict__ xs, T* __restrict__ x,
                                                   const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   __shared__ double part[8][33];
   const int i = blockIdx.y, rows = P.ni + 2 * P.rm;
@@ -811,9 +821,9 @@ void dense_build(const Grid& c, const DensePlan& P, const double* stencil, int r
     }
   }
   const int t = (rm + TB - 1) / TB;
-  launch_k(k_gemm_batched, dim3(t * ((ni + TB - 1) / TB), w.count), 256, 0, st, w);
-  launch_k(k_gemm_batched, dim3(t * t, r.count), 256, 0, st, r);
-  launch_k(k_gemm_batched, dim3(t * t, l.count), 256, 0, st, l);
+  launch_pdl(k_gemm_batched, dim3(t * ((ni + TB - 1) / TB), w.count), 256, 0, st, w);
+  launch_pdl(k_gemm_batched, dim3(t * t, r.count), 256, 0, st, r);
+  launch_pdl(k_gemm_batched, dim3(t * t, l.count), 256, 0, st, l);
   cholesky_inverse(S, work, P.ns, 2 * rm, d_info, st, 1, 0);
 }
 void dense_build32(const DensePlan& P, const double* store, float* store32, cudaStream_t st) {
@@ -829,11 +839,11 @@ template <typename T, typename S>
 static void dissected_solve(const DensePlan& P, const S* store, int ld, const int* perm, double* vec, const T* b, T* x,
                             const KrylovState* ks, cudaStream_t st) {
   double* xs = vec + (size_t)P.parts * (P.ni + 2 * P.rm);
-  launch_k(k_dis_parts<T, S>, dim3((P.ni + 2 * P.rm + kDisRows - 1) / kDisRows, P.parts), 256, sizeof(double) * P.ni, st,
+  launch_pdl(k_dis_parts<T, S>, dim3((P.ni + 2 * P.rm + kDisRows - 1) / kDisRows, P.parts), 256, sizeof(double) * P.ni, st,
            P, store, perm, b, vec, ks);
-  launch_k(k_dis_schur<T, S>, (P.ns + 7) / 8, 256, sizeof(double) * ld, st, P, store + P.parts * dis_part(P), ld, perm, b,
+  launch_pdl(k_dis_schur<T, S>, (P.ns + 7) / 8, 256, sizeof(double) * ld, st, P, store + P.parts * dis_part(P), ld, perm, b,
            (const double*)vec, xs, x, ks);
-  launch_k(k_dis_back<T, S>, dim3((P.ni + 31) / 32, P.parts), 256, 0, st, P, store, perm, (const double*)vec,
+  launch_pdl(k_dis_back<T, S>, dim3((P.ni + 31) / 32, P.parts), 256, 0, st, P, store, perm, (const double*)vec,
            (const double*)xs, x, ks);
 }
 
@@ -862,7 +872,7 @@ void launch_dense_solve<double>(const DensePlan& P, const double* store, const f
     dissected_solve<double, double>(P, store, P.ns, perm, vec, b, x, ks, st);
     return;
   }
-  launch_k(k_dense_solve<double>, (P.n + 7) / 8, 256, sizeof(double) * P.n, st, store, P.n, perm, b, x, ks);
+  launch_pdl(k_dense_solve<double>, (P.n + 7) / 8, 256, sizeof(double) * P.n, st, store, P.n, perm, b, x, ks);
 }
 template <>
 void launch_dense_solve<float>(const DensePlan& P, const double*, const float* store32, const int* perm, double* vec,
@@ -872,7 +882,7 @@ void launch_dense_solve<float>(const DensePlan& P, const double*, const float* s
     return;
   }
   const int ld = dense_ld32(P.n);
-  launch_k(k_dense_solve_f32<float>, (P.n + 7) / 8, 256, sizeof(double) * ld, st, store32, P.n, ld, perm, b, x, ks);
+  launch_pdl(k_dense_solve_f32<float>, (P.n + 7) / 8, 256, sizeof(double) * ld, st, store32, P.n, ld, perm, b, x, ks);
 }
 
 }  // namespace vf

@@ -35,6 +35,7 @@ template <> struct V16<double> {
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_dot(long long n3, const T* __restrict__ a, const T* __restrict__ b,
                                                      double* partials, KrylovState* ks, int slot) {
+  pdl_enter();
   if (ks->done && slot != SLOT_FNORM && slot != SLOT_RZ_INIT && slot != SLOT_OUTER && slot != SLOT_PLAIN) return;
   using H = V16<T>;
   using V = typename H::V;
@@ -51,6 +52,7 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_cg_update(long long n3, T* __restrict__ x, const T* __restrict__ p,
                                                            T* __restrict__ r, const T* __restrict__ Ap,
                                                            double* partials, KrylovState* ks, double* hist) {
+  pdl_enter();
   if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
@@ -75,6 +77,7 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update(long long n3, T* __re
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_dot_fcg(long long n3, const T* __restrict__ r, const T* __restrict__ z,
                                                          const T* __restrict__ Ap, double* partials, KrylovState* ks) {
+  pdl_enter();
   if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
@@ -94,6 +97,7 @@ __global__ void __launch_bounds__(kVecThreads) k_dot_fcg(long long n3, const T* 
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_p_update(long long n3, T* __restrict__ p, const T* __restrict__ z,
                                                           const KrylovState* ks) {
+  pdl_enter();
   if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
@@ -116,6 +120,7 @@ __global__ void __launch_bounds__(kVecThreads) k_p_update(long long n3, T* __res
 __global__ void __launch_bounds__(kVecThreads) k_cg_update_split(long long n3, double* __restrict__ r,
                                                                  const double* __restrict__ Ap, float* __restrict__ r32,
                                                                  double* partials, KrylovState* ks, double* hist) {
+  pdl_enter();
   if (ks->done) return;
   const double alpha = ks->alpha;
   const long long n4 = n3 / 4;
@@ -142,6 +147,7 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update_split(long long n3, d
 __global__ void __launch_bounds__(kVecThreads) k_p_update_split(long long n3, double* __restrict__ x,
                                                                 double* __restrict__ p, const float* __restrict__ z,
                                                                 KrylovState* ks) {
+  pdl_enter();
   const int it = ks->it;
   const bool do_x = it > ks->x_it;
   const bool do_p = !ks->done;
@@ -187,6 +193,7 @@ __global__ void __launch_bounds__(kVecThreads) k_dot_fcg_split(long long n3, con
                                                                const float* __restrict__ z,
                                                                const double* __restrict__ Ap, double* partials,
                                                                KrylovState* ks) {
+  pdl_enter();
   if (ks->done) return;
   const long long n4 = n3 / 4;
   const float4* rv = reinterpret_cast<const float4*>(r);
@@ -211,6 +218,7 @@ __global__ void k_scale64(long long n3, const double* x, double* y, double sc) {
 template <typename T>
 __global__ void k_jacobi_precond(int n, const T* __restrict__ r, const T* __restrict__ minv,
                                  const uint8_t* __restrict__ mask, T* __restrict__ z, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     const uint8_t m = mask[p];
@@ -233,6 +241,7 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_update(long long n3, T* 
                                                                T* __restrict__ r, const T* __restrict__ Ap,
                                                                const T* __restrict__ minv, double* partials,
                                                                KrylovState* ks, double* hist) {
+  pdl_enter();
   if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
@@ -260,6 +269,7 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_jacobi_direction(long long n3, T* __restrict__ p,
                                                                   const T* __restrict__ r, const T* __restrict__ minv,
                                                                   const KrylovState* ks) {
+  pdl_enter();
   if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
@@ -277,6 +287,7 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_direction(long long n3, 
 
 template <typename T>
 __global__ void k_copy(long long n3, const T* __restrict__ s, T* __restrict__ d, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   const long long n16 = n3 * (long long)sizeof(T) / 16;   // 16-byte chunks
   const float4* sv = reinterpret_cast<const float4*>(s);
@@ -352,6 +363,7 @@ __global__ void k_power_init(long long n, T* __restrict__ x, const uint8_t* __re
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_power_norm(long long n3, const T* __restrict__ x, double* partials,
                                                             KrylovState* ks) {
+  pdl_enter();
   using H = V16<T>;
   using V = typename H::V;
   const long long nv = n3 / H::W;
@@ -365,7 +377,8 @@ __global__ void __launch_bounds__(kVecThreads) k_power_norm(long long n3, const 
 }
 
 template <typename T>
-__global__ void k_power_normalize(long long n, const T* y, T* x, const KrylovState* ks) {   // (in place)
+__global__ void k_power_normalize(long long n, const T* y, T* x, const KrylovState* ks) {
+  pdl_enter();   // (in place)
   const T inv = ks->rr > 0.0 ? (T)(1.0 / sqrt(ks->rr)) : (T)0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     x[i] = y[i] * inv;
@@ -424,11 +437,11 @@ void launch_power_init(const Grid& g, T* x, const uint8_t* mask, cudaStream_t st
 }
 template <typename T>
 void launch_power_norm(const Grid& g, const T* x, double* partials, KrylovState* ks, cudaStream_t st) {
-  launch_k(k_power_norm<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, partials, ks);
+  launch_pdl(k_power_norm<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, partials, ks);
 }
 template <typename T>
 void launch_power_normalize(const Grid& g, const T* y, T* x, const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_power_normalize<T>, vec_blocks(3LL * g.n), kVecThreads, 0, st, 3LL * g.n, y, x, ks);
+  launch_pdl(k_power_normalize<T>, vec_blocks(3LL * g.n), kVecThreads, 0, st, 3LL * g.n, y, x, ks);
 }
 #define VF_INST_POWER(T)                                                                                   \
   template void launch_power_init<T>(const Grid&, T*, const uint8_t*, cudaStream_t);                       \
@@ -444,38 +457,38 @@ void launch_power_omega(const KrylovState* ks, double omega_rel, double safety, 
 
 template <typename T>
 void launch_dot(const Grid& g, const T* a, const T* b, double* partials, KrylovState* ks, int slot, cudaStream_t st) {
-  launch_k(k_dot<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, a, b, partials, ks, slot);
+  launch_pdl(k_dot<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, a, b, partials, ks, slot);
 }
 template <typename T>
 void launch_cg_update(const Grid& g, T* x, const T* p, T* r, const T* Ap, double* partials, KrylovState* ks,
                       double* hist, cudaStream_t st) {
-  launch_k(k_cg_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, p, r, Ap, partials, ks, hist);
+  launch_pdl(k_cg_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, p, r, Ap, partials, ks, hist);
 }
 template <typename T>
 void launch_p_update(const Grid& g, T* p, const T* z, KrylovState* ks, cudaStream_t st) {
-  launch_k(k_p_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, p, z, ks);
+  launch_pdl(k_p_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, p, z, ks);
 }
 template <typename T>
 void launch_jacobi_precond(const Grid& g, const T* r, const T* minv3, const uint8_t* mask, T* z,
                            const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_jacobi_precond<T>, vec_blocks(g.n), kVecThreads, 0, st, g.n, r, minv3, mask, z, ks);
+  launch_pdl(k_jacobi_precond<T>, vec_blocks(g.n), kVecThreads, 0, st, g.n, r, minv3, mask, z, ks);
 }
 template <typename T>
 void launch_jacobi_update(const Grid& g, T* x, const T* p, T* r, const T* Ap, const T* minv3, double* partials,
                           KrylovState* ks, double* hist, cudaStream_t st) {
-  launch_k(k_jacobi_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, p, r, Ap, minv3,
+  launch_pdl(k_jacobi_update<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, x, p, r, Ap, minv3,
            partials, ks, hist);
 }
 template <typename T>
 void launch_jacobi_direction(const Grid& g, T* p, const T* r, const T* minv3, const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_jacobi_direction<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, p, r, minv3, ks);
+  launch_pdl(k_jacobi_direction<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, p, r, minv3, ks);
 }
 template <typename T>
 void launch_copy_vec(const Grid& g, const T* src, T* dst, const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_copy<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, src, dst, ks);
+  launch_pdl(k_copy<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, src, dst, ks);
 }
 void launch_norm2_f64(const Grid& g, const double* v, double* partials, KrylovState* ks, int slot, cudaStream_t st) {
-  launch_k(k_dot<double>, vec_blocks(3LL * g.n / 2), kVecThreads, 0, st, 3LL * g.n, v, v, partials, ks, slot);
+  launch_pdl(k_dot<double>, vec_blocks(3LL * g.n / 2), kVecThreads, 0, st, 3LL * g.n, v, v, partials, ks, slot);
 }
 void launch_ir_prepare(const Grid& g, const double* r64, float* r32, KrylovState* ks, cudaStream_t st) {
   launch_k(k_ir_prepare, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, r64, r32, ks);
@@ -505,14 +518,14 @@ void launch_sub_from(const Grid& g, const double* f, double* r, cudaStream_t st)
 
 void launch_cg_update_split(const Grid& g, double* r, const double* Ap, float* r32, double* partials,
                             KrylovState* ks, double* hist, cudaStream_t st) {
-  launch_k(k_cg_update_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, r, Ap, r32, partials, ks, hist);
+  launch_pdl(k_cg_update_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, r, Ap, r32, partials, ks, hist);
 }
 void launch_p_update_split(const Grid& g, double* x, double* p, const float* z, KrylovState* ks, cudaStream_t st) {
-  launch_k(k_p_update_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, x, p, z, ks);
+  launch_pdl(k_p_update_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, x, p, z, ks);
 }
 void launch_dot_fcg_split(const Grid& g, const float* r, const float* z, const double* Ap, double* partials,
                           KrylovState* ks, cudaStream_t st) {
-  launch_k(k_dot_fcg_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
+  launch_pdl(k_dot_fcg_split, vec_blocks(3LL * g.n / 4), kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
 }
 void launch_scale64(const Grid& g, const double* x, double* y, double sc, cudaStream_t st) {
   launch_k(k_scale64, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, x, y, sc);
@@ -521,7 +534,7 @@ void launch_scale64(const Grid& g, const double* x, double* y, double sc, cudaSt
 template <typename T>
 void launch_dot_fcg(const Grid& g, const T* r, const T* z, const T* Ap, double* partials, KrylovState* ks,
                     cudaStream_t st) {
-  launch_k(k_dot_fcg<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
+  launch_pdl(k_dot_fcg<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, r, z, Ap, partials, ks);
 }
 
 #define VF_INST(T)                                                                                            \

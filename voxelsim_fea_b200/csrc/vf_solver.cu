@@ -432,8 +432,7 @@ void prolong_level(vf_solver* s, int li, const T* ec, T* x, KrylovState* ks) {
     return;
   }
   T* t = Sel<T>::w(l, 1);
-  cudaMemsetAsync(t, 0, sizeof(T) * 3 * (size_t)l.g.n, s->st);
-  launch_prolong_add<T>(c.g, ec, l.g, l.mask, t, ks, s->st);
+  launch_prolong_set<T>(c.g, ec, l.g, l.mask, t, ks, s->st);
   SweepStep st;
   st.omega_dev = s->d_spc + li;
   st.c1_dev = s->d_one;
@@ -529,8 +528,7 @@ void learned_stage(vf_solver* s, const T* r, T* z, KrylovState* ks) {
     Level& cl = s->L[li];
     Level& f = s->L[li - 1];
     T* target = (li == 1) ? c : Sel<T>::w(f, 0);
-    cudaMemsetAsync(target, 0, sizeof(T) * 3 * (size_t)f.g.n, s->st);
-    launch_prolong_add<T>(cl.g, Sel<T>::w(cl, 0), f.g, f.mask, target, ks, s->st);
+    launch_prolong_set<T>(cl.g, Sel<T>::w(cl, 0), f.g, f.mask, target, ks, s->st);
   }
   level_op<T>(s, 0, EPI_APPLY, c, Ac, nullptr, kk, s->d_partials, SLOT_GDEN);
   launch_dot<T>(l0.g, c, r1, s->d_partials, kk, SLOT_GNUM, s->st);

@@ -17,6 +17,7 @@ namespace {
 __global__ void __launch_bounds__(256) k_restrict_d(Grid f, const double* __restrict__ rf, Grid c,
                                                     const uint8_t* __restrict__ cm, double* __restrict__ rc,
                                                     const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   const int nx1 = c.lx + 1, ny1 = c.ly + 1, nint = nx1 * ny1 * (c.lz + 1);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += gridDim.x * blockDim.x) {
@@ -43,6 +44,7 @@ __global__ void __launch_bounds__(256) k_restrict_d(Grid f, const double* __rest
 __global__ void __launch_bounds__(256) k_restrict_f(Grid f, const float* __restrict__ rf, Grid c,
                                                     const uint8_t* __restrict__ cm, float* __restrict__ rc,
                                                     const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   const int nx1 = c.lx + 1, ny1 = c.ly + 1, nint = nx1 * ny1 * (c.lz + 1);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += gridDim.x * blockDim.x) {
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(256) k_restrict_first(Grid f, const T* __restr
                                                         const uint8_t* __restrict__ cm, T* __restrict__ rc,
                                                         const T* __restrict__ minvc, const double* __restrict__ wdev,
                                                         T* __restrict__ uc, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   const T w = (T)(*wdev);
   const int nx1 = c.lx + 1, ny1 = c.ly + 1, nint = nx1 * ny1 * (c.lz + 1);
@@ -130,42 +133,7 @@ __global__ void __launch_bounds__(256) k_restrict_first(Grid f, const T* __restr
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_prolong_add(Grid c, const T* __restrict__ ec, Grid f,
-                                                     const uint8_t* __restrict__ fm, T* __restrict__ uf,
-                                                     const KrylovState* ks) {
-  if (ks && ks->done) return;
-  const int nx1 = f.lx + 1, ny1 = f.ly + 1, nint = nx1 * ny1 * (f.lz + 1);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += gridDim.x * blockDim.x) {
-    const int x = t % nx1, rr = t / nx1, y = rr % ny1, z = rr / ny1;
-    const int p = f.idx(x, y, z);
-    const uint8_t m = fm[p];
-    if (!m) continue;
-    // all eight coarse corners, weight 0 on the unused ones: the loads are
-    // independent (one latency) and x0+1 <= c.lx+1 stays on the padded grid
-    const int x0 = x >> 1, y0 = y >> 1, z0 = z >> 1;
-    const T wx[2] = {(x & 1) ? (T)0.5 : (T)1, (x & 1) ? (T)0.5 : (T)0};
-    const T wy[2] = {(y & 1) ? (T)0.5 : (T)1, (y & 1) ? (T)0.5 : (T)0};
-    const T wz[2] = {(z & 1) ? (T)0.5 : (T)1, (z & 1) ? (T)0.5 : (T)0};
-    T e0 = 0, e1 = 0, e2 = 0;
-#pragma unroll
-    for (int kz = 0; kz < 2; ++kz)
-#pragma unroll
-      for (int ky = 0; ky < 2; ++ky)
-#pragma unroll
-        for (int kx = 0; kx < 2; ++kx) {
-          const T w = wx[kx] * wy[ky] * wz[kz];
-          const long long q = 3 * (long long)c.idx(x0 + kx, y0 + ky, z0 + kz);
-          e0 += w * __ldg(ec + q); e1 += w * __ldg(ec + q + 1); e2 += w * __ldg(ec + q + 2);
-        }
-    const long long p3 = 3 * (long long)p;
-    if (m & 1) uf[p3] += e0;
-    if (m & 2) uf[p3 + 1] += e1;
-    if (m & 4) uf[p3 + 2] += e2;
-  }
-}
-
-// The same prolongation, four consecutive storage nodes of a row per thread:
+// Prolongation, four consecutive storage nodes of a row per thread:
 // their 12 values are 48 contiguous, 16-byte aligned bytes (px is a multiple
 // of 4), read and written as whole vectors.
 template <typename T> struct Vec12;
@@ -202,10 +170,12 @@ template <> struct Vec12<double> {
 // only where a weight is non-zero (an even fine coordinate has one parent on
 // that axis).  The sums keep the order of the 8-corner loop over (kz, ky, kx)
 // with the zero-weight terms left out, which does not change them.
-template <typename T>
+// SET: u = P e instead of u += P e (zero on the DOFs that are not free).
+template <typename T, bool SET>
 __global__ void __launch_bounds__(256) k_prolong_add4(Grid c, const T* __restrict__ ec, Grid f,
                                                       const uint8_t* __restrict__ fm, T* __restrict__ uf,
                                                       const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   const int gpr = f.px / 4;                        // 4-node groups per storage row
   const long long ngroups = (long long)gpr * (f.ly + 1) * (f.lz + 1);
@@ -216,9 +186,14 @@ __global__ void __launch_bounds__(256) k_prolong_add4(Grid c, const T* __restric
     const int y = (int)(rr % (f.ly + 1)), z = (int)(rr / (f.ly + 1));
     const int p0 = f.idx(-1, y, z) + 4 * gx;        // storage x = 4 gx .. 4 gx + 3
     const uint32_t m4 = *reinterpret_cast<const uint32_t*>(fm + p0);
-    if (!m4) continue;
+    if (!SET && !m4) continue;
     Vec12<T> u;
-    u.load(uf + 3LL * p0);
+    if (SET) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) u.at(k) = (T)0;
+    } else {
+      u.load(uf + 3LL * p0);
+    }
     const int y0 = y >> 1, z0 = z >> 1;
     const int ny = (y & 1) ? 2 : 1, nz = (z & 1) ? 2 : 1;
     const T wy[2] = {(y & 1) ? (T)0.5 : (T)1, (y & 1) ? (T)0.5 : (T)0};
@@ -272,6 +247,7 @@ template <typename T>
 __global__ void k_jacobi_from_zero(Grid g, const T* __restrict__ b, const T* __restrict__ minv,
                                    const uint8_t* __restrict__ mask, T w0, const double* __restrict__ wdev,
                                    T* __restrict__ u, const KrylovState* ks) {
+  pdl_enter();
   if (ks && ks->done) return;
   const T w = wdev ? (T)(*wdev) : w0;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < g.n; p += gridDim.x * blockDim.x) {
@@ -294,18 +270,18 @@ inline int blocks_for(long long n) {
 template <>
 void launch_restrict<double>(const Grid& f, const double* rf, const Grid& c, const uint8_t* cmask, double* rc,
                              const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_restrict_d, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c, cmask, rc, ks);
+  launch_pdl(k_restrict_d, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c, cmask, rc, ks);
 }
 template <>
 void launch_restrict<float>(const Grid& f, const float* rf, const Grid& c, const uint8_t* cmask, float* rc,
                             const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_restrict_f, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c, cmask, rc, ks);
+  launch_pdl(k_restrict_f, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c, cmask, rc, ks);
 }
 
 template <typename T>
 void launch_restrict_first(const Grid& f, const T* rf, const Grid& c, const uint8_t* cmask, T* rc, const T* minvc,
                            const double* wdev, T* uc, const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_restrict_first<T>, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c,
+  launch_pdl(k_restrict_first<T>, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c,
            cmask, rc, minvc, wdev, uc, ks);
 }
 template void launch_restrict_first<float>(const Grid&, const float*, const Grid&, const uint8_t*, float*,
@@ -316,16 +292,24 @@ template void launch_restrict_first<double>(const Grid&, const double*, const Gr
 template <typename T>
 void launch_prolong_add(const Grid& c, const T* ec, const Grid& f, const uint8_t* fmask, T* uf,
                         const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_prolong_add4<T>, blocks_for((long long)(f.px / 4) * (f.ly + 1) * (f.lz + 1)), 256, 0, st, c, ec, f, fmask,
-           uf, ks);
+  launch_pdl(k_prolong_add4<T, false>, blocks_for((long long)(f.px / 4) * (f.ly + 1) * (f.lz + 1)), 256, 0, st, c, ec, f,
+             fmask, uf, ks);
+}
+template <typename T>
+void launch_prolong_set(const Grid& c, const T* ec, const Grid& f, const uint8_t* fmask, T* uf,
+                        const KrylovState* ks, cudaStream_t st) {
+  launch_pdl(k_prolong_add4<T, true>, blocks_for((long long)(f.px / 4) * (f.ly + 1) * (f.lz + 1)), 256, 0, st, c, ec, f,
+             fmask, uf, ks);
 }
 
 template <typename T>
 void launch_jacobi_from_zero(const Grid& g, const T* b, const T* minv3, const uint8_t* mask, double omega,
                              const double* omega_dev, T* u, const KrylovState* ks, cudaStream_t st) {
-  launch_k(k_jacobi_from_zero<T>, blocks_for(g.n), 256, 0, st, g, b, minv3, mask, (T)omega, omega_dev, u, ks);
+  launch_pdl(k_jacobi_from_zero<T>, blocks_for(g.n), 256, 0, st, g, b, minv3, mask, (T)omega, omega_dev, u, ks);
 }
 
+template void launch_prolong_set<double>(const Grid&, const double*, const Grid&, const uint8_t*, double*, const KrylovState*, cudaStream_t);
+template void launch_prolong_set<float>(const Grid&, const float*, const Grid&, const uint8_t*, float*, const KrylovState*, cudaStream_t);
 template void launch_prolong_add<double>(const Grid&, const double*, const Grid&, const uint8_t*, double*, const KrylovState*, cudaStream_t);
 template void launch_prolong_add<float>(const Grid&, const float*, const Grid&, const uint8_t*, float*, const KrylovState*, cudaStream_t);
 template void launch_jacobi_from_zero<double>(const Grid&, const double*, const double*, const uint8_t*, double, const double*, double*, const KrylovState*, cudaStream_t);

@@ -677,6 +677,7 @@ struct WideBlocks {
 template <typename T, typename S, int R, int EPI>
 __global__ void __launch_bounds__(128) k_wide_op(Grid g, OpArgs a, const S* __restrict__ stc,
                                                  const T* __restrict__ sqd) {
+  pdl_enter();
   using L = WideLayout<S, R>;
   using A = typename std::conditional<sizeof(T) == 8, double, float>::type;
   constexpr int G = L::G;
@@ -830,9 +831,9 @@ template void launch_wide_compress<double, 2>(const Grid&, const double*, const 
 template <typename T, typename S, int R>
 void launch_wide_op(const Grid& g, int epi, const OpArgs& a, const S* stc, const T* sqrtd, cudaStream_t st) {
   const int blocks = wide_op_grid_blocks(g);
-  if (epi == EPI_APPLY) launch_k(k_wide_op<T, S, R, EPI_APPLY>, blocks, 128, 0, st, g, a, stc, sqrtd);
-  else if (epi == EPI_SMOOTH) launch_k(k_wide_op<T, S, R, EPI_SMOOTH>, blocks, 128, 0, st, g, a, stc, sqrtd);
-  else launch_k(k_wide_op<T, S, R, EPI_RESID>, blocks, 128, 0, st, g, a, stc, sqrtd);
+  if (epi == EPI_APPLY) launch_pdl(k_wide_op<T, S, R, EPI_APPLY>, blocks, 128, 0, st, g, a, stc, sqrtd);
+  else if (epi == EPI_SMOOTH) launch_pdl(k_wide_op<T, S, R, EPI_SMOOTH>, blocks, 128, 0, st, g, a, stc, sqrtd);
+  else launch_pdl(k_wide_op<T, S, R, EPI_RESID>, blocks, 128, 0, st, g, a, stc, sqrtd);
 }
 template void launch_wide_op<float, __half, 2>(const Grid&, int, const OpArgs&, const __half*, const float*, cudaStream_t);
 template void launch_wide_op<float, float, 2>(const Grid&, int, const OpArgs&, const float*, const float*, cudaStream_t);
