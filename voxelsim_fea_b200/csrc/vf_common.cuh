@@ -16,7 +16,6 @@
 #include <stdint.h>
 
 #include <atomic>
-#include <cstdlib>
 #include <string>
 #include <type_traits>
 #include <utility>
@@ -40,17 +39,19 @@ inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
 // kernel that calls pdl_enter() first may be launched with launch_pdl: it is
 // then scheduled while its predecessor in the stream (or graph) still runs and
 // waits in pdl_enter() for that to complete, so its launch and ramp are not
-// added to the chain.  Only grids that fit the device beside what is running
-// do this: the early blocks of a long kernel would hold slots that the
-// predecessor's last wave needs (measured on the 256x128x128 bracket with
-// every kernel launched early: 0.337 -> 0.379 s).
+// added to the chain.  Only grids of at most a block per SM do this: the early
+// blocks of larger ones are packed onto the SMs that drain first and hold
+// slots that the predecessor's last wave needs.  Per iteration, none / up to
+// 148 / up to 300 blocks early: 64x32x32 195 / 183 / 185 us, 96x80x64 323 /
+// 315 / 337, 128x64x64 FP64 539 / 533 / 641; the 64x16x16 reference solve
+// 5.42 / 4.96 / 4.96 ms.
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
 }
-inline long long pdl_blocks() { static long long v = getenv("VF_PDL") ? atoi(getenv("VF_PDL")) : 64; return v; }
+constexpr long long kPdlBlocks = 148;   // one block per SM at most
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-  if ((long long)grid.x * grid.y * grid.z > pdl_blocks()) {
+  if ((long long)grid.x * grid.y * grid.z > kPdlBlocks) {
     launch_k(kern, grid, block, smem, st, std::forward<Args>(args)...);
     return;
   }
