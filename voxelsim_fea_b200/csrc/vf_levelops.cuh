@@ -1,0 +1,130 @@
+// Device pieces shared by the kernels that apply assembled Galerkin levels
+// (vf_stencil.cu, vf_wide.cu): 16-byte chunks of the symmetric
+// scaled storages and the rows of a reach-R operator.
+#pragma once
+
+#include <cuda_fp16.h>
+#include <string.h>
+
+#include "vf_common.cuh"
+
+namespace vf {
+
+__device__ __forceinline__ bool inside(const Grid& g, int x, int y, int z) {
+  return x >= 0 && x <= g.lx && y >= 0 && y <= g.ly && z >= 0 && z <= g.lz;
+}
+
+// position of value k < 6 of SymLayout in the diagonal block
+__host__ __device__ constexpr int diag_r(int k) { return k < 3 ? 0 : (k < 5 ? 1 : 2); }
+__host__ __device__ constexpr int diag_c(int k) { return k < 3 ? k : (k < 5 ? k - 2 : 2); }
+
+// One 16-byte chunk of stencil values, unpacked to the accumulation type.
+template <typename S, typename A> struct Chunk;
+template <> struct Chunk<__half, float> {
+  float v[8];
+  __device__ __forceinline__ void load(const __half* base) {
+    const uint4 w = __ldg(reinterpret_cast<const uint4*>(base));
+    const unsigned ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      __half2 h;
+      memcpy(&h, &ws[i], 4);
+      const float2 f = __half22float2(h);
+      v[2 * i] = f.x; v[2 * i + 1] = f.y;
+    }
+  }
+};
+template <> struct Chunk<float, float> {
+  float v[4];
+  __device__ __forceinline__ void load(const float* base) {
+    const float4 w = __ldg(reinterpret_cast<const float4*>(base));
+    v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+  }
+};
+template <> struct Chunk<double, double> {
+  double v[2];
+  __device__ __forceinline__ void load(const double* base) {
+    const double2 w = __ldg(reinterpret_cast<const double2*>(base));
+    v[0] = w.x; v[1] = w.y;
+  }
+};
+
+// ---- rows of a reach-R operator (WideLayout) --------------------------------
+// The linear storage offset of upper block u (positive), or 0 for the diagonal
+// block and the padding slots past it.
+template <typename L>
+__device__ __forceinline__ int wide_shift(const Grid& g, int u) {
+  constexpr int R = (L::W - 1) / 2, W = L::W, SC = L::NB / 2;
+  if (u >= L::NU) return 0;
+  const int s = SC + 1 + u;
+  return ((s / (W * W) - R) * g.py + (s / W) % W - R) * g.px + s % W - R;
+}
+
+__device__ __forceinline__ uint4 ldg_chunk(const void* p) {
+  // volatile: a batch's loads stay together, ahead of its arithmetic
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+template <typename S, typename A> __device__ __forceinline__ A chunk_value(const uint4& c, int i);
+template <> __device__ __forceinline__ float chunk_value<__half, float>(const uint4& c, int i) {
+  const unsigned w = i < 2 ? c.x : (i < 4 ? c.y : (i < 6 ? c.z : c.w));
+  __half2 h;
+  memcpy(&h, &w, 4);
+  return (i & 1) ? __high2float(h) : __low2float(h);
+}
+template <> __device__ __forceinline__ float chunk_value<float, float>(const uint4& c, int i) {
+  return __uint_as_float(i == 0 ? c.x : (i == 1 ? c.y : (i == 2 ? c.z : c.w)));
+}
+template <> __device__ __forceinline__ double chunk_value<double, double>(const uint4& c, int i) {
+  return i == 0 ? __hiloint2double((int)c.y, (int)c.x) : __hiloint2double((int)c.w, (int)c.z);
+}
+
+// acc (the rows of node p) += the blocks of lane `lane` (of L::G lanes): own
+// block u = lane + G*JJ applied to node p + shift, and the transposed block u
+// of node p - shift (lane and slot are the same there).  V(shift, up, v) gives
+// D^1/2 u of those nodes: ghost and pad nodes hold zeros, and a reach-2
+// neighbour past the shell lands, in linear storage, on a ghost or pad node of
+// the next row or plane or outside the array (zero as well), so no neighbour
+// needs a test; only the address of the transposed block is kept in the array.
+// The loads of JB slots stand together, ahead of their products.
+template <typename S> struct WideBatch { static constexpr int JB = sizeof(S) == 2 ? 4 : 2; };
+template <typename S, typename A, typename L, int J0 = 0, typename SH, typename VF>
+__device__ __forceinline__ void wide_rows(const S* __restrict__ stc, int p, int lane, A (&acc)[3], SH shift_of, VF V) {
+  constexpr int VPC = L::VPC, JB = WideBatch<S>::JB;
+  constexpr int C0 = 9 * J0 / VPC, C1 = (9 * (J0 + JB) - 1) / VPC;      // own chunks of the batch
+  constexpr int ND = (9 + VPC - 1) / VPC + 1;                           // chunks a block may straddle
+  const S* own = stc + L::off((long long)p * L::G + lane, 0);
+  uint4 co[C1 - C0 + 1], cd[JB][ND];
+  int sh[JB];
+#pragma unroll
+  for (int j = 0; j < JB; ++j) sh[j] = shift_of(lane + L::G * (J0 + j));
+#pragma unroll
+  for (int c = C0; c <= C1; ++c) co[c - C0] = ldg_chunk(own + c * 32 * VPC);
+#pragma unroll
+  for (int j = 0; j < JB; ++j) {
+    const int k0 = 9 * (J0 + j), q = p - sh[j];
+    const S* base = stc + L::off((long long)(q < 0 ? 0 : q) * L::G + lane, 0);
+#pragma unroll
+    for (int c = 0; c < ND; ++c)
+      if (k0 / VPC + c <= (k0 + 8) / VPC) cd[j][c] = ldg_chunk(base + (k0 / VPC + c) * 32 * VPC);
+  }
+#pragma unroll
+  for (int j = 0; j < JB; ++j) {
+    const int k0 = 9 * (J0 + j);
+    A vu[3], vd[3];
+    V(sh[j], vu, vd);
+    if (lane + L::G * (J0 + j) >= L::NU) vd[0] = vd[1] = vd[2] = (A)0;   // the diagonal block is applied once
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int k = k0 + 3 * r + c;
+        acc[r] += chunk_value<S, A>(co[k / VPC - C0], k % VPC) * vu[c];
+        acc[c] += chunk_value<S, A>(cd[j][k / VPC - k0 / VPC], k % VPC) * vd[r];
+      }
+  }
+  if constexpr (J0 + JB < L::NJ) wide_rows<S, A, L, J0 + JB>(stc, p, lane, acc, shift_of, V);
+}
+
+}  // namespace vf

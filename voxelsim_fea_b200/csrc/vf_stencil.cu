@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "vf_common.cuh"
+#include "vf_levelops.cuh"
 #include "vf_reduce.cuh"
 
 namespace vf {
@@ -484,8 +485,6 @@ template <typename S> __device__ __forceinline__ S st_from(double v);
 template <> __device__ __forceinline__ float st_from<float>(double v) { return (float)v; }
 template <> __device__ __forceinline__ double st_from<double>(double v) { return v; }
 template <> __device__ __forceinline__ __half st_from<__half>(double v) { return __double2half(v); }
-__host__ __device__ constexpr int diag_r(int k) { return k < 3 ? 0 : (k < 5 ? 1 : 2); }
-__host__ __device__ constexpr int diag_c(int k) { return k < 3 ? k : (k < 5 ? k - 2 : 2); }
 
 template <typename S>
 __global__ void k_stencil_compress(Grid g, const double* __restrict__ st, const uint8_t* __restrict__ mask,
@@ -526,37 +525,6 @@ __global__ void k_stencil_compress(Grid g, const double* __restrict__ st, const 
     for (int k = 123; k < 128; ++k) stc[L::off(p, k)] = st_from<S>(0.0);
   }
 }
-
-// One 16-byte chunk of stencil values, unpacked to the accumulation type.
-template <typename S, typename A> struct Chunk;
-template <> struct Chunk<__half, float> {
-  float v[8];
-  __device__ __forceinline__ void load(const __half* base) {
-    const uint4 w = __ldg(reinterpret_cast<const uint4*>(base));
-    const unsigned ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      __half2 h;
-      memcpy(&h, &ws[i], 4);
-      const float2 f = __half22float2(h);
-      v[2 * i] = f.x; v[2 * i + 1] = f.y;
-    }
-  }
-};
-template <> struct Chunk<float, float> {
-  float v[4];
-  __device__ __forceinline__ void load(const float* base) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(base));
-    v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
-  }
-};
-template <> struct Chunk<double, double> {
-  double v[2];
-  __device__ __forceinline__ void load(const double* base) {
-    const double2 w = __ldg(reinterpret_cast<const double2*>(base));
-    v[0] = w.x; v[1] = w.y;
-  }
-};
 
 constexpr int SX = 32, SY = 8;   // node tile of the marching stencil kernel
 

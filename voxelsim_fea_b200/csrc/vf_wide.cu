@@ -36,13 +36,13 @@
 // blocks s > center (9 values each) of A~ = D^-1/2 A D^-1/2, FP16 for the
 // FP32 V-cycle, warp-chunked so a warp loads one 16-byte chunk of 32
 // consecutive nodes at once; the lower blocks are read transposed from the
-// neighbour that stores them.  One thread per padded node; the vector is read
-// through the L1 (the coarse levels are small).
+// neighbour that stores them.
 #include <cuda_fp16.h>
 
 #include <type_traits>
 
 #include "vf_common.cuh"
+#include "vf_levelops.cuh"
 #include "vf_reduce.cuh"
 
 namespace vf {
@@ -56,10 +56,6 @@ __host__ __device__ constexpr int wide_nb(int R) { return (2 * R + 1) * (2 * R +
 __device__ __forceinline__ double tw(int d) { return d == 0 ? 1.0 : ((d == 1 || d == -1) ? 0.5 : 0.0); }
 // ceil(v / 2) for any sign
 __device__ __forceinline__ int ceil_half(int v) { return v >= 0 ? (v + 1) / 2 : -((-v) / 2); }
-
-__device__ __forceinline__ bool inside(const Grid& g, int x, int y, int z) {
-  return x >= 0 && x <= g.lx && y >= 0 && y <= g.ly && z >= 0 && z <= g.lz;
-}
 
 __device__ __forceinline__ void interior_xyz(const Grid& g, long long t, int& x, int& y, int& z) {
   const int nx1 = g.lx + 1, ny1 = g.ly + 1;
@@ -585,151 +581,122 @@ __global__ void k_wide_compress(Grid g, const double* __restrict__ st, const uin
   }
 }
 
-// One 16-byte chunk, unpacked to the accumulation type.
-template <typename S, typename A> struct WChunk;
-template <> struct WChunk<__half, float> {
-  float v[8];
-  __device__ __forceinline__ void load(const __half* base) {
-    const uint4 w = __ldg(reinterpret_cast<const uint4*>(base));
-    const unsigned ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      __half2 h;
-      memcpy(&h, &ws[i], 4);
-      const float2 f = __half22float2(h);
-      v[2 * i] = f.x;
-      v[2 * i + 1] = f.y;
-    }
-  }
-};
-template <> struct WChunk<float, float> {
-  float v[4];
-  __device__ __forceinline__ void load(const float* base) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(base));
-    v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
-  }
-};
-template <> struct WChunk<double, double> {
-  double v[2];
-  __device__ __forceinline__ void load(const double* base) {
-    const double2 w = __ldg(reinterpret_cast<const double2*>(base));
-    v[0] = w.x; v[1] = w.y;
-  }
-};
-
-// The 9 values of slot jj of virtual node v (chunks straddled as needed).
-template <typename S, typename A, typename L, int JJ>
-__device__ __forceinline__ void load_block(const S* __restrict__ stc, long long v, A (&blk)[9]) {
-  constexpr int VPC = L::VPC, K0 = 9 * JJ;
-#pragma unroll
-  for (int j = K0 / VPC; j <= (K0 + 8) / VPC; ++j) {
-    WChunk<S, A> ch;
-    ch.load(stc + L::off(v, j * VPC));
-#pragma unroll
-    for (int i = 0; i < VPC; ++i) {
-      const int k = j * VPC + i;
-      if (k >= K0 && k < K0 + 9) blk[k - K0] = ch.v[i];
-    }
-  }
-}
-
-template <typename S, typename A, typename L, int JJ>
-struct WideBlocks {
-  // acc (this node's rows) += own block u = lane + G*JJ applied to the
-  // neighbour p + off(s); for an upper block also the transposed upper block
-  // u of the node p - off(s) (lane and slot are the same there).
-  template <typename VF>
-  __device__ __forceinline__ static void run(const S* __restrict__ stc, const Grid& g, int p, int lane, int x, int y,
-                                             int z, A (&acc)[3], VF V) {
-    constexpr int R = (L::W - 1) / 2, W = L::W, SC = L::NB / 2;
-    const int u = lane + L::G * JJ;
-    if (u < L::NBLK) {
-      const int s = (u == L::NU) ? SC : SC + 1 + u;
-      const int dx = s % W - R, dy = (s / W) % W - R, dz = s / (W * W) - R;
-      const long long v = (long long)p * L::G + lane;
-      if (inside(g, x + dx, y + dy, z + dz)) {
-        const int q = g.idx(x + dx, y + dy, z + dz);
-        A blk[9];
-        load_block<S, A, L, JJ>(stc, v, blk);
-        const A v0 = V(q, 0), v1 = V(q, 1), v2 = V(q, 2);
-#pragma unroll
-        for (int r = 0; r < 3; ++r) acc[r] += blk[3 * r] * v0 + blk[3 * r + 1] * v1 + blk[3 * r + 2] * v2;
-      }
-      if (u < L::NU && inside(g, x - dx, y - dy, z - dz)) {
-        const int q = g.idx(x - dx, y - dy, z - dz);
-        A blk[9];
-        load_block<S, A, L, JJ>(stc, (long long)q * L::G + lane, blk);
-        const A w0 = V(q, 0), w1 = V(q, 1), w2 = V(q, 2);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc[c] += blk[c] * w0 + blk[3 + c] * w1 + blk[6 + c] * w2;
-      }
-    }
-    if constexpr (JJ + 1 < L::NJ) WideBlocks<S, A, L, JJ + 1>::run(stc, g, p, lane, x, y, z, acc, V);
-  }
-};
-
 // y = mask(D^1/2 A~ D^1/2 u) with the epilogues of the other level kernels
 // (APPLY, SMOOTH with the Chebyshev step fields, RESID; a null rhs reads as
-// zero).  G = 8 lanes per node: each lane applies its own blocks and the
-// transposed blocks of the same lane and slot of the lower neighbours, the
-// partial sums meet through warp shuffles, and lanes 0..2 write component
-// 0..2 of the node.
+// zero; no fused dot product: the PCG's reductions run on level 0).  G = 8
+// lanes per node: each lane applies its own blocks and the transposed blocks
+// of the same lane and slot of the lower neighbours, the partial sums meet
+// through warp shuffles, and lanes 0..2 write component 0..2 of the node.
+//
+// A CTA owns 16 nodes of a row, one round of its threads: it stages v = D^1/2 u
+// of them and their reach-2 halo in shared memory with one set of loads, and
+// the operator's loads depend on no branch and no table in global memory
+// (wide_rows).  Bound by the latency of those loads on small levels and by the
+// L1 on large ones.  Against a form that walked the 8 block slots of a lane
+// behind bounds tests and read u and the scale from global memory at every
+// neighbour: 64x32x32 part 185 -> 165 us an iteration, 96x80x64 315 -> 303,
+// 128x64x64 FP64 534 -> 520, 256x128x128 1,401 -> 1,381.  Larger tiles (16 x 2 x 2,
+// 16 x 4 x 4 nodes, several rounds) were no faster at any size: fewer CTAs to
+// hide the loads.
+template <typename T> struct Node3;   // 3 values of a node in shared memory
+template <> struct Node3<float> {
+  float4 v;
+  __device__ __forceinline__ void get(float (&o)[3]) const { const float4 t = v; o[0] = t.x; o[1] = t.y; o[2] = t.z; }
+  __device__ __forceinline__ void set(float a, float b, float c) { v = make_float4(a, b, c, 0.f); }
+};
+template <> struct Node3<double> {
+  double v[3];
+  __device__ __forceinline__ void get(double (&o)[3]) const { o[0] = v[0]; o[1] = v[1]; o[2] = v[2]; }
+  __device__ __forceinline__ void set(double a, double b, double c) { v[0] = a; v[1] = b; v[2] = c; }
+};
+constexpr int kWideTX = 16;
+
 template <typename T, typename S, int R, int EPI>
-__global__ void __launch_bounds__(128) k_wide_op(Grid g, OpArgs a, const S* __restrict__ stc,
-                                                 const T* __restrict__ sqd) {
+__global__ void __launch_bounds__(kWideTX * 8)
+    k_wide_op(Grid g, OpArgs a, const S* __restrict__ stc, const T* __restrict__ sqd) {
   pdl_enter();
   using L = WideLayout<S, R>;
-  using A = typename std::conditional<sizeof(T) == 8, double, float>::type;
-  constexpr int G = L::G;
+  using A = T;
+  constexpr int G = L::G, TX = kWideTX, HX = TX + 2 * R, HY = 1 + 2 * R, HZ = 1 + 2 * R, NT = TX * G;
+  __shared__ Node3<T> sv[HX * HY * HZ];
+  __shared__ int s_shift[G * L::NJ], s_delta[G * L::NJ];
   KrylovState* ks = a.ks;
   if (ks && ks->done) return;
   const T* __restrict__ u = (const T*)a.u;
   T* out = (T*)a.out;
   const T* b = (const T*)a.b;
-  const T* __restrict__ minv = (const T*)a.minv;
-  const uint8_t* __restrict__ mask = a.mask;
+  const T* __restrict__ minv = (const T*)(EPI == EPI_APPLY ? a.apply_minv : a.minv);
   const T w = a.omega_dev ? (T)(*a.omega_dev) : (T)a.omega;
   const T* dprev = (const T*)a.dprev;
   T* dout = (T*)a.dout;
   const T c1 = a.c1_dev ? (T)(*a.c1_dev) : (T)0;
-  auto V = [&](int q, int c) -> A { return (A)__ldg(sqd + 3LL * q + c) * (A)__ldg(u + 3LL * q + c); };
-  double dot = 0.0;
-  // whole warps iterate together (the shuffles need every lane)
-  const long long nv = ((long long)g.n * G + 31) / 32 * 32;
-  for (long long vv = blockIdx.x * (long long)blockDim.x + threadIdx.x; vv < nv;
-       vv += (long long)gridDim.x * blockDim.x) {
-    const int p = (int)(vv / G), lane = (int)(vv % G);
-    int x = -1, y = -1, z = -1;
-    if (p < g.n) decode(g, p, x, y, z);
-    const bool in = p < g.n && inside(g, x, y, z);
-    const uint8_t m = in ? mask[p] : (uint8_t)0;
-    A acc[3] = {(A)0, (A)0, (A)0};
-    if (m) WideBlocks<S, A, L, 0>::run(stc, g, p, lane, x, y, z, acc, V);
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    }
-    if (!in || lane >= 3) continue;
-    const int c = lane;
-    const long long pc = 3LL * p + c;
-    const A ac = c == 0 ? acc[0] : (c == 1 ? acc[1] : acc[2]);
-    const T kc = ((m >> c) & 1) ? (T)(ac * (A)sqd[pc]) : (T)0;
-    const T bc = b ? b[pc] : (T)0;
-    if (EPI == EPI_APPLY) {
-      out[pc] = a.apply_minv ? kc * __ldg((const T*)a.apply_minv + pc) : kc;
-      if (a.dot_partials) dot += (double)u[pc] * (double)kc;
-    } else if (EPI == EPI_SMOOTH) {
-      const T u0 = u[pc];
-      T o = u0 + (((m >> c) & 1) ? w * (minv[pc] * (bc - kc)) : (T)0);
-      if (dprev) o += c1 * dprev[pc];
-      out[pc] = o;
-      if (dout) dout[pc] = o - u0;
-    } else {
-      out[pc] = bc - kc;
-    }
+  const int ntx = (g.lx + TX) / TX;
+  const int X0 = (blockIdx.x % ntx) * TX, y = blockIdx.x / ntx % (g.ly + 1), z = blockIdx.x / (ntx * (g.ly + 1));
+  if (threadIdx.x < G * L::NJ) {
+    constexpr int W = L::W, SC = L::NB / 2;
+    const int uu = threadIdx.x, s = uu < L::NU ? SC + 1 + uu : SC;
+    s_shift[uu] = wide_shift<L>(g, uu);
+    s_delta[uu] = ((s / (W * W) - R) * HY + (s / W) % W - R) * HX + s % W - R;
   }
-  if (EPI == EPI_APPLY && a.dot_partials && ks) reduce_and_finalize(dot, a.dot_partials, ks, a.dot_slot, nullptr);
+  // halo nodes outside the grid read as zero, like the ghost shell
+#pragma unroll
+  for (int i0 = 0; i0 < HX * HY * HZ; i0 += NT) {
+    const int i = i0 + threadIdx.x;
+    const int hx = X0 - R + i % HX, hy = y - R + i / HX % HY, hz = z - R + i / (HX * HY);
+    T v0 = 0, v1 = 0, v2 = 0;
+    if (i < HX * HY * HZ && inside(g, hx, hy, hz)) {
+      const long long q = 3LL * g.idx(hx, hy, hz);
+      v0 = __ldg(sqd + q) * __ldg(u + q);
+      v1 = __ldg(sqd + q + 1) * __ldg(u + q + 1);
+      v2 = __ldg(sqd + q + 2) * __ldg(u + q + 2);
+    }
+    if (i < HX * HY * HZ) sv[i].set(v0, v1, v2);
+  }
+  const int tx = threadIdx.x / G, lane = threadIdx.x % G, x = X0 + tx;
+  const bool in = inside(g, x, y, z);
+  const int p = in ? g.idx(x, y, z) : 0;
+  const int c = lane < 3 ? lane : 0;
+  const long long pc = 3LL * p + c;
+  T bc = 0, u0 = 0, mi = 0, dp = 0;
+  const uint8_t m = __ldg(a.mask + p);
+  const bool fr = (m >> c) & 1;
+  const A sq = (A)__ldg(sqd + pc);
+  if (lane < 3) {
+    if (EPI != EPI_APPLY && b) bc = b[pc];
+    if (EPI != EPI_RESID) u0 = __ldg(u + pc);
+    if (EPI != EPI_RESID && minv) mi = __ldg(minv + pc);
+    if (EPI == EPI_SMOOTH && dprev) dp = dprev[pc];
+  }
+  __syncthreads();
+  A acc[3] = {(A)0, (A)0, (A)0};
+  const int c0 = (R * HY + R) * HX + tx + R;
+  int slot = 0;
+  auto SH = [&](int uu) { return s_shift[uu]; };
+  auto V = [&](int, A (&vu)[3], A (&vd)[3]) {
+    const int d = s_delta[lane + G * slot];
+    ++slot;
+    sv[c0 + d].get(vu);
+    sv[c0 - d].get(vd);
+  };
+  wide_rows<S, A, L>(stc, p, lane, acc, SH, V);
+#pragma unroll
+  for (int o = 1; o < G; o <<= 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+  }
+  if (!in || lane >= 3) return;
+  const A ac = c == 0 ? acc[0] : (c == 1 ? acc[1] : acc[2]);
+  const T kc = fr ? (T)(ac * sq) : (T)0;
+  if (EPI == EPI_APPLY) {
+    out[pc] = minv ? kc * mi : kc;
+  } else if (EPI == EPI_SMOOTH) {
+    T o = u0 + (fr ? w * (mi * (bc - kc)) : (T)0);
+    if (dprev) o += c1 * dp;
+    out[pc] = o;
+    if (dout) dout[pc] = o - u0;
+  } else {
+    out[pc] = bc - kc;
+  }
 }
 
 // Dense row-major A of a reach-R level (reference node order, DOF 3*node + c),
@@ -830,16 +797,15 @@ template void launch_wide_compress<double, 2>(const Grid&, const double*, const 
 
 template <typename T, typename S, int R>
 void launch_wide_op(const Grid& g, int epi, const OpArgs& a, const S* stc, const T* sqrtd, cudaStream_t st) {
-  const int blocks = wide_op_grid_blocks(g);
-  if (epi == EPI_APPLY) launch_pdl(k_wide_op<T, S, R, EPI_APPLY>, blocks, 128, 0, st, g, a, stc, sqrtd);
-  else if (epi == EPI_SMOOTH) launch_pdl(k_wide_op<T, S, R, EPI_SMOOTH>, blocks, 128, 0, st, g, a, stc, sqrtd);
-  else launch_pdl(k_wide_op<T, S, R, EPI_RESID>, blocks, 128, 0, st, g, a, stc, sqrtd);
+  const unsigned blocks = (unsigned)((g.lx + kWideTX) / kWideTX) * (g.ly + 1) * (g.lz + 1);
+  if (epi == EPI_APPLY) launch_pdl(k_wide_op<T, S, R, EPI_APPLY>, blocks, kWideTX * 8, 0, st, g, a, stc, sqrtd);
+  else if (epi == EPI_SMOOTH) launch_pdl(k_wide_op<T, S, R, EPI_SMOOTH>, blocks, kWideTX * 8, 0, st, g, a, stc, sqrtd);
+  else launch_pdl(k_wide_op<T, S, R, EPI_RESID>, blocks, kWideTX * 8, 0, st, g, a, stc, sqrtd);
 }
 template void launch_wide_op<float, __half, 2>(const Grid&, int, const OpArgs&, const __half*, const float*, cudaStream_t);
 template void launch_wide_op<float, float, 2>(const Grid&, int, const OpArgs&, const float*, const float*, cudaStream_t);
 template void launch_wide_op<double, double, 2>(const Grid&, int, const OpArgs&, const double*, const double*,
                                                 cudaStream_t);
-int wide_op_grid_blocks(const Grid& g) { return blocks_for((long long)g.n * 8, 128, 148LL * 32); }
 
 int wide_dense_assemble(const Grid& c, int R, const double* stencil, const uint8_t* cmask, double* A, int n,
                         cudaStream_t st) {
