@@ -73,8 +73,8 @@ unsigned long long graph_kernel_nodes(cudaGraph_t g) {
 
 struct Level {
   Grid g{};
-  int zchunk = 0;          // modal kernel: z-planes per CTA (< 0: one even wave)
-  int szchunk = 0;         // marching stencil kernel: z-planes per CTA
+  int zchunk[2] = {0, 0};  // modal kernel, FP32 / FP64: z-planes per CTA (< 0: one even wave)
+  int szchunk[2] = {0, 0}; // marching stencil kernel, FP32 / FP64: z-planes per CTA
   uint8_t* mask = nullptr;
   bool galerkin = false;   // operator is the assembled stencil
   double* E64 = nullptr; double* mu64 = nullptr; double* minv64 = nullptr; double* st64 = nullptr;
@@ -263,16 +263,16 @@ void compress_sym64(vf_solver* s, Level& l) {
 template <> void level_sym_op<double>(vf_solver* s, Level& l, int epi, const OpArgs& a) {
   if (!l.sym64_ok) compress_sym64(s, l);
   if (l.reach == 2) launch_wide_op<double, double, 2>(l.g, epi, a, l.sym64, l.sq64, s->st);
-  else launch_stencil_sym_op<double, double>(l.g, epi, a, l.sym64, l.sq64, l.szchunk, s->st);
+  else launch_stencil_sym_op<double, double>(l.g, epi, a, l.sym64, l.sq64, l.szchunk[1], s->st);
 }
 template <> void level_sym_op<float>(vf_solver* s, Level& l, int epi, const OpArgs& a) {
   if (l.reach == 2) {
     if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) launch_wide_op<float, __half, 2>(l.g, epi, a, l.sym16, l.sq32, s->st);
     else launch_wide_op<float, float, 2>(l.g, epi, a, l.sym32, l.sq32, s->st);
   } else if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) {
-    launch_stencil_sym_op<float, __half>(l.g, epi, a, l.sym16, l.sq32, l.szchunk, s->st);
+    launch_stencil_sym_op<float, __half>(l.g, epi, a, l.sym16, l.sq32, l.szchunk[0], s->st);
   } else {
-    launch_stencil_sym_op<float, float>(l.g, epi, a, l.sym32, l.sq32, l.szchunk, s->st);
+    launch_stencil_sym_op<float, float>(l.g, epi, a, l.sym32, l.sq32, l.szchunk[0], s->st);
   }
 }
 
@@ -317,8 +317,9 @@ void level_op(vf_solver* s, int li, int epi, const T* u, T* out, const T* b, Kry
     launch_fine_op<T>(l.g, epi, a, s->st);
   } else {
     const ModalConst& mc = s->lame ? s->mc_lame : s->mc;
-    if (s->o.fine_kernel == VF_FINE_MODAL_CPASYNC || !launch_modal_tma<T>(l.g, epi, a, mc, l.zchunk, s->st))
-      launch_modal_op<T>(l.g, epi, a, mc, 8, l.zchunk > 0 ? l.zchunk : auto_zchunk(l.g, 0), s->st);
+    const int zc = l.zchunk[sizeof(T) == 8 ? 1 : 0];
+    if (s->o.fine_kernel == VF_FINE_MODAL_CPASYNC || !launch_modal_tma<T>(l.g, epi, a, mc, zc, s->st))
+      launch_modal_op<T>(l.g, epi, a, mc, 8, zc > 0 ? zc : auto_zchunk(l.g, 0), s->st);
   }
 }
 
@@ -892,12 +893,85 @@ void nn_refresh_features(vf_solver* s) {
 
 // ---------------------------------------------------------------------------
 // autotuner: z-planes per CTA of the marching kernels, per level, timed with
-// CUDA events on the FP32 Jacobi sweep (the kernel the V-cycle runs most);
-// the choice is cached per (grid, kernel form) for the process.
+// CUDA events on the kernel that the iteration runs on it most: the sweep in
+// the V-cycle's precision, and for the FP64 PCG around an FP32 V-cycle also the
+// FP64 fine operator.  (Each precision has its own choice: the FP64 stencil
+// sweep of a 64x32x32 level takes 27 us at 33 planes and 57 us at 11, where
+// the FP32 one is as fast.)  The choice is cached per (grid, kernel form) for
+// the process.
 // ---------------------------------------------------------------------------
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int>, int> g_tune_cache;
 int auto_zchunk(const Grid& g, int requested);
+
+template <typename T>
+int autotune_level(vf_solver* s, int li, int epi, cudaEvent_t t0, cudaEvent_t t1) {
+  Level& l = s->L[li];
+  constexpr int q = sizeof(T) == 8 ? 1 : 0;
+  const bool stencil = l.galerkin && s->o.coarse_storage != VF_STENCIL_FULL && l.reach == 1;
+  const bool modal = !l.galerkin && s->o.fine_kernel == VF_FINE_MODAL;
+  if (!stencil && !modal) return VF_OK;
+  if (modal && s->o.modal_zchunk != 0) return VF_OK;   // fixed by the caller
+  int& choice = stencil ? l.szchunk[q] : l.zchunk[q];
+  const auto key = std::make_tuple(l.g.lx, l.g.ly, l.g.lz, (stencil ? 1 + s->o.coarse_storage : 0) + 8 * q);
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tune_cache.find(key);
+    if (it != g_tune_cache.end()) {
+      choice = it->second;
+      return VF_OK;
+    }
+  }
+  const int planes = l.g.lz + 1;
+  // CTAs of a candidate; candidates that leave SMs idle while a finer split
+  // would fill them are not considered (a short level is latency bound)
+  const long long tiles = stencil ? (long long)((l.g.lx + 32) / 32) * ((l.g.ly + 8) / 8)
+                                  : (long long)((l.g.lx + 31) / 31) * ((l.g.ly + 7) / 7);
+  auto ctas = [&](int c) { return tiles * ((planes + c - 1) / c); };
+  const long long floor_ctas = std::min<long long>(148, ctas(modal ? 2 : 1));
+  // every distinct z-chunk ceil(planes / n) for n = 1..64 z-ranges: the
+  // last wave of CTAs can be anywhere from nearly empty to full, and which
+  // split fills it best depends on the tile count and the residency
+  std::vector<int> cand;
+  const int base = stencil ? sym_zchunk(l.g) : auto_zchunk(l.g, 0);
+  cand.push_back(base);
+  // (the TMA modal kernel's one-wave split, z-chunk -1, is not a candidate:
+  // it is ~3 % faster on the 256x128x128 level but its CTAs march
+  // neighbouring tiles at different z, so the tile halos miss L2 and the
+  // DRAM traffic grows from 219 to 336 MB per sweep)
+  for (int n = 1; n <= 64; ++n) {
+    const int c = (planes + n - 1) / n;
+    if (c >= 1 && (modal ? c >= 2 : true) && ctas(c) >= floor_ctas &&
+        std::find(cand.begin(), cand.end(), c) == cand.end())
+      cand.push_back(c);
+  }
+  T *u = Sel<T>::w(l, 0), *out = Sel<T>::w(l, 1), *b = Sel<T>::w(l, 3);
+  auto run = [&]() { level_op<T>(s, li, epi, u, out, b, nullptr, nullptr, 0); };
+  // two passes, minimum per candidate: the first pass also brings the
+  // clocks up after the set-up, which would otherwise favour late candidates
+  std::vector<float> tmin(cand.size(), 1e30f);
+  for (int pass = 0; pass < 2; ++pass)
+    for (size_t ci = 0; ci < cand.size(); ++ci) {
+      choice = cand[ci];
+      run();   // warm
+      VF_TRY(cudaEventRecord(t0, s->st));
+      for (int r = 0; r < 6; ++r) run();
+      VF_TRY(cudaEventRecord(t1, s->st));
+      VF_TRY(cudaEventSynchronize(t1));
+      VF_CHECK_LAUNCH();
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, t0, t1);
+      tmin[ci] = std::min(tmin[ci], ms);
+    }
+  int best = base;
+  float best_ms = 1e30f;
+  for (size_t ci = 0; ci < cand.size(); ++ci)
+    if (tmin[ci] < best_ms) { best_ms = tmin[ci]; best = cand[ci]; }
+  choice = best;
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  g_tune_cache[key] = best;
+  return VF_OK;
+}
 
 int autotune_levels(vf_solver* s) {
   cudaEvent_t t0 = nullptr, t1 = nullptr;
@@ -907,69 +981,14 @@ int autotune_levels(vf_solver* s) {
     cudaEvent_t a, b;
     ~Ev() { cudaEventDestroy(a); cudaEventDestroy(b); }
   } ev{t0, t1};
+  const bool f64 = s->o.precision == VF_PREC_FP64;
   for (size_t li = 0; li < s->L.size(); ++li) {
-    Level& l = s->L[li];
-    const bool stencil = l.galerkin && s->o.coarse_storage != VF_STENCIL_FULL && l.reach == 1;
-    const bool modal = !l.galerkin && s->o.fine_kernel == VF_FINE_MODAL;
-    if (!stencil && !modal) continue;
-    if (modal && s->o.modal_zchunk != 0) continue;   // fixed by the caller
-    const auto key = std::make_tuple(l.g.lx, l.g.ly, l.g.lz, stencil ? 1 + s->o.coarse_storage : 0);
-    {
-      std::lock_guard<std::mutex> lk(g_tune_mu);
-      auto it = g_tune_cache.find(key);
-      if (it != g_tune_cache.end()) {
-        (stencil ? l.szchunk : l.zchunk) = it->second;
-        continue;
-      }
-    }
-    const int planes = l.g.lz + 1;
-    // CTAs of a candidate; candidates that leave SMs idle while a finer split
-    // would fill them are not considered (a short level is latency bound)
-    const long long tiles = stencil ? (long long)((l.g.lx + 32) / 32) * ((l.g.ly + 8) / 8)
-                                    : (long long)((l.g.lx + 31) / 31) * ((l.g.ly + 7) / 7);
-    auto ctas = [&](int c) { return tiles * ((planes + c - 1) / c); };
-    const long long floor_ctas = std::min<long long>(148, ctas(modal ? 2 : 1));
-    // every distinct z-chunk ceil(planes / n) for n = 1..64 z-ranges: the
-    // last wave of CTAs can be anywhere from nearly empty to full, and which
-    // split fills it best depends on the tile count and the residency
-    std::vector<int> cand;
-    const int base = stencil ? sym_zchunk(l.g) : auto_zchunk(l.g, 0);
-    cand.push_back(base);
-    // (the TMA modal kernel's one-wave split, z-chunk -1, is not a candidate:
-    // it is ~3 % faster on the 256x128x128 level but its CTAs march
-    // neighbouring tiles at different z, so the tile halos miss L2 and the
-    // DRAM traffic grows from 219 to 336 MB per sweep)
-    for (int n = 1; n <= 64; ++n) {
-      const int c = (planes + n - 1) / n;
-      if (c >= 1 && (modal ? c >= 2 : true) && ctas(c) >= floor_ctas &&
-          std::find(cand.begin(), cand.end(), c) == cand.end())
-        cand.push_back(c);
-    }
-    // two passes, minimum per candidate: the first pass also brings the
-    // clocks up after the set-up, which would otherwise favour late candidates
-    std::vector<float> tmin(cand.size(), 1e30f);
-    for (int pass = 0; pass < 2; ++pass)
-      for (size_t ci = 0; ci < cand.size(); ++ci) {
-        (stencil ? l.szchunk : l.zchunk) = cand[ci];
-        level_op<float>(s, (int)li, EPI_SMOOTH, l.w32[0], l.w32[1], l.w32[3], nullptr, nullptr, 0);   // warm
-        VF_TRY(cudaEventRecord(t0, s->st));
-        for (int r = 0; r < 6; ++r)
-          level_op<float>(s, (int)li, EPI_SMOOTH, l.w32[0], l.w32[1], l.w32[3], nullptr, nullptr, 0);
-        VF_TRY(cudaEventRecord(t1, s->st));
-        VF_TRY(cudaEventSynchronize(t1));
-        VF_CHECK_LAUNCH();
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, t0, t1);
-        tmin[ci] = std::min(tmin[ci], ms);
-      }
-    int best = base;
-    float best_ms = 1e30f;
-    for (size_t ci = 0; ci < cand.size(); ++ci)
-      if (tmin[ci] < best_ms) { best_ms = tmin[ci]; best = cand[ci]; }
-    (stencil ? l.szchunk : l.zchunk) = best;
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache[key] = best;
+    const int rc = f64 ? autotune_level<double>(s, (int)li, EPI_SMOOTH, t0, t1)
+                       : autotune_level<float>(s, (int)li, EPI_SMOOTH, t0, t1);
+    if (rc) return rc;
   }
+  if (s->o.precision == VF_PREC_MIXED && s->o.mixed_mode == VF_MIXED_OUTER64)
+    return autotune_level<double>(s, 0, EPI_APPLY, t0, t1);
   return VF_OK;
 }
 
@@ -988,8 +1007,8 @@ int upload_tables(vf_solver* s) {
   s->mc = vf::modal_constants(s->nu, false);
   s->mc_lame = vf::modal_constants(s->nu, true);
   for (auto& l : s->L) {
-    l.zchunk = auto_zchunk(l.g, s->o.modal_zchunk);
-    l.szchunk = sym_zchunk(l.g);
+    l.zchunk[0] = l.zchunk[1] = auto_zchunk(l.g, s->o.modal_zchunk);
+    l.szchunk[0] = l.szchunk[1] = sym_zchunk(l.g);
   }
   std::vector<double> G(8 * 576), GL(16 * 576);
   galerkin_child_tables(s->tab, G.data());
@@ -2244,7 +2263,12 @@ void share_operator(vf_solver* c, const vf_solver* m) {
   for (size_t i = 0; i < c->L.size(); ++i) {
     Level& d = c->L[i];
     const Level& sl = m->L[i];
-    d.g = sl.g; d.zchunk = sl.zchunk; d.szchunk = sl.szchunk; d.mask = sl.mask; d.galerkin = sl.galerkin;
+    d.g = sl.g; 
+    for (int q = 0; q < 2; ++q) {
+      d.zchunk[q] = sl.zchunk[q];
+      d.szchunk[q] = sl.szchunk[q];
+    }
+    d.mask = sl.mask; d.galerkin = sl.galerkin;
     d.E64 = sl.E64; d.mu64 = sl.mu64; d.minv64 = sl.minv64; d.st64 = sl.st64;
     d.E32 = sl.E32; d.mu32 = sl.mu32; d.minv32 = sl.minv32; d.st32 = sl.st32;
     d.sym64 = sl.sym64; d.sq64 = sl.sq64; d.sym32 = sl.sym32; d.sym16 = sl.sym16; d.sq32 = sl.sq32;
