@@ -215,6 +215,13 @@ template <typename T> bool launch_modal_tma(const Grid& g, int epi, const OpArgs
                                             cudaStream_t st);
 bool modal_tma_supported();
 
+// vf_coarse.cu -- the coarsest level's Jacobi sweeps from zero in one launch;
+// false (nothing launched) when the level does not fit or there is one sweep
+template <typename T>
+bool launch_coarse_jacobi(const Grid& g, const T* b, T* x, const T* minv3, const uint8_t* mask, const T* E, const T* mu,
+                          const ModalConst& mc, int sweeps, double omega, const double* omega_dev,
+                          const KrylovState* ks, cudaStream_t st);
+
 // vf_stencil.cu -- assembled 27-point block stencils (Galerkin levels)
 template <typename T> void launch_stencil_op(const Grid& g, int epi, const OpArgs& a, const T* stencil, cudaStream_t st);
 template <typename T> int stencil_op_grid_blocks(const Grid& g);
