@@ -13,8 +13,13 @@
 // Backward-weight: dW[tap][co][ci] = sum_v dY[v][co] X[v + off(tap)][ci] is a
 // GEMM with M = co, N = ci and K = voxels (mma.m16n8k16).  A CTA takes a group
 // of taps and a strided set of voxel tiles; both operands come out of shared
-// memory through ldmatrix.trans.  Per-CTA partial sums are reduced in a fixed
-// order (deterministic).
+// memory through ldmatrix.trans.  A warp keeps 16 co x 16 ci for every tap of
+// the group in registers, so a row of 16 voxels costs one load of dY and one of
+// X per tap for two products per tap (one tap, 8 ci at a time and both operands
+// loaded for each product, the shared-memory pipe was the bound: 32-32
+// channels on 68x52x36 voxels 127 us); with few channels the warps share the
+// rows of a tile.  Per-CTA partial sums are reduced in a fixed order
+// (deterministic).
 #include <cuda_bf16.h>
 
 #include <atomic>
@@ -38,9 +43,6 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)_
 __device__ __forceinline__ void ldsm_x4_t(unsigned a, unsigned& r0, unsigned& r1, unsigned& r2, unsigned& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(a));
-}
-__device__ __forceinline__ void ldsm_x2_t(unsigned a, unsigned& r0, unsigned& r1) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(a));
 }
 __device__ __forceinline__ void mma16816(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
                                          unsigned b0, unsigned b1) {
@@ -73,39 +75,47 @@ __device__ __forceinline__ int halo_index(int hx, int hy, int hz) { return (hz *
 // ---------------------------------------------------------------------------
 template <int CIN, int COUT>
 struct WgradCfg {
-  static constexpr int frags(int taps) { return taps * (COUT / 16) * (CIN / 8); }
-  static constexpr int TAPS = frags(27) <= 128 ? 27 : (frags(9) <= 128 ? 9 : (frags(3) <= 128 ? 3 : 1));
-  static constexpr int F = frags(TAPS);
-  static constexpr int NF = (F + 7) / 8;   // fragments per warp
-  static constexpr int DP = COUT + 8;      // smem stride of a dY voxel
+  static constexpr int MT = COUT / 16, NP = CIN / 16, COMB = MT * NP;   // 16 x 16 blocks of (co, ci)
+  static constexpr int CPW = COMB <= 8 ? 1 : COMB / 8;                  // blocks per warp
+  static constexpr int KS = COMB < 8 ? 8 / COMB : 1;                    // warps sharing a block: rows of the tile
+  static constexpr int TAPS = CPW == 1 ? 9 : 3;                         // 8 CPW TAPS accumulators per thread
+  static constexpr int DP = COUT + 8;                                   // smem stride of a dY voxel
   static constexpr size_t smem() {
     return sizeof(bf16) * ((size_t)NHALO * (CIN + 8) + (size_t)OTX * OTY * OTZ * DP);
   }
+  static_assert(KS == 1 || sizeof(float) * TAPS * COUT * CIN <= smem(), "the shared sum reuses the tile's memory");
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(NTHREADS) k_conv3_wgrad(const bf16* __restrict__ x, const bf16* __restrict__ dy,
-                                                           float* __restrict__ partial, int X, int Y, int Z) {
+__global__ void __launch_bounds__(NTHREADS, 2)
+    k_conv3_wgrad(const bf16* __restrict__ x, const bf16* __restrict__ dy, float* __restrict__ partial, int X, int Y,
+                  int Z) {
   using Cfg = WgradCfg<CIN, COUT>;
-  constexpr int CP = CIN + 8, DP = Cfg::DP, NF = Cfg::NF, F = Cfg::F, TAPS = Cfg::TAPS;
-  constexpr int MT = COUT / 16, NTI = CIN / 8;
+  constexpr int CP = CIN + 8, DP = Cfg::DP, TAPS = Cfg::TAPS, KS = Cfg::KS, CPW = Cfg::CPW;
   extern __shared__ __align__(16) unsigned char smem[];
   bf16* sX = reinterpret_cast<bf16*>(smem);
   bf16* sD = sX + NHALO * CP;   // [256 tile voxels][DP], voxel = (tz*8 + ty)*16 + tx
   const int tx = (X + OTX - 1) / OTX, ty = (Y + OTY - 1) / OTY, tz = (Z + OTZ - 1) / OTZ;
   const int ntiles = tx * ty * tz;
   const int tap0 = blockIdx.y * TAPS;
+  const int ddz = tap0 / 9, ddy0 = tap0 / 3 % 3;   // halo offsets (d + 1) of the group's first tap
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float acc[NF][4];
+  const int comb0 = KS > 1 ? warp % Cfg::COMB : warp, part = KS > 1 ? warp / Cfg::COMB : 0;
+  float acc[CPW][TAPS][2][4];
 #pragma unroll
-  for (int f = 0; f < NF; ++f)
+  for (int q = 0; q < CPW; ++q)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) acc[f][k] = 0.f;
+    for (int t = 0; t < TAPS; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[q][t][h][k] = 0.f;
   // A = dY^T (m = co, k = voxel), from [voxel][co]: ldmatrix.trans, row = voxel
   const int a_v = (lane & 7) + ((lane >> 4) & 1) * 8;
   const int a_c = ((lane >> 3) & 1) * 8;
-  // B = X shifted (k = voxel, n = ci), from [voxel][ci]: ldmatrix.trans, row = voxel (lanes 0..15)
+  // B = X shifted (k = voxel, n = ci), from [voxel][ci]: two 8-channel halves per load
   const int b_v = (lane & 7) + ((lane >> 3) & 1) * 8;
+  const int b_c = (lane >> 4) * 8;
 
 #pragma unroll 1
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -125,47 +135,77 @@ __global__ void __launch_bounds__(NTHREADS) k_conv3_wgrad(const bf16* __restrict
       }
     }
     __syncthreads();
-#pragma unroll
-    for (int j = 0; j < NF; ++j) {
-      const int f = warp + 8 * j;
-      if (f >= F) break;
-      const int tap = f / (MT * NTI), rem = f % (MT * NTI), mt = rem / NTI, nt = rem % NTI;
-      const int tg = tap0 + tap;
-      const int ddz = tg / 9, ddy = (tg / 3) % 3, ddx = tg % 3;   // halo offsets (d + 1)
 #pragma unroll 1
-      for (int row = 0; row < OTY * OTZ; ++row) {
-        const int ry = row % OTY, rz = row / OTY;
-        unsigned a0, a1, a2, a3, b0, b1;
+    for (int row = part; row < OTY * OTZ; row += KS) {
+      const int ry = row % OTY, rz = row / OTY;
+#pragma unroll
+      for (int q = 0; q < CPW; ++q) {
+        const int comb = comb0 + 8 * q, mt = comb / Cfg::NP, np = comb % Cfg::NP;
+        unsigned a0, a1, a2, a3;
         ldsm_x4_t(smem_u32(sD + (row * OTX + a_v) * DP + mt * 16 + a_c), a0, a1, a2, a3);
-        ldsm_x2_t(smem_u32(sX + halo_index((b_v & 15) + ddx, ry + ddy, rz + ddz) * CP + nt * 8), b0, b1);
-        mma16816(acc[j], a0, a1, a2, a3, b0, b1);
+        const unsigned xb = smem_u32(sX + halo_index(b_v, ry + ddy0, rz + ddz) * CP + np * 16 + b_c);
+#pragma unroll
+        for (int tap = 0; tap < TAPS; ++tap) {
+          unsigned b0, b1, b2, b3;
+          ldsm_x4_t(xb + (unsigned)(halo_index(tap % 3, tap / 3, 0) * CP * sizeof(bf16)), b0, b1, b2, b3);
+          mma16816(acc[q][tap][0], a0, a1, a2, a3, b0, b1);
+          mma16816(acc[q][tap][1], a0, a1, a2, a3, b2, b3);
+        }
       }
     }
   }
   // partial[block][tap][co][ci] for the taps of this group
   const int g = lane >> 2, tig = lane & 3;
-  float* dst = partial + (long long)blockIdx.x * 27 * COUT * CIN;
+  float* dst = partial + (long long)blockIdx.x * 27 * COUT * CIN + (long long)tap0 * COUT * CIN;
+  float* sum = reinterpret_cast<float*>(smem);
+#pragma unroll 1
+  for (int k = 0; k < KS; ++k) {
+    if (KS > 1) __syncthreads();
+    if (KS > 1 && part != k) continue;
 #pragma unroll
-  for (int j = 0; j < NF; ++j) {
-    const int f = warp + 8 * j;
-    if (f >= F) break;
-    const int tap = f / (MT * NTI), rem = f % (MT * NTI), mt = rem / NTI, nt = rem % NTI;
-    const int tg = tap0 + tap;
-    const int co = mt * 16 + g, ci = nt * 8 + 2 * tig;
-    float* d = dst + ((long long)tg * COUT + co) * CIN + ci;
-    d[0] = acc[j][0];
-    d[1] = acc[j][1];
-    d[8 * CIN] = acc[j][2];
-    d[8 * CIN + 1] = acc[j][3];
+    for (int q = 0; q < CPW; ++q) {
+      const int comb = comb0 + 8 * q, mt = comb / Cfg::NP, np = comb % Cfg::NP;
+#pragma unroll
+      for (int tap = 0; tap < TAPS; ++tap)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int co = mt * 16 + g, ci = np * 16 + h * 8 + 2 * tig;
+          float* d = (KS > 1 ? sum : dst) + ((long long)tap * COUT + co) * CIN + ci;
+          const float* v = acc[q][tap][h];
+          const bool add = KS > 1 && k > 0;
+          d[0] = add ? d[0] + v[0] : v[0];
+          d[1] = add ? d[1] + v[1] : v[1];
+          d[8 * CIN] = add ? d[8 * CIN] + v[2] : v[2];
+          d[8 * CIN + 1] = add ? d[8 * CIN + 1] + v[3] : v[3];
+        }
+    }
+  }
+  if (KS > 1) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < TAPS * COUT * CIN; i += NTHREADS) dst[i] = sum[i];
   }
 }
 
-__global__ void k_reduce_partials(const float* __restrict__ partial, int nparts, long long n, float* __restrict__ out,
-                                  int accumulate) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < nparts; ++b) s += partial[(long long)b * n + i];
-    out[i] = accumulate ? out[i] + s : s;
+// Sums of the per-CTA partials in a fixed order: 8 threads per value take every
+// eighth partial (one thread per value walked all of them, 21 us for 27,648
+// values of 148 partials).
+__global__ void __launch_bounds__(256) k_reduce_partials(const float* __restrict__ partial, int nparts, long long n,
+                                                         float* __restrict__ out, int accumulate) {
+  __shared__ float s[8][33];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  const long long i = blockIdx.x * 32LL + lane;
+  float v = 0.f;
+  if (i < n) {
+#pragma unroll 4
+    for (int b = grp; b < nparts; b += 8) v += __ldg(partial + (long long)b * n + i);
+  }
+  s[grp][lane] = v;
+  __syncthreads();
+  if (grp == 0 && i < n) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += s[k][lane];
+    out[i] = accumulate ? out[i] + t : t;
   }
 }
 
@@ -175,16 +215,18 @@ int conv_wgrad_t(const void* x, const void* dy, float* dw, float* work, size_t w
   using Cfg = WgradCfg<CIN, COUT>;
   const size_t per = sizeof(float) * 27 * COUT * CIN;
   const long long tiles = (long long)((X + OTX - 1) / OTX) * ((Y + OTY - 1) / OTY) * ((Z + OTZ - 1) / OTZ);
-  long long nb = std::min<long long>(tiles, 148);
-  nb = std::min<long long>(nb, (long long)(work_bytes / per));
-  if (nb < 1) return -1;
   constexpr size_t smem = Cfg::smem();
   static std::atomic<int> per_dev[kMaxDevices];
-  kernel_prepare(per_dev, k_conv3_wgrad<CIN, COUT>, smem, NTHREADS);
-  launch_k(k_conv3_wgrad<CIN, COUT>, dim3((unsigned)nb, 27 / Cfg::TAPS), dim3(NTHREADS), smem, st,
+  const int per_sm = kernel_prepare(per_dev, k_conv3_wgrad<CIN, COUT>, smem, NTHREADS);
+  // one resident wave over the tap groups (148 CTAs a group were a wave and a half)
+  constexpr int groups = 27 / Cfg::TAPS;
+  long long nb = std::min<long long>(tiles, std::min(148, std::max(1, 148 * per_sm / groups)));
+  nb = std::min<long long>(nb, (long long)(work_bytes / per));
+  if (nb < 1) return -1;
+  launch_k(k_conv3_wgrad<CIN, COUT>, dim3((unsigned)nb, groups), dim3(NTHREADS), smem, st,
            (const bf16*)x, (const bf16*)dy, work, X, Y, Z);
   const long long n = 27LL * COUT * CIN;
-  launch_k(k_reduce_partials, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (const float*)work, (int)nb, n,
+  launch_k(k_reduce_partials, dim3((unsigned)((n + 31) / 32)), dim3(256), 0, st, (const float*)work, (int)nb, n,
            dw, accumulate);
   return 0;
 }
