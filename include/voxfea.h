@@ -404,6 +404,10 @@ int vf_nn_conv3d_backward_data(const void* dy, const void* w_t, const void* gate
 int vf_nn_conv3d_backward_weight(const void* x, const void* dy, float* dw, int32_t accumulate,
                                  float* work, size_t work_bytes, int32_t X, int32_t Y, int32_t Z,
                                  int32_t cin, int32_t cout, void* stream);
+/* db[cout] (FP32) = sum over the nvox voxels of dy (BF16); work: at least
+ * 148 x cout floats of caller-provided scratch; cout 16, 32 or 64. */
+int vf_nn_conv3d_backward_bias(const void* dy, float* db, float* work, size_t work_bytes, int64_t nvox, int32_t cout,
+                               void* stream);
 size_t vf_nn_wgrad_workspace(int32_t cin, int32_t cout, int32_t X, int32_t Y, int32_t Z);
 
 /* The learned stage inside the solver's preconditioner: after the V-cycle,

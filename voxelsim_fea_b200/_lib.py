@@ -145,6 +145,7 @@ def _declare(L):
         "vf_nn_conv3d_backward_data": (ctypes.c_int, [_P, _P, _P, _P, _I32, _I32, _I32, _I32, _I32, _P]),
         "vf_nn_conv3d_backward_weight": (ctypes.c_int, [_P, _P, _P, _I32, _P, ctypes.c_size_t, _I32, _I32, _I32,
                                                         _I32, _I32, _P]),
+        "vf_nn_conv3d_backward_bias": (ctypes.c_int, [_P, _P, _P, ctypes.c_size_t, ctypes.c_int64, _I32, _P]),
         "vf_nn_wgrad_workspace": (ctypes.c_size_t, [_I32, _I32, _I32, _I32, _I32]),
         "vf_learned_param_count": (ctypes.c_int64, []),
         "vf_learned_configure": (ctypes.c_int, [_P, _I32, _P, ctypes.c_int64, _I32]),

@@ -209,6 +209,41 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const float* __restrict
   }
 }
 
+// Bias gradient: column sums of dY.  A thread keeps 8 consecutive channels (16
+// bytes a voxel) of every gridDim-th group of voxels; a block's threads of the
+// same channels, then the blocks, are summed in a fixed order.  (As a
+// conversion to FP32 and a generic reduction: 35 us for 32 channels on
+// 68x52x36 voxels, the bytes take 1.5.)
+constexpr int kBiasBlocks = 148;
+template <int COUT>
+__global__ void __launch_bounds__(NTHREADS) k_bias_grad(const bf16* __restrict__ dy, long long nvox,
+                                                        float* __restrict__ partial) {
+  constexpr int CH = COUT / 8, VOX = NTHREADS / CH;
+  __shared__ float s[NTHREADS][9];
+  const int ch = threadIdx.x % CH, v0 = threadIdx.x / CH;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (long long v = (long long)blockIdx.x * VOX + v0; v < nvox; v += (long long)gridDim.x * VOX) {
+    const uint4 p = __ldg(reinterpret_cast<const uint4*>(dy + v * COUT) + ch);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&p);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 f = __bfloat1622float2(h[k]);
+      acc[2 * k] += f.x;
+      acc[2 * k + 1] += f.y;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s[threadIdx.x][k] = acc[k];
+  __syncthreads();
+  if (threadIdx.x < COUT) {
+    const int c = threadIdx.x;
+    float t = 0.f;
+    for (int v = 0; v < VOX; ++v) t += s[v * CH + c / 8][c % 8];
+    partial[(long long)blockIdx.x * COUT + c] = t;
+  }
+}
+
 template <int CIN, int COUT>
 int conv_wgrad_t(const void* x, const void* dy, float* dw, float* work, size_t work_bytes, int X, int Y, int Z,
                  int accumulate, cudaStream_t st) {
@@ -290,6 +325,21 @@ int vf_nn_conv3d_backward_weight(const void* x, const void* dy, float* dw, int32
   if (!x || !dy || !dw || !work || X < 1 || Y < 1 || Z < 1) return VF_ERR_ARG;
   if (vf::nn_conv_wgrad(cin, cout, x, dy, dw, work, work_bytes, X, Y, Z, accumulate, (cudaStream_t)stream))
     return VF_ERR_ARG;
+  return cudaPeekAtLastError() == cudaSuccess ? VF_OK : VF_ERR_CUDA;
+}
+
+int vf_nn_conv3d_backward_bias(const void* dy, float* db, float* work, size_t work_bytes, int64_t nvox, int32_t cout,
+                               void* stream) {
+  using namespace vf;
+  if (!dy || !db || !work || nvox < 1 || work_bytes < sizeof(float) * kBiasBlocks * (size_t)cout) return VF_ERR_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  const bf16* d = (const bf16*)dy;
+  const int nb = (int)std::min<long long>(kBiasBlocks, (nvox * cout / 8 + NTHREADS - 1) / NTHREADS);
+  if (cout == 16) launch_k(k_bias_grad<16>, nb, NTHREADS, 0, st, d, (long long)nvox, work);
+  else if (cout == 32) launch_k(k_bias_grad<32>, nb, NTHREADS, 0, st, d, (long long)nvox, work);
+  else if (cout == 64) launch_k(k_bias_grad<64>, nb, NTHREADS, 0, st, d, (long long)nvox, work);
+  else return VF_ERR_ARG;
+  launch_k(k_reduce_partials, (cout + 31) / 32, 256, 0, st, (const float*)work, nb, (long long)cout, db, 0);
   return cudaPeekAtLastError() == cudaSuccess ? VF_OK : VF_ERR_CUDA;
 }
 

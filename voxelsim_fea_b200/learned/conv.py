@@ -78,6 +78,18 @@ def conv3d_backward_weight(x, dy):
     return dw
 
 
+def conv3d_backward_bias(dy):
+    """db (Cout,) FP32 = sum of dy (Z,Y,X,Cout) BF16 over the voxels."""
+    cout = dy.shape[3]
+    dy = dy.contiguous()
+    work = torch.empty(148 * cout, device=dy.device, dtype=torch.float32)
+    db = torch.empty(cout, device=dy.device, dtype=torch.float32)
+    rc = _lib.load().vf_nn_conv3d_backward_bias(_ptr(dy), _ptr(db), _ptr(work), 4 * work.numel(), dy.numel() // cout,
+                                                cout, _stream())
+    _check(rc, "vf_nn_conv3d_backward_bias")
+    return db
+
+
 class Conv3dFn(torch.autograd.Function):
     """y = conv(x, w) + b with the libvoxfea kernels in both directions
     (BF16 output, or FP32 with ``out_f32``)."""
@@ -94,7 +106,7 @@ class Conv3dFn(torch.autograd.Function):
         dy = dy.to(torch.bfloat16).contiguous()
         dx = conv3d_backward_data(dy, wb) if ctx.needs_input_grad[0] else None
         dw = conv3d_backward_weight(x, dy) if ctx.needs_input_grad[1] else None
-        db = dy.float().sum(dim=(0, 1, 2)) if ctx.needs_input_grad[2] else None
+        db = conv3d_backward_bias(dy) if ctx.needs_input_grad[2] else None
         return dx, dw, db, None
 
 
