@@ -40,7 +40,6 @@ using namespace modal;
 
 constexpr int TX = 32;
 constexpr int TY = 8;
-constexpr int NSTAGE = 4;
 
 // widths (elements) of the boxes: u / rhs / diagonal rows cover the 33 nodes
 // of the halo tile (3 values each), modulus rows the 32 voxel columns; plus
@@ -54,6 +53,11 @@ constexpr int rup128(int b) { return (b + 127) / 128 * 128; }
 template <typename T, bool LAME, int EPI>
 struct Layout {
   static constexpr int L = Pack<T>::L;
+  // Stages of the ring: planes s - 1 and s in use, the others in flight.  The
+  // sweep with a second modulus gets by with one plane in flight: four stages
+  // leave it one CTA per SM (256x128x128: 119 -> 90 us, 96x80x64: 22.5 -> 18.4).
+  static constexpr int NSTAGE = (LAME && EPI == EPI_SMOOTH) ? 3 : 4;
+  static constexpr int AHEAD = NSTAGE - 2;
   static constexpr int U = rup128((TY + 1) * Box<T>::W * (int)sizeof(T));   // one lane
   static constexpr int E = rup128(TY * Box<T>::WE * (int)sizeof(T));
   static constexpr int B = rup128(TY * Box<T>::W * (int)sizeof(T));
@@ -95,6 +99,7 @@ __global__ void __launch_bounds__(TX * TY, 2)
   using O = Pack<T>;
   using P = typename O::P;
   using Lay = Layout<T, LAME, EPI>;
+  constexpr int NSTAGE = Lay::NSTAGE, AHEAD = Lay::AHEAD;
   constexpr int L = O::L;
   constexpr int W = Box<T>::W, WE = Box<T>::WE, AL = Box<T>::A;
   KrylovState* ks = a.ks;
@@ -190,16 +195,26 @@ __global__ void __launch_bounds__(TX * TY, 2)
     const int gs = gbase + s;
     const int st = gs % NSTAGE, sp = (gs + NSTAGE - 1) % NSTAGE;
     const bool arrived = mbar_wait_bounded(&bar[st], (unsigned)((gs / NSTAGE) & 1));
-    // the barrier also marks step s-1 done everywhere: stage (s+2) is free
+    // the barrier also marks step s-1 done everywhere: stage (s + AHEAD) is free
     if (__syncthreads_or(!arrived)) return false;
-    if (leader && s + 2 < nsteps) issue(s + 2);
+    if (leader && s + AHEAD < nsteps) issue(s + AHEAD);
     // free-mask bytes: this step's were loaded one step ahead (mk_next),
     // the next step's are requested now, far from their use
     uint8_t mk[L];
+    T dp[EPI == EPI_SMOOTH ? L : 1][3];
 #pragma unroll
     for (int l = 0; l < L; ++l) {
       mk[l] = mk_next[l];
       const int zs = z0[l] + s;   // output plane of step s + 1
+      // the previous step's update (Chebyshev) is used at the end of the step: its
+      // loads pass beside the step's arithmetic
+      if (EPI == EPI_SMOOTH) {
+        const int zo = z0[l] + s - 1;
+        const bool use = dprev != nullptr && s >= 2 && out_col && zo < oend[l];
+        const T* q = dprev + (use ? 3 * ((zo + 1) * sz + colbase) : 0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) dp[l][c] = use ? q[c] : (T)0;
+      }
       mk_next[l] = (s + 1 >= 2 && s + 1 < nsteps && out_col && zs < oend[l]) ? __ldg(mask + (zs + 1) * sz + colbase)
                                                                              : (uint8_t)0;
     }
@@ -285,7 +300,7 @@ __global__ void __launch_bounds__(TX * TY, 2)
                 T o0 = u0 + ((m8 & 1) ? w * (d0 * (b0 - k0)) : (T)0);
                 T o1 = u1 + ((m8 & 2) ? w * (d1 * (b1 - k1)) : (T)0);
                 T o2 = u2 + ((m8 & 4) ? w * (d2 * (b2 - k2)) : (T)0);
-                if (dprev) { o0 += c1 * dprev[p3]; o1 += c1 * dprev[p3 + 1]; o2 += c1 * dprev[p3 + 2]; }
+                if (dprev) { o0 += c1 * dp[l][0]; o1 += c1 * dp[l][1]; o2 += c1 * dp[l][2]; }
                 out[p3] = o0; out[p3 + 1] = o1; out[p3 + 2] = o2;
                 if (dout) { dout[p3] = o0 - u0; dout[p3 + 1] = o1 - u1; dout[p3 + 2] = o2 - u2; }
                 if (a.dot_partials) dot += (double)b0 * (double)o0 + (double)b1 * (double)o1 + (double)b2 * (double)o2;
@@ -304,9 +319,9 @@ __global__ void __launch_bounds__(TX * TY, 2)
 
   P Fa[3][4], Fb[3][4];
   int failed_at = -1;   // running index of the step whose copies did not arrive
-  // Segments: a new segment's first two loads go to the stages of steps
-  // gbase-4 and gbase-3, whose last readers (steps gbase-3 and gbase-2) every
-  // thread has left once the leader is past step gbase-1's first barrier.
+  // Segments: a new segment's first loads go to the stages of steps
+  // gbase-NSTAGE .. gbase-3, whose last readers (at the latest step gbase-2)
+  // every thread has left once the leader is past step gbase-1's first barrier.
 #pragma unroll 1
   for (long long u0 = ub; u0 < ue;) {
     const int tile = (int)(u0 / NP);
@@ -337,8 +352,9 @@ __global__ void __launch_bounds__(TX * TY, 2)
 #pragma unroll
       for (int m = 0; m < 4; ++m) { hiPrev[c][m] = O::zero(); Fa[c][m] = O::zero(); Fb[c][m] = O::zero(); }
     if (leader) {
-      issue(0);
-      issue(1);
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k)
+        if (k < nsteps) issue(k);
     }
 #pragma unroll
     for (int l = 0; l < L; ++l) mk_next[l] = 0;   // steps 0 and 1 write no output

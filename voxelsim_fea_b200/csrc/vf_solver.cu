@@ -938,16 +938,14 @@ int autotune_level(vf_solver* s, int li, int epi, cudaEvent_t t0, cudaEvent_t t1
   std::vector<int> cand;
   const int base = stencil ? sym_zchunk(l.g) : auto_zchunk(l.g, 0);
   cand.push_back(base);
-  // (the TMA modal kernel's one-wave split, z-chunk -1, is not a candidate:
-  // it is ~3 % faster on the 256x128x128 level but its CTAs march
-  // neighbouring tiles at different z, so the tile halos miss L2 and the
-  // DRAM traffic grows from 219 to 336 MB per sweep)
+  // (and the TMA modal kernel's even one-wave split)
   for (int n = 1; n <= 64; ++n) {
     const int c = (planes + n - 1) / n;
     if (c >= 1 && (modal ? c >= 2 : true) && ctas(c) >= floor_ctas &&
         std::find(cand.begin(), cand.end(), c) == cand.end())
       cand.push_back(c);
   }
+  if (modal) cand.push_back(-1);
   T *u = Sel<T>::w(l, 0), *out = Sel<T>::w(l, 1), *b = Sel<T>::w(l, 3);
   auto run = [&]() { level_op<T>(s, li, epi, u, out, b, nullptr, nullptr, 0); };
   // two passes, minimum per candidate: the first pass also brings the
