@@ -50,6 +50,7 @@ EXPORTS = (
     "vf_vcycle", "vf_inv_diagonal", "vf_time_kernel", "vf_get_stream", "vf_launch_count",
     "vf_apply_noalloc",
     "vf_nn_conv3d_forward", "vf_nn_conv3d_backward_data", "vf_nn_conv3d_backward_weight",
+    "vf_nn_conv3d_backward_bias",
     "vf_nn_wgrad_workspace", "vf_learned_param_count", "vf_learned_configure", "vf_learned_info",
     "vf_learned_input", "vf_learned_apply", "vf_level_mask", "vf_mg_propagate", "vf_solve_block",
     "vf_solve_batch", "vf_inside_points", "vf_inside_grid", "vf_element_displacement",
