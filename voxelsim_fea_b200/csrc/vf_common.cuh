@@ -245,21 +245,22 @@ int sym_zchunk(const Grid& g);
 void launch_galerkin_from_fine(const Grid& f, const double* E, const double* mu, const uint8_t* fmask,
                                const Grid& c, double* stencil_c, const double* Gtab, int lame, cudaStream_t st);
 
-// vf_wide.cu -- reach-R Galerkin levels (coarse space with a smoothed prolongation).
-// Scaled symmetric storage of a reach-R stencil, split over G = 8 lanes per
-// node: block u of a node -- the upper blocks s = center + 1 + u (u < NU)
+// vf_wide.cu -- reach-R Galerkin levels (coarse space with a smoothed
+// prolongation) and 27-block ones in the same form.
+// Scaled symmetric storage of a reach-R stencil, split over G lanes per node
+// (8 of 64 slots for reach 2, 4 of 16 for reach 1): block u of a node -- the upper blocks s = center + 1 + u (u < NU)
 // and the diagonal block (u = NU), 9 values each -- belongs to lane u % G,
 // slot u / G; a lane holds NJ blocks (9 NJ values, zero padded).  Storage is
 // warp-chunked over virtual nodes v = p * G + lane: 16-byte chunk j of 32
-// consecutive virtual nodes is contiguous, so the 32 lanes of a warp (4
-// nodes) load one chunk each in one 512-byte transaction.
+// consecutive virtual nodes is contiguous, so the 32 lanes of a warp load one
+// chunk each in one 512-byte transaction.
 template <typename S, int R> struct WideLayout {
   static constexpr int W = 2 * R + 1, NB = W * W * W, NU = NB / 2;
-  static constexpr int G = 8;
+  static constexpr int G = R == 1 ? 4 : 8;
   static constexpr int NBLK = NU + 1;
   static constexpr int NJ = (NBLK + G - 1) / G;
-  static constexpr int NVL = (NJ * 9 + 7) / 8 * 8;
   static constexpr int VPC = 16 / (int)sizeof(S);
+  static constexpr int NVL = (NJ * 9 + VPC - 1) / VPC * VPC;
   static constexpr int NCH = NVL / VPC;
   using Q = typename std::conditional<sizeof(S) == 8, double, float>::type;
   __host__ __device__ static constexpr long long off(long long v, int k) {

@@ -41,13 +41,6 @@ template <> struct Chunk<float, float> {
     v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
   }
 };
-template <> struct Chunk<double, double> {
-  double v[2];
-  __device__ __forceinline__ void load(const double* base) {
-    const double2 w = __ldg(reinterpret_cast<const double2*>(base));
-    v[0] = w.x; v[1] = w.y;
-  }
-};
 
 // ---- rows of a reach-R operator (WideLayout) --------------------------------
 // The linear storage offset of upper block u (positive), or 0 for the diagonal
@@ -80,51 +73,52 @@ template <> __device__ __forceinline__ double chunk_value<double, double>(const 
   return i == 0 ? __hiloint2double((int)c.y, (int)c.x) : __hiloint2double((int)c.w, (int)c.z);
 }
 
-// acc (the rows of node p) += the blocks of lane `lane` (of L::G lanes): own
-// block u = lane + G*JJ applied to node p + shift, and the transposed block u
-// of node p - shift (lane and slot are the same there).  V(shift, up, v) gives
-// D^1/2 u of those nodes: ghost and pad nodes hold zeros, and a reach-2
-// neighbour past the shell lands, in linear storage, on a ghost or pad node of
-// the next row or plane or outside the array (zero as well), so no neighbour
-// needs a test; only the address of the transposed block is kept in the array.
-// The loads of JB slots stand together, ahead of their products.
+// A batch of JB block slots J0 .. J0 + JB - 1 of lane `lane` (of L::G lanes) of
+// node p: own block u = lane + G*J applied to node p + shift, and the transposed
+// block u of node p - shift (lane and slot are the same there).  V(slot, vu, vd)
+// gives D^1/2 u of those nodes; ghost nodes hold zeros, so no neighbour needs a
+// test, only the address of the transposed block is kept in the array.  load()
+// depends on nothing but the node, so it may stand ahead of the staging of u.
 template <typename S> struct WideBatch { static constexpr int JB = sizeof(S) == 2 ? 4 : 2; };
-template <typename S, typename A, typename L, int J0 = 0, typename SH, typename VF>
-__device__ __forceinline__ void wide_rows(const S* __restrict__ stc, int p, int lane, A (&acc)[3], SH shift_of, VF V) {
-  constexpr int VPC = L::VPC, JB = WideBatch<S>::JB;
-  constexpr int C0 = 9 * J0 / VPC, C1 = (9 * (J0 + JB) - 1) / VPC;      // own chunks of the batch
-  constexpr int ND = (9 + VPC - 1) / VPC + 1;                           // chunks a block may straddle
-  const S* own = stc + L::off((long long)p * L::G + lane, 0);
-  uint4 co[C1 - C0 + 1], cd[JB][ND];
-  int sh[JB];
+template <typename S, typename L, int JB> struct RowBatch {
+  static constexpr int VPC = L::VPC;
+  static constexpr int NC = (9 * JB + VPC - 2) / VPC + 1;    // own chunks JB blocks may straddle
+  static constexpr int ND = (9 + VPC - 2) / VPC + 1;         // chunks a block may straddle
+  uint4 co[NC], cd[JB][ND];
+
+  template <int J0> __device__ __forceinline__ void load(const Grid& g, const S* __restrict__ stc, int p, int lane) {
+    constexpr int C0 = 9 * J0 / VPC, C1 = (9 * (J0 + JB) - 1) / VPC;
+    static_assert(C1 - C0 < NC, "chunks of a batch");
+    const S* own = stc + L::off((long long)p * L::G + lane, 0);
 #pragma unroll
-  for (int j = 0; j < JB; ++j) sh[j] = shift_of(lane + L::G * (J0 + j));
+    for (int c = C0; c <= C1; ++c) co[c - C0] = ldg_chunk(own + c * 32 * VPC);
 #pragma unroll
-  for (int c = C0; c <= C1; ++c) co[c - C0] = ldg_chunk(own + c * 32 * VPC);
+    for (int j = 0; j < JB; ++j) {
+      const int k0 = 9 * (J0 + j), q = p - wide_shift<L>(g, lane + L::G * (J0 + j));
+      const S* base = stc + L::off((long long)(q < 0 ? 0 : q) * L::G + lane, 0);
 #pragma unroll
-  for (int j = 0; j < JB; ++j) {
-    const int k0 = 9 * (J0 + j), q = p - sh[j];
-    const S* base = stc + L::off((long long)(q < 0 ? 0 : q) * L::G + lane, 0);
-#pragma unroll
-    for (int c = 0; c < ND; ++c)
-      if (k0 / VPC + c <= (k0 + 8) / VPC) cd[j][c] = ldg_chunk(base + (k0 / VPC + c) * 32 * VPC);
+      for (int c = 0; c < ND; ++c)
+        if (k0 / VPC + c <= (k0 + 8) / VPC) cd[j][c] = ldg_chunk(base + (k0 / VPC + c) * 32 * VPC);
+    }
   }
+  template <int J0, typename A, typename VF> __device__ __forceinline__ void apply(int lane, A (&acc)[3], VF V) const {
+    constexpr int C0 = 9 * J0 / VPC;
 #pragma unroll
-  for (int j = 0; j < JB; ++j) {
-    const int k0 = 9 * (J0 + j);
-    A vu[3], vd[3];
-    V(sh[j], vu, vd);
-    if (lane + L::G * (J0 + j) >= L::NU) vd[0] = vd[1] = vd[2] = (A)0;   // the diagonal block is applied once
+    for (int j = 0; j < JB; ++j) {
+      const int k0 = 9 * (J0 + j);
+      A vu[3], vd[3];
+      V(J0 + j, vu, vd);
+      if (lane + L::G * (J0 + j) >= L::NU) vd[0] = vd[1] = vd[2] = (A)0;   // the diagonal block is applied once
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+      for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int k = k0 + 3 * r + c;
-        acc[r] += chunk_value<S, A>(co[k / VPC - C0], k % VPC) * vu[c];
-        acc[c] += chunk_value<S, A>(cd[j][k / VPC - k0 / VPC], k % VPC) * vd[r];
-      }
+        for (int c = 0; c < 3; ++c) {
+          const int k = k0 + 3 * r + c;
+          acc[r] += chunk_value<S, A>(co[k / VPC - C0], k % VPC) * vu[c];
+          acc[c] += chunk_value<S, A>(cd[j][k / VPC - k0 / VPC], k % VPC) * vd[r];
+        }
+    }
   }
-  if constexpr (J0 + JB < L::NJ) wide_rows<S, A, L, J0 + JB>(stc, p, lane, acc, shift_of, V);
-}
+};
 
 }  // namespace vf

@@ -74,13 +74,13 @@ unsigned long long graph_kernel_nodes(cudaGraph_t g) {
 struct Level {
   Grid g{};
   int zchunk[2] = {0, 0};  // modal kernel, FP32 / FP64: z-planes per CTA (< 0: one even wave)
-  int szchunk[2] = {0, 0}; // marching stencil kernel, FP32 / FP64: z-planes per CTA
+  int szchunk = 0;         // marching stencil kernel (FP32): z-planes per CTA
   uint8_t* mask = nullptr;
   bool galerkin = false;   // operator is the assembled stencil
   double* E64 = nullptr; double* mu64 = nullptr; double* minv64 = nullptr; double* st64 = nullptr;
   float* E32 = nullptr; float* mu32 = nullptr; float* minv32 = nullptr; float* st32 = nullptr;
-  // symmetric scaled stencils (Galerkin levels): 123 values per node + sqrt(diag)
-  // (reach 2: WideLayout, 568 values per node)
+  // symmetric scaled stencils (Galerkin levels) + sqrt(diag): WideLayout, or
+  // SymLayout where row_form says so
   double* sym64 = nullptr; double* sq64 = nullptr;
   float* sym32 = nullptr; __half* sym16 = nullptr; float* sq32 = nullptr;
   // sym64 / sq64 hold the current stencil: built at set-up for an FP64
@@ -254,26 +254,49 @@ int nlev(const vf_solver* s) { return use_mg(s) ? (int)s->L.size() : 1; }
 // ---------------------------------------------------------------------------
 // operator dispatch on one level
 // ---------------------------------------------------------------------------
+// Kernel form and storage of a Galerkin level: rows of nodes (vf_wide.cu,
+// WideLayout) for reach 2, for FP64 and for small levels; the marching kernel
+// (vf_stencil.cu, SymLayout) for the FP32 V-cycle's reach-1 levels of more
+// than 20,000 nodes.  On small levels the march has too few CTAs to hide its
+// loads, on large ones it re-reads fewer values.  An iteration with the march /
+// the rows on level 1: FP32, 17 x 9 x 9 nodes 105 / 101 us, 33 x 17 x 17 152 /
+// 147, 41 x 21 x 21 159 / 156, 49 x 25 x 25 189 / 196, 129 x 65 x 65 1,332 /
+// 1,418; FP64, 41 x 25 x 21 233 / 221, 65 x 33 x 33 473 / 466, 129 x 65 x 65
+// 2,445 / 2,385.
+constexpr long long kRowFormNodes = 20000;
+template <typename T> bool row_form(const Level& l) {
+  return l.reach == 2 || sizeof(T) == 8 || (long long)(l.g.lx + 1) * (l.g.ly + 1) * (l.g.lz + 1) <= kRowFormNodes;
+}
+template <typename T, typename S> size_t sym_count(const Level& l) {
+  if (l.reach == 2) return WideLayout<S, 2>::count(l.g.n);
+  return row_form<T>(l) ? WideLayout<S, 1>::count(l.g.n) : SymLayout<S>::count(l.g.n);
+}
+template <typename T, typename S> void sym_compress(vf_solver* s, Level& l, S* sym, T* sq) {
+  if (l.reach == 2) { launch_wide_compress<S, 2>(l.g, l.st64, l.mask, sym, sq, s->st); return; }
+  if constexpr (sizeof(T) == 4)
+    if (!row_form<T>(l)) { launch_stencil_compress<S>(l.g, l.st64, l.mask, sym, sq, s->st); return; }
+  launch_wide_compress<S, 1>(l.g, l.st64, l.mask, sym, sq, s->st);
+}
+template <typename T, typename S>
+void sym_op(vf_solver* s, Level& l, int epi, const OpArgs& a, const S* sym, const T* sq) {
+  if (l.reach == 2) { launch_wide_op<T, S, 2>(l.g, epi, a, sym, sq, s->st); return; }
+  if constexpr (sizeof(T) == 4)
+    if (!row_form<T>(l)) { launch_stencil_sym_op<T, S>(l.g, epi, a, sym, sq, l.szchunk, s->st); return; }
+  launch_wide_op<T, S, 1>(l.g, epi, a, sym, sq, s->st);
+}
+
 template <typename T> void level_sym_op(vf_solver* s, Level& l, int epi, const OpArgs& a);
 void compress_sym64(vf_solver* s, Level& l) {
-  if (l.reach == 2) launch_wide_compress<double, 2>(l.g, l.st64, l.mask, l.sym64, l.sq64, s->st);
-  else launch_stencil_compress<double>(l.g, l.st64, l.mask, l.sym64, l.sq64, s->st);
+  sym_compress<double, double>(s, l, l.sym64, l.sq64);
   l.sym64_ok = true;
 }
 template <> void level_sym_op<double>(vf_solver* s, Level& l, int epi, const OpArgs& a) {
   if (!l.sym64_ok) compress_sym64(s, l);
-  if (l.reach == 2) launch_wide_op<double, double, 2>(l.g, epi, a, l.sym64, l.sq64, s->st);
-  else launch_stencil_sym_op<double, double>(l.g, epi, a, l.sym64, l.sq64, l.szchunk[1], s->st);
+  sym_op<double, double>(s, l, epi, a, l.sym64, l.sq64);
 }
 template <> void level_sym_op<float>(vf_solver* s, Level& l, int epi, const OpArgs& a) {
-  if (l.reach == 2) {
-    if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) launch_wide_op<float, __half, 2>(l.g, epi, a, l.sym16, l.sq32, s->st);
-    else launch_wide_op<float, float, 2>(l.g, epi, a, l.sym32, l.sq32, s->st);
-  } else if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) {
-    launch_stencil_sym_op<float, __half>(l.g, epi, a, l.sym16, l.sq32, l.szchunk[0], s->st);
-  } else {
-    launch_stencil_sym_op<float, float>(l.g, epi, a, l.sym32, l.sq32, l.szchunk[0], s->st);
-  }
+  if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) sym_op<float, __half>(s, l, epi, a, l.sym16, l.sq32);
+  else sym_op<float, float>(s, l, epi, a, l.sym32, l.sq32);
 }
 
 int auto_zchunk(const Grid& g, int requested);
@@ -793,18 +816,11 @@ int build_levels(vf_solver* s) {
       VF_ALLOC(l.st64, 9 * nblk * n);
       if (s->o.coarse_storage == VF_STENCIL_FULL) VF_ALLOC(l.st32, 243 * n);
       else {
-        using W64 = WideLayout<double, 2>;
-        using W32 = WideLayout<float, 2>;
-        using W16 = WideLayout<__half, 2>;
-        const bool wide = l.reach == 2;
-        const size_t c64 = wide ? W64::count(n) : SymLayout<double>::count(n);
-        const size_t c32 = wide ? W32::count(n) : SymLayout<float>::count(n);
-        const size_t c16 = wide ? W16::count(n) : SymLayout<__half>::count(n);
-        VF_ALLOC(l.sym64, c64);
+        VF_ALLOC(l.sym64, (sym_count<double, double>(l)));
         VF_ALLOC(l.sq64, 3 * n);
         VF_ALLOC(l.sq32, 3 * n);
-        if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) VF_ALLOC(l.sym16, c16);
-        else VF_ALLOC(l.sym32, c32);
+        if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) VF_ALLOC(l.sym16, (sym_count<float, __half>(l)));
+        else VF_ALLOC(l.sym32, (sym_count<float, float>(l)));
       }
     }
     for (int k = 0; k < 4; ++k) {
@@ -911,11 +927,11 @@ template <typename T>
 int autotune_level(vf_solver* s, int li, int epi, cudaEvent_t t0, cudaEvent_t t1) {
   Level& l = s->L[li];
   constexpr int q = sizeof(T) == 8 ? 1 : 0;
-  const bool stencil = l.galerkin && s->o.coarse_storage != VF_STENCIL_FULL && l.reach == 1;
+  const bool stencil = l.galerkin && s->o.coarse_storage != VF_STENCIL_FULL && !row_form<T>(l);
   const bool modal = !l.galerkin && s->o.fine_kernel == VF_FINE_MODAL;
   if (!stencil && !modal) return VF_OK;
   if (modal && s->o.modal_zchunk != 0) return VF_OK;   // fixed by the caller
-  int& choice = stencil ? l.szchunk[q] : l.zchunk[q];
+  int& choice = stencil ? l.szchunk : l.zchunk[q];
   const auto key = std::make_tuple(l.g.lx, l.g.ly, l.g.lz, (stencil ? 1 + s->o.coarse_storage : 0) + 8 * q);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1009,7 +1025,7 @@ int upload_tables(vf_solver* s) {
   s->mc_lame = vf::modal_constants(s->nu, true);
   for (auto& l : s->L) {
     l.zchunk[0] = l.zchunk[1] = auto_zchunk(l.g, s->o.modal_zchunk);
-    l.szchunk[0] = l.szchunk[1] = sym_zchunk(l.g);
+    l.szchunk = sym_zchunk(l.g);
   }
   std::vector<double> G(8 * 576), GL(16 * 576);
   galerkin_child_tables(s->tab, G.data());
@@ -1431,20 +1447,11 @@ int vf_set_material(vf_solver* s, const double* E, const double* nu_elem, uint32
       if (lame) launch_convert<double, float>(l.mu64, l.mu32, n, s->st);
     } else if (s->o.coarse_storage == VF_STENCIL_FULL) {
       launch_convert<double, float>(l.st64, l.st32, 243 * n, s->st);
-    } else if (l.reach == 2) {
-      l.sym64_ok = false;
-      if (s->o.precision == VF_PREC_FP64) compress_sym64(s, l);
-      if (s->o.coarse_storage == VF_STENCIL_SYM_HALF)
-        launch_wide_compress<__half, 2>(l.g, l.st64, l.mask, l.sym16, l.sq32, s->st);
-      else
-        launch_wide_compress<float, 2>(l.g, l.st64, l.mask, l.sym32, l.sq32, s->st);
     } else {
       l.sym64_ok = false;
       if (s->o.precision == VF_PREC_FP64) compress_sym64(s, l);
-      if (s->o.coarse_storage == VF_STENCIL_SYM_HALF)
-        launch_stencil_compress<__half>(l.g, l.st64, l.mask, l.sym16, l.sq32, s->st);
-      else
-        launch_stencil_compress<float>(l.g, l.st64, l.mask, l.sym32, l.sq32, s->st);
+      if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) sym_compress<float, __half>(s, l, l.sym16, l.sq32);
+      else sym_compress<float, float>(s, l, l.sym32, l.sq32);
     }
     launch_convert<double, float>(l.minv64, l.minv32, 3 * n, s->st);
     finalized[i] = 1;
@@ -2264,11 +2271,9 @@ void share_operator(vf_solver* c, const vf_solver* m) {
   for (size_t i = 0; i < c->L.size(); ++i) {
     Level& d = c->L[i];
     const Level& sl = m->L[i];
-    d.g = sl.g; 
-    for (int q = 0; q < 2; ++q) {
-      d.zchunk[q] = sl.zchunk[q];
-      d.szchunk[q] = sl.szchunk[q];
-    }
+    d.g = sl.g;
+    for (int q = 0; q < 2; ++q) d.zchunk[q] = sl.zchunk[q];
+    d.szchunk = sl.szchunk;
     d.mask = sl.mask; d.galerkin = sl.galerkin;
     d.E64 = sl.E64; d.mu64 = sl.mu64; d.minv64 = sl.minv64; d.st64 = sl.st64;
     d.E32 = sl.E32; d.mu32 = sl.mu32; d.minv32 = sl.minv32; d.st32 = sl.st32;

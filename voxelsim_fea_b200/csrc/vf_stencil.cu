@@ -462,7 +462,8 @@ void launch_stencil_diag(const Grid& c, double* stencil, const uint8_t* cmask, d
 }
 
 // ---------------------------------------------------------------------------
-// Symmetric, diagonally scaled Galerkin stencils (default coarse storage).
+// Symmetric, diagonally scaled Galerkin stencils (default coarse storage), the
+// form of the FP32 V-cycle's large 27-block levels (vf_wide.cu has the others).
 //
 // A Galerkin operator is symmetric, so only the diagonal block (6 values) and
 // the 13 "upper" neighbour blocks (offsets s = 14..26, 9 values each) are
@@ -700,7 +701,6 @@ void launch_stencil_compress(const Grid& g, const double* st, const uint8_t* mas
 }
 template void launch_stencil_compress<__half>(const Grid&, const double*, const uint8_t*, __half*, float*, cudaStream_t);
 template void launch_stencil_compress<float>(const Grid&, const double*, const uint8_t*, float*, float*, cudaStream_t);
-template void launch_stencil_compress<double>(const Grid&, const double*, const uint8_t*, double*, double*, cudaStream_t);
 
 // z-planes per CTA of the marching stencil kernel: about 4 CTAs per SM.
 int sym_zchunk(const Grid& g) {
@@ -723,6 +723,5 @@ void launch_stencil_sym_op(const Grid& g, int epi, const OpArgs& a, const S* stc
 }
 template void launch_stencil_sym_op<float, __half>(const Grid&, int, const OpArgs&, const __half*, const float*, int, cudaStream_t);
 template void launch_stencil_sym_op<float, float>(const Grid&, int, const OpArgs&, const float*, const float*, int, cudaStream_t);
-template void launch_stencil_sym_op<double, double>(const Grid&, int, const OpArgs&, const double*, const double*, int, cudaStream_t);
 
 }  // namespace vf

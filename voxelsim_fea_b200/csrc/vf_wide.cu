@@ -31,8 +31,8 @@
 // Full stencils: st[(s*9 + 3r + c) * n + p], s = ((dz+R)*W + (dy+R))*W + (dx+R),
 // W = 2R+1: coupling of DOF r of node p with DOF c of node p + (dx,dy,dz).
 //
-// Apply (V-cycle): symmetric, diagonally scaled storage as on the 27-block
-// levels (vf_stencil.cu) -- the diagonal block (6 values) and the upper
+// Apply (V-cycle), also of the 27-block levels in FP64 and of the small ones:
+// symmetric, diagonally scaled storage -- the diagonal block and the upper
 // blocks s > center (9 values each) of A~ = D^-1/2 A D^-1/2, FP16 for the
 // FP32 V-cycle, warp-chunked so a warp loads one 16-byte chunk of 32
 // consecutive nodes at once; the lower blocks are read transposed from the
@@ -583,21 +583,24 @@ __global__ void k_wide_compress(Grid g, const double* __restrict__ st, const uin
 
 // y = mask(D^1/2 A~ D^1/2 u) with the epilogues of the other level kernels
 // (APPLY, SMOOTH with the Chebyshev step fields, RESID; a null rhs reads as
-// zero; no fused dot product: the PCG's reductions run on level 0).  G = 8
+// zero; no fused dot product: the PCG's reductions run on level 0).  L::G
 // lanes per node: each lane applies its own blocks and the transposed blocks
 // of the same lane and slot of the lower neighbours, the partial sums meet
 // through warp shuffles, and lanes 0..2 write component 0..2 of the node.
 //
-// A CTA owns 16 nodes of a row, one round of its threads: it stages v = D^1/2 u
-// of them and their reach-2 halo in shared memory with one set of loads, and
-// the operator's loads depend on no branch and no table in global memory
-// (wide_rows).  Bound by the latency of those loads on small levels and by the
-// L1 on large ones.  Against a form that walked the 8 block slots of a lane
-// behind bounds tests and read u and the scale from global memory at every
-// neighbour: 64x32x32 part 185 -> 165 us an iteration, 96x80x64 315 -> 303,
-// 128x64x64 FP64 534 -> 520, 256x128x128 1,401 -> 1,381.  Larger tiles (16 x 2 x 2,
-// 16 x 4 x 4 nodes, several rounds) were no faster at any size: fewer CTAs to
-// hide the loads.
+// A CTA owns 8 (reach 2) or 16 (reach 1) nodes of a row, one round of its 64
+// threads: it stages v = D^1/2 u of them and their halo in shared memory with
+// one set of loads, and the operator's loads depend on no branch, no table and
+// not on u: the first batch is issued before anything else (RowBatch).  Bound
+// by the latency of the loads on small levels and by the L1 on large ones.
+// Against a form that walked the 8 block slots of a lane behind bounds tests
+// and read u and the scale from global memory at every neighbour: 64x32x32
+// part 185 -> 165 us an iteration, 96x80x64 315 -> 303, 128x64x64 FP64 534 ->
+// 520, 256x128x128 1,401 -> 1,381.  The first batch ahead of the staging: 162 ->
+// 153, 299 -> 286, 518 -> 507, 1,345 -> 1,333.  8 nodes a CTA instead of 16 on the
+// reach-2 levels: 96x48x48 199 -> 189, 128x64x64 FP64 483 -> 466, others equal;
+// larger tiles (32 x 1, 16 x 2 x 2, 16 x 4 x 4 nodes) and the slots split over
+// 2 or 4 times the threads were slower or equal at every size.
 template <typename T> struct Node3;   // 3 values of a node in shared memory
 template <> struct Node3<float> {
   float4 v;
@@ -609,19 +612,28 @@ template <> struct Node3<double> {
   __device__ __forceinline__ void get(double (&o)[3]) const { o[0] = v[0]; o[1] = v[1]; o[2] = v[2]; }
   __device__ __forceinline__ void set(double a, double b, double c) { v[0] = a; v[1] = b; v[2] = c; }
 };
-constexpr int kWideTX = 16;
+constexpr int wide_tx(int R) { return R == 1 ? 16 : 8; }   // nodes of a CTA
+
+// f(integral constants I, I + STEP, ... < N)
+template <int I, int N, int STEP, typename F> __device__ __forceinline__ void for_slots(F f) {
+  if constexpr (I < N) {
+    f(std::integral_constant<int, I>{});
+    for_slots<I + STEP, N, STEP>(f);
+  }
+}
 
 template <typename T, typename S, int R, int EPI>
-__global__ void __launch_bounds__(kWideTX * 8)
+__global__ void __launch_bounds__(wide_tx(R) * WideLayout<S, R>::G)
     k_wide_op(Grid g, OpArgs a, const S* __restrict__ stc, const T* __restrict__ sqd) {
   pdl_enter();
   using L = WideLayout<S, R>;
   using A = T;
-  constexpr int G = L::G, TX = kWideTX, HX = TX + 2 * R, HY = 1 + 2 * R, HZ = 1 + 2 * R, NT = TX * G;
+  constexpr int G = L::G, TX = wide_tx(R), HX = TX + 2 * R, HY = 1 + 2 * R, HZ = 1 + 2 * R, NT = TX * G;
+  constexpr int JB = WideBatch<S>::JB;
   __shared__ Node3<T> sv[HX * HY * HZ];
-  __shared__ int s_shift[G * L::NJ], s_delta[G * L::NJ];
+  __shared__ int s_delta[G * L::NJ];
   KrylovState* ks = a.ks;
-  if (ks && ks->done) return;
+  const int done = ks ? ks->done : 0;
   const T* __restrict__ u = (const T*)a.u;
   T* out = (T*)a.out;
   const T* b = (const T*)a.b;
@@ -632,10 +644,15 @@ __global__ void __launch_bounds__(kWideTX * 8)
   const T c1 = a.c1_dev ? (T)(*a.c1_dev) : (T)0;
   const int ntx = (g.lx + TX) / TX;
   const int X0 = (blockIdx.x % ntx) * TX, y = blockIdx.x / ntx % (g.ly + 1), z = blockIdx.x / (ntx * (g.ly + 1));
+  const int tx = threadIdx.x / G, lane = threadIdx.x % G, x = X0 + tx;
+  const bool in = inside(g, x, y, z);
+  const int p = in ? g.idx(x, y, z) : 0;
+  RowBatch<S, L, JB> rb;
+  rb.template load<0>(g, stc, p, lane);
+  if (done) return;
   if (threadIdx.x < G * L::NJ) {
     constexpr int W = L::W, SC = L::NB / 2;
     const int uu = threadIdx.x, s = uu < L::NU ? SC + 1 + uu : SC;
-    s_shift[uu] = wide_shift<L>(g, uu);
     s_delta[uu] = ((s / (W * W) - R) * HY + (s / W) % W - R) * HX + s % W - R;
   }
   // halo nodes outside the grid read as zero, like the ghost shell
@@ -652,9 +669,6 @@ __global__ void __launch_bounds__(kWideTX * 8)
     }
     if (i < HX * HY * HZ) sv[i].set(v0, v1, v2);
   }
-  const int tx = threadIdx.x / G, lane = threadIdx.x % G, x = X0 + tx;
-  const bool in = inside(g, x, y, z);
-  const int p = in ? g.idx(x, y, z) : 0;
   const int c = lane < 3 ? lane : 0;
   const long long pc = 3LL * p + c;
   T bc = 0, u0 = 0, mi = 0, dp = 0;
@@ -670,15 +684,16 @@ __global__ void __launch_bounds__(kWideTX * 8)
   __syncthreads();
   A acc[3] = {(A)0, (A)0, (A)0};
   const int c0 = (R * HY + R) * HX + tx + R;
-  int slot = 0;
-  auto SH = [&](int uu) { return s_shift[uu]; };
-  auto V = [&](int, A (&vu)[3], A (&vd)[3]) {
+  auto V = [&](int slot, A (&vu)[3], A (&vd)[3]) {
     const int d = s_delta[lane + G * slot];
-    ++slot;
     sv[c0 + d].get(vu);
     sv[c0 - d].get(vd);
   };
-  wide_rows<S, A, L>(stc, p, lane, acc, SH, V);
+  rb.template apply<0>(lane, acc, V);
+  for_slots<JB, L::NJ, JB>([&](auto j) {
+    rb.template load<decltype(j)::value>(g, stc, p, lane);
+    rb.template apply<decltype(j)::value>(lane, acc, V);
+  });
 #pragma unroll
   for (int o = 1; o < G; o <<= 1) {
 #pragma unroll
@@ -791,21 +806,24 @@ void launch_wide_compress(const Grid& g, const double* st, const uint8_t* mask, 
                           typename WideLayout<S, R>::Q* sqrtd, cudaStream_t st_) {
   launch_k(k_wide_compress<S, R>, blocks_for((long long)g.n * WideLayout<S, R>::G * WideLayout<S, R>::NJ, 128), 128, 0, st_, g, st, mask, stc, sqrtd);
 }
-template void launch_wide_compress<__half, 2>(const Grid&, const double*, const uint8_t*, __half*, float*, cudaStream_t);
-template void launch_wide_compress<float, 2>(const Grid&, const double*, const uint8_t*, float*, float*, cudaStream_t);
-template void launch_wide_compress<double, 2>(const Grid&, const double*, const uint8_t*, double*, double*, cudaStream_t);
 
 template <typename T, typename S, int R>
 void launch_wide_op(const Grid& g, int epi, const OpArgs& a, const S* stc, const T* sqrtd, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((g.lx + kWideTX) / kWideTX) * (g.ly + 1) * (g.lz + 1);
-  if (epi == EPI_APPLY) launch_pdl(k_wide_op<T, S, R, EPI_APPLY>, blocks, kWideTX * 8, 0, st, g, a, stc, sqrtd);
-  else if (epi == EPI_SMOOTH) launch_pdl(k_wide_op<T, S, R, EPI_SMOOTH>, blocks, kWideTX * 8, 0, st, g, a, stc, sqrtd);
-  else launch_pdl(k_wide_op<T, S, R, EPI_RESID>, blocks, kWideTX * 8, 0, st, g, a, stc, sqrtd);
+  constexpr int TX = wide_tx(R), NT = TX * WideLayout<S, R>::G;
+  const unsigned blocks = (unsigned)((g.lx + TX) / TX) * (g.ly + 1) * (g.lz + 1);
+  if (epi == EPI_APPLY) launch_pdl(k_wide_op<T, S, R, EPI_APPLY>, blocks, NT, 0, st, g, a, stc, sqrtd);
+  else if (epi == EPI_SMOOTH) launch_pdl(k_wide_op<T, S, R, EPI_SMOOTH>, blocks, NT, 0, st, g, a, stc, sqrtd);
+  else launch_pdl(k_wide_op<T, S, R, EPI_RESID>, blocks, NT, 0, st, g, a, stc, sqrtd);
 }
-template void launch_wide_op<float, __half, 2>(const Grid&, int, const OpArgs&, const __half*, const float*, cudaStream_t);
-template void launch_wide_op<float, float, 2>(const Grid&, int, const OpArgs&, const float*, const float*, cudaStream_t);
-template void launch_wide_op<double, double, 2>(const Grid&, int, const OpArgs&, const double*, const double*,
-                                                cudaStream_t);
+#define VF_INST_WIDE(T, S)                                                                                          \
+  template void launch_wide_op<T, S, 1>(const Grid&, int, const OpArgs&, const S*, const T*, cudaStream_t);         \
+  template void launch_wide_op<T, S, 2>(const Grid&, int, const OpArgs&, const S*, const T*, cudaStream_t);         \
+  template void launch_wide_compress<S, 1>(const Grid&, const double*, const uint8_t*, S*, T*, cudaStream_t);       \
+  template void launch_wide_compress<S, 2>(const Grid&, const double*, const uint8_t*, S*, T*, cudaStream_t);
+VF_INST_WIDE(float, __half)
+VF_INST_WIDE(float, float)
+VF_INST_WIDE(double, double)
+#undef VF_INST_WIDE
 
 int wide_dense_assemble(const Grid& c, int R, const double* stencil, const uint8_t* cmask, double* A, int n,
                         cudaStream_t st) {
