@@ -32,19 +32,47 @@ template <> struct V16<double> {
   __device__ __forceinline__ static V mul(V a, V b) { return make_double2(a.x * b.x, a.y * b.y); }
 };
 
+// A pass over nv 16-byte (or larger) items: op(item, i) for the items this
+// thread owns, in order.  Two items are loaded at a time, the first two before
+// go() looks at the solver state: short vectors are bound by the chain state ->
+// loads -> reduction, and the two read latencies pass at once.  (An item past
+// the end is loaded from index 0 and dropped.)  False: go() said no.  With the
+// shorter reduction tail (vf_reduce.cuh) a Jacobi iteration on 61x43x37 took 20.4
+// us instead of 22.6, on 31x17x19 15.4 instead of 19.7, a V-cycle PCG iteration on
+// 64x32x32 142.5 instead of 146.6; long vectors are as fast either way.
+template <typename LD, typename GO, typename OP>
+__device__ __forceinline__ bool vec_pass(long long nv, LD ld, GO go, OP op) {
+  const long long step = (long long)gridDim.x * blockDim.x;
+  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  auto a = ld(i < nv ? i : 0), b = ld(i + step < nv ? i + step : 0);
+  if (!go()) return false;
+  while (i < nv) {
+    op(a, i);
+    if (i + step < nv) op(b, i + step);
+    i += 2 * step;
+    if (i < nv) {
+      a = ld(i);
+      b = ld(i + step < nv ? i + step : 0);
+    }
+  }
+  return true;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_dot(long long n3, const T* __restrict__ a, const T* __restrict__ b,
                                                      double* partials, KrylovState* ks, int slot) {
   pdl_enter();
-  if (ks->done && slot != SLOT_FNORM && slot != SLOT_RZ_INIT && slot != SLOT_OUTER && slot != SLOT_PLAIN) return;
   using H = V16<T>;
   using V = typename H::V;
-  const long long nv = n3 / H::W;
   const V* av = reinterpret_cast<const V*>(a);
   const V* bv = reinterpret_cast<const V*>(b);
+  struct I { V a, b; };
   double s = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x)
-    s += H::dot(__ldg(av + i), __ldg(bv + i));
+  const bool go = vec_pass(
+      n3 / H::W, [&](long long i) { return I{__ldg(av + i), __ldg(bv + i)}; },
+      [&] { return !(ks->done && slot != SLOT_FNORM && slot != SLOT_RZ_INIT && slot != SLOT_OUTER && slot != SLOT_PLAIN); },
+      [&](const I& v, long long) { s += H::dot(v.a, v.b); });
+  if (!go) return;
   reduce_and_finalize(s, partials, ks, slot, nullptr);
 }
 
@@ -53,23 +81,25 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update(long long n3, T* __re
                                                            T* __restrict__ r, const T* __restrict__ Ap,
                                                            double* partials, KrylovState* ks, double* hist) {
   pdl_enter();
-  if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
-  const T alpha = (T)ks->alpha;
-  const long long nv = n3 / H::W;
   V* xv = reinterpret_cast<V*>(x);
   V* rv = reinterpret_cast<V*>(r);
   const V* pv = reinterpret_cast<const V*>(p);
   const V* av = reinterpret_cast<const V*>(Ap);
+  struct I { V x, p, r, a; };
+  T alpha = (T)0;
   double s = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
-    const V pi = __ldg(pv + i), ai = __ldg(av + i);
-    xv[i] = H::axpy(alpha, pi, xv[i]);
-    const V ri = H::axpy(-alpha, ai, rv[i]);
-    rv[i] = ri;
-    s += H::dot(ri, ri);
-  }
+  const bool go = vec_pass(
+      n3 / H::W, [&](long long i) { return I{xv[i], __ldg(pv + i), rv[i], __ldg(av + i)}; },
+      [&] { alpha = (T)ks->alpha; return !ks->done; },
+      [&](const I& v, long long i) {
+        xv[i] = H::axpy(alpha, v.p, v.x);
+        const V ri = H::axpy(-alpha, v.a, v.r);
+        rv[i] = ri;
+        s += H::dot(ri, ri);
+      });
+  if (!go) return;
   reduce_and_finalize(s, partials, ks, SLOT_RR, hist);
 }
 
@@ -78,19 +108,20 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_dot_fcg(long long n3, const T* __restrict__ r, const T* __restrict__ z,
                                                          const T* __restrict__ Ap, double* partials, KrylovState* ks) {
   pdl_enter();
-  if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
-  const long long nv = n3 / H::W;
   const V* rv = reinterpret_cast<const V*>(r);
   const V* zv = reinterpret_cast<const V*>(z);
   const V* av = reinterpret_cast<const V*>(Ap);
+  struct I { V r, z, a; };
   double s1 = 0.0, s2 = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
-    const V zz = __ldg(zv + i);
-    s1 += H::dot(__ldg(rv + i), zz);
-    s2 += H::dot(zz, __ldg(av + i));
-  }
+  const bool go = vec_pass(
+      n3 / H::W, [&](long long i) { return I{__ldg(rv + i), __ldg(zv + i), __ldg(av + i)}; }, [&] { return !ks->done; },
+      [&](const I& v, long long) {
+        s1 += H::dot(v.r, v.z);
+        s2 += H::dot(v.z, v.a);
+      });
+  if (!go) return;
   reduce2_and_finalize(s1, s2, partials, ks, SLOT_FCG);
 }
 
@@ -98,16 +129,21 @@ template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_p_update(long long n3, T* __restrict__ p, const T* __restrict__ z,
                                                           const KrylovState* ks) {
   pdl_enter();
-  if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
-  const bool restart = ks->restart != 0;
-  const T beta = restart ? (T)0 : (T)ks->beta;
-  const long long nv = n3 / H::W;
   V* pv = reinterpret_cast<V*>(p);
   const V* zv = reinterpret_cast<const V*>(z);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x)
-    pv[i] = restart ? __ldg(zv + i) : H::axpy(beta, pv[i], __ldg(zv + i));
+  struct I { V p, z; };
+  bool restart = false;
+  T beta = (T)0;
+  vec_pass(
+      n3 / H::W, [&](long long i) { return I{pv[i], __ldg(zv + i)}; },
+      [&] {
+        restart = ks->restart != 0;
+        beta = restart ? (T)0 : (T)ks->beta;
+        return !ks->done;
+      },
+      [&](const I& v, long long i) { pv[i] = restart ? v.z : H::axpy(beta, v.p, v.z); });
 }
 
 // FP64 outer PCG around an FP32 preconditioner: the FP64 recurrences of x,
@@ -121,22 +157,23 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update_split(long long n3, d
                                                                  const double* __restrict__ Ap, float* __restrict__ r32,
                                                                  double* partials, KrylovState* ks, double* hist) {
   pdl_enter();
-  if (ks->done) return;
-  const double alpha = ks->alpha;
-  const long long n4 = n3 / 4;
   double2* rv = reinterpret_cast<double2*>(r);
   const double2* av = reinterpret_cast<const double2*>(Ap);
   float4* r4 = reinterpret_cast<float4*>(r32);
-  double s = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const double2 a0 = __ldg(av + 2 * i), a1 = __ldg(av + 2 * i + 1);
-    double2 q0 = rv[2 * i], q1 = rv[2 * i + 1];
-    q0.x = fma(-alpha, a0.x, q0.x); q0.y = fma(-alpha, a0.y, q0.y);
-    q1.x = fma(-alpha, a1.x, q1.x); q1.y = fma(-alpha, a1.y, q1.y);
-    rv[2 * i] = q0; rv[2 * i + 1] = q1;
-    r4[i] = make_float4((float)q0.x, (float)q0.y, (float)q1.x, (float)q1.y);
-    s += q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
-  }
+  struct I { double2 a0, a1, q0, q1; };
+  double alpha = 0.0, s = 0.0;
+  const bool go = vec_pass(
+      n3 / 4, [&](long long i) { return I{__ldg(av + 2 * i), __ldg(av + 2 * i + 1), rv[2 * i], rv[2 * i + 1]}; },
+      [&] { alpha = ks->alpha; return !ks->done; },
+      [&](const I& v, long long i) {
+        double2 q0 = v.q0, q1 = v.q1;
+        q0.x = fma(-alpha, v.a0.x, q0.x); q0.y = fma(-alpha, v.a0.y, q0.y);
+        q1.x = fma(-alpha, v.a1.x, q1.x); q1.y = fma(-alpha, v.a1.y, q1.y);
+        rv[2 * i] = q0; rv[2 * i + 1] = q1;
+        r4[i] = make_float4((float)q0.x, (float)q0.y, (float)q1.x, (float)q1.y);
+        s += q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y;
+      });
+  if (!go) return;
   reduce_and_finalize(s, partials, ks, SLOT_RR, hist);
 }
 
@@ -148,42 +185,43 @@ __global__ void __launch_bounds__(kVecThreads) k_p_update_split(long long n3, do
                                                                 double* __restrict__ p, const float* __restrict__ z,
                                                                 KrylovState* ks) {
   pdl_enter();
-  const int it = ks->it;
-  const bool do_x = it > ks->x_it;
-  const bool do_p = !ks->done;
-  if (!do_x && !do_p) return;
-  const double alpha = do_x ? ks->alpha : 0.0;
-  const bool restart = ks->restart != 0;
-  const double beta = restart ? 0.0 : ks->beta;
-  const long long n4 = n3 / 4;
   double2* xv = reinterpret_cast<double2*>(x);
   double2* pv = reinterpret_cast<double2*>(p);
   const float4* zv = reinterpret_cast<const float4*>(z);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    double2 p0 = pv[2 * i], p1 = pv[2 * i + 1];
-    if (do_x) {
-      double2 x0 = xv[2 * i], x1 = xv[2 * i + 1];
-      x0.x = fma(alpha, p0.x, x0.x); x0.y = fma(alpha, p0.y, x0.y);
-      x1.x = fma(alpha, p1.x, x1.x); x1.y = fma(alpha, p1.y, x1.y);
-      xv[2 * i] = x0; xv[2 * i + 1] = x1;
-    }
-    if (do_p) {
-      const float4 zz = __ldg(zv + i);
-      p0.x = fma(beta, p0.x, (double)zz.x); p0.y = fma(beta, p0.y, (double)zz.y);
-      p1.x = fma(beta, p1.x, (double)zz.z); p1.y = fma(beta, p1.y, (double)zz.w);
-      pv[2 * i] = p0; pv[2 * i + 1] = p1;
-    }
-  }
+  struct I { double2 p0, p1, x0, x1; float4 z; };
+  int it = 0;
+  bool do_x = false, do_p = false;
+  double alpha = 0.0, beta = 0.0;
+  const bool go = vec_pass(
+      n3 / 4, [&](long long i) { return I{pv[2 * i], pv[2 * i + 1], xv[2 * i], xv[2 * i + 1], __ldg(zv + i)}; },
+      [&] {
+        it = ks->it;
+        do_x = it > ks->x_it;
+        do_p = !ks->done;
+        alpha = do_x ? ks->alpha : 0.0;
+        beta = ks->restart != 0 ? 0.0 : ks->beta;
+        return do_x || do_p;
+      },
+      [&](const I& v, long long i) {
+        double2 p0 = v.p0, p1 = v.p1;
+        if (do_x) {
+          double2 x0 = v.x0, x1 = v.x1;
+          x0.x = fma(alpha, p0.x, x0.x); x0.y = fma(alpha, p0.y, x0.y);
+          x1.x = fma(alpha, p1.x, x1.x); x1.y = fma(alpha, p1.y, x1.y);
+          xv[2 * i] = x0; xv[2 * i + 1] = x1;
+        }
+        if (do_p) {
+          p0.x = fma(beta, p0.x, (double)v.z.x); p0.y = fma(beta, p0.y, (double)v.z.y);
+          p1.x = fma(beta, p1.x, (double)v.z.z); p1.y = fma(beta, p1.y, (double)v.z.w);
+          pv[2 * i] = p0; pv[2 * i + 1] = p1;
+        }
+      });
+  if (!go) return;
   if (do_x) {   // last CTA: this iteration's alpha p is in x
     __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      const unsigned prev = atomicAdd(&ks->counter[11], 1u);
-      if (prev == gridDim.x - 1) {
-        ks->x_it = it;
-        ks->counter[11] = 0u;
-        __threadfence();
-      }
+    if (threadIdx.x == 0 && atomicAdd(&ks->counter[11], 1u) == gridDim.x - 1) {
+      ks->x_it = it;
+      ks->counter[11] = 0u;
     }
   }
 }
@@ -194,18 +232,20 @@ __global__ void __launch_bounds__(kVecThreads) k_dot_fcg_split(long long n3, con
                                                                const double* __restrict__ Ap, double* partials,
                                                                KrylovState* ks) {
   pdl_enter();
-  if (ks->done) return;
-  const long long n4 = n3 / 4;
   const float4* rv = reinterpret_cast<const float4*>(r);
   const float4* zv = reinterpret_cast<const float4*>(z);
   const double2* av = reinterpret_cast<const double2*>(Ap);
+  struct I { float4 r, z; double2 a0, a1; };
   double s1 = 0.0, s2 = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const float4 rr = __ldg(rv + i), zz = __ldg(zv + i);
-    const double2 a0 = __ldg(av + 2 * i), a1 = __ldg(av + 2 * i + 1);
-    s1 += (double)rr.x * zz.x + (double)rr.y * zz.y + (double)rr.z * zz.z + (double)rr.w * zz.w;
-    s2 += (double)zz.x * a0.x + (double)zz.y * a0.y + (double)zz.z * a1.x + (double)zz.w * a1.y;
-  }
+  const bool go = vec_pass(
+      n3 / 4, [&](long long i) { return I{__ldg(rv + i), __ldg(zv + i), __ldg(av + 2 * i), __ldg(av + 2 * i + 1)}; },
+      [&] { return !ks->done; },
+      [&](const I& v, long long) {
+        const float4 rr = v.r, zz = v.z;
+        s1 += (double)rr.x * zz.x + (double)rr.y * zz.y + (double)rr.z * zz.z + (double)rr.w * zz.w;
+        s2 += (double)zz.x * v.a0.x + (double)zz.y * v.a0.y + (double)zz.z * v.a1.x + (double)zz.w * v.a1.y;
+      });
+  if (!go) return;
   reduce2_and_finalize(s1, s2, partials, ks, SLOT_FCG);
 }
 
@@ -242,25 +282,27 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_update(long long n3, T* 
                                                                const T* __restrict__ minv, double* partials,
                                                                KrylovState* ks, double* hist) {
   pdl_enter();
-  if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
-  const T alpha = (T)ks->alpha;
-  const long long nv = n3 / H::W;
   V* xv = reinterpret_cast<V*>(x);
   V* rv = reinterpret_cast<V*>(r);
   const V* pv = reinterpret_cast<const V*>(p);
   const V* av = reinterpret_cast<const V*>(Ap);
   const V* mv = reinterpret_cast<const V*>(minv);
+  struct I { V x, p, r, a, m; };
+  T alpha = (T)0;
   double s = 0.0, sz = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
-    const V pi = __ldg(pv + i), ai = __ldg(av + i), mi = __ldg(mv + i);
-    xv[i] = H::axpy(alpha, pi, xv[i]);
-    const V ri = H::axpy(-alpha, ai, rv[i]);
-    rv[i] = ri;
-    s += H::dot(ri, ri);
-    sz += H::dot(ri, H::mul(mi, ri));
-  }
+  const bool go = vec_pass(
+      n3 / H::W, [&](long long i) { return I{xv[i], __ldg(pv + i), rv[i], __ldg(av + i), __ldg(mv + i)}; },
+      [&] { alpha = (T)ks->alpha; return !ks->done; },
+      [&](const I& v, long long i) {
+        xv[i] = H::axpy(alpha, v.p, v.x);
+        const V ri = H::axpy(-alpha, v.a, v.r);
+        rv[i] = ri;
+        s += H::dot(ri, ri);
+        sz += H::dot(ri, H::mul(v.m, ri));
+      });
+  if (!go) return;
   reduce_rr_rz(s, sz, partials, ks, hist);
 }
 
@@ -270,19 +312,25 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_direction(long long n3, 
                                                                   const T* __restrict__ r, const T* __restrict__ minv,
                                                                   const KrylovState* ks) {
   pdl_enter();
-  if (ks->done) return;
   using H = V16<T>;
   using V = typename H::V;
-  const bool restart = ks->restart != 0;
-  const T beta = restart ? (T)0 : (T)ks->beta;
-  const long long nv = n3 / H::W;
   V* pv = reinterpret_cast<V*>(p);
   const V* rv = reinterpret_cast<const V*>(r);
   const V* mv = reinterpret_cast<const V*>(minv);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
-    const V z = H::mul(__ldg(mv + i), __ldg(rv + i));
-    pv[i] = restart ? z : H::axpy(beta, pv[i], z);
-  }
+  struct I { V p, r, m; };
+  bool restart = false;
+  T beta = (T)0;
+  vec_pass(
+      n3 / H::W, [&](long long i) { return I{pv[i], __ldg(rv + i), __ldg(mv + i)}; },
+      [&] {
+        restart = ks->restart != 0;
+        beta = restart ? (T)0 : (T)ks->beta;
+        return !ks->done;
+      },
+      [&](const I& v, long long i) {
+        const V z = H::mul(v.m, v.r);
+        pv[i] = restart ? z : H::axpy(beta, v.p, z);
+      });
 }
 
 template <typename T>

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(TX * TY, 2)
   constexpr int L = O::L;
   constexpr int W = Box<T>::W, WE = Box<T>::WE, AL = Box<T>::A;
   KrylovState* ks = a.ks;
-  if (ks && ks->done) return;
+  const int done = ks ? ks->done : 0;   // (tested once the barriers stand)
 
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(TX * TY, 2)
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
+  if (done) return;
 
   // stages and mbarrier phases follow the CTA's running step count gbase + s
   auto issue = [&](int s) {   // leader only

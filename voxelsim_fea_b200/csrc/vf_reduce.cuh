@@ -56,7 +56,26 @@ __device__ __forceinline__ double block_sum(double v) {
   return t;
 }
 
-__device__ inline void finalize_slot(KrylovState* ks, int slot, double total, double* hist) {
+// Block-wide sums of two values at once; valid in thread 0.
+__device__ __forceinline__ void block_sum2(double& a, double& b) {
+  __shared__ double2 s_warp2[32];
+  a = warp_sum(a);
+  b = warp_sum(b);
+  const int t0 = lin_tid();
+  const int lane = t0 & 31, w = t0 >> 5;
+  __syncthreads();
+  if (lane == 0) s_warp2[w] = make_double2(a, b);
+  __syncthreads();
+  if (w == 0) {
+    const double2 v = (lane < ((lin_nthreads() + 31) >> 5)) ? s_warp2[lane] : make_double2(0.0, 0.0);
+    a = warp_sum(v.x);
+    b = warp_sum(v.y);
+  }
+}
+
+// What the finalize does with a sum.  `in` is the state before this kernel,
+// read by the last CTA beside its partials rather than after their sum.
+__device__ inline void finalize_slot(KrylovState* ks, const KrylovState& in, int slot, double total, double* hist) {
   switch (slot) {
     case SLOT_PAP: {
       ks->pAp = total;
@@ -64,40 +83,40 @@ __device__ inline void finalize_slot(KrylovState* ks, int slot, double total, do
         ks->done = 1; ks->status = KS_NONFINITE;
       } else if (total == 0.0) {
         ks->done = 1;
-        ks->status = (ks->resid < ks->tol) ? KS_CONVERGED : KS_BREAKDOWN;
+        ks->status = (in.resid < in.tol) ? KS_CONVERGED : KS_BREAKDOWN;
       } else {
-        ks->alpha = ks->rz / total;
+        ks->alpha = in.rz / total;
       }
       break;
     }
     case SLOT_RR: {
       ks->rr = total;
-      const int it = ks->it + 1;
+      const int it = in.it + 1;
       ks->it = it;
-      const double ratio = sqrt(total) / ks->fnorm;
+      const double ratio = sqrt(total) / in.fnorm;
       ks->resid = ratio;
-      if (hist) hist[ks->it_base + it - 1] = ratio * ks->hist_scale;
+      if (hist) hist[in.it_base + it - 1] = ratio * in.hist_scale;
       if (!(ratio == ratio)) { ks->done = 1; ks->status = KS_NONFINITE; break; }
-      if (ratio < ks->tol) { ks->done = 1; ks->status = KS_CONVERGED; break; }
-      if (ratio < ks->best) ks->best = ratio;
-      if (ks->stall_guard && it >= 10 && ratio > 5.0 * ks->best) {
+      if (ratio < in.tol) { ks->done = 1; ks->status = KS_CONVERGED; break; }
+      if (ratio < in.best) ks->best = ratio;
+      if (in.stall_guard && it >= 10 && ratio > 5.0 * fmin(ratio, in.best)) {
         ks->done = 1; ks->status = KS_STALLED; break;
       }
-      if (total < ks->rr_trigger) { ks->done = 1; ks->status = KS_RELIABLE; break; }
-      if (ks->it_trigger > 0 && it >= ks->it_trigger) { ks->done = 1; ks->status = KS_RELIABLE; break; }
-      if (it >= ks->max_it) { ks->done = 1; ks->status = KS_MAXIT; }
+      if (total < in.rr_trigger) { ks->done = 1; ks->status = KS_RELIABLE; break; }
+      if (in.it_trigger > 0 && it >= in.it_trigger) { ks->done = 1; ks->status = KS_RELIABLE; break; }
+      if (it >= in.max_it) { ks->done = 1; ks->status = KS_MAXIT; }
       break;
     }
     case SLOT_RZ: {
       ks->rz_new = total;
-      if (ks->rz == 0.0) { ks->restart = 1; ks->beta = 0.0; }
-      else { ks->restart = 0; ks->beta = total / ks->rz; }
+      if (in.rz == 0.0) { ks->restart = 1; ks->beta = 0.0; }
+      else { ks->restart = 0; ks->beta = total / in.rz; }
       ks->rz = total;
       break;
     }
     case SLOT_RZ_INIT: ks->rz = total; ks->restart = 0; break;
     case SLOT_FNORM: ks->fnorm = sqrt(total); break;
-    case SLOT_OUTER: ks->rr = total; ks->resid = sqrt(total) / ks->fnorm; break;
+    case SLOT_OUTER: ks->rr = total; ks->resid = sqrt(total) / in.fnorm; break;
     case SLOT_GNUM: ks->gnum = total; break;
     case SLOT_GDEN: ks->gden = total; break;
     default: ks->rr = total; break;
@@ -114,16 +133,17 @@ __device__ __forceinline__ void sum_partials2(const double* partials, int nb, do
     ta += v.x;
     tb += v.y;
   }
-  a = block_sum(ta);
-  b = block_sum(tb);
+  block_sum2(ta, tb);
+  a = ta;
+  b = tb;
 }
 
 // Jacobi-PCG: r.r and r.z in one pass; the last CTA finalizes r.r (ratio,
 // history, stopping tests) and, if the iteration goes on, r.z (beta)
 __device__ inline void reduce_rr_rz(double rr, double rz, double* partials, KrylovState* ks, double* hist) {
   __shared__ bool s_last3;
-  const double sa = block_sum(rr);
-  const double sb = block_sum(rz);
+  double sa = rr, sb = rz;
+  block_sum2(sa, sb);
   const int tid = lin_tid();
   const unsigned nb = lin_nblocks();
   if (tid == 0) {
@@ -135,13 +155,14 @@ __device__ inline void reduce_rr_rz(double rr, double rz, double* partials, Kryl
   __syncthreads();
   if (!s_last3) return;
   __threadfence();
+  KrylovState in;
+  if (tid == 0) in = *ks;
   double ta, tb;
   sum_partials2(partials, (int)nb, ta, tb);
   if (tid == 0) {
-    finalize_slot(ks, SLOT_RR, ta, hist);
-    if (!ks->done) finalize_slot(ks, SLOT_RZ, tb, nullptr);
+    finalize_slot(ks, in, SLOT_RR, ta, hist);
+    if (!ks->done) finalize_slot(ks, in, SLOT_RZ, tb, nullptr);
     ks->counter[SLOT_RR] = 0u;
-    __threadfence();
   }
 }
 
@@ -149,8 +170,8 @@ __device__ inline void reduce_rr_rz(double rr, double rz, double* partials, Kryl
 // both together.  Used by the flexible-CG beta.
 __device__ inline void reduce2_and_finalize(double a, double b, double* partials, KrylovState* ks, int slot) {
   __shared__ bool s_last2;
-  const double sa = block_sum(a);
-  const double sb = block_sum(b);
+  double sa = a, sb = b;
+  block_sum2(sa, sb);
   const int tid = lin_tid();
   const unsigned nb = lin_nblocks();
   if (tid == 0) {
@@ -163,17 +184,17 @@ __device__ inline void reduce2_and_finalize(double a, double b, double* partials
   __syncthreads();
   if (!s_last2) return;
   __threadfence();
+  const double pAp = tid == 0 ? ks->pAp : 0.0;
   double ta, tb;
   sum_partials2(partials, (int)nb, ta, tb);
   if (tid == 0) {
     // FCG(1): p_new = z - (z.Ap / p.Ap) p; alpha next = (r.z) / (p_new.Ap_new)
     ks->rz_new = ta;
     ks->zap = tb;
-    if (ks->pAp != 0.0) { ks->restart = 0; ks->beta = -tb / ks->pAp; }
+    if (pAp != 0.0) { ks->restart = 0; ks->beta = -tb / pAp; }
     else { ks->restart = 1; ks->beta = 0.0; }
     ks->rz = ta;
     ks->counter[slot] = 0u;
-    __threadfence();
   }
 }
 
@@ -194,15 +215,16 @@ __device__ inline void reduce_and_finalize(double v, double* partials, KrylovSta
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  KrylovState in;
+  if (tid == 0) in = *ks;
   double t = 0.0;
   // (through L2, several in flight: the partials come from other SMs)
 #pragma unroll 4
   for (int i = tid; i < (int)nb; i += lin_nthreads()) t += __ldcg(partials + i);
   t = block_sum(t);
   if (tid == 0) {
-    finalize_slot(ks, slot, t, hist);
+    finalize_slot(ks, in, slot, t, hist);
     ks->counter[slot] = 0u;
-    __threadfence();
   }
 }
 
