@@ -122,15 +122,27 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_
 // and keeps the upper face's forces for the next step, so a node's value is
 // loaded once per tile and a voxel costs ~170 operations instead of the 576
 // products per node of the gather form below.  The caller's arrays are in
-// reference order with rows of any alignment, so planes are staged with plain
-// coalesced loads, one plane ahead in registers, three planes in shared
-// memory; the corner forces are exchanged through a double buffer (one barrier
-// a plane).  251x127x129 voxels: 387 us (gather) -> 161 us; 48x24x24: 29 -> 12 us
-// (there also without a clearing launch and the host's 24x24 tables).
+// reference order with rows of any alignment, so planes are staged with
+// 8-byte asynchronous copies, two planes ahead in a ring of four (staged
+// through registers they cost spills and waits: 161 us where it is 118 now);
+// the corner forces are exchanged through a double buffer, one barrier a
+// plane.  Bound by the FP64 and shared-memory instructions of 16 warps an SM
+// (the 24 modes of a voxel and their forces fill the registers).  251x127x129
+// voxels: 387 us (gather) -> 118 us; 48x24x24: 29 -> 12 us (there also without a
+// clearing launch and the host's 24x24 tables).
 constexpr int kMX = 32, kMY = 8;
-constexpr int kRow = 3 * (kMX + 1) + 1, kPlane = (kMY + 1) * kRow;   // 33 x 9 halo nodes
-constexpr size_t kMarchSmem = sizeof(double) * (3 * kPlane + 2 * 3 * 3 * kMY * kMX);
+constexpr int kRow = 3 * (kMX + 1), kPlane = (kMY + 1) * kRow;   // 33 x 9 halo nodes
+constexpr size_t kMarchSmem = sizeof(double) * (4 * kPlane + 2 * 3 * 3 * kMY * kMX);
 struct March { int ntx, nty, zchunk, units; };
+
+// 8-byte asynchronous copy to shared memory; zeros where !in
+__device__ __forceinline__ void copy8(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 __global__ void __launch_bounds__(kThreads, 2)
     k_apply_march(int nx, int ny, int nz, const double* __restrict__ E, const uint8_t* __restrict__ mask,
@@ -140,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   using O = vf::modal::Pack<double>;
   extern __shared__ double smem[];
   double (*s_u)[kPlane] = reinterpret_cast<double (*)[kPlane]>(smem);
-  double (*s_c)[3][3][kMY][kMX] = reinterpret_cast<double (*)[3][3][kMY][kMX]>(smem + 3 * kPlane);
+  double (*s_c)[3][3][kMY][kMX] = reinterpret_cast<double (*)[3][3][kMY][kMX]>(smem + 4 * kPlane);
   const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + kMX * ty;
   const int nx1 = nx + 1, ny1 = ny + 1;
   constexpr int NL = (3 * (kMX + 1) * (kMY + 1) + kThreads - 1) / kThreads;   // halo values per thread
@@ -154,57 +166,52 @@ __global__ void __launch_bounds__(kThreads, 2)
     const bool elem_col = Xc >= 0 && Xc < nx && Yc >= 0 && Yc < ny;
     const double* Ecol = E + (elem_col ? ((long long)Xc * ny + Yc) * nz : 0);
     const int node_col = out_col ? Xc + nx1 * Yc : 0;
-    int goff[NL], soff[NL];   // this thread's halo values: offset within a plane of u (-1: outside), in s_u
+    int goff[NL];   // this thread's halo values tid + q * kThreads: offset within a plane of u (-1: outside)
 #pragma unroll
     for (int q = 0; q < NL; ++q) {
-      const int e = tid + q * kThreads, j = e / (3 * (kMX + 1)), i = e % (3 * (kMX + 1));
+      const int e = tid + q * kThreads, j = e / kRow, i = e % kRow;
       const int gx = X0 - 1 + i / 3, gy = Y0 - 1 + j;
-      soff[q] = j < kMY + 1 ? j * kRow + i : -1;
       goff[q] = (j < kMY + 1 && gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) ? 3 * (gx + nx1 * gy) + i % 3 : -1;
     }
-    double pre[NL];
-    auto fetch = [&](int z) {
+    auto fetch = [&](int z, int b) {
+      const bool zin = z >= 0 && z <= nz;
+      const double* up = u + (zin ? 3LL * nx1 * ny1 * z : 0);
 #pragma unroll
       for (int q = 0; q < NL; ++q)
-        pre[q] = (goff[q] >= 0 && z >= 0 && z <= nz) ? __ldg(u + 3LL * nx1 * ny1 * z + goff[q]) : 0.0;
+        if (tid + q * kThreads < kPlane) copy8(&s_u[b][tid + q * kThreads], up + max(goff[q], 0), zin && goff[q] >= 0);
     };
-    auto store = [&](int b) {
+    double hiPrev[3][4], Fp[3][4];
 #pragma unroll
-      for (int q = 0; q < NL; ++q)
-        if (soff[q] >= 0) s_u[b][soff[q]] = pre[q];
-    };
-    double hiPrev[3][4], Fp[3][4], own[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      own[c] = 0.0;
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
       for (int m = 0; m < 4; ++m) { hiPrev[c][m] = 0.0; Fp[c][m] = 0.0; }
-    }
     // plane s of this unit is z = zb - 1 + s; layer s lies between planes s - 1 and s
     const int nsteps = ze - zb + 2;
     __syncthreads();   // the previous unit's readers are done
-    fetch(zb - 1);
-    store(0);
-    fetch(zb);
+    fetch(zb - 1, 0);
+    copy_commit();
+    fetch(zb, 1);
+    copy_commit();
     double En = 0.0;
     uint8_t mk = 0;
+    copy_wait1();
     __syncthreads();
 #pragma unroll 1
     for (int s = 0; s < nsteps; ++s) {
       const int z = zb - 1 + s;
-      if (s + 1 < nsteps) store((s + 1) % 3);
-      if (s + 2 < nsteps) fetch(z + 2);
+      // (slot (s + 2) & 3 was last read before the barrier of step s - 1)
+      if (s + 2 < nsteps) fetch(z + 2, (s + 2) & 3);
+      copy_commit();
       const double Ee = En;   // of layer s
       En = (elem_col && z >= 0 && z < nz && s + 1 < nsteps) ? __ldg(Ecol + z) : 0.0;
       const uint8_t m8 = mk;
       mk = (out_col && s >= 1 && z >= 0 && z <= nz) ? __ldg(mask + node_col + (long long)nx1 * ny1 * z) : (uint8_t)0;
-      const double* us = s_u[s % 3] + ty * kRow + 3 * tx;
-      double Fc[3][4], u0[3];
+      const double* us = s_u[s & 3] + ty * kRow + 3 * tx;
+      double Fc[3][4];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const double u00 = us[c], u10 = us[3 + c], u01 = us[kRow + c], u11 = us[kRow + 3 + c];
         const double e0 = u10 + u00, e1 = u10 - u00, e2 = u11 + u01, e3 = u11 - u01;
-        u0[c] = u00;
         Fc[c][0] = e0 + e2;
         Fc[c][1] = e1 + e3;
         Fc[c][2] = e2 - e0;
@@ -237,6 +244,10 @@ __global__ void __launch_bounds__(kThreads, 2)
           s_c[s & 1][1][c][ty][tx] = t2 - t3;
           s_c[s & 1][2][c][ty][tx] = t2 + t3;
         }
+        double own[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) own[c] = s_u[(s - 1) & 3][ty * kRow + 3 * tx + c];
+        copy_wait1();   // plane s + 1 of this thread; the barrier makes it all threads'
         __syncthreads();
         if (s >= 2 && out_col) {
           const long long p3 = 3 * (node_col + (long long)nx1 * ny1 * (z - 1));
@@ -250,14 +261,13 @@ __global__ void __launch_bounds__(kThreads, 2)
           }
         }
       } else {
+        copy_wait1();
         __syncthreads();
       }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        own[c] = u0[c];
+      for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int m = 0; m < 4; ++m) Fp[c][m] = Fc[c][m];
-      }
     }
   }
   finish_dot(dot, dot_out, partials, counters, slot);
