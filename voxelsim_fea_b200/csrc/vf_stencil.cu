@@ -484,7 +484,6 @@ namespace {
 
 template <typename S> __device__ __forceinline__ S st_from(double v);
 template <> __device__ __forceinline__ float st_from<float>(double v) { return (float)v; }
-template <> __device__ __forceinline__ double st_from<double>(double v) { return v; }
 template <> __device__ __forceinline__ __half st_from<__half>(double v) { return __double2half(v); }
 
 template <typename S>
