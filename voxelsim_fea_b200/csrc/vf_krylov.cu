@@ -505,7 +505,11 @@ void launch_power_omega(const KrylovState* ks, double omega_rel, double safety, 
 
 template <typename T>
 void launch_dot(const Grid& g, const T* a, const T* b, double* partials, KrylovState* ks, int slot, cudaStream_t st) {
-  launch_pdl(k_dot<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, a, b, partials, ks, slot);
+  // a sum taken once per solve keeps the full grid: its partial sums, and with
+  // the first r.z every step length after it, stay the same to the last bit
+  const bool once = slot == SLOT_RZ_INIT || slot == SLOT_FNORM || slot == SLOT_OUTER || slot == SLOT_PLAIN;
+  const int blocks = once ? kVecBlocks : vec_blocks(3LL * g.n / V16<T>::W);
+  launch_pdl(k_dot<T>, blocks, kVecThreads, 0, st, 3LL * g.n, a, b, partials, ks, slot);
 }
 template <typename T>
 void launch_cg_update(const Grid& g, T* x, const T* p, T* r, const T* Ap, double* partials, KrylovState* ks,
@@ -536,7 +540,7 @@ void launch_copy_vec(const Grid& g, const T* src, T* dst, const KrylovState* ks,
   launch_pdl(k_copy<T>, vec_blocks(3LL * g.n / V16<T>::W), kVecThreads, 0, st, 3LL * g.n, src, dst, ks);
 }
 void launch_norm2_f64(const Grid& g, const double* v, double* partials, KrylovState* ks, int slot, cudaStream_t st) {
-  launch_pdl(k_dot<double>, vec_blocks(3LL * g.n / 2), kVecThreads, 0, st, 3LL * g.n, v, v, partials, ks, slot);
+  launch_dot<double>(g, v, v, partials, ks, slot, st);
 }
 void launch_ir_prepare(const Grid& g, const double* r64, float* r32, KrylovState* ks, cudaStream_t st) {
   launch_k(k_ir_prepare, kVecBlocks, kVecThreads, 0, st, 3LL * g.n, r64, r32, ks);

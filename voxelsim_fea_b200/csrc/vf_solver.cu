@@ -1074,19 +1074,19 @@ int power_level(vf_solver* s, int li) {
   init_ks(*s->h_ks, 1.0, 1, 0, 0, 1.0);
   VF_TRY(cudaMemcpyAsync(s->ks, s->h_ks, sizeof(KrylovState), cudaMemcpyHostToDevice, s->st));
   Level& l = s->L[li];
-  // lambda = ||D^-1 A x|| for the last, unit x.  In between the iterate only
-  // needs to stay in range: an eigenvalue of D^-1 A is at most a few dozen, so
-  // it is scaled to unit length every 8 steps, and a step is one launch (it
-  // was three: product, scaling with its reduction, normalisation)
+  // lambda = ||D^-1 A x|| for the last, unit x; the product is one launch with
+  // its scaling.  The iterate is scaled to unit length after every step: every 8
+  // steps were 0.3-0.5 ms less set-up (64x32x32 1.46 / 1.98 ms, 128x64x64 FP64
+  // 4.2 / 5.0), but rounded the iterate differently, and the damping, the Chebyshev
+  // interval and the smoothed transfers follow it: displacements inside voids,
+  // which a residual does not pin, moved by 1e-9.
   float *x = l.w32[0], *y = l.w32[1];
   launch_power_init<float>(l.g, x, l.mask, s->st);
   const int steps = std::max(2, s->o.power_iters);
   for (int k = 0; k < steps; ++k) {
     level_op<float>(s, li, EPI_APPLY, x, y, nullptr, nullptr, nullptr, 0, nullptr, l.minv32);
-    if (k == steps - 1 || k == steps - 2 || k % 8 == 7) {
-      launch_power_norm<float>(l.g, y, s->d_partials, s->ks, s->st);
-      if (k < steps - 1) launch_power_normalize<float>(l.g, y, y, s->ks, s->st);
-    }
+    launch_power_norm<float>(l.g, y, s->d_partials, s->ks, s->st);
+    if (k < steps - 1) launch_power_normalize<float>(l.g, y, y, s->ks, s->st);
     std::swap(x, y);
   }
   launch_power_omega(s->ks, s->o.omega_rel, 1.1, s->d_omega + li, s->d_lambda + li, s->st);
