@@ -39,9 +39,9 @@ size_t coarse_values(const Grid& g) { return 9 * (size_t)g.nodes_ref() + 24 * (s
 
 template <typename T, bool LAME>
 __global__ void __launch_bounds__(kCoarseThreads, 1)
-    k_coarse_jacobi(Grid g, const T* __restrict__ b, T* __restrict__ x, const T* __restrict__ minv,
+    k_coarse_jacobi(Grid g, const T* b, T* __restrict__ x, const T* __restrict__ minv,
                     const uint8_t* __restrict__ mask, const T* __restrict__ E, const T* __restrict__ MU, ModalConst mc,
-                    int sweeps, T w0, const double* __restrict__ wdev, const KrylovState* ks) {
+                    int sweeps, T w0, const double* wdev, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
   using O = Scalar<T>;

@@ -45,6 +45,14 @@ inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
 // 148 / up to 300 blocks early: 64x32x32 195 / 183 / 185 us, 96x80x64 323 /
 // 315 / 337, 128x64x64 FP64 539 / 533 / 641; the 64x16x16 reference solve
 // 5.42 / 4.96 / 4.96 ms.
+//
+// What the predecessor writes is read through plain pointers there, neither
+// const __restrict__ nor by __ldg: the read-only path is specified for data
+// that nobody writes while the kernel exists, and here the writer still runs
+// (its lines may be kept, its loads moved above the wait).  Set-up data --
+// operators, masks, diagonals, tables -- may take it: a launch right behind
+// their writer is an ordinary one.  (tests/test_early_launch_loads.py reads the
+// sources for this.)
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -284,7 +292,7 @@ template <typename S, int R>
 void launch_wide_compress(const Grid& g, const double* st, const uint8_t* mask, S* stc,
                           typename WideLayout<S, R>::Q* sqrtd, cudaStream_t st_);
 template <typename T, typename S, int R>
-void launch_wide_op(const Grid& g, int epi, const OpArgs& a, const S* stc, const T* sqrtd, cudaStream_t st);
+void launch_wide_op(const Grid& g, int epi, const OpArgs& a, const S* stc, const T* sqrtd, bool early, cudaStream_t st);
 int wide_dense_assemble(const Grid& c, int R, const double* stencil, const uint8_t* cmask, double* A, int n,
                         cudaStream_t st);
 void launch_galerkin_from_stencil(const Grid& f, const double* stencil_f, const Grid& c, double* stencil_c, cudaStream_t st);

@@ -334,7 +334,7 @@ __global__ void k_convert_pad(const double* __restrict__ A, float* __restrict__ 
 // padded FP32 copy in k_dense_solve_f32).
 template <typename T>
 __global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int* __restrict__ perm,
-                              const T* __restrict__ b, T* __restrict__ x, const KrylovState* ks) {
+                              const T* b, T* __restrict__ x, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];
@@ -366,7 +366,7 @@ __global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int*
 // row per warp), products accumulated in FP64.
 template <typename T>
 __global__ void k_dense_solve_f32(const float* __restrict__ Ainv, int n, int ld, const int* __restrict__ perm,
-                                  const T* __restrict__ b, T* __restrict__ x, const KrylovState* ks) {
+                                  const T* b, T* __restrict__ x, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];   // ld values, zero past n
@@ -630,7 +630,7 @@ constexpr int kDisRows = 32;   // rows per block: the staged vector serves four 
 // y_i = [Z_i; W_i^T] b_i
 template <typename T, typename S>
 __global__ void __launch_bounds__(256) k_dis_parts(DensePlan P, const S* __restrict__ store,
-                                                   const int* __restrict__ perm, const T* __restrict__ b,
+                                                   const int* __restrict__ perm, const T* b,
                                                    double* __restrict__ y, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
@@ -651,8 +651,8 @@ __global__ void __launch_bounds__(256) k_dis_parts(DensePlan P, const S* __restr
 // x_s = S^-1 (b_s - the parts' W^T b); S in rows of ld values
 template <typename T, typename S>
 __global__ void __launch_bounds__(256) k_dis_schur(DensePlan P, const S* __restrict__ Sinv, int ld,
-                                                   const int* __restrict__ perm, const T* __restrict__ b,
-                                                   const double* __restrict__ y, double* __restrict__ xs,
+                                                   const int* __restrict__ perm, const T* b, const double* y,
+                                                   double* __restrict__ xs,
                                                    T* __restrict__ x, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
@@ -680,8 +680,8 @@ __global__ void __launch_bounds__(256) k_dis_schur(DensePlan P, const S* __restr
 // x_i = (Z_i b_i) - W_i x_s: lanes take 32 rows, warps share the separators' DOFs
 template <typename T, typename S>
 __global__ void __launch_bounds__(256) k_dis_back(DensePlan P, const S* __restrict__ store,
-                                                  const int* __restrict__ perm, const double* __restrict__ y,
-                                                  const double* __restrict__ xs, T* __restrict__ x,
+                                                  const int* __restrict__ perm, const double* y, const double* xs,
+                                                  T* __restrict__ x,
                                                   const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;

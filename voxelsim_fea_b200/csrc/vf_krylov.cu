@@ -59,7 +59,7 @@ __device__ __forceinline__ bool vec_pass(long long nv, LD ld, GO go, OP op) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_dot(long long n3, const T* __restrict__ a, const T* __restrict__ b,
+__global__ void __launch_bounds__(kVecThreads) k_dot(long long n3, const T* a, const T* b,
                                                      double* partials, KrylovState* ks, int slot) {
   pdl_enter();
   using H = V16<T>;
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kVecThreads) k_dot(long long n3, const T* __re
   struct I { V a, b; };
   double s = 0.0;
   const bool go = vec_pass(
-      n3 / H::W, [&](long long i) { return I{__ldg(av + i), __ldg(bv + i)}; },
+      n3 / H::W, [&](long long i) { return I{av[i], bv[i]}; },
       [&] { return !(ks->done && slot != SLOT_FNORM && slot != SLOT_RZ_INIT && slot != SLOT_OUTER && slot != SLOT_PLAIN); },
       [&](const I& v, long long) { s += H::dot(v.a, v.b); });
   if (!go) return;
@@ -77,8 +77,8 @@ __global__ void __launch_bounds__(kVecThreads) k_dot(long long n3, const T* __re
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_cg_update(long long n3, T* __restrict__ x, const T* __restrict__ p,
-                                                           T* __restrict__ r, const T* __restrict__ Ap,
+__global__ void __launch_bounds__(kVecThreads) k_cg_update(long long n3, T* __restrict__ x, const T* p,
+                                                           T* __restrict__ r, const T* Ap,
                                                            double* partials, KrylovState* ks, double* hist) {
   pdl_enter();
   using H = V16<T>;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update(long long n3, T* __re
   T alpha = (T)0;
   double s = 0.0;
   const bool go = vec_pass(
-      n3 / H::W, [&](long long i) { return I{xv[i], __ldg(pv + i), rv[i], __ldg(av + i)}; },
+      n3 / H::W, [&](long long i) { return I{xv[i], pv[i], rv[i], av[i]}; },
       [&] { alpha = (T)ks->alpha; return !ks->done; },
       [&](const I& v, long long i) {
         xv[i] = H::axpy(alpha, v.p, v.x);
@@ -105,8 +105,8 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update(long long n3, T* __re
 
 // (r.z, z.Ap) in one pass -> flexible-CG beta
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_dot_fcg(long long n3, const T* __restrict__ r, const T* __restrict__ z,
-                                                         const T* __restrict__ Ap, double* partials, KrylovState* ks) {
+__global__ void __launch_bounds__(kVecThreads) k_dot_fcg(long long n3, const T* r, const T* z, const T* Ap,
+                                                         double* partials, KrylovState* ks) {
   pdl_enter();
   using H = V16<T>;
   using V = typename H::V;
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kVecThreads) k_dot_fcg(long long n3, const T* 
   struct I { V r, z, a; };
   double s1 = 0.0, s2 = 0.0;
   const bool go = vec_pass(
-      n3 / H::W, [&](long long i) { return I{__ldg(rv + i), __ldg(zv + i), __ldg(av + i)}; }, [&] { return !ks->done; },
+      n3 / H::W, [&](long long i) { return I{rv[i], zv[i], av[i]}; }, [&] { return !ks->done; },
       [&](const I& v, long long) {
         s1 += H::dot(v.r, v.z);
         s2 += H::dot(v.z, v.a);
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kVecThreads) k_dot_fcg(long long n3, const T* 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_p_update(long long n3, T* __restrict__ p, const T* __restrict__ z,
+__global__ void __launch_bounds__(kVecThreads) k_p_update(long long n3, T* __restrict__ p, const T* z,
                                                           const KrylovState* ks) {
   pdl_enter();
   using H = V16<T>;
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kVecThreads) k_p_update(long long n3, T* __res
   bool restart = false;
   T beta = (T)0;
   vec_pass(
-      n3 / H::W, [&](long long i) { return I{pv[i], __ldg(zv + i)}; },
+      n3 / H::W, [&](long long i) { return I{pv[i], zv[i]}; },
       [&] {
         restart = ks->restart != 0;
         beta = restart ? (T)0 : (T)ks->beta;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kVecThreads) k_p_update(long long n3, T* __res
 // values per thread step (n3 is a multiple of 12): two double2 and one
 // float4 access per vector.
 __global__ void __launch_bounds__(kVecThreads) k_cg_update_split(long long n3, double* __restrict__ r,
-                                                                 const double* __restrict__ Ap, float* __restrict__ r32,
+                                                                 const double* Ap, float* __restrict__ r32,
                                                                  double* partials, KrylovState* ks, double* hist) {
   pdl_enter();
   double2* rv = reinterpret_cast<double2*>(r);
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update_split(long long n3, d
   struct I { double2 a0, a1, q0, q1; };
   double alpha = 0.0, s = 0.0;
   const bool go = vec_pass(
-      n3 / 4, [&](long long i) { return I{__ldg(av + 2 * i), __ldg(av + 2 * i + 1), rv[2 * i], rv[2 * i + 1]}; },
+      n3 / 4, [&](long long i) { return I{av[2 * i], av[2 * i + 1], rv[2 * i], rv[2 * i + 1]}; },
       [&] { alpha = ks->alpha; return !ks->done; },
       [&](const I& v, long long i) {
         double2 q0 = v.q0, q1 = v.q1;
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kVecThreads) k_cg_update_split(long long n3, d
 // the one whose residual test ended the solve, when p stays -- tracked by
 // ks->x_it, which the last CTA advances.
 __global__ void __launch_bounds__(kVecThreads) k_p_update_split(long long n3, double* __restrict__ x,
-                                                                double* __restrict__ p, const float* __restrict__ z,
+                                                                double* __restrict__ p, const float* z,
                                                                 KrylovState* ks) {
   pdl_enter();
   double2* xv = reinterpret_cast<double2*>(x);
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kVecThreads) k_p_update_split(long long n3, do
   bool do_x = false, do_p = false;
   double alpha = 0.0, beta = 0.0;
   const bool go = vec_pass(
-      n3 / 4, [&](long long i) { return I{pv[2 * i], pv[2 * i + 1], xv[2 * i], xv[2 * i + 1], __ldg(zv + i)}; },
+      n3 / 4, [&](long long i) { return I{pv[2 * i], pv[2 * i + 1], xv[2 * i], xv[2 * i + 1], zv[i]}; },
       [&] {
         it = ks->it;
         do_x = it > ks->x_it;
@@ -227,9 +227,8 @@ __global__ void __launch_bounds__(kVecThreads) k_p_update_split(long long n3, do
 }
 
 // (r.z, z.Ap) with r, z FP32 and Ap FP64 -> flexible-CG beta
-__global__ void __launch_bounds__(kVecThreads) k_dot_fcg_split(long long n3, const float* __restrict__ r,
-                                                               const float* __restrict__ z,
-                                                               const double* __restrict__ Ap, double* partials,
+__global__ void __launch_bounds__(kVecThreads) k_dot_fcg_split(long long n3, const float* r, const float* z,
+                                                               const double* Ap, double* partials,
                                                                KrylovState* ks) {
   pdl_enter();
   const float4* rv = reinterpret_cast<const float4*>(r);
@@ -238,7 +237,7 @@ __global__ void __launch_bounds__(kVecThreads) k_dot_fcg_split(long long n3, con
   struct I { float4 r, z; double2 a0, a1; };
   double s1 = 0.0, s2 = 0.0;
   const bool go = vec_pass(
-      n3 / 4, [&](long long i) { return I{__ldg(rv + i), __ldg(zv + i), __ldg(av + 2 * i), __ldg(av + 2 * i + 1)}; },
+      n3 / 4, [&](long long i) { return I{rv[i], zv[i], av[2 * i], av[2 * i + 1]}; },
       [&] { return !ks->done; },
       [&](const I& v, long long) {
         const float4 rr = v.r, zz = v.z;
@@ -256,7 +255,7 @@ __global__ void k_scale64(long long n3, const double* x, double* y, double sc) {
 }
 
 template <typename T>
-__global__ void k_jacobi_precond(int n, const T* __restrict__ r, const T* __restrict__ minv,
+__global__ void k_jacobi_precond(int n, const T* r, const T* __restrict__ minv,
                                  const uint8_t* __restrict__ mask, T* __restrict__ z, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
@@ -277,8 +276,8 @@ __global__ void k_jacobi_precond(int n, const T* __restrict__ r, const T* __rest
 // vectors are bound by: a job on a 61x43x37 grid 92.9 -> 55.9 ms (with the
 // smaller grids of vec_blocks and several chunks per look at the state).
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_jacobi_update(long long n3, T* __restrict__ x, const T* __restrict__ p,
-                                                               T* __restrict__ r, const T* __restrict__ Ap,
+__global__ void __launch_bounds__(kVecThreads) k_jacobi_update(long long n3, T* __restrict__ x, const T* p,
+                                                               T* __restrict__ r, const T* Ap,
                                                                const T* __restrict__ minv, double* partials,
                                                                KrylovState* ks, double* hist) {
   pdl_enter();
@@ -293,7 +292,7 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_update(long long n3, T* 
   T alpha = (T)0;
   double s = 0.0, sz = 0.0;
   const bool go = vec_pass(
-      n3 / H::W, [&](long long i) { return I{xv[i], __ldg(pv + i), rv[i], __ldg(av + i), __ldg(mv + i)}; },
+      n3 / H::W, [&](long long i) { return I{xv[i], pv[i], rv[i], av[i], __ldg(mv + i)}; },
       [&] { alpha = (T)ks->alpha; return !ks->done; },
       [&](const I& v, long long i) {
         xv[i] = H::axpy(alpha, v.p, v.x);
@@ -309,7 +308,7 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_update(long long n3, T* 
 // p = Minv r + beta p (r is zero on the DOFs that are not free)
 template <typename T>
 __global__ void __launch_bounds__(kVecThreads) k_jacobi_direction(long long n3, T* __restrict__ p,
-                                                                  const T* __restrict__ r, const T* __restrict__ minv,
+                                                                  const T* r, const T* __restrict__ minv,
                                                                   const KrylovState* ks) {
   pdl_enter();
   using H = V16<T>;
@@ -321,7 +320,7 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_direction(long long n3, 
   bool restart = false;
   T beta = (T)0;
   vec_pass(
-      n3 / H::W, [&](long long i) { return I{pv[i], __ldg(rv + i), __ldg(mv + i)}; },
+      n3 / H::W, [&](long long i) { return I{pv[i], rv[i], __ldg(mv + i)}; },
       [&] {
         restart = ks->restart != 0;
         beta = restart ? (T)0 : (T)ks->beta;
@@ -334,14 +333,14 @@ __global__ void __launch_bounds__(kVecThreads) k_jacobi_direction(long long n3, 
 }
 
 template <typename T>
-__global__ void k_copy(long long n3, const T* __restrict__ s, T* __restrict__ d, const KrylovState* ks) {
+__global__ void k_copy(long long n3, const T* s, T* __restrict__ d, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
   const long long n16 = n3 * (long long)sizeof(T) / 16;   // 16-byte chunks
   const float4* sv = reinterpret_cast<const float4*>(s);
   float4* dv = reinterpret_cast<float4*>(d);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n16; i += (long long)gridDim.x * blockDim.x)
-    dv[i] = __ldg(sv + i);
+    dv[i] = sv[i];
 }
 
 // Mixed precision: r32 = r64 / ||r64|| (inner solves see a unit right-hand
@@ -409,7 +408,7 @@ __global__ void k_power_init(long long n, T* __restrict__ x, const uint8_t* __re
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_power_norm(long long n3, const T* __restrict__ x, double* partials,
+__global__ void __launch_bounds__(kVecThreads) k_power_norm(long long n3, const T* x, double* partials,
                                                             KrylovState* ks) {
   pdl_enter();
   using H = V16<T>;
@@ -418,7 +417,7 @@ __global__ void __launch_bounds__(kVecThreads) k_power_norm(long long n3, const 
   const V* xv = reinterpret_cast<const V*>(x);
   double s = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
-    const V v = __ldg(xv + i);
+    const V v = xv[i];
     s += H::dot(v, v);
   }
   reduce_and_finalize(s, partials, ks, SLOT_PLAIN, nullptr);

@@ -278,11 +278,11 @@ template <typename T, typename S> void sym_compress(vf_solver* s, Level& l, S* s
   launch_wide_compress<S, 1>(l.g, l.st64, l.mask, sym, sq, s->st);
 }
 template <typename T, typename S>
-void sym_op(vf_solver* s, Level& l, int epi, const OpArgs& a, const S* sym, const T* sq) {
-  if (l.reach == 2) { launch_wide_op<T, S, 2>(l.g, epi, a, sym, sq, s->st); return; }
+void sym_op(vf_solver* s, Level& l, int epi, const OpArgs& a, const S* sym, const T* sq, bool early = true) {
+  if (l.reach == 2) { launch_wide_op<T, S, 2>(l.g, epi, a, sym, sq, early, s->st); return; }
   if constexpr (sizeof(T) == 4)
     if (!row_form<T>(l)) { launch_stencil_sym_op<T, S>(l.g, epi, a, sym, sq, l.szchunk, s->st); return; }
-  launch_wide_op<T, S, 1>(l.g, epi, a, sym, sq, s->st);
+  launch_wide_op<T, S, 1>(l.g, epi, a, sym, sq, early, s->st);
 }
 
 template <typename T> void level_sym_op(vf_solver* s, Level& l, int epi, const OpArgs& a);
@@ -291,8 +291,9 @@ void compress_sym64(vf_solver* s, Level& l) {
   l.sym64_ok = true;
 }
 template <> void level_sym_op<double>(vf_solver* s, Level& l, int epi, const OpArgs& a) {
-  if (!l.sym64_ok) compress_sym64(s, l);
-  sym_op<double, double>(s, l, epi, a, l.sym64, l.sq64);
+  const bool fresh = !l.sym64_ok;   // (the operator right behind its own set-up does not start early)
+  if (fresh) compress_sym64(s, l);
+  sym_op<double, double>(s, l, epi, a, l.sym64, l.sq64, !fresh);
 }
 template <> void level_sym_op<float>(vf_solver* s, Level& l, int epi, const OpArgs& a) {
   if (s->o.coarse_storage == VF_STENCIL_SYM_HALF) sym_op<float, __half>(s, l, epi, a, l.sym16, l.sq32);

@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(SX * SY, 4) k_sym_march(Grid g, OpArgs a, cons
 
   KrylovState* ks = a.ks;
   if (ks && ks->done) return;
-  const T* __restrict__ u = (const T*)a.u;
+  const T* u = (const T*)a.u;
   // out may be the step field dprev (the smoothed prolongation updates x in
   // place: each element is read and written by the same thread); a null rhs
   // reads as zero
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(SX * SY, 4) k_sym_march(Grid g, OpArgs a, cons
       const bool ok = hoff[q] >= 0;
       const long long p3 = ok ? 3LL * ((long long)(zz + 1) * sz + hoff[q]) : 0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) pv[q][c] = ok ? (A)__ldg(sqd + p3 + c) * (A)__ldg(u + p3 + c) : (A)0;
+      for (int c = 0; c < 3; ++c) pv[q][c] = ok ? (A)__ldg(sqd + p3 + c) * (A)u[p3 + c] : (A)0;
     }
   };
   auto store = [&](int zz) {

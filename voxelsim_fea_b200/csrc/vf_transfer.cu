@@ -14,7 +14,7 @@ namespace vf {
 
 namespace {
 
-__global__ void __launch_bounds__(256) k_restrict_d(Grid f, const double* __restrict__ rf, Grid c,
+__global__ void __launch_bounds__(256) k_restrict_d(Grid f, const double* rf, Grid c,
                                                     const uint8_t* __restrict__ cm, double* __restrict__ rc,
                                                     const KrylovState* ks) {
   pdl_enter();
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) k_restrict_d(Grid f, const double* __rest
   }
 }
 
-__global__ void __launch_bounds__(256) k_restrict_f(Grid f, const float* __restrict__ rf, Grid c,
+__global__ void __launch_bounds__(256) k_restrict_f(Grid f, const float* rf, Grid c,
                                                     const uint8_t* __restrict__ cm, float* __restrict__ rc,
                                                     const KrylovState* ks) {
   pdl_enter();
@@ -59,8 +59,8 @@ __global__ void __launch_bounds__(256) k_restrict_f(Grid f, const float* __restr
         // multiple of 4 nodes long): four float2 loads and one float
         const long long q = 3 * (long long)f.idx(2 * X - 1, 2 * Y + dy, 2 * Z + dz);
         const float2* q2 = reinterpret_cast<const float2*>(rf + q);
-        const float2 v01 = __ldg(q2), v23 = __ldg(q2 + 1), v45 = __ldg(q2 + 2), v67 = __ldg(q2 + 3);
-        const float v8 = __ldg(rf + q + 8);
+        const float2 v01 = q2[0], v23 = q2[1], v45 = q2[2], v67 = q2[3];
+        const float v8 = rf[q + 8];
         const float r[9] = {v01.x, v01.y, v23.x, v23.y, v45.x, v45.y, v67.x, v67.y, v8};
 #pragma unroll
         for (int dx = -1; dx <= 1; ++dx) {
@@ -82,9 +82,9 @@ __global__ void __launch_bounds__(256) k_restrict_f(Grid f, const float* __restr
 // uc = w * (Minv rc), the same sums and products as k_restrict_* followed by
 // k_jacobi_from_zero (ghost entries of uc stay untouched: they hold zeros).
 template <typename T>
-__global__ void __launch_bounds__(256) k_restrict_first(Grid f, const T* __restrict__ rf, Grid c,
+__global__ void __launch_bounds__(256) k_restrict_first(Grid f, const T* rf, Grid c,
                                                         const uint8_t* __restrict__ cm, T* __restrict__ rc,
-                                                        const T* __restrict__ minvc, const double* __restrict__ wdev,
+                                                        const T* __restrict__ minvc, const double* wdev,
                                                         T* __restrict__ uc, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(256) k_restrict_first(Grid f, const T* __restr
         for (int dy = -1; dy <= 1; ++dy) {
           const long long q = 3 * (long long)f.idx(2 * X - 1, 2 * Y + dy, 2 * Z + dz);
           const float2* q2 = reinterpret_cast<const float2*>(rf + q);
-          const float2 v01 = __ldg(q2), v23 = __ldg(q2 + 1), v45 = __ldg(q2 + 2), v67 = __ldg(q2 + 3);
-          const float v8 = __ldg(rf + q + 8);
+          const float2 v01 = q2[0], v23 = q2[1], v45 = q2[2], v67 = q2[3];
+          const float v8 = rf[q + 8];
           const float r[9] = {v01.x, v01.y, v23.x, v23.y, v45.x, v45.y, v67.x, v67.y, v8};
 #pragma unroll
           for (int dx = -1; dx <= 1; ++dx) {
@@ -172,7 +172,7 @@ template <> struct Vec12<double> {
 // with the zero-weight terms left out, which does not change them.
 // SET: u = P e instead of u += P e (zero on the DOFs that are not free).
 template <typename T, bool SET>
-__global__ void __launch_bounds__(256) k_prolong_add4(Grid c, const T* __restrict__ ec, Grid f,
+__global__ void __launch_bounds__(256) k_prolong_add4(Grid c, const T* ec, Grid f,
                                                       const uint8_t* __restrict__ fm, T* __restrict__ uf,
                                                       const KrylovState* ks) {
   pdl_enter();
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256) k_prolong_add4(Grid c, const T* __restric
           const bool ld = kz < nz && ky < ny && need[ci];
           const long long q = ld ? 3 * (long long)c.idx(2 * gx - 1 + ci, y0 + ky, z0 + kz) : 0;
 #pragma unroll
-          for (int cc = 0; cc < 3; ++cc) cv[kz][ky][ci][cc] = ld ? __ldg(ec + q + cc) : (T)0;
+          for (int cc = 0; cc < 3; ++cc) cv[kz][ky][ci][cc] = ld ? ec[q + cc] : (T)0;
         }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(256) k_prolong_add4(Grid c, const T* __restric
 }
 
 template <typename T>
-__global__ void k_jacobi_from_zero(Grid g, const T* __restrict__ b, const T* __restrict__ minv,
-                                   const uint8_t* __restrict__ mask, T w0, const double* __restrict__ wdev,
+__global__ void k_jacobi_from_zero(Grid g, const T* b, const T* __restrict__ minv,
+                                   const uint8_t* __restrict__ mask, T w0, const double* wdev,
                                    T* __restrict__ u, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;

@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(wide_tx(R) * WideLayout<S, R>::G)
   __shared__ int s_delta[G * L::NJ];
   KrylovState* ks = a.ks;
   const int done = ks ? ks->done : 0;
-  const T* __restrict__ u = (const T*)a.u;
+  const T* u = (const T*)a.u;
   T* out = (T*)a.out;
   const T* b = (const T*)a.b;
   const T* __restrict__ minv = (const T*)(EPI == EPI_APPLY ? a.apply_minv : a.minv);
@@ -663,9 +663,9 @@ __global__ void __launch_bounds__(wide_tx(R) * WideLayout<S, R>::G)
     T v0 = 0, v1 = 0, v2 = 0;
     if (i < HX * HY * HZ && inside(g, hx, hy, hz)) {
       const long long q = 3LL * g.idx(hx, hy, hz);
-      v0 = __ldg(sqd + q) * __ldg(u + q);
-      v1 = __ldg(sqd + q + 1) * __ldg(u + q + 1);
-      v2 = __ldg(sqd + q + 2) * __ldg(u + q + 2);
+      v0 = __ldg(sqd + q) * u[q];
+      v1 = __ldg(sqd + q + 1) * u[q + 1];
+      v2 = __ldg(sqd + q + 2) * u[q + 2];
     }
     if (i < HX * HY * HZ) sv[i].set(v0, v1, v2);
   }
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(wide_tx(R) * WideLayout<S, R>::G)
   const A sq = (A)__ldg(sqd + pc);
   if (lane < 3) {
     if (EPI != EPI_APPLY && b) bc = b[pc];
-    if (EPI != EPI_RESID) u0 = __ldg(u + pc);
+    if (EPI != EPI_RESID) u0 = u[pc];
     if (EPI != EPI_RESID && minv) mi = __ldg(minv + pc);
     if (EPI == EPI_SMOOTH && dprev) dp = dprev[pc];
   }
@@ -808,16 +808,20 @@ void launch_wide_compress(const Grid& g, const double* st, const uint8_t* mask, 
 }
 
 template <typename T, typename S, int R>
-void launch_wide_op(const Grid& g, int epi, const OpArgs& a, const S* stc, const T* sqrtd, cudaStream_t st) {
+void launch_wide_op(const Grid& g, int epi, const OpArgs& a, const S* stc, const T* sqrtd, bool early, cudaStream_t st) {
   constexpr int TX = wide_tx(R), NT = TX * WideLayout<S, R>::G;
   const unsigned blocks = (unsigned)((g.lx + TX) / TX) * (g.ly + 1) * (g.lz + 1);
-  if (epi == EPI_APPLY) launch_pdl(k_wide_op<T, S, R, EPI_APPLY>, blocks, NT, 0, st, g, a, stc, sqrtd);
-  else if (epi == EPI_SMOOTH) launch_pdl(k_wide_op<T, S, R, EPI_SMOOTH>, blocks, NT, 0, st, g, a, stc, sqrtd);
-  else launch_pdl(k_wide_op<T, S, R, EPI_RESID>, blocks, NT, 0, st, g, a, stc, sqrtd);
+  auto go = [&](auto kern) {
+    if (early) launch_pdl(kern, blocks, NT, 0, st, g, a, stc, sqrtd);
+    else launch_k(kern, blocks, NT, 0, st, g, a, stc, sqrtd);
+  };
+  if (epi == EPI_APPLY) go(k_wide_op<T, S, R, EPI_APPLY>);
+  else if (epi == EPI_SMOOTH) go(k_wide_op<T, S, R, EPI_SMOOTH>);
+  else go(k_wide_op<T, S, R, EPI_RESID>);
 }
 #define VF_INST_WIDE(T, S)                                                                                          \
-  template void launch_wide_op<T, S, 1>(const Grid&, int, const OpArgs&, const S*, const T*, cudaStream_t);         \
-  template void launch_wide_op<T, S, 2>(const Grid&, int, const OpArgs&, const S*, const T*, cudaStream_t);         \
+  template void launch_wide_op<T, S, 1>(const Grid&, int, const OpArgs&, const S*, const T*, bool, cudaStream_t);   \
+  template void launch_wide_op<T, S, 2>(const Grid&, int, const OpArgs&, const S*, const T*, bool, cudaStream_t);   \
   template void launch_wide_compress<S, 1>(const Grid&, const double*, const uint8_t*, S*, T*, cudaStream_t);       \
   template void launch_wide_compress<S, 2>(const Grid&, const double*, const uint8_t*, S*, T*, cudaStream_t);
 VF_INST_WIDE(float, __half)
