@@ -2383,9 +2383,11 @@ int vf_solve_block(vf_solver* s, const double* F, int32_t k, double tol, int32_t
     vf_solver* c = s->children[j];
     const bool had_graphs = c->chunk[0] || c->chunk[1] || c->chunk[2] || c->chunk[3];
     const double* oldA = c->d_Ainv;
+    const bool old_lame = c->lame;
     share_operator(c, s);
-    // graphs hold operator pointers and option-dependent launch sequences: re-capture on change
-    if (had_graphs && (oldA != c->d_Ainv))
+    // graphs hold operator pointers, one or two moduli and option-dependent launch
+    // sequences: re-capture on change
+    if (had_graphs && (oldA != c->d_Ainv || old_lame != c->lame))
       for (auto& gexe : c->chunk)
         if (gexe) { cudaGraphExecDestroy(gexe); gexe = nullptr; }
     solvers.push_back(c);
