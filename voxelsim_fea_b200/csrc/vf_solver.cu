@@ -73,7 +73,7 @@ unsigned long long graph_kernel_nodes(cudaGraph_t g) {
 
 struct Level {
   Grid g{};
-  int zchunk[2] = {0, 0};  // modal kernel, FP32 / FP64: z-planes per CTA (< 0: one even wave)
+  int zchunk = 0;          // modal kernel: z-planes per CTA (< 0: one even wave)
   int szchunk = 0;         // marching stencil kernel (FP32): z-planes per CTA
   uint8_t* mask = nullptr;
   bool galerkin = false;   // operator is the assembled stencil
@@ -186,7 +186,7 @@ struct vf_solver {
   // own their vectors, Krylov state, stream and graphs (vf_solve_block)
   std::vector<vf_solver*> children;
   bool is_child = false;
-  bool tuned = false;
+  int tuned_for = -1;           // material kind (lame) whose launch shapes the levels hold; -1: not tuned
 };
 
 namespace {
@@ -341,7 +341,7 @@ void level_op(vf_solver* s, int li, int epi, const T* u, T* out, const T* b, Kry
     launch_fine_op<T>(l.g, epi, a, s->st);
   } else {
     const ModalConst& mc = s->lame ? s->mc_lame : s->mc;
-    const int zc = l.zchunk[sizeof(T) == 8 ? 1 : 0];
+    const int zc = l.zchunk;
     if (s->o.fine_kernel == VF_FINE_MODAL_CPASYNC || !launch_modal_tma<T>(l.g, epi, a, mc, zc, s->st))
       launch_modal_op<T>(l.g, epi, a, mc, 8, zc > 0 ? zc : auto_zchunk(l.g, 0), s->st);
   }
@@ -913,27 +913,28 @@ void nn_refresh_features(vf_solver* s) {
 
 // ---------------------------------------------------------------------------
 // autotuner: z-planes per CTA of the marching kernels, per level, timed with
-// CUDA events on the kernel that the iteration runs on it most: the sweep in
-// the V-cycle's precision, and for the FP64 PCG around an FP32 V-cycle also the
-// FP64 fine operator.  (Each precision has its own choice: the FP64 stencil
-// sweep of a 64x32x32 level takes 27 us at 33 planes and 57 us at 11, where
-// the FP32 one is as fast.)  The choice is cached per (grid, kernel form) for
-// the process.
+// CUDA events on the kernel that the iteration runs on it most, the sweep in
+// the V-cycle's precision; the other fine operators of the solver take the same
+// split.  (The FP64 operator of a mixed solve is fastest at the FP32 sweep's split:
+// both 11 planes on 96x80x64 with two moduli, 2 on 64x32x32, one wave on
+// 256x128x128, where timing its candidates too cost the first solve 36 ms.)
+// The choice is cached for the process by what it was timed on: device, grid,
+// kernel form, precision and, for the fine kernel, one or two moduli.
 // ---------------------------------------------------------------------------
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, int> g_tune_cache;
+std::map<std::array<int, 7>, int> g_tune_cache;
 int auto_zchunk(const Grid& g, int requested);
 
 template <typename T>
-int autotune_level(vf_solver* s, int li, int epi, cudaEvent_t t0, cudaEvent_t t1) {
+int autotune_level(vf_solver* s, int li, cudaEvent_t t0, cudaEvent_t t1) {
   Level& l = s->L[li];
-  constexpr int q = sizeof(T) == 8 ? 1 : 0;
   const bool stencil = l.galerkin && s->o.coarse_storage != VF_STENCIL_FULL && !row_form<T>(l);
   const bool modal = !l.galerkin && s->o.fine_kernel == VF_FINE_MODAL;
   if (!stencil && !modal) return VF_OK;
   if (modal && s->o.modal_zchunk != 0) return VF_OK;   // fixed by the caller
-  int& choice = stencil ? l.szchunk : l.zchunk[q];
-  const auto key = std::make_tuple(l.g.lx, l.g.ly, l.g.lz, (stencil ? 1 + s->o.coarse_storage : 0) + 8 * q);
+  int& choice = stencil ? l.szchunk : l.zchunk;
+  const std::array<int, 7> key{s->device, l.g.lx, l.g.ly, l.g.lz, stencil ? 1 + s->o.coarse_storage : 0, (int)sizeof(T),
+                               modal && s->lame ? 1 : 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_cache.find(key);
@@ -964,25 +965,33 @@ int autotune_level(vf_solver* s, int li, int epi, cudaEvent_t t0, cudaEvent_t t1
   }
   if (modal) cand.push_back(-1);
   T *u = Sel<T>::w(l, 0), *out = Sel<T>::w(l, 1), *b = Sel<T>::w(l, 3);
-  auto run = [&]() { level_op<T>(s, li, epi, u, out, b, nullptr, nullptr, 0); };
-  // two passes, minimum per candidate: the first pass also brings the
-  // clocks up after the set-up, which would otherwise favour late candidates
+  auto run = [&]() { level_op<T>(s, li, EPI_SMOOTH, u, out, b, nullptr, nullptr, 0); };
+  // two passes, minimum per candidate: the first also brings the clocks up
+  // after the set-up, which would otherwise favour late candidates, and takes
+  // two launches of each; the second takes six of those within 1.3 times the
+  // best (14 launches of each were half of a process's first set-up)
   std::vector<float> tmin(cand.size(), 1e30f);
-  for (int pass = 0; pass < 2; ++pass)
+  float best_ms = 1e30f;
+  for (int pass = 0; pass < 2 && cand.size() > 1; ++pass) {
+    const float limit = pass ? 1.3f * best_ms : 1e30f;
+    const int reps = pass ? 6 : 2;
     for (size_t ci = 0; ci < cand.size(); ++ci) {
+      if (pass && tmin[ci] > limit) continue;
       choice = cand[ci];
       run();   // warm
       VF_TRY(cudaEventRecord(t0, s->st));
-      for (int r = 0; r < 6; ++r) run();
+      for (int r = 0; r < reps; ++r) run();
       VF_TRY(cudaEventRecord(t1, s->st));
       VF_TRY(cudaEventSynchronize(t1));
       VF_CHECK_LAUNCH();
       float ms = 0.f;
       cudaEventElapsedTime(&ms, t0, t1);
-      tmin[ci] = std::min(tmin[ci], ms);
+      tmin[ci] = std::min(tmin[ci], ms / reps);
+      best_ms = std::min(best_ms, tmin[ci]);
     }
+  }
   int best = base;
-  float best_ms = 1e30f;
+  best_ms = 1e30f;
   for (size_t ci = 0; ci < cand.size(); ++ci)
     if (tmin[ci] < best_ms) { best_ms = tmin[ci]; best = cand[ci]; }
   choice = best;
@@ -1001,12 +1010,9 @@ int autotune_levels(vf_solver* s) {
   } ev{t0, t1};
   const bool f64 = s->o.precision == VF_PREC_FP64;
   for (size_t li = 0; li < s->L.size(); ++li) {
-    const int rc = f64 ? autotune_level<double>(s, (int)li, EPI_SMOOTH, t0, t1)
-                       : autotune_level<float>(s, (int)li, EPI_SMOOTH, t0, t1);
+    const int rc = f64 ? autotune_level<double>(s, (int)li, t0, t1) : autotune_level<float>(s, (int)li, t0, t1);
     if (rc) return rc;
   }
-  if (s->o.precision == VF_PREC_MIXED && s->o.mixed_mode == VF_MIXED_OUTER64)
-    return autotune_level<double>(s, 0, EPI_APPLY, t0, t1);
   return VF_OK;
 }
 
@@ -1025,7 +1031,7 @@ int upload_tables(vf_solver* s) {
   s->mc = vf::modal_constants(s->nu, false);
   s->mc_lame = vf::modal_constants(s->nu, true);
   for (auto& l : s->L) {
-    l.zchunk[0] = l.zchunk[1] = auto_zchunk(l.g, s->o.modal_zchunk);
+    l.zchunk = auto_zchunk(l.g, s->o.modal_zchunk);
     l.szchunk = sym_zchunk(l.g);
   }
   std::vector<double> G(8 * 576), GL(16 * 576);
@@ -1517,11 +1523,11 @@ int vf_set_material(vf_solver* s, const double* E, const double* nu_elem, uint32
   }
   if (s->nn) nn_refresh_features(s);
   VF_CHECK_LAUNCH();
-  if (s->o.autotune && !s->tuned && use_mg(s)) {
+  if (s->o.autotune && s->tuned_for != (lame ? 1 : 0) && use_mg(s)) {
     // the kernels' shapes are baked into the captured graphs: tune before any capture
     int rc = autotune_levels(s);
     if (rc) return rc;
-    s->tuned = true;
+    s->tuned_for = lame ? 1 : 0;
     for (auto& gexe : s->chunk)
       if (gexe) { cudaGraphExecDestroy(gexe); gexe = nullptr; }
   }
@@ -2273,7 +2279,7 @@ void share_operator(vf_solver* c, const vf_solver* m) {
     Level& d = c->L[i];
     const Level& sl = m->L[i];
     d.g = sl.g;
-    for (int q = 0; q < 2; ++q) d.zchunk[q] = sl.zchunk[q];
+    d.zchunk = sl.zchunk;
     d.szchunk = sl.szchunk;
     d.mask = sl.mask; d.galerkin = sl.galerkin;
     d.E64 = sl.E64; d.mu64 = sl.mu64; d.minv64 = sl.minv64; d.st64 = sl.st64;
@@ -2385,8 +2391,8 @@ int vf_solve_block(vf_solver* s, const double* F, int32_t k, double tol, int32_t
     const double* oldA = c->d_Ainv;
     const bool old_lame = c->lame;
     share_operator(c, s);
-    // graphs hold operator pointers, one or two moduli and option-dependent launch
-    // sequences: re-capture on change
+    // graphs hold operator pointers, one or two moduli (and the launch shapes tuned
+    // for them) and option-dependent launch sequences: re-capture on change
     if (had_graphs && (oldA != c->d_Ainv || old_lame != c->lame))
       for (auto& gexe : c->chunk)
         if (gexe) { cudaGraphExecDestroy(gexe); gexe = nullptr; }
