@@ -15,14 +15,17 @@
 //   * at most kMaxBlocks blocks of 256 threads, i.e. (nx+1)(ny+1)(nz+1) <=
 //     kMaxNodes grid nodes; larger grids are rejected with VF_ERR_ARG;
 //   * every call on a device shares the one array and it keeps the last call's
-//     contents; successive calls take successive completion counters of a
-//     ring, and a call's last block clears its own and the one half a ring
-//     ahead, so a counter that an overlap spoilt does not stay spoilt.
+//     contents; successive calls on a device take successive completion
+//     counters of a ring, and a call's last block clears its own and the one
+//     half a ring ahead, so a counter that an overlap spoilt does not stay
+//     spoilt.  A captured call would keep its counter for every replay: it
+//     takes one outside the ring, cleared by a memset node ahead of the kernel;
 //     Calls whose kernels overlap on the GPU (different streams, no ordering)
 //     race on the array and give wrong results: order them on one stream;
 //   * the first call on each device looks up the array's device address
-//     (cudaGetSymbolAddress with that device current) and keeps it for the
-//     process; make that first call before any stream capture.  A
+//     (cudaGetSymbolAddress with that device current), keeps it for the
+//     process and loads both forms' kernels; make that first call, on any
+//     grid, before any stream capture.  A
 //     cudaDeviceReset tears the module down with the context, so the kept
 //     address is stale afterwards: make no call on that device after a reset;
 //   * u, y and u_dot_y must not overlap: threads read u at neighbouring nodes
@@ -50,8 +53,8 @@ constexpr int kMaxBlocks = 32768;
 constexpr long long kMaxNodes = (long long)kMaxBlocks * kThreads;   // 8,388,608 nodes
 constexpr int kMaxDevices = 64;
 constexpr int kRing = 64;
-// [0, kMaxBlocks) doubles: per-block partials; then kRing unsigned counters.
-constexpr size_t kScratchBytes = sizeof(double) * kMaxBlocks + kRing * sizeof(unsigned);
+// [0, kMaxBlocks) doubles: per-block partials; then the ring's counters and the captured calls'.
+constexpr size_t kScratchBytes = sizeof(double) * kMaxBlocks + (kRing + 1) * sizeof(unsigned);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -59,29 +62,12 @@ struct KeParam { double k[576]; };
 
 unsigned char* g_scratch_addr[kMaxDevices] = {};
 std::mutex g_scratch_mu;
-std::atomic<unsigned> g_call{0};
-
-// Device address of g_noalloc_scratch on the current device (set up once per device).
-int scratch_for_device(unsigned char** out) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return VF_ERR_NO_DEVICE;
-  std::lock_guard<std::mutex> lock(g_scratch_mu);
-  if (!g_scratch_addr[dev]) {
-    void* p = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-    if (e != cudaSuccess || !p) {
-      vf::g_last_error = std::string("cudaGetSymbolAddress(g_noalloc_scratch): ") + cudaGetErrorString(e);
-      return VF_ERR_CUDA;
-    }
-    g_scratch_addr[dev] = (unsigned char*)p;
-  }
-  *out = g_scratch_addr[dev];
-  return VF_OK;
-}
+std::atomic<unsigned> g_call[kMaxDevices];
+std::atomic<int> g_march_ready[vf::kMaxDevices];
 
 // Block sum in a fixed order; the last block sums the partials in order.
 __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_out, double* __restrict__ partials,
-                                           unsigned int* __restrict__ counters, unsigned slot) {
+                                           unsigned int* __restrict__ counters, unsigned slot, unsigned heal) {
   __shared__ double s_w[kThreads / 32];
   __shared__ bool s_last;
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
@@ -112,7 +98,7 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_
     for (int w = 0; w < kThreads / 32; ++w) tot += s_w[w];
     *dot_out = tot;
     counters[slot] = 0u;
-    counters[(slot + kRing / 2) % kRing] = 0u;
+    counters[heal] = 0u;
   }
 }
 
@@ -147,7 +133,7 @@ __device__ __forceinline__ void copy_wait1() { asm volatile("cp.async.wait_group
 __global__ void __launch_bounds__(kThreads, 2)
     k_apply_march(int nx, int ny, int nz, const double* __restrict__ E, const uint8_t* __restrict__ mask,
                   const double* __restrict__ u, double* __restrict__ y, double* __restrict__ dot_out,
-                  double* __restrict__ partials, unsigned int* __restrict__ counters, unsigned slot,
+                  double* __restrict__ partials, unsigned int* __restrict__ counters, unsigned slot, unsigned heal,
                   const vf::ModalConst mc, March mp) {
   using O = vf::modal::Pack<double>;
   extern __shared__ double smem[];
@@ -270,7 +256,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int m = 0; m < 4; ++m) Fp[c][m] = Fc[c][m];
     }
   }
-  finish_dot(dot, dot_out, partials, counters, slot);
+  finish_dot(dot, dot_out, partials, counters, slot, heal);
 }
 
 // The operator as a node-centric gather over KE, one thread per node: better
@@ -281,7 +267,7 @@ __global__ void __launch_bounds__(kThreads) k_apply_noalloc(int nx, int ny, int 
                                                             double* __restrict__ dot_out,
                                                             double* __restrict__ partials,
                                                             unsigned int* __restrict__ counters, unsigned slot,
-                                                            const KeParam K) {
+                                                            unsigned heal, const KeParam K) {
   const int nx1 = nx + 1, ny1 = ny + 1;
   const long long nn = (long long)nx1 * ny1 * (nz + 1);
   const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -323,7 +309,7 @@ __global__ void __launch_bounds__(kThreads) k_apply_noalloc(int nx, int ny, int 
     y[3 * r] = a0; y[3 * r + 1] = a1; y[3 * r + 2] = a2;
     dot = u[3 * r] * a0 + u[3 * r + 1] * a1 + u[3 * r + 2] * a2;
   }
-  finish_dot(dot, dot_out, partials, counters, slot);
+  finish_dot(dot, dot_out, partials, counters, slot, heal);
 }
 
 // Planes per chunk of the marching form: the split whose waves of two blocks
@@ -347,6 +333,32 @@ March march_plan(int nx, int ny, int nz) {
   }
   m.units = (int)(tiles * ((planes + m.zchunk - 1) / m.zchunk));
   return m;
+}
+
+// The current device and the address of g_noalloc_scratch on it; the first time
+// on a device, with both kernels loaded (so that a later capture loads nothing).
+int scratch_for_device(int* device, unsigned char** out) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return VF_ERR_NO_DEVICE;
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
+  if (!g_scratch_addr[dev]) {
+    void* p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+    if (e != cudaSuccess || !p) {
+      vf::g_last_error = std::string("cudaGetSymbolAddress(g_noalloc_scratch): ") + cudaGetErrorString(e);
+      return VF_ERR_CUDA;
+    }
+    cudaFuncAttributes at;
+    if ((e = cudaFuncGetAttributes(&at, k_apply_noalloc)) != cudaSuccess) {
+      vf::g_last_error = std::string("vf_apply_noalloc: ") + cudaGetErrorString(e);
+      return VF_ERR_CUDA;
+    }
+    vf::kernel_prepare(g_march_ready, k_apply_march, kMarchSmem, kThreads);
+    g_scratch_addr[dev] = (unsigned char*)p;
+  }
+  *device = dev;
+  *out = g_scratch_addr[dev];
+  return VF_OK;
 }
 
 }  // namespace
@@ -379,23 +391,34 @@ extern "C" int vf_apply_noalloc(int32_t nx, int32_t ny, int32_t nz, double nu, c
       return VF_ERR_ARG;
     }
   }
+  int dev = 0;
   unsigned char* base = nullptr;
-  int rc = scratch_for_device(&base);
+  int rc = scratch_for_device(&dev, &base);
   if (rc) return rc;
   double* partials = (double*)base;
   unsigned int* counters = (unsigned int*)(base + sizeof(double) * kMaxBlocks);
-  const unsigned slot = g_call.fetch_add(1) % kRing;
   cudaStream_t st = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(st, &cap);
+  unsigned slot = kRing, heal = kRing;
+  if (e == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    slot = g_call[dev].fetch_add(1) % kRing;
+    heal = (slot + kRing / 2) % kRing;
+  } else if (e == cudaSuccess) {
+    e = cudaMemsetAsync(counters + slot, 0, sizeof(unsigned int), st);
+  }
+  if (e != cudaSuccess) {
+    vf::g_last_error = std::string("vf_apply_noalloc: ") + cudaGetErrorString(e);
+    return VF_ERR_CUDA;
+  }
   // The marching form computes whole 31 x 7 tiles: where less than a fifth of
   // their columns are nodes of the grid the gather form is no slower (gather /
   // marching form, us: 3x40x3000 51 / 92, 2x100x400 24 / 38, 1x1x100000 43 /
   // 406; above the line 10x3x200 24 / 10, 30x6x1000 29 / 14, 61x43x37 23 / 12).
   const March m = march_plan(nx, ny, nz);
   if (5LL * (nx + 1) * (ny + 1) >= (long long)m.ntx * (kMX - 1) * m.nty * (kMY - 1)) {
-    static std::atomic<int> per_dev[vf::kMaxDevices];
-    vf::kernel_prepare(per_dev, k_apply_march, kMarchSmem, kThreads);
     vf::launch_k(k_apply_march, dim3((unsigned)std::min(m.units, kMaxBlocks)), dim3(kMX, kMY), kMarchSmem, st, nx, ny,
-                 nz, E, free_mask, u, y, u_dot_y, partials, counters, slot, vf::modal_constants(nu, false), m);
+                 nz, E, free_mask, u, y, u_dot_y, partials, counters, slot, heal, vf::modal_constants(nu, false), m);
   } else {
     KeParam K;
     double tab[1728], b0[144];
@@ -403,9 +426,9 @@ extern "C" int vf_apply_noalloc(int32_t nx, int32_t ny, int32_t nz, double nu, c
     for (int i = 0; i < 576; ++i) K.k[i] = tab[i];
     const int blocks = (int)((nn + kThreads - 1) / kThreads);
     vf::launch_k(k_apply_noalloc, blocks, kThreads, 0, st, nx, ny, nz, E, free_mask, u, y, u_dot_y, partials, counters,
-                 slot, K);
+                 slot, heal, K);
   }
-  const cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     vf::g_last_error = std::string("vf_apply_noalloc launch: ") + cudaGetErrorString(e);
     return VF_ERR_CUDA;
