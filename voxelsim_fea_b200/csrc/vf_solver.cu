@@ -470,7 +470,7 @@ void coarse_solve(vf_solver* s, int li, const T* b, T* x, KrylovState* ks) {
   Level& l = s->L[li];
   if (s->o.coarsest == VF_COARSEST_CHOLESKY && s->d_Ainv) {
     launch_dense_solve<T>(s->dense, s->d_Ainv, s->d_Ainv32, s->d_dense_perm, s->d_dense_vec, b, x, ks, s->st);
-  } else if (l.galerkin ||
+  } else if (l.galerkin || s->o.fine_kernel != VF_FINE_MODAL ||   // (the one-launch sweeps are the modal operator)
              !launch_coarse_jacobi<T>(l.g, b, x, Sel<T>::minv(l), l.mask, Sel<T>::E(l), s->lame ? Sel<T>::mu(l) : nullptr,
                                       s->lame ? s->mc_lame : s->mc, s->o.coarse_sweeps, s->o.omega, s->d_omega + li,
                                       ks, s->st)) {
