@@ -317,6 +317,7 @@ size_t dense_store32_count(const DensePlan& P);   // floats of their FP32 copy
 size_t dense_work_count(const DensePlan& P);      // doubles of the set-up's scratch
 size_t dense_perm_count(const DensePlan& P);
 size_t dense_vec_count(const DensePlan& P);       // doubles of a solve's intermediate vectors (one per stream)
+constexpr int kDenseNoRow = 0x7f7f7f7f;           // dense_build: every pivot was positive
 int dense_assemble(const Grid& c, const double* stencil, const uint8_t* cmask, double* A, int n, cudaStream_t st);
 int dense_ld32(int n);   // row stride (floats) of the padded FP32 inverse
 void dense_prepare_smem();

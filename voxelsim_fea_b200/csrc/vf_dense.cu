@@ -47,9 +47,10 @@ __global__ void k_dense_assemble(Grid c, const double* __restrict__ st, const ui
 // 1024 threads, one per (row t, column c) of the block; the panel solve and
 // the block-row solve of the inverse phase then multiply by linv instead of
 // substituting row by row.
-// (blockIdx.x: matrix of a batch, sA / sL values apart.)
+// (blockIdx.x: matrix of a batch, sA / sL values apart.  info: the least of
+// row0 + n * matrix + row over the rows whose pivot was not positive.)
 __global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int k, int nb, int* info, double* linv,
-                                                           size_t sA, size_t sL) {
+                                                           size_t sA, size_t sL, int row0) {
   pdl_enter();
   A += sA * blockIdx.x;
   linv += sL * blockIdx.x;
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(NB * NB, 1) k_potrf_diag(double* A, int n, int
     if (t == j && c == j) {
       F[j][j] = piv;
       rec[j] = rinv;
-      if (bad && *info == 0) *info = k + j + 1;
+      if (bad) atomicMin(info, row0 + n * (int)blockIdx.x + k + j);
     }
     if (t > j && t < nb) {
       const double lt = L[t][j] * rinv;
@@ -420,14 +421,15 @@ static size_t cholesky_work(int n, int batch) {
 
 // A (batch matrices n x n, sA values apart, lower parts) is overwritten by L;
 // work (cholesky_work) receives Y = L^-1 and the inverted diagonal blocks;
-// A <- Y^T Y = A^-1.  d_info > 0 flags a non-positive pivot.  bw: A[i][j] == 0
+// A <- Y^T Y = A^-1.  d_info receives the first row without a positive pivot,
+// row0 + n * matrix + row, where it is below d_info's value.  bw: A[i][j] == 0
 // for |i - j| > bw (a stencil operator in lexicographic node order is banded).
 // A Cholesky factor keeps the band, so the panel solve and the trailing update
 // of block column k only touch the rows below it that lie within the band: the
 // rows they skip would receive exact zeros (the factor is the same bit for
 // bit).
 static void cholesky_inverse(double* A, double* work, int n, int bw, int* d_info, cudaStream_t st, int batch,
-                             size_t sA) {
+                             size_t sA, int row0) {
   const int nbk = (n + NB - 1) / NB;
   const size_t sY = (size_t)n * n, sL = (size_t)nbk * NB * NB;
   double* linv_all = work + sY * batch;
@@ -435,7 +437,7 @@ static void cholesky_inverse(double* A, double* work, int n, int bw, int* d_info
   for (int k = 0; k < n; k += NB) {
     const int nb = (n - k < NB) ? (n - k) : NB;
     double* linv = linv_all + (size_t)(k / NB) * NB * NB;
-    launch_pdl(k_potrf_diag, batch, NB * NB, 0, st, A, n, k, nb, d_info, linv, sA, sL);
+    launch_pdl(k_potrf_diag, batch, NB * NB, 0, st, A, n, k, nb, d_info, linv, sA, sL, row0);
     // rows > k + nb - 1 + bw of columns k .. k + nb - 1 are zero
     const int rest = std::min(n, k + nb + bw) - (k + nb);
     if (rest > 0) {
@@ -777,17 +779,18 @@ void launch_dense_perm(const Grid& c, const DensePlan& P, int* perm, cudaStream_
 }
 
 // The coarsest operator's explicit inverse, or the dissected one's blocks, in
-// `store`, from the level's full stencil.  d_info > 0: a non-positive pivot.
+// `store`, from the level's full stencil.  d_info: kDenseNoRow, or the index in
+// the permutation table of the first row without a positive pivot.
 void dense_build(const Grid& c, const DensePlan& P, const double* stencil, int reach, const uint8_t* cmask,
                  double* store, double* work, int* d_info, cudaStream_t st) {
-  cudaMemsetAsync(d_info, 0, sizeof(int), st);
+  cudaMemsetAsync(d_info, 0x7f, sizeof(int), st);   // (kDenseNoRow)
   if (P.parts == 1) {
     if (reach > 1) wide_dense_assemble(c, reach, stencil, cmask, store, P.n, st);
     else dense_assemble(c, stencil, cmask, store, P.n, st);
     // DOF bandwidth of the reach-R stencil in reference node order
     const long long nx1 = c.lx + 1, ny1 = c.ly + 1;
     const long long bw = 3LL * std::max(reach, 1) * (1 + nx1 + nx1 * ny1) + 2;
-    cholesky_inverse(store, work, P.n, (int)std::min<long long>(bw, P.n), d_info, st, 1, 0);
+    cholesky_inverse(store, work, P.n, (int)std::min<long long>(bw, P.n), d_info, st, 1, 0, 0);
     return;
   }
   const size_t sp = dis_part(P), blk = (size_t)P.rm * P.rm;
@@ -801,7 +804,7 @@ void dense_build(const Grid& c, const DensePlan& P, const double* stencil, int r
            store, coup);
   launch_k(k_dis_pad, dim3(4, P.parts), 256, 0, st, P, store);
   // within a part the DOFs run plane by plane: the band is reach + 1 planes
-  cholesky_inverse(store, work, P.ni, P.rm + P.m, d_info, st, P.parts, sp);
+  cholesky_inverse(store, work, P.ni, P.rm + P.m, d_info, st, P.parts, sp, 0);
   GemmBatch w{}, r{}, l{};
   w.alpha = 1.0;
   r.alpha = l.alpha = -1.0;
@@ -824,7 +827,7 @@ void dense_build(const Grid& c, const DensePlan& P, const double* stencil, int r
   launch_pdl(k_gemm_batched, dim3(t * ((ni + TB - 1) / TB), w.count), 256, 0, st, w);
   launch_pdl(k_gemm_batched, dim3(t * t, r.count), 256, 0, st, r);
   launch_pdl(k_gemm_batched, dim3(t * t, l.count), 256, 0, st, l);
-  cholesky_inverse(S, work, P.ns, 2 * rm, d_info, st, 1, 0);
+  cholesky_inverse(S, work, P.ns, 2 * rm, d_info, st, 1, 0, P.parts * P.ni);
 }
 void dense_build32(const DensePlan& P, const double* store, float* store32, cudaStream_t st) {
   const size_t head = P.parts == 1 ? 0 : P.parts * dis_part(P);

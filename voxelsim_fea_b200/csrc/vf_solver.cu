@@ -1152,8 +1152,15 @@ int build_dense_coarsest(vf_solver* s) {
   int info = 0;
   VF_TRY(cudaMemcpyAsync(&info, s->d_info, sizeof(int), cudaMemcpyDeviceToHost, sd));
   VF_TRY(cudaStreamSynchronize(sd));
-  if (info != 0) {
-    s->err = "coarsest-level Cholesky: non-positive pivot at row " + std::to_string(info - 1) +
+  if (info != kDenseNoRow) {
+    // the row's DOF, in the coarse operator's own order whatever the dissection's
+    int at = 0;
+    VF_TRY(cudaMemcpyAsync(&at, s->d_dense_perm + info, sizeof(int), cudaMemcpyDeviceToHost, sd));
+    VF_TRY(cudaStreamSynchronize(sd));
+    const Grid& g = lc.g;
+    const int p = at / 3, x = p % g.px - 1, y = p / g.px % g.py - 1, z = p / (g.px * g.py) - 1;
+    const int row = 3 * (x + (g.lx + 1) * (y + (g.ly + 1) * z)) + at % 3;
+    s->err = "coarsest-level Cholesky: non-positive pivot at row " + std::to_string(row) +
              " (singular coarse operator: is the part supported?)";
     return VF_ERR_BREAKDOWN;
   }
