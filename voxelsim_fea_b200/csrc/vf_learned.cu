@@ -28,6 +28,7 @@
 
 #include "vf_common.cuh"
 #include "vf_nn.cuh"
+#include "vf_workspace.cuh"
 
 namespace vf {
 
@@ -259,7 +260,7 @@ namespace {
 template <typename P>
 cudaError_t nn_alloc(NnStage* s, P** p, size_t count, cudaStream_t st) {
   void* q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(P));
+  cudaError_t e = device_malloc(&q, std::max<size_t>(count, 1) * sizeof(P));
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(q, 0, std::max<size_t>(count, 1) * sizeof(P), st);   // ordered with the solver stream
   s->allocs.push_back(q);

@@ -212,12 +212,7 @@ namespace {
 template <typename T>
 int dalloc(vf_solver* s, T** p, size_t count) {
   void* q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-  if (e == cudaErrorMemoryAllocation) {   // what the stateless calls keep may be in the way
-    cudaGetLastError();
-    workspace_trim();
-    e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-  }
+  cudaError_t e = device_malloc(&q, std::max<size_t>(count, 1) * sizeof(T));
   if (e != cudaSuccess) {
     s->err = std::string("cudaMalloc(") + std::to_string(count * sizeof(T)) + " B): " + cudaGetErrorString(e);
     return VF_ERR_NOMEM;

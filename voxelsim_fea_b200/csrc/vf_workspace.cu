@@ -45,4 +45,14 @@ void workspace_trim() {
   cudaGetLastError();
 }
 
+cudaError_t device_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    workspace_trim();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 }  // namespace vf

@@ -8,7 +8,8 @@
 // stream-ordered memory pool per device instead: it keeps at most
 // kPoolKeepBytes between calls, is safe for any number of threads and streams
 // (the allocator orders reuse itself), and workspace_trim gives what it keeps
-// back -- a solver's allocation that fails does that before it gives up.
+// back -- every other device allocation of the library (device_malloc) does
+// that before it gives up.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -23,6 +24,8 @@ constexpr size_t kPoolKeepBytes = (size_t)512 << 20;
 cudaMemPool_t workspace_pool();
 // Gives the pool's unused memory on the current device back.
 void workspace_trim();
+// cudaMalloc that, out of memory, first takes back what the pool keeps.
+cudaError_t device_malloc(void** p, size_t bytes);
 
 struct Workspace {
   std::vector<void*> p;
@@ -38,7 +41,7 @@ struct Workspace {
     const size_t bytes = count * sizeof(T) + 16;
     void* q = nullptr;
     for (int attempt = 0; attempt < 2; ++attempt) {
-      const cudaError_t e = pool ? cudaMallocFromPoolAsync(&q, bytes, pool, st) : cudaMalloc(&q, bytes);
+      const cudaError_t e = pool ? cudaMallocFromPoolAsync(&q, bytes, pool, st) : device_malloc(&q, bytes);
       if (e == cudaSuccess) {
         p.push_back(q);
         *out = (T*)q;
