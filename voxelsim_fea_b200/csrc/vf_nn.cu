@@ -186,15 +186,15 @@ __global__ void __launch_bounds__(NTHREADS, 2)
   }
 }
 
-// Sums of the per-CTA partials in a fixed order: 8 threads per value take every
-// eighth partial (one thread per value walked all of them, 21 us for 27,648
-// values of 148 partials).
+// Sums of the per-CTA partials in a fixed order, in FP64: 8 threads per value
+// take every eighth partial (one thread per value walked all of them, 21 us for
+// 27,648 values of 148 partials).
 __global__ void __launch_bounds__(256) k_reduce_partials(const float* __restrict__ partial, int nparts, long long n,
                                                          float* __restrict__ out, int accumulate) {
-  __shared__ float s[8][33];
+  __shared__ double s[8][33];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const long long i = blockIdx.x * 32LL + lane;
-  float v = 0.f;
+  double v = 0.0;
   if (i < n) {
 #pragma unroll 4
     for (int b = grp; b < nparts; b += 8) v += __ldg(partial + (long long)b * n + i);
@@ -202,10 +202,10 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const float* __restrict
   s[grp][lane] = v;
   __syncthreads();
   if (grp == 0 && i < n) {
-    float t = 0.f;
+    double t = 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += s[k][lane];
-    out[i] = accumulate ? out[i] + t : t;
+    out[i] = accumulate ? out[i] + (float)t : (float)t;
   }
 }
 
@@ -244,6 +244,18 @@ __global__ void __launch_bounds__(NTHREADS) k_bias_grad(const bf16* __restrict__
   }
 }
 
+// Partials (CTAs of a tap group) of a weight gradient whose `ks` warps share a
+// block of channels: whole waves of resident CTAs, and at least so many that a
+// warp adds up no more rows than with 148 partials of one warp each.  The FP32
+// accumulators of the MMA truncate, so the error grows with the rows added up.
+// 36 x 52 x 68 voxels, one wave / by this rule, error against FP64 and time: 64-64
+// channels 32 partials 7.0e-6, 259 us / 164 partials 5.3e-7, 297 us; 64-32 98
+// partials 1.8e-6, 110 us / 197 partials 5.1e-7, 119 us.
+int wgrad_parts(int ks, int groups, int per_sm) {
+  const int need = (148 + ks - 1) / ks, room = 148 * std::min(per_sm, 2);
+  return room * ((need * groups + room - 1) / room) / groups;
+}
+
 template <int CIN, int COUT>
 int conv_wgrad_t(const void* x, const void* dy, float* dw, float* work, size_t work_bytes, int X, int Y, int Z,
                  int accumulate, cudaStream_t st) {
@@ -253,9 +265,8 @@ int conv_wgrad_t(const void* x, const void* dy, float* dw, float* work, size_t w
   constexpr size_t smem = Cfg::smem();
   static std::atomic<int> per_dev[kMaxDevices];
   const int per_sm = kernel_prepare(per_dev, k_conv3_wgrad<CIN, COUT>, smem, NTHREADS);
-  // one resident wave over the tap groups (148 CTAs a group were a wave and a half)
   constexpr int groups = 27 / Cfg::TAPS;
-  long long nb = std::min<long long>(tiles, std::min(148, std::max(1, 148 * per_sm / groups)));
+  long long nb = std::min<long long>(tiles, wgrad_parts(Cfg::KS, groups, per_sm));
   nb = std::min<long long>(nb, (long long)(work_bytes / per));
   if (nb < 1) return -1;
   launch_k(k_conv3_wgrad<CIN, COUT>, dim3((unsigned)nb, groups), dim3(NTHREADS), smem, st,
@@ -268,12 +279,20 @@ int conv_wgrad_t(const void* x, const void* dy, float* dw, float* work, size_t w
 
 }  // namespace
 
+#define VF_NN_PAIRS(F) F(16, 16) F(16, 32) F(32, 16) F(32, 32) F(32, 64) F(64, 32) F(64, 64)
+
 size_t nn_wgrad_work_bytes(int cin, int cout, int X, int Y, int Z) {
   const long long tiles = (long long)((X + OTX - 1) / OTX) * ((Y + OTY - 1) / OTY) * ((Z + OTZ - 1) / OTZ);
-  return sizeof(float) * 27 * (size_t)cin * cout * (size_t)std::max<long long>(1, std::min<long long>(tiles, 148));
+  long long parts = 148;
+#define VF_NN_PARTS(I, O)                                                                   \
+  if (cin == I && cout == O) {                                                              \
+    using C = WgradCfg<I, O>;                                                               \
+    parts = std::max(wgrad_parts(C::KS, 27 / C::TAPS, 1), wgrad_parts(C::KS, 27 / C::TAPS, 2)); \
+  }
+  VF_NN_PAIRS(VF_NN_PARTS)
+#undef VF_NN_PARTS
+  return sizeof(float) * 27 * (size_t)cin * cout * (size_t)std::max<long long>(1, std::min<long long>(tiles, parts));
 }
-
-#define VF_NN_PAIRS(F) F(16, 16) F(16, 32) F(32, 16) F(32, 32) F(32, 64) F(64, 32) F(64, 64)
 
 template <int CIN, int COUT> int conv_forward_tc(const NnConvArgs& a, cudaStream_t st);   // vf_nn_tc.cu
 
