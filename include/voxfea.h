@@ -385,7 +385,8 @@ int vf_inside_grid(const double* verts, int64_t nv, const int64_t* faces, int64_
  * weights [27][cout][cin] BF16 with tap = (dz+1)*9 + (dy+1)*3 + (dx+1)
  * (cross-correlation, the torch conv3d convention).  FP32 accumulation on the
  * tensor cores.  (cin, cout) in {(16,16) (16,32) (32,16) (32,32) (32,64)
- * (64,32) (64,64)}; other pairs return VF_ERR_ARG.  `stream`: cudaStream_t. */
+ * (64,32) (64,64)}; other pairs return VF_ERR_ARG, and so do tensors (in, w, out,
+ * dy, dx, x) that do not start on 16 bytes.  `stream`: cudaStream_t. */
 /* out = relu?(conv(in, w) + bias + skip); bias (FP32, cout), skip (BF16, cout
  * channels) optional; out_f32 non-NULL writes FP32 instead of BF16 `out`. */
 int vf_nn_conv3d_forward(const void* in, const void* w, const float* bias, const void* skip,

@@ -322,11 +322,19 @@ int nn_conv_wgrad(int cin, int cout, const void* x, const void* dy, float* dw, f
 // ---------------------------------------------------------------------------
 #include "../../include/voxfea.h"
 
+namespace {
+// The kernels move activations, weights and results 16 bytes at a time.
+bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr, const void* d = nullptr) {
+  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d) & 15) == 0;
+}
+}  // namespace
+
 extern "C" {
 
 int vf_nn_conv3d_forward(const void* in, const void* w, const float* bias, const void* skip, int32_t relu, void* out,
                          float* out_f32, int32_t X, int32_t Y, int32_t Z, int32_t cin, int32_t cout, void* stream) {
-  if (!in || !w || (!out && !out_f32) || X < 1 || Y < 1 || Z < 1) return VF_ERR_ARG;
+  if (!in || !w || (!out && !out_f32) || X < 1 || Y < 1 || Z < 1 || !aligned16(in, w, out_f32 ? out_f32 : out))
+    return VF_ERR_ARG;
   vf::NnConvArgs a{in, w, bias, skip, nullptr, out, out_f32, X, Y, Z, relu ? 1 : 0};
   if (vf::nn_conv_forward(cin, cout, a, (cudaStream_t)stream)) return VF_ERR_ARG;
   return cudaPeekAtLastError() == cudaSuccess ? VF_OK : VF_ERR_CUDA;
@@ -334,7 +342,7 @@ int vf_nn_conv3d_forward(const void* in, const void* w, const float* bias, const
 
 int vf_nn_conv3d_backward_data(const void* dy, const void* w_t, const void* gate, void* dx, int32_t X, int32_t Y,
                                int32_t Z, int32_t cin, int32_t cout, void* stream) {
-  if (!dy || !w_t || !dx || X < 1 || Y < 1 || Z < 1) return VF_ERR_ARG;
+  if (!dy || !w_t || !dx || X < 1 || Y < 1 || Z < 1 || !aligned16(dy, w_t, dx)) return VF_ERR_ARG;
   vf::NnConvArgs a{dy, w_t, nullptr, nullptr, gate, dx, nullptr, X, Y, Z, 0};
   if (vf::nn_conv_forward(cout, cin, a, (cudaStream_t)stream)) return VF_ERR_ARG;
   return cudaPeekAtLastError() == cudaSuccess ? VF_OK : VF_ERR_CUDA;
@@ -343,7 +351,7 @@ int vf_nn_conv3d_backward_data(const void* dy, const void* w_t, const void* gate
 int vf_nn_conv3d_backward_weight(const void* x, const void* dy, float* dw, int32_t accumulate, float* work,
                                  size_t work_bytes, int32_t X, int32_t Y, int32_t Z, int32_t cin, int32_t cout,
                                  void* stream) {
-  if (!x || !dy || !dw || !work || X < 1 || Y < 1 || Z < 1) return VF_ERR_ARG;
+  if (!x || !dy || !dw || !work || X < 1 || Y < 1 || Z < 1 || !aligned16(x, dy)) return VF_ERR_ARG;
   if (vf::nn_conv_wgrad(cin, cout, x, dy, dw, work, work_bytes, X, Y, Z, accumulate, (cudaStream_t)stream))
     return VF_ERR_ARG;
   return cudaPeekAtLastError() == cudaSuccess ? VF_OK : VF_ERR_CUDA;
@@ -352,7 +360,8 @@ int vf_nn_conv3d_backward_weight(const void* x, const void* dy, float* dw, int32
 int vf_nn_conv3d_backward_bias(const void* dy, float* db, float* work, size_t work_bytes, int64_t nvox, int32_t cout,
                                void* stream) {
   using namespace vf;
-  if (!dy || !db || !work || nvox < 1 || work_bytes < sizeof(float) * kBiasBlocks * (size_t)cout) return VF_ERR_ARG;
+  if (!dy || !db || !work || nvox < 1 || work_bytes < sizeof(float) * kBiasBlocks * (size_t)cout || !aligned16(dy))
+    return VF_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   const bf16* d = (const bf16*)dy;
   const int nb = (int)std::min<long long>(kBiasBlocks, (nvox * cout / 8 + NTHREADS - 1) / NTHREADS);

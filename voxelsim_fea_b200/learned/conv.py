@@ -28,6 +28,13 @@ def _check(rc, what):
         raise RuntimeError(f"{what} failed: {_lib.load().vf_status_string(rc).decode()}")
 
 
+def _dense(t):
+    """t contiguous and on a 16-byte boundary, as the kernels' loads want it (a
+    view may start anywhere in its storage)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def conv3d_forward(x, w_bf16, bias=None, skip=None, relu=False, out_f32=False):
     """y = relu?(conv(x, w) + bias + skip); x (Z,Y,X,Cin) BF16, w (27,Cout,Cin) BF16."""
     Z, Y, X, cin = x.shape
@@ -59,7 +66,8 @@ def conv3d_backward_data(dy, w_bf16, gate=None):
     cin = w_bf16.shape[2]
     dx = torch.empty((Z, Y, X, cin), device=dy.device, dtype=torch.bfloat16)
     wt = mirror_transpose(w_bf16)
-    rc = _lib.load().vf_nn_conv3d_backward_data(_ptr(dy.contiguous()), _ptr(wt), _ptr(gate), _ptr(dx), X, Y, Z,
+    dy = _dense(dy)
+    rc = _lib.load().vf_nn_conv3d_backward_data(_ptr(dy), _ptr(wt), _ptr(gate), _ptr(dx), X, Y, Z,
                                                 cin, cout, _stream())
     _check(rc, "vf_nn_conv3d_backward_data")
     return dx
@@ -72,7 +80,8 @@ def conv3d_backward_weight(x, dy):
     nbytes = L.vf_nn_wgrad_workspace(cin, cout, X, Y, Z)
     work = torch.empty(nbytes // 4, device=x.device, dtype=torch.float32)
     dw = torch.empty((27, cout, cin), device=x.device, dtype=torch.float32)
-    rc = L.vf_nn_conv3d_backward_weight(_ptr(x), _ptr(dy.contiguous()), _ptr(dw), 0, _ptr(work), nbytes, X, Y, Z,
+    x, dy = _dense(x), _dense(dy)
+    rc = L.vf_nn_conv3d_backward_weight(_ptr(x), _ptr(dy), _ptr(dw), 0, _ptr(work), nbytes, X, Y, Z,
                                         cin, cout, _stream())
     _check(rc, "vf_nn_conv3d_backward_weight")
     return dw
@@ -81,7 +90,7 @@ def conv3d_backward_weight(x, dy):
 def conv3d_backward_bias(dy):
     """db (Cout,) FP32 = sum of dy (Z,Y,X,Cout) BF16 over the voxels."""
     cout = dy.shape[3]
-    dy = dy.contiguous()
+    dy = _dense(dy)
     work = torch.empty(148 * cout, device=dy.device, dtype=torch.float32)
     db = torch.empty(cout, device=dy.device, dtype=torch.float32)
     rc = _lib.load().vf_nn_conv3d_backward_bias(_ptr(dy), _ptr(db), _ptr(work), 4 * work.numel(), dy.numel() // cout,
@@ -96,14 +105,14 @@ class Conv3dFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w, b, out_f32=False):
-        wb = w.to(torch.bfloat16).contiguous()
+        wb = _dense(w.to(torch.bfloat16))
         ctx.save_for_backward(x, wb)
-        return conv3d_forward(x.contiguous(), wb, bias=b, out_f32=out_f32)
+        return conv3d_forward(_dense(x), wb, bias=b, out_f32=out_f32)
 
     @staticmethod
     def backward(ctx, dy):
         x, wb = ctx.saved_tensors
-        dy = dy.to(torch.bfloat16).contiguous()
+        dy = _dense(dy.to(torch.bfloat16))
         dx = conv3d_backward_data(dy, wb) if ctx.needs_input_grad[0] else None
         dw = conv3d_backward_weight(x, dy) if ctx.needs_input_grad[1] else None
         db = conv3d_backward_bias(dy) if ctx.needs_input_grad[2] else None
