@@ -99,6 +99,20 @@ def conv3d_backward_bias(dy):
     return db
 
 
+class _BiasGradFn(torch.autograd.Function):
+    """conv3d_backward_bias, differentiable in dy (a linear map: its own
+    gradient is the channel's, broadcast over the voxels)."""
+
+    @staticmethod
+    def forward(ctx, dy):
+        ctx.shape = dy.shape
+        return conv3d_backward_bias(dy)
+
+    @staticmethod
+    def backward(ctx, g):
+        return g.to(torch.bfloat16).expand(ctx.shape)
+
+
 class Conv3dFn(torch.autograd.Function):
     """y = conv(x, w) + b with the libvoxfea kernels in both directions
     (BF16 output, or FP32 with ``out_f32``)."""
@@ -115,7 +129,9 @@ class Conv3dFn(torch.autograd.Function):
         dy = _dense(dy.to(torch.bfloat16))
         dx = conv3d_backward_data(dy, wb) if ctx.needs_input_grad[0] else None
         dw = conv3d_backward_weight(x, dy) if ctx.needs_input_grad[1] else None
-        db = conv3d_backward_bias(dy) if ctx.needs_input_grad[2] else None
+        db = None
+        if ctx.needs_input_grad[2]:   # (dy requires a gradient only where a second derivative is taken)
+            db = _BiasGradFn.apply(dy) if dy.requires_grad else conv3d_backward_bias(dy)
         return dx, dw, db, None
 
 
