@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(kTczThreads) k_conv3_tcz(NnConvArgs a, int zc,
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   // this thread's 16-byte pieces of an input plane: channel chunk and voxel
-  // (offset in the volume's plane, -1 outside), place in a ring slot
+  // (offset in the volume's plane in 16-byte pieces, -1 outside; in values it would
+  // leave 32 bits on planes of 2^31 values), place in a ring slot
   int goff[L::NPRE], soff[L::NPRE];
 #pragma unroll
   for (int q = 0; q < L::NPRE; ++q) {
@@ -298,15 +299,14 @@ __global__ void __launch_bounds__(kTczThreads) k_conv3_tcz(NnConvArgs a, int zc,
     const int hx = v % HCX, hy = v / HCX, x = X0 - 1 + hx, y = Y0 - 1 + hy;
     const bool own = worker && kc < L::KC;
     soff[q] = own ? (int)(kc * L::CHUNK_A + hy * L::ROW + hx * 16) : -1;
-    goff[q] = own && x >= 0 && x < X && y >= 0 && y < Y ? (y * X + x) * CIN + kc * 8 : -1;
+    goff[q] = own && x >= 0 && x < X && y >= 0 && y < Y ? (y * X + x) * L::KC + kc : -1;
   }
   uint4 pre[L::NPRE];
   auto fetch = [&](int zz) {
-    const bf16* p = in + (long long)zz * Y * X * CIN;
+    const uint4* p = reinterpret_cast<const uint4*>(in + (long long)zz * Y * X * CIN);
 #pragma unroll
     for (int q = 0; q < L::NPRE; ++q)
-      pre[q] = (goff[q] >= 0 && zz >= 0 && zz < Z) ? __ldg(reinterpret_cast<const uint4*>(p + goff[q]))
-                                                   : make_uint4(0u, 0u, 0u, 0u);
+      pre[q] = (goff[q] >= 0 && zz >= 0 && zz < Z) ? __ldg(p + goff[q]) : make_uint4(0u, 0u, 0u, 0u);
   };
   auto store = [&](int zz) {
     unsigned char* dst = sIn + ((zz - zb + 1) & 3) * L::PLANE;
