@@ -242,11 +242,20 @@ def assemble(descr, masks, dims):
     _lib.check(_lib.load().vf_assemble_grid(nx, ny, nz, n, _lib.ptr(roles), ptrs, _lib.ptr(meta), 0,
                                             _lib.ptr(active), _lib.ptr(bits), _lib.ptr(force),
                                             ctypes.byref(n_act), ctypes.byref(n_fix)), None, "assemble")
-    # (the supports touch few nodes: expand those alone, in the same ascending order)
+    return active.astype(bool), _fixed_dofs(bits, n_fix.value), force, bits
+
+
+def _fixed_dofs(bits, count):
+    """The `count` fixed DOFs in ascending order from the nodes' fixed bits.  The
+    supported nodes alone are expanded where at most a third of the DOFs is fixed
+    (811,265 nodes: 1.7 ms against 12 for all of them with 1 % fixed, 6.4 against 12
+    with 20 %, but 32 against 20 with every node fixed)."""
+    bit = np.arange(3, dtype=np.uint8)
+    if count > bits.size:
+        return np.flatnonzero(((bits[:, None] >> bit) & 1).ravel()).astype(np.int64)
     nodes = np.flatnonzero(bits)
-    fixed = ((bits[nodes, None] >> np.arange(3, dtype=np.uint8)) & 1).astype(bool)
-    fixed_dofs = (3 * nodes[:, None] + np.arange(3))[fixed].astype(np.int64)
-    return active.astype(bool), fixed_dofs, force, bits
+    fixed = ((bits[nodes, None] >> bit) & 1).astype(bool)
+    return (3 * nodes[:, None] + np.arange(3))[fixed].astype(np.int64)
 
 
 def drop_unsupported_islands_bits(active, fixed_bits, dims):
