@@ -333,13 +333,12 @@ __global__ void k_convert_pad(const double* __restrict__ A, float* __restrict__ 
 // x = Ainv b on the coarsest level; b gathered into shared memory in FP64,
 // products accumulated in FP64 (Ainv in FP64; the FP32 V-cycle reads the
 // padded FP32 copy in k_dense_solve_f32).
-template <typename T>
-__global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int* __restrict__ perm,
-                              const T* b, T* __restrict__ x, const KrylovState* ks) {
+__global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int* __restrict__ perm, const double* b,
+                              double* __restrict__ x, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) sb[i] = (double)b[__ldg(perm + i)];
+  for (int i = threadIdx.x; i < n; i += blockDim.x) sb[i] = b[__ldg(perm + i)];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
@@ -357,7 +356,7 @@ __global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int*
     double s = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) x[__ldg(perm + i)] = (T)s;
+    if (lane == 0) x[__ldg(perm + i)] = s;
   }
 }
 
@@ -365,9 +364,8 @@ __global__ void k_dense_solve(const double* __restrict__ Ainv, int n, const int*
 // zero-padded past n), each lane streaming float4s, eight in flight per lane
 // (4 KB per warp: enough bytes in flight to approach the HBM rate with one
 // row per warp), products accumulated in FP64.
-template <typename T>
 __global__ void k_dense_solve_f32(const float* __restrict__ Ainv, int n, int ld, const int* __restrict__ perm,
-                                  const T* b, T* __restrict__ x, const KrylovState* ks) {
+                                  const float* b, float* __restrict__ x, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
   extern __shared__ double sb[];   // ld values, zero past n
@@ -399,7 +397,7 @@ __global__ void k_dense_solve_f32(const float* __restrict__ Ainv, int n, int ld,
     double s = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) x[__ldg(perm + i)] = (T)s;
+    if (lane == 0) x[__ldg(perm + i)] = (float)s;
   }
 }
 
@@ -856,9 +854,8 @@ static void dissected_solve(const DensePlan& P, const S* store, int ld, const in
 void dense_prepare_smem() {
   const int bytes = (int)sizeof(double) * 16384;
   auto allow = [&](const void* f) { cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
-  allow((const void*)k_dense_solve<double>);
-  allow((const void*)k_dense_solve<float>);
-  allow((const void*)k_dense_solve_f32<float>);
+  allow((const void*)k_dense_solve);
+  allow((const void*)k_dense_solve_f32);
   allow((const void*)k_dis_parts<double, double>);
   allow((const void*)k_dis_parts<float, float>);
   allow((const void*)k_dis_schur<double, double>);
@@ -875,7 +872,7 @@ void launch_dense_solve<double>(const DensePlan& P, const double* store, const f
     dissected_solve<double, double>(P, store, P.ns, perm, vec, b, x, ks, st);
     return;
   }
-  launch_pdl(k_dense_solve<double>, (P.n + 7) / 8, 256, sizeof(double) * P.n, st, store, P.n, perm, b, x, ks);
+  launch_pdl(k_dense_solve, (P.n + 7) / 8, 256, sizeof(double) * P.n, st, store, P.n, perm, b, x, ks);
 }
 template <>
 void launch_dense_solve<float>(const DensePlan& P, const double*, const float* store32, const int* perm, double* vec,
@@ -885,7 +882,7 @@ void launch_dense_solve<float>(const DensePlan& P, const double*, const float* s
     return;
   }
   const int ld = dense_ld32(P.n);
-  launch_pdl(k_dense_solve_f32<float>, (P.n + 7) / 8, 256, sizeof(double) * ld, st, store32, P.n, ld, perm, b, x, ks);
+  launch_pdl(k_dense_solve_f32, (P.n + 7) / 8, 256, sizeof(double) * ld, st, store32, P.n, ld, perm, b, x, ks);
 }
 
 }  // namespace vf

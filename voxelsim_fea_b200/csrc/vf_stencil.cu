@@ -24,7 +24,6 @@
 //     diagonal}; zero their rows/columns; Jacobi inverse diagonal.
 #include <cuda_fp16.h>
 
-#include <type_traits>
 
 #include "vf_common.cuh"
 #include "vf_levelops.cuh"
@@ -541,7 +540,7 @@ __global__ void __launch_bounds__(SX * SY, 4) k_sym_march(Grid g, OpArgs a, cons
                                                            const T* __restrict__ sqd, int zchunk) {
   pdl_enter();
   using Lay = SymLayout<S>;
-  using A = typename std::conditional<sizeof(T) == 8, double, float>::type;
+  using A = T;
   constexpr int VPC = Lay::VPC;
   constexpr int HX = SX + 2, HY = SY + 2, NH = HX * HY;
   constexpr int NTH = SX * SY;
