@@ -1,6 +1,5 @@
-"""vf_apply_noalloc on a grid with more tiles than blocks may be launched
-(32,768): blocks take a second unit, with the ring of staged planes, its copy
-groups and the double-buffered corner forces carried over -- against a plain FP64
+"""vf_apply_noalloc on very long grids one voxel thick, with more tiles than blocks
+may be launched (32,768): the gather form takes them -- against a plain FP64
 evaluation, 1e-13 of the largest value."""
 
 import numpy as np
@@ -10,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dims", [(1_030_000, 1, 1), (1_030_000, 1, 2)])
-def test_more_units_than_blocks(gpu, dims):
+def test_more_tiles_than_blocks(gpu, dims):
     import torch
     from oracle import hex8
     from voxelsim_fea_b200 import _lib

@@ -73,7 +73,6 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-  __syncthreads();
   if ((tid & 31) == 0) s_w[tid >> 5] = dot;
   __syncthreads();
   if (tid == 0) {
@@ -87,8 +86,7 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_
   if (!s_last) return;
   __threadfence();
   double s = 0.0;
-#pragma unroll 4
-  for (int i = tid; i < (int)gridDim.x; i += kThreads) s += __ldcg(partials + i);
+  for (int i = tid; i < (int)gridDim.x; i += kThreads) s += ((volatile double*)partials)[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((tid & 31) == 0) s_w[tid >> 5] = s;
@@ -119,7 +117,7 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_
 constexpr int kMX = 32, kMY = 8;
 constexpr int kRow = 3 * (kMX + 1), kPlane = (kMY + 1) * kRow;   // 33 x 9 halo nodes
 constexpr size_t kMarchSmem = sizeof(double) * (4 * kPlane + 2 * 3 * 3 * kMY * kMX);
-struct March { int ntx, nty, zchunk, units; };
+struct March { int ntx, nty, zchunk; long long units, steps; };
 
 // 8-byte asynchronous copy to shared memory; zeros where !in
 __device__ __forceinline__ void copy8(double* dst, const double* src, bool in) {
@@ -143,124 +141,121 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int nx1 = nx + 1, ny1 = ny + 1;
   constexpr int NL = (3 * (kMX + 1) * (kMY + 1) + kThreads - 1) / kThreads;   // halo values per thread
   double dot = 0.0;
-#pragma unroll 1
-  for (int unit = blockIdx.x; unit < mp.units; unit += gridDim.x) {
-    const int X0 = unit % mp.ntx * (kMX - 1), Y0 = unit / mp.ntx % mp.nty * (kMY - 1);
-    const int zb = unit / (mp.ntx * mp.nty) * mp.zchunk, ze = min(zb + mp.zchunk, nz + 1);
-    const int Xc = X0 - 1 + tx, Yc = Y0 - 1 + ty;
-    const bool out_col = tx >= 1 && ty >= 1 && Xc <= nx && Yc <= ny;
-    const bool elem_col = Xc >= 0 && Xc < nx && Yc >= 0 && Yc < ny;
-    const double* Ecol = E + (elem_col ? ((long long)Xc * ny + Yc) * nz : 0);
-    const int node_col = out_col ? Xc + nx1 * Yc : 0;
-    int goff[NL];   // this thread's halo values tid + q * kThreads: offset within a plane of u (-1: outside)
+  const int unit = blockIdx.x;
+  const int X0 = unit % mp.ntx * (kMX - 1), Y0 = unit / mp.ntx % mp.nty * (kMY - 1);
+  const int zb = unit / (mp.ntx * mp.nty) * mp.zchunk, ze = min(zb + mp.zchunk, nz + 1);
+  const int Xc = X0 - 1 + tx, Yc = Y0 - 1 + ty;
+  const bool out_col = tx >= 1 && ty >= 1 && Xc <= nx && Yc <= ny;
+  const bool elem_col = Xc >= 0 && Xc < nx && Yc >= 0 && Yc < ny;
+  const double* Ecol = E + (elem_col ? ((long long)Xc * ny + Yc) * nz : 0);
+  const int node_col = out_col ? Xc + nx1 * Yc : 0;
+  int goff[NL];   // this thread's halo values tid + q * kThreads: offset within a plane of u (-1: outside)
 #pragma unroll
-    for (int q = 0; q < NL; ++q) {
-      const int e = tid + q * kThreads, j = e / kRow, i = e % kRow;
-      const int gx = X0 - 1 + i / 3, gy = Y0 - 1 + j;
-      goff[q] = (j < kMY + 1 && gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) ? 3 * (gx + nx1 * gy) + i % 3 : -1;
+  for (int q = 0; q < NL; ++q) {
+    const int e = tid + q * kThreads, j = e / kRow, i = e % kRow;
+    const int gx = X0 - 1 + i / 3, gy = Y0 - 1 + j;
+    goff[q] = (j < kMY + 1 && gx >= 0 && gx <= nx && gy >= 0 && gy <= ny) ? 3 * (gx + nx1 * gy) + i % 3 : -1;
+  }
+  auto fetch = [&](int z, int b) {
+    const bool zin = z >= 0 && z <= nz;
+    const double* up = u + (zin ? 3LL * nx1 * ny1 * z : 0);
+#pragma unroll
+    for (int q = 0; q < NL; ++q)
+      if (tid + q * kThreads < kPlane) copy8(&s_u[b][tid + q * kThreads], up + max(goff[q], 0), zin && goff[q] >= 0);
+  };
+  double hiPrev[3][4], Fp[3][4];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) { hiPrev[c][m] = 0.0; Fp[c][m] = 0.0; }
+  // plane s of this unit is z = zb - 1 + s; layer s lies between planes s - 1 and s
+  const int nsteps = ze - zb + 2;
+  fetch(zb - 1, 0);
+  copy_commit();
+  fetch(zb, 1);
+  copy_commit();
+  double En = 0.0;
+  uint8_t mk = 0;
+  copy_wait1();
+  __syncthreads();
+#pragma unroll 1
+  for (int s = 0; s < nsteps; ++s) {
+    const int z = zb - 1 + s;
+    // (slot (s + 2) & 3 was last read before the barrier of step s - 1)
+    if (s + 2 < nsteps) fetch(z + 2, (s + 2) & 3);
+    copy_commit();
+    const double Ee = En;   // of layer s
+    En = (elem_col && z >= 0 && z < nz && s + 1 < nsteps) ? __ldg(Ecol + z) : 0.0;
+    const uint8_t m8 = mk;
+    mk = (out_col && s >= 1 && z >= 0 && z <= nz) ? __ldg(mask + node_col + (long long)nx1 * ny1 * z) : (uint8_t)0;
+    const double* us = s_u[s & 3] + ty * kRow + 3 * tx;
+    double Fc[3][4];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double u00 = us[c], u10 = us[3 + c], u01 = us[kRow + c], u11 = us[kRow + 3 + c];
+      const double e0 = u10 + u00, e1 = u10 - u00, e2 = u11 + u01, e3 = u11 - u01;
+      Fc[c][0] = e0 + e2;
+      Fc[c][1] = e1 + e3;
+      Fc[c][2] = e2 - e0;
+      Fc[c][3] = e3 - e1;
     }
-    auto fetch = [&](int z, int b) {
-      const bool zin = z >= 0 && z <= nz;
-      const double* up = u + (zin ? 3LL * nx1 * ny1 * z : 0);
-#pragma unroll
-      for (int q = 0; q < NL; ++q)
-        if (tid + q * kThreads < kPlane) copy8(&s_u[b][tid + q * kThreads], up + max(goff[q], 0), zin && goff[q] >= 0);
-    };
-    double hiPrev[3][4], Fp[3][4];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int m = 0; m < 4; ++m) { hiPrev[c][m] = 0.0; Fp[c][m] = 0.0; }
-    // plane s of this unit is z = zb - 1 + s; layer s lies between planes s - 1 and s
-    const int nsteps = ze - zb + 2;
-    __syncthreads();   // the previous unit's readers are done
-    fetch(zb - 1, 0);
-    copy_commit();
-    fetch(zb, 1);
-    copy_commit();
-    double En = 0.0;
-    uint8_t mk = 0;
-    copy_wait1();
-    __syncthreads();
-#pragma unroll 1
-    for (int s = 0; s < nsteps; ++s) {
-      const int z = zb - 1 + s;
-      // (slot (s + 2) & 3 was last read before the barrier of step s - 1)
-      if (s + 2 < nsteps) fetch(z + 2, (s + 2) & 3);
-      copy_commit();
-      const double Ee = En;   // of layer s
-      En = (elem_col && z >= 0 && z < nz && s + 1 < nsteps) ? __ldg(Ecol + z) : 0.0;
-      const uint8_t m8 = mk;
-      mk = (out_col && s >= 1 && z >= 0 && z <= nz) ? __ldg(mask + node_col + (long long)nx1 * ny1 * z) : (uint8_t)0;
-      const double* us = s_u[s & 3] + ty * kRow + 3 * tx;
-      double Fc[3][4];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const double u00 = us[c], u10 = us[3 + c], u01 = us[kRow + c], u11 = us[kRow + 3 + c];
-        const double e0 = u10 + u00, e1 = u10 - u00, e2 = u11 + u01, e3 = u11 - u01;
-        Fc[c][0] = e0 + e2;
-        Fc[c][1] = e1 + e3;
-        Fc[c][2] = e2 - e0;
-        Fc[c][3] = e3 - e1;
-      }
-      if (s >= 1) {
-        double A[3][8], B[3][8];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int m = 0; m < 4; ++m) {
-            A[c][m] = Fp[c][m] + Fc[c][m];
-            A[c][m + 4] = Fc[c][m] - Fp[c][m];
-          }
-        vf::modal::modal_physics<O, double, double>(A, B, Ee, Ee, mc);
-        double c00[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          double acc[4];
-          acc[0] = hiPrev[c][0] - B[c][4];
-          hiPrev[c][0] = B[c][4];
-#pragma unroll
-          for (int m = 1; m < 4; ++m) {
-            acc[m] = hiPrev[c][m] + (B[c][m] - B[c][m + 4]);
-            hiPrev[c][m] = B[c][m] + B[c][m + 4];
-          }
-          const double t0 = acc[0] - acc[2], t1 = acc[1] - acc[3], t2 = acc[0] + acc[2], t3 = acc[1] + acc[3];
-          c00[c] = t0 - t1;
-          s_c[s & 1][0][c][ty][tx] = t0 + t1;
-          s_c[s & 1][1][c][ty][tx] = t2 - t3;
-          s_c[s & 1][2][c][ty][tx] = t2 + t3;
-        }
-        double own[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) own[c] = s_u[(s - 1) & 3][ty * kRow + 3 * tx + c];
-        copy_wait1();   // plane s + 1 of this thread; the barrier makes it all threads'
-        __syncthreads();
-        if (s >= 2 && out_col) {
-          const long long p3 = 3 * (node_col + (long long)nx1 * ny1 * (z - 1));
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const double v = (c00[c] + s_c[s & 1][0][c][ty][tx - 1]) +
-                             (s_c[s & 1][1][c][ty - 1][tx] + s_c[s & 1][2][c][ty - 1][tx - 1]);
-            const double k = ((m8 >> c) & 1) ? v : 0.0;
-            y[p3 + c] = k;
-            dot += own[c] * k;
-          }
-        }
-      } else {
-        copy_wait1();
-        __syncthreads();
-      }
+    if (s >= 1) {
+      double A[3][8], B[3][8];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int m = 0; m < 4; ++m) Fp[c][m] = Fc[c][m];
+        for (int m = 0; m < 4; ++m) {
+          A[c][m] = Fp[c][m] + Fc[c][m];
+          A[c][m + 4] = Fc[c][m] - Fp[c][m];
+        }
+      vf::modal::modal_physics<O, double, double>(A, B, Ee, Ee, mc);
+      double c00[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        double acc[4];
+        acc[0] = hiPrev[c][0] - B[c][4];
+        hiPrev[c][0] = B[c][4];
+#pragma unroll
+        for (int m = 1; m < 4; ++m) {
+          acc[m] = hiPrev[c][m] + (B[c][m] - B[c][m + 4]);
+          hiPrev[c][m] = B[c][m] + B[c][m + 4];
+        }
+        const double t0 = acc[0] - acc[2], t1 = acc[1] - acc[3], t2 = acc[0] + acc[2], t3 = acc[1] + acc[3];
+        c00[c] = t0 - t1;
+        s_c[s & 1][0][c][ty][tx] = t0 + t1;
+        s_c[s & 1][1][c][ty][tx] = t2 - t3;
+        s_c[s & 1][2][c][ty][tx] = t2 + t3;
+      }
+      double own[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) own[c] = s_u[(s - 1) & 3][ty * kRow + 3 * tx + c];
+      copy_wait1();   // plane s + 1 of this thread; the barrier makes it all threads'
+      __syncthreads();
+      if (s >= 2 && out_col) {
+        const long long p3 = 3 * (node_col + (long long)nx1 * ny1 * (z - 1));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const double v = (c00[c] + s_c[s & 1][0][c][ty][tx - 1]) +
+                           (s_c[s & 1][1][c][ty - 1][tx] + s_c[s & 1][2][c][ty - 1][tx - 1]);
+          const double k = ((m8 >> c) & 1) ? v : 0.0;
+          y[p3 + c] = k;
+          dot += own[c] * k;
+        }
+      }
+    } else {
+      copy_wait1();
+      __syncthreads();
     }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int m = 0; m < 4; ++m) Fp[c][m] = Fc[c][m];
   }
   finish_dot(dot, dot_out, partials, counters, slot, heal);
 }
 
 // The operator as a node-centric gather over KE, one thread per node: better
-// only on grids too thin to fill the marching form's tiles.
+// on grids too thin to fill the marching form's tiles.
 __global__ void __launch_bounds__(kThreads) k_apply_noalloc(int nx, int ny, int nz, const double* __restrict__ E,
                                                             const uint8_t* __restrict__ mask,
                                                             const double* __restrict__ u, double* __restrict__ y,
@@ -319,19 +314,20 @@ March march_plan(int nx, int ny, int nz) {
   m.ntx = (nx + kMX - 1) / (kMX - 1);
   m.nty = (ny + kMY - 1) / (kMY - 1);
   const long long tiles = (long long)m.ntx * m.nty, planes = nz + 1, room = 2 * 148;
-  long long best = -1;
+  m.steps = -1;
   m.zchunk = (int)planes;
-  for (long long n = 1; n <= planes && n <= 4096; ++n) {
-    const long long zc = (planes + n - 1) / n;
+  // (the most chunks of each number of waves; past eight or so waves more
+  // chunks only add their two extra steps)
+  for (long long w = (tiles + room - 1) / room, w1 = w + 10; w < w1; ++w) {
+    const long long n = std::min(planes, std::max(1LL, w * room / tiles)), zc = (planes + n - 1) / n;
     const long long waves = (tiles * ((planes + zc - 1) / zc) + room - 1) / room;
-    const long long cost = waves * (zc + 2);
-    if (best < 0 || cost < best) {
-      best = cost;
+    if (m.steps < 0 || waves * (zc + 2) < m.steps) {
+      m.steps = waves * (zc + 2);
       m.zchunk = (int)zc;
     }
-    if (tiles * n > 8 * room) break;   // (more chunks only add their two extra steps)
+    if (tiles * n > 8 * room) break;
   }
-  m.units = (int)(tiles * ((planes + m.zchunk - 1) / m.zchunk));
+  m.units = tiles * ((planes + m.zchunk - 1) / m.zchunk);
   return m;
 }
 
@@ -411,14 +407,19 @@ extern "C" int vf_apply_noalloc(int32_t nx, int32_t ny, int32_t nz, double nu, c
     vf::g_last_error = std::string("vf_apply_noalloc: ") + cudaGetErrorString(e);
     return VF_ERR_CUDA;
   }
-  // The marching form computes whole 31 x 7 tiles: where less than a fifth of
-  // their columns are nodes of the grid the gather form is no slower (gather /
-  // marching form, us: 3x40x3000 51 / 92, 2x100x400 24 / 38, 1x1x100000 43 /
-  // 406; above the line 10x3x200 24 / 10, 30x6x1000 29 / 14, 61x43x37 23 / 12).
+  // The marching form takes a step's time however many of its tiles' 31 x 7
+  // columns are nodes of the grid, the gather form a node's and an element's
+  // time: in us about 5 + 1.3 steps (waves of units, two more planes each than
+  // they own) against 9 + 0.03 per 1,000 nodes + 0.07 per 1,000 elements, and
+  // about 13 more on the host, half of which count.  Marching / gather form, the
+  // kernels: 100x100x100 47 / 112, 10000x10x10 49 / 109, 30x6x1000 16 / 30, 15x7x4000 47 / 56,
+  // 200x1x200 16.1 / 16.5; on the other side 7x7x8000 80 / 56, 1x200x200 36 / 19, 3x40x3000
+  // 88 / 53, 1x1x100000 390 / 45, 2000000x1x1 1,081 / 315.
   const March m = march_plan(nx, ny, nz);
-  if (5LL * (nx + 1) * (ny + 1) >= (long long)m.ntx * (kMX - 1) * m.nty * (kMY - 1)) {
-    vf::launch_k(k_apply_march, dim3((unsigned)std::min(m.units, kMaxBlocks)), dim3(kMX, kMY), kMarchSmem, st, nx, ny,
-                 nz, E, free_mask, u, y, u_dot_y, partials, counters, slot, heal, vf::modal_constants(nu, false), m);
+  const double gather_us = 9.0 + 3e-5 * (double)nn + 7e-5 * (double)nx * ny * nz + 8.0;
+  if (m.units <= kMaxBlocks && 5.0 + 1.3 * (double)m.steps < gather_us) {
+    vf::launch_k(k_apply_march, dim3((unsigned)m.units), dim3(kMX, kMY), kMarchSmem, st, nx, ny, nz, E,
+                 free_mask, u, y, u_dot_y, partials, counters, slot, heal, vf::modal_constants(nu, false), m);
   } else {
     KeParam K;
     double tab[1728], b0[144];
