@@ -79,10 +79,12 @@ template <> __device__ __forceinline__ double chunk_value<double, double>(const 
 // gives D^1/2 u of those nodes; ghost nodes hold zeros, so no neighbour needs a
 // test, only the address of the transposed block is kept in the array.  load()
 // depends on nothing but the node, so it may stand ahead of the staging of u.
-// apply() adds a block's three products of a row as one sum, a row of the own
-// block, then a column of the transposed one: the order is part of the result
+// In FP32 apply() adds a block's three products of a row as one sum, a row of the
+// own block, then a column of the transposed one: the order is part of the result
 // (summed product by product into acc, the FP32 V-cycle differed by 1e-7 and a
 // two-material displacement to a residual of 1e-11 by up to 2e-9 inside the void).
+// FP64 sums product by product, 2-3 % of its V-cycle faster (256x128x128 1,784 /
+// 1,832 us), as its order moves results by rounding only.
 template <typename S> struct WideBatch { static constexpr int JB = sizeof(S) == 2 ? 4 : 2; };
 template <typename S, typename L, int JB> struct RowBatch {
   static constexpr int VPC = L::VPC;
@@ -119,10 +121,20 @@ template <typename S, typename L, int JB> struct RowBatch {
         bu[k] = chunk_value<S, A>(co[(k0 + k) / VPC - C0], (k0 + k) % VPC);
         bd[k] = chunk_value<S, A>(cd[j][(k0 + k) / VPC - k0 / VPC], (k0 + k) % VPC);
       }
+      if constexpr (sizeof(A) == 4) {
 #pragma unroll
-      for (int r = 0; r < 3; ++r) acc[r] += bu[3 * r] * vu[0] + bu[3 * r + 1] * vu[1] + bu[3 * r + 2] * vu[2];
+        for (int r = 0; r < 3; ++r) acc[r] += bu[3 * r] * vu[0] + bu[3 * r + 1] * vu[1] + bu[3 * r + 2] * vu[2];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) acc[c] += bd[c] * vd[0] + bd[3 + c] * vd[1] + bd[6 + c] * vd[2];
+        for (int c = 0; c < 3; ++c) acc[c] += bd[c] * vd[0] + bd[3 + c] * vd[1] + bd[6 + c] * vd[2];
+      } else {
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            acc[r] += bu[3 * r + c] * vu[c];
+            acc[c] += bd[3 * r + c] * vd[r];
+          }
+      }
     }
   }
 };
