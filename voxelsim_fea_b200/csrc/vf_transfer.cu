@@ -14,72 +14,55 @@ namespace vf {
 
 namespace {
 
-__global__ void __launch_bounds__(256) k_restrict_d(Grid f, const double* rf, Grid c,
-                                                    const uint8_t* __restrict__ cm, double* __restrict__ rc,
-                                                    const KrylovState* ks) {
-  pdl_enter();
-  if (ks && ks->done) return;
-  const int nx1 = c.lx + 1, ny1 = c.ly + 1, nint = nx1 * ny1 * (c.lz + 1);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += gridDim.x * blockDim.x) {
-    const int X = t % nx1, rr = t / nx1, Y = rr % ny1, Z = rr / ny1;
-    double a0 = 0, a1 = 0, a2 = 0;
+// The weighted sum of the 27 fine nodes around coarse node (X, Y, Z).  The three
+// of a row, 2X-1 .. 2X+1, are 9 consecutive values that start on two values'
+// boundary (storage x = 2X, rows a multiple of 4 nodes long): four two-value
+// loads and one of one.
+template <typename T> struct Pair;
+template <> struct Pair<float> { using V = float2; };
+template <> struct Pair<double> { using V = double2; };
+template <typename T>
+__device__ __forceinline__ void restrict_sum(const Grid& f, const T* rf, int X, int Y, int Z, T& a0, T& a1, T& a2) {
+  using V = typename Pair<T>::V;
+  a0 = a1 = a2 = 0;
 #pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
+  for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
-      for (int dy = -1; dy <= 1; ++dy)
+    for (int dy = -1; dy <= 1; ++dy) {
+      const long long q = 3 * (long long)f.idx(2 * X - 1, 2 * Y + dy, 2 * Z + dz);
+      const V* q2 = reinterpret_cast<const V*>(rf + q);
+      const V v01 = q2[0], v23 = q2[1], v45 = q2[2], v67 = q2[3];
+      const T r[9] = {v01.x, v01.y, v23.x, v23.y, v45.x, v45.y, v67.x, v67.y, rf[q + 8]};
 #pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const double w = (dx ? 0.5 : 1.0) * (dy ? 0.5 : 1.0) * (dz ? 0.5 : 1.0);
-          const long long q = 3 * (long long)f.idx(2 * X + dx, 2 * Y + dy, 2 * Z + dz);
-          a0 += w * rf[q]; a1 += w * rf[q + 1]; a2 += w * rf[q + 2];
-        }
-    const int p = c.idx(X, Y, Z);
-    const uint8_t m = cm[p];
-    rc[3 * (long long)p] = (m & 1) ? a0 : 0.0;
-    rc[3 * (long long)p + 1] = (m & 2) ? a1 : 0.0;
-    rc[3 * (long long)p + 2] = (m & 4) ? a2 : 0.0;
-  }
+      for (int dx = -1; dx <= 1; ++dx) {
+        const T w = (dx ? (T)0.5 : (T)1) * (dy ? (T)0.5 : (T)1) * (dz ? (T)0.5 : (T)1);
+        const int o = 3 * (dx + 1);
+        a0 += w * r[o]; a1 += w * r[o + 1]; a2 += w * r[o + 2];
+      }
+    }
 }
 
-__global__ void __launch_bounds__(256) k_restrict_f(Grid f, const float* rf, Grid c,
-                                                    const uint8_t* __restrict__ cm, float* __restrict__ rc,
-                                                    const KrylovState* ks) {
+template <typename T>
+__global__ void __launch_bounds__(256) k_restrict(Grid f, const T* rf, Grid c, const uint8_t* __restrict__ cm,
+                                                  T* __restrict__ rc, const KrylovState* ks) {
   pdl_enter();
   if (ks && ks->done) return;
   const int nx1 = c.lx + 1, ny1 = c.ly + 1, nint = nx1 * ny1 * (c.lz + 1);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += gridDim.x * blockDim.x) {
     const int X = t % nx1, rr = t / nx1, Y = rr % ny1, Z = rr / ny1;
-    float a0 = 0, a1 = 0, a2 = 0;
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-      for (int dy = -1; dy <= 1; ++dy) {
-        // the three fine nodes 2X-1 .. 2X+1 of this row are 9 consecutive
-        // values starting on an 8-byte boundary (storage x = 2X, rows a
-        // multiple of 4 nodes long): four float2 loads and one float
-        const long long q = 3 * (long long)f.idx(2 * X - 1, 2 * Y + dy, 2 * Z + dz);
-        const float2* q2 = reinterpret_cast<const float2*>(rf + q);
-        const float2 v01 = q2[0], v23 = q2[1], v45 = q2[2], v67 = q2[3];
-        const float v8 = rf[q + 8];
-        const float r[9] = {v01.x, v01.y, v23.x, v23.y, v45.x, v45.y, v67.x, v67.y, v8};
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const float w = (dx ? 0.5f : 1.0f) * (dy ? 0.5f : 1.0f) * (dz ? 0.5f : 1.0f);
-          const int o = 3 * (dx + 1);
-          a0 += w * r[o]; a1 += w * r[o + 1]; a2 += w * r[o + 2];
-        }
-      }
+    T a0, a1, a2;
+    restrict_sum<T>(f, rf, X, Y, Z, a0, a1, a2);
     const int p = c.idx(X, Y, Z);
     const uint8_t m = cm[p];
-    rc[3 * (long long)p] = (m & 1) ? a0 : 0.0f;
-    rc[3 * (long long)p + 1] = (m & 2) ? a1 : 0.0f;
-    rc[3 * (long long)p + 2] = (m & 4) ? a2 : 0.0f;
+    rc[3 * (long long)p] = (m & 1) ? a0 : (T)0;
+    rc[3 * (long long)p + 1] = (m & 2) ? a1 : (T)0;
+    rc[3 * (long long)p + 2] = (m & 4) ? a2 : (T)0;
   }
 }
 
 // Restriction fused with the coarse level's first smoothing step from zero:
 // the restricted residual rc (kept: the coarse level's right-hand side) and
-// uc = w * (Minv rc), the same sums and products as k_restrict_* followed by
+// uc = w * (Minv rc), the same sums and products as k_restrict followed by
 // k_jacobi_from_zero (ghost entries of uc stay untouched: they hold zeros).
 template <typename T>
 __global__ void __launch_bounds__(256) k_restrict_first(Grid f, const T* rf, Grid c,
@@ -92,36 +75,8 @@ __global__ void __launch_bounds__(256) k_restrict_first(Grid f, const T* rf, Gri
   const int nx1 = c.lx + 1, ny1 = c.ly + 1, nint = nx1 * ny1 * (c.lz + 1);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nint; t += gridDim.x * blockDim.x) {
     const int X = t % nx1, rr = t / nx1, Y = rr % ny1, Z = rr / ny1;
-    T a0 = 0, a1 = 0, a2 = 0;
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-        for (int dy = -1; dy <= 1; ++dy) {
-          const long long q = 3 * (long long)f.idx(2 * X - 1, 2 * Y + dy, 2 * Z + dz);
-          const float2* q2 = reinterpret_cast<const float2*>(rf + q);
-          const float2 v01 = q2[0], v23 = q2[1], v45 = q2[2], v67 = q2[3];
-          const float v8 = rf[q + 8];
-          const float r[9] = {v01.x, v01.y, v23.x, v23.y, v45.x, v45.y, v67.x, v67.y, v8};
-#pragma unroll
-          for (int dx = -1; dx <= 1; ++dx) {
-            const float wt = (dx ? 0.5f : 1.0f) * (dy ? 0.5f : 1.0f) * (dz ? 0.5f : 1.0f);
-            const int o = 3 * (dx + 1);
-            a0 += wt * r[o]; a1 += wt * r[o + 1]; a2 += wt * r[o + 2];
-          }
-        }
-    } else {
-#pragma unroll
-      for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-        for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-          for (int dx = -1; dx <= 1; ++dx) {
-            const double wt = (dx ? 0.5 : 1.0) * (dy ? 0.5 : 1.0) * (dz ? 0.5 : 1.0);
-            const long long q = 3 * (long long)f.idx(2 * X + dx, 2 * Y + dy, 2 * Z + dz);
-            a0 += wt * rf[q]; a1 += wt * rf[q + 1]; a2 += wt * rf[q + 2];
-          }
-    }
+    T a0, a1, a2;
+    restrict_sum<T>(f, rf, X, Y, Z, a0, a1, a2);
     const int p = c.idx(X, Y, Z);
     const uint8_t m = cm[p];
     const long long p3 = 3 * (long long)p;
@@ -267,16 +222,14 @@ inline int blocks_for(long long n) {
 
 }  // namespace
 
-template <>
-void launch_restrict<double>(const Grid& f, const double* rf, const Grid& c, const uint8_t* cmask, double* rc,
-                             const KrylovState* ks, cudaStream_t st) {
-  launch_pdl(k_restrict_d, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c, cmask, rc, ks);
+template <typename T>
+void launch_restrict(const Grid& f, const T* rf, const Grid& c, const uint8_t* cmask, T* rc, const KrylovState* ks,
+                     cudaStream_t st) {
+  launch_pdl(k_restrict<T>, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c, cmask, rc,
+             ks);
 }
-template <>
-void launch_restrict<float>(const Grid& f, const float* rf, const Grid& c, const uint8_t* cmask, float* rc,
-                            const KrylovState* ks, cudaStream_t st) {
-  launch_pdl(k_restrict_f, blocks_for((long long)(c.lx + 1) * (c.ly + 1) * (c.lz + 1)), 256, 0, st, f, rf, c, cmask, rc, ks);
-}
+template void launch_restrict<float>(const Grid&, const float*, const Grid&, const uint8_t*, float*, const KrylovState*, cudaStream_t);
+template void launch_restrict<double>(const Grid&, const double*, const Grid&, const uint8_t*, double*, const KrylovState*, cudaStream_t);
 
 template <typename T>
 void launch_restrict_first(const Grid& f, const T* rf, const Grid& c, const uint8_t* cmask, T* rc, const T* minvc,
