@@ -713,8 +713,11 @@ __global__ void __launch_bounds__(256) k_dis_back(DensePlan P, const S* __restri
 // 60 per block step of 32 columns, 2.5e-8 per n^3 (both measured on 10,920
 // DOFs: 342 steps, 32 ms of products), 8 bytes per value read at 4.5 TB/s, and
 // for a split 150 of set-up launches and 8 per use for the two more kernels.
-// It keeps the explicit inverse up to about 700 DOFs, and splits 10,920 of them
-// into 7 parts of 1,260 (a 100x52x36 job, FP64: 99 -> 34 ms).
+// It splits 10,920 DOFs into 7 parts of 1,260 (a 100x52x36 job, FP64: 99 -> 34 ms).
+// Whole set-up and 80 V-cycles of FP64 two-level solvers, as chosen / explicit
+// inverse, ms: 735 DOFs one piece 4.35, 945 4.80 / 4.71, 1,155 4.65 / 5.14, 2,835 6.7 /
+// 8.4, 4,563 9.0 / 15.6, 9,405 16.9 / 54.6, 15,249 31 / 216; reach 2: 1,617 10.6 / 10.5, 3,159
+// 13.9 / 16.8, 14,625 57 / 230.  No other number of parts was more than 2 % better.
 DensePlan dense_plan(const Grid& c, int reach) {
   DensePlan best{};
   const int dims[3] = {c.lx + 1, c.ly + 1, c.lz + 1};

@@ -112,7 +112,7 @@ __device__ __forceinline__ void finish_dot(double dot, double* __restrict__ dot_
 // the corner forces are exchanged through a double buffer, one barrier a
 // plane.  Bound by the FP64 and shared-memory instructions of 16 warps an SM
 // (the 24 modes of a voxel and their forces fill the registers).  251x127x129
-// voxels: 387 us (gather) -> 118 us; 48x24x24: 29 -> 12 us (there also without a
+// voxels: 387 us (gather) -> 117 us; 48x24x24: 29 -> 9.3 us (there also without a
 // clearing launch and the host's 24x24 tables).
 constexpr int kMX = 32, kMY = 8;
 constexpr int kRow = 3 * (kMX + 1), kPlane = (kMY + 1) * kRow;   // 33 x 9 halo nodes
